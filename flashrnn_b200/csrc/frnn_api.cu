@@ -20,23 +20,24 @@ static bool cell_dims(int cell, CellDims* d) {
   return false;
 }
 
-LoopKernel get_fwd_kernel(int cell, int kt, int nt) {
+// The lane loops (head dims up to 256) and the streamed loops of a kernel family (kernel_cell) and direction.
+static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt) {
   switch (cell) {
-    case CELL_LSTM: return get_fwd_kernel_lstm(kt, nt);
-    case CELL_GRU: return get_fwd_kernel_gru(kt, nt);
-    case CELL_ELMAN: return get_fwd_kernel_elman(kt, nt);
-    case CELL_ELMAN_CLIP: return get_fwd_kernel_elmanc(kt, nt);
-    case CELL_SLSTM: return get_fwd_kernel_slstm(kt, nt);
+    case CELL_LSTM: return bwd ? lane_bwd_lstm(kt, u, nt) : lane_fwd_lstm(kt, u, nt);
+    case CELL_GRU: return bwd ? lane_bwd_gru(kt, u, nt) : lane_fwd_gru(kt, u, nt);
+    case CELL_ELMAN: return bwd ? lane_bwd_elman(kt, u, nt) : lane_fwd_elman(kt, u, nt);
+    case CELL_ELMAN_CLIP: return bwd ? lane_bwd_elmanc(kt, u, nt) : lane_fwd_elmanc(kt, u, nt);
+    case CELL_SLSTM: return bwd ? lane_bwd_slstm(kt, u, nt) : lane_fwd_slstm(kt, u, nt);
   }
-  return LoopKernel{nullptr, 0, nullptr};
+  return LaneKernel{nullptr, 0, 0};
 }
-LoopKernel get_bwd_kernel(int cell, int kt, int nt, int mpw) {
+static LoopKernel stream_kernel(int cell, bool bwd, int nt) {
   switch (cell) {
-    case CELL_LSTM: return get_bwd_kernel_lstm(kt, nt, mpw);
-    case CELL_GRU: return get_bwd_kernel_gru(kt, nt, mpw);
-    case CELL_ELMAN: return get_bwd_kernel_elman(kt, nt, mpw);
-    case CELL_ELMAN_CLIP: return get_bwd_kernel_elmanc(kt, nt, mpw);
-    case CELL_SLSTM: return get_bwd_kernel_slstm(kt, nt, mpw);
+    case CELL_LSTM: return bwd ? stream_bwd_lstm(nt) : stream_fwd_lstm(nt);
+    case CELL_GRU: return bwd ? stream_bwd_gru(nt) : stream_fwd_gru(nt);
+    case CELL_ELMAN: return bwd ? stream_bwd_elman(nt) : stream_fwd_elman(nt);
+    case CELL_ELMAN_CLIP: return bwd ? stream_bwd_elmanc(nt) : stream_fwd_elmanc(nt);
+    case CELL_SLSTM: return bwd ? stream_bwd_slstm(nt) : stream_fwd_slstm(nt);
   }
   return LoopKernel{nullptr, 0, nullptr};
 }
@@ -56,32 +57,22 @@ static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 constexpr size_t kMaxDynSmem = 227 * 1024;
 constexpr size_t kStatusBytes = 256;
 
+// head dims above 256 take the streamed kernels
+static bool streamed(const frnn_problem& pr) { return pr.D > 256; }
+
+// Scratch of a plan: status block, then what the plan's kernels need.  Only the streamed loops repack R for the forward pass.
 struct WsLayout { size_t rpack_fwd, rpack_bwd, grads, dg0, total; };
-static WsLayout workspace_layout(const frnn_problem& pr, const CellDims& cd) {
+static WsLayout workspace_layout(const frnn_problem& pr, const CellDims& cd, int units) {
   WsLayout w;
   const size_t rbytes = (size_t)cd.Gr * pr.N * pr.D * pr.D * 2;
   size_t off = kStatusBytes;
-  w.rpack_fwd = off; off = align_up(off + rbytes, 256);
-  w.rpack_bwd = off; off = align_up(off + rbytes, 256);
-  w.grads = off; off = align_up(off + ((size_t)cd.Gr * pr.N * pr.D * pr.D + (size_t)cd.Gt * pr.N * pr.D) * 4, 256);
+  w.rpack_fwd = off; if (streamed(pr)) off = align_up(off + rbytes, 256);
+  w.rpack_bwd = off; if (pr.training) off = align_up(off + (streamed(pr) ? rbytes : rt_pack_bytes(cd.Gr, pr.N, pr.D, units)), 256);
+  w.grads = off; if (pr.training) off = align_up(off + ((size_t)cd.Gr * pr.N * pr.D * pr.D + (size_t)cd.Gt * pr.N * pr.D) * 4, 256);
   w.dg0 = off;
-  if (pr.cell == CELL_GRU) off = align_up(off + (size_t)pr.B * pr.T * pr.N * pr.D * 2, 256);
+  if (pr.training && pr.cell == CELL_GRU) off = align_up(off + (size_t)pr.B * pr.T * pr.N * pr.D * 2, 256);
   w.total = off;
   return w;
-}
-
-// Backward exchange scheme of a tile: reduce-scatter (returns MPW = CS / Gr) where that kernel exists and fits,
-// else all-gather (0).
-// head dims above 256 take the streamed kernels (lookup key kt = 0)
-static bool streamed(const frnn_problem& pr) { return pr.D > 256; }
-static int kernel_kt(const frnn_problem& pr) { return streamed(pr) ? 0 : pr.D / 16; }
-
-static int bwd_mpw(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
-  if (streamed(pr) || cs <= 1 || cs % cd.Gr) return 0;
-  const int U = pr.D / cs, threads = 2 * cd.Gr * U, mpw = cs / cd.Gr;
-  const LoopKernel k = get_bwd_kernel(kernel_cell(pr), pr.D / 16, bt / 8, mpw);
-  if (!k.fn || threads > k.max_threads || k.smem_bytes(pr.D, U, threads) > kMaxDynSmem) return 0;
-  return mpw;
 }
 
 // A tile (cluster size, batch tile) is usable when both loop kernels exist for it, the CTA fits the
@@ -96,6 +87,12 @@ static bool wide_gates_problem(const frnn_problem& pr) {
 }
 static int plan_threads(const CellDims& cd, int units, int bt) { return bt == kWideBatchTile ? kWideThreads : 2 * cd.Gr * units; }
 
+// Rows / 8 the lane loops run a plan's batch tile with (the activation cache and every result are the same whatever it is).
+// 16-row tiles reuse a fragment of R for two products but hold twice the items per lane.  Measured at batches that fill the GPU (clk per
+// step of all CTAs, 8 against 16 rows): forward LSTM D = 64 8887 / 11285, sLSTM 9283 / 12485, LSTM D = 128 8130 / 8214, but GRU D = 64
+// 8512 / 7320; reverse LSTM D = 64 9881 / 11400, GRU 8524 / 12100, sLSTM 7378 / 9263, but LSTM D = 128 (clusters) 10718 / 8900.
+static int lane_nt(const frnn_problem& pr, bool bwd, int cs, int bt) { return bt >= 16 && (bwd ? cs > 1 : pr.cell == CELL_GRU && cs == 1) ? 2 : 1; }
+
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
   const int D = pr.D;
   if (bt == kWideBatchTile) return cs == 1 && wide_problem(pr);  // 128-row tensor-core loops: one CTA per head and tile
@@ -105,12 +102,17 @@ static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) 
   const int U = D / cs;
   if (U % 16 || ((U / 16) & (U / 16 - 1))) return false;  // 16 * power of two
   if (bt != 8 && bt != 16 && bt != 32) return false;
-  const int kt = kernel_kt(pr), nt = bt / 8, threads = 2 * cd.Gr * U;
-  const LoopKernel f = get_fwd_kernel(kernel_cell(pr), kt, nt), b = get_bwd_kernel(kernel_cell(pr), kt, nt, 0);
-  if (!f.fn || !b.fn) return false;
-  if (threads > f.max_threads || threads > b.max_threads || threads < 32) return false;
-  if (f.smem_bytes(D, U, threads) > kMaxDynSmem || b.smem_bytes(D, U, threads) > kMaxDynSmem) return false;
-  return true;
+  // a CTA owns at most 512 gate-row halves (256 from head dim 256, 384 from 192 up: the registers that hold R), and with
+  // 32-row tiles at most 192 gate rows
+  const int threads = 2 * cd.Gr * U;
+  if (threads > (streamed(pr) || D < 192 ? 512 : D < 256 ? 384 : 256)) return false;
+  if (bt == 32 && (streamed(pr) || cd.Gr * U > 192)) return false;
+  if (streamed(pr)) {
+    const LoopKernel f = stream_kernel(kernel_cell(pr), false, bt / 8), b = stream_kernel(kernel_cell(pr), true, bt / 8);
+    return f.smem_bytes(D, U, threads) <= kMaxDynSmem && b.smem_bytes(D, U, threads) <= kMaxDynSmem;
+  }
+  return lane_kernel(kernel_cell(pr), false, D / 16, U, lane_nt(pr, false, cs, bt)).fn &&
+         lane_kernel(kernel_cell(pr), true, D / 16, U, lane_nt(pr, true, cs, bt)).fn;
 }
 
 static int sm_count_cached();
@@ -212,7 +214,7 @@ static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_pl
   // one bf16 pair per (item, slot, step) in the time loops' own order; batch rows padded to whole tiles
   const uint64_t rows = (uint64_t)((pr->B + cbt - 1) / cbt) * cbt;
   pl.cache_bytes = rows * pr->T * pl.cache_slots * pr->N * pr->D * 2;
-  const WsLayout w = workspace_layout(*pr, cd);
+  const WsLayout w = workspace_layout(*pr, cd, pl.units_per_cta);
   pl.workspace_bytes = w.total;
   pl.grads_offset = w.grads;
   pl.grads_count = (uint64_t)cd.Gr * pr->N * pr->D * pr->D + (uint64_t)cd.Gt * pr->N * pr->D;
@@ -228,7 +230,7 @@ static int check_plan(const frnn_plan* pl, CellDims* cd) {
   if (!tile_ok(pl->prob, *cd, pl->cluster_size, pl->batch_tile)) return FRNN_ERR_PLAN;
   if (pl->units_per_cta * pl->cluster_size != pl->prob.D) return FRNN_ERR_PLAN;
   if (pl->threads != plan_threads(*cd, pl->units_per_cta, pl->batch_tile)) return FRNN_ERR_PLAN;
-  if (pl->workspace_bytes != workspace_layout(pl->prob, *cd).total) return FRNN_ERR_PLAN;
+  if (pl->workspace_bytes != workspace_layout(pl->prob, *cd, pl->units_per_cta).total) return FRNN_ERR_PLAN;
   if (pl->wide_forward && !(pl->wide_forward == 1 && wide_gates_problem(pl->prob) && pl->cluster_size == 1 && pl->batch_tile == 16))
     return FRNN_ERR_PLAN;
   return FRNN_OK;
@@ -250,19 +252,18 @@ static bool resolve_strides(const int64_t (&in)[4], const long long (&dense)[4],
   return true;
 }
 
-static cudaError_t launch_loop(const LoopKernel& k, const frnn_plan& pl, const LoopParams& lp, cudaStream_t stream) {
-  const size_t smem = k.smem_bytes(pl.prob.D, pl.units_per_cta, pl.threads);
+static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int rows, const frnn_plan& pl, const LoopParams& lp, cudaStream_t stream) {
   // always the fixed maximum, never this plan's own size: the attribute belongs to the kernel, not to the launch, and a
   // second host thread launching the same instantiation with a larger tile must not find it lowered in between
-  cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
   if (e != cudaSuccess) return e;
   if (pl.cluster_size > 8) {  // clusters of more than 8 CTAs are a non-portable size: opt in
-    e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)pl.cluster_size, (unsigned)((pl.prob.B + pl.batch_tile - 1) / pl.batch_tile), (unsigned)pl.prob.N);
-  cfg.blockDim = dim3((unsigned)pl.threads, 1, 1);
+  cfg.gridDim = dim3((unsigned)pl.cluster_size, (unsigned)((pl.prob.B + rows - 1) / rows), (unsigned)pl.prob.N);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -273,7 +274,18 @@ static cudaError_t launch_loop(const LoopKernel& k, const frnn_plan& pl, const L
   cfg.attrs = attr;
   cfg.numAttrs = pl.cluster_size > 1 ? 1 : 0;
   void* args[1] = {const_cast<LoopParams*>(&lp)};
-  return cudaLaunchKernelExC(&cfg, k.fn, args);
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+static cudaError_t launch_stream(const LoopKernel& k, const frnn_plan& pl, const LoopParams& lp, cudaStream_t stream) {
+  return launch_loop(k.fn, pl.threads, k.smem_bytes(pl.prob.D, pl.units_per_cta, pl.threads), pl.batch_tile, pl, lp, stream);
+}
+static int launch_lane(const frnn_plan& pl, bool bwd, const LoopParams& lp, cudaStream_t stream) {
+  const frnn_problem& pr = pl.prob;
+  const int kt = pr.D / 16, nt = lane_nt(pr, bwd, pl.cluster_size, pl.batch_tile);
+  const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(kernel_cell(pr), bwd, kt, pl.units_per_cta, nt)
+                       : bwd              ? lane_bwd_floor(pr.cell, kt, pl.units_per_cta, nt)
+                                          : lane_fwd_floor(pr.cell, kt, pl.units_per_cta, nt);
+  return k.fn ? (int)launch_loop(k.fn, k.threads, k.smem, 8 * nt, pl, lp, stream) : FRNN_ERR_PLAN;
 }
 
 static int sm_count_cached() {
@@ -360,20 +372,20 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
       !aligned16(a->workspace) || (a->cache && !aligned16(a->cache)))
     return FRNN_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const WsLayout w = workspace_layout(pr, cd);
+  const WsLayout w = workspace_layout(pr, cd, plan->units_per_cta);
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   const long long nd = (long long)pr.N * pr.D;
   const long long wx_dense[4] = {(long long)pr.T * cd.Gw * nd, cd.Gw * nd, nd, pr.D};
   long long wxs[4];
   if (!resolve_strides(a->wx_stride, wx_dense, wxs)) return FRNN_ERR_ALIGN;
 
+  const bool lane = !streamed(pr) && !is_wide(*plan) && !plan->wide_forward;
   // keep_packed_r: the workspace is left as the previous call left it (R fragments kept, status block not cleared, so
-  // an expired wait of an earlier step stays on record until the caller reads it)
-  cudaError_t e = plan->keep_packed_r ? cudaSuccess : cudaMemsetAsync(ws, 0, kStatusBytes, stream);
+  // an expired wait of an earlier step stays on record until the caller reads it).  The lane loops clear the block themselves.
+  cudaError_t e = plan->keep_packed_r || lane ? cudaSuccess : cudaMemsetAsync(ws, 0, kStatusBytes, stream);
   if (e != cudaSuccess) return (int)e;
   if (a->last && !aligned16(a->last)) return FRNN_ERR_ALIGN;
-  // `last`: one strided device copy of states[:, :, T-1] behind the time loop.  (Storing it from inside the forward
-  // kernel, after the loop, cost the C2 forward loop 6 %: the longer live ranges changed its register allocation.)
+  // `last`: the lane loops store it; behind the others one strided device copy of states[:, :, T-1]
   auto copy_last = [&]() -> cudaError_t {
     if (!a->last) return cudaSuccess;
     const size_t row = (size_t)pr.N * pr.D * (pr.dtype_state == FRNN_DTYPE_F32 ? 4 : 2);
@@ -392,11 +404,14 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
                                  reinterpret_cast<unsigned*>(ws), pr.B, pr.T, pr.N, pr.forward_clip, plan->test_drop_exchange, stream);
     return (int)(e == cudaSuccess ? copy_last() : e);
   }
-  if (!plan->keep_packed_r) e = launch_pack_recurrent(a->R, ws + w.rpack_fwd, cd.Gr, pr.N, pr.D, 0, stream);
+  if (!lane && !plan->keep_packed_r) e = launch_pack_recurrent(a->R, ws + w.rpack_fwd, cd.Gr, pr.N, pr.D, 0, stream);
   if (e != cudaSuccess) return (int)e;
 
   LoopParams lp = {};
   lp.Wx = static_cast<const elem_t*>(a->Wx);
+  lp.R = static_cast<const elem_t*>(a->R);
+  lp.last = a->last;
+  lp.clear_status = !plan->keep_packed_r;
   lp.Rpack = reinterpret_cast<const uint4*>(ws + w.rpack_fwd);
   lp.bias = static_cast<const elem_t*>(a->b);
   lp.s0 = a->s0;
@@ -409,10 +424,9 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
   lp.fclip = pr.forward_clip; lp.gclip = pr.grad_clip; lp.grad_cut = pr.grad_cut;
   lp.test_drop = plan->test_drop_exchange;
   lp.wx_sb = wxs[0]; lp.wx_st = wxs[1]; lp.wx_sg = wxs[2]; lp.wx_sn = wxs[3];
-  const LoopKernel k = plan->probe_noop_cell ? get_fwd_kernel_floor(kernel_cell(pr), kernel_kt(pr), plan->batch_tile / 8)
-                                             : get_fwd_kernel(kernel_cell(pr), kernel_kt(pr), plan->batch_tile / 8);
-  if (!k.fn) return FRNN_ERR_PLAN;
-  e = launch_loop(k, *plan, lp, stream);
+  if (lane) return launch_lane(*plan, false, lp, stream);
+  if (plan->probe_noop_cell) return FRNN_ERR_PLAN;
+  e = launch_stream(stream_kernel(kernel_cell(pr), false, plan->batch_tile / 8), *plan, lp, stream);
   return (int)(e == cudaSuccess ? copy_last() : e);
 }
 
@@ -436,7 +450,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
       !aligned16(a->ds0) || !aligned16(a->workspace) || (a->cache && !aligned16(a->cache)))
     return FRNN_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const WsLayout w = workspace_layout(pr, cd);
+  const WsLayout w = workspace_layout(pr, cd, plan->units_per_cta);
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   float* grads = reinterpret_cast<float*>(ws + w.grads);
   const size_t nR = (size_t)cd.Gr * pr.N * pr.D * pr.D, nb = (size_t)cd.Gt * pr.N * pr.D;
@@ -446,7 +460,10 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   if (!resolve_strides(a->dstates_stride, ds_dense, dss)) return FRNN_ERR_ALIGN;
 
   cudaError_t e = cudaSuccess;
-  if (parts & FRNN_PART_LOOP) {
+  if ((parts & FRNN_PART_LOOP) && !is_wide(*plan) && !streamed(pr)) {
+    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, plan->units_per_cta, grads, nR + nb, reinterpret_cast<unsigned*>(ws), stream);
+    if (e != cudaSuccess) return (int)e;
+  } else if (parts & FRNN_PART_LOOP) {
     e = cudaMemsetAsync(ws, 0, kStatusBytes, stream);
     if (e != cudaSuccess) return (int)e;
     e = cudaMemsetAsync(grads, 0, (nR + nb) * sizeof(float), stream);
@@ -480,11 +497,13 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   lp.test_drop = plan->test_drop_exchange;
   lp.ds_ss = dss[0]; lp.ds_sb = dss[1]; lp.ds_st = dss[2]; lp.ds_sn = dss[3];
   if (parts & FRNN_PART_LOOP) {
-    const int mpw = bwd_mpw(pr, cd, plan->cluster_size, plan->batch_tile);
-    const LoopKernel k = plan->probe_noop_cell ? get_bwd_kernel_floor(kernel_cell(pr), kernel_kt(pr), plan->batch_tile / 8, mpw)
-                                               : get_bwd_kernel(kernel_cell(pr), kernel_kt(pr), plan->batch_tile / 8, mpw);
-    if (!k.fn) return FRNN_ERR_PLAN;
-    e = launch_loop(k, *plan, lp, stream);
+    if (!streamed(pr)) {
+      rc = launch_lane(*plan, true, lp, stream);
+      if (rc) return rc;
+    } else {
+      if (plan->probe_noop_cell) return FRNN_ERR_PLAN;
+      e = launch_stream(stream_kernel(kernel_cell(pr), true, plan->batch_tile / 8), *plan, lp, stream);
+    }
     if (e != cudaSuccess) return (int)e;
   }
   // measured on B200: the tcgen05 kernel wins from head_dim 128 up (C2 0.167 vs 0.212 ms, C3 0.263 vs 0.304 ms) and at

@@ -38,6 +38,37 @@ __global__ void pack_recurrent_kernel(const elem_t* __restrict__ R, uint4* __res
   out[idx] = v;
 }
 
+// In front of a reverse lane loop, one launch: R^T as the 16-byte fragments its warps keep in registers, the fp32 gradients
+// and the status block zeroed.  One thread builds the two fragments (rows 2 gid and 2 gid + 1 of a 16-row tile of p) of one
+// lane: eight consecutive gate rows k = 8 tig .. of the CTA's K = Gr * U (an odd last k-step: four).
+//   out[((((n * CS + c) * D/16 + mt) * KP + kp) * 2 + row parity) * 32 + lane], KP = ceil(K / 32)
+__global__ void bwd_prepare_kernel(const elem_t* __restrict__ R, uint4* __restrict__ out, int Gr, int N, int D, int U, int KP,
+                                   size_t nfrag, float4* __restrict__ grads, size_t ngrads4, unsigned* __restrict__ status) {
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx < 64) status[idx] = 0u;
+  for (size_t i = idx; i < ngrads4; i += (size_t)gridDim.x * blockDim.x) grads[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (idx >= nfrag) return;
+  const int lane = (int)(idx & 31), gid = lane >> 2, tig = lane & 3, K = Gr * U, CS = D / U;
+  size_t r = idx >> 5;
+  const int kp = (int)(r % KP); r /= KP;
+  const int mt = (int)(r % (D / 16)); r /= (D / 16);
+  const int c = (int)(r % CS), n = (int)(r / CS);
+  const bool pair = kp * 32 + 32 <= K;
+  const int k0 = kp * 32 + tig * (pair ? 8 : 4), ne = pair ? 8 : 4, g = k0 / U, u0 = k0 - g * U;
+  const unsigned* src = reinterpret_cast<const unsigned*>(R + ((((size_t)g * N + n) * D + (size_t)c * U + u0) * D + mt * 16 + 2 * gid));
+  unsigned w[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = e < ne ? __ldg(src + (size_t)e * (D / 2)) : 0u;
+  uint4 lo, hi;
+  lo.x = __byte_perm(w[0], w[1], 0x5410); lo.y = __byte_perm(w[2], w[3], 0x5410);
+  lo.z = __byte_perm(w[4], w[5], 0x5410); lo.w = __byte_perm(w[6], w[7], 0x5410);
+  hi.x = __byte_perm(w[0], w[1], 0x7632); hi.y = __byte_perm(w[2], w[3], 0x7632);
+  hi.z = __byte_perm(w[4], w[5], 0x7632); hi.w = __byte_perm(w[6], w[7], 0x7632);
+  uint4* dst = out + (idx >> 5) * 64 + lane;
+  dst[0] = lo;
+  dst[32] = hi;
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // dR.  For one R gate g and head n:  C[d][p] = sum_k A_k[d] * H_k[p],  k = b*T + t,
 //   A_k = delta of gate g at (b,t) (a row of dWx, or of the GRU side buffer), H_k = h_{t-1}[b] (a row of
@@ -191,6 +222,18 @@ cudaError_t launch_pack_recurrent(const void* R, void* out, int Gr, int N, int D
   const int threads = 256;
   pack_recurrent_kernel<<<(unsigned)((total + threads - 1) / threads), threads, 0, stream>>>(
       static_cast<const elem_t*>(R), static_cast<uint4*>(out), Gr, N, D, transpose);
+  return cudaGetLastError();
+}
+
+size_t rt_pack_bytes(int Gr, int N, int D, int U) { return (size_t)N * (D / U) * (D / 16) * ((Gr * U + 31) / 32) * 64 * 16; }
+
+cudaError_t launch_bwd_prepare(const void* R, void* out, int Gr, int N, int D, int U, float* grads, size_t ngrads, unsigned* status,
+                               cudaStream_t stream) {
+  const size_t nfrag = rt_pack_bytes(Gr, N, D, U) / 32;
+  const int threads = 128;
+  bwd_prepare_kernel<<<(unsigned)((nfrag + threads - 1) / threads), threads, 0, stream>>>(
+      static_cast<const elem_t*>(R), static_cast<uint4*>(out), Gr, N, D, U, (Gr * U + 31) / 32, nfrag, reinterpret_cast<float4*>(grads),
+      ngrads / 4, status);
   return cudaGetLastError();
 }
 

@@ -4,41 +4,46 @@
 
 namespace FRNN_NS {
 
-// head dims (D = 16*KT) and batch tiles (BT = 8*NT) the time-loop kernels are instantiated for
-#define FRNN_FOREACH_KT(X, ...) X(1, __VA_ARGS__) X(2, __VA_ARGS__) X(4, __VA_ARGS__) X(6, __VA_ARGS__) X(8, __VA_ARGS__) X(12, __VA_ARGS__) X(16, __VA_ARGS__)
+// (head dim / 16, units per CTA) the lane loops are instantiated for
+#define FRNN_FOREACH_KT_U(X) X(1, 16) X(2, 16) X(2, 32) X(4, 16) X(4, 32) X(4, 64) X(6, 16) X(6, 32) X(8, 16) X(8, 32) X(8, 64) \
+  X(12, 32) X(16, 16) X(16, 32)
+#define FRNN_FOREACH_KT_U_FEW_GATES(X) X(12, 64)
+#define FRNN_FOREACH_KT_U_ONE_GATE(X) X(8, 128) X(16, 64) X(16, 128)
 constexpr int kNumKT = 7;
 constexpr int kKTs[kNumKT] = {1, 2, 4, 6, 8, 12, 16};
-constexpr int kNumNT = 3;
-constexpr int kNTs[kNumNT] = {1, 2, 4};
 
 // head dims above 256 (multiples of 64 up to kStreamMaxD) run the streamed kernels: kStreamKT k-steps of R per warp
 // in registers, U = kStreamU units per CTA, cluster size D / kStreamU (up to 16, non-portable above 8)
 // (kStreamKT, kStreamU, kStreamMaxD: frnn_common.cuh)
 
+struct LaneKernel {
+  const void* fn;  // kernel entry; null: no such instantiation
+  int threads;
+  size_t smem;
+};
 struct LoopKernel {
   const void* fn;      // kernel entry
   int max_threads;     // __launch_bounds__ of the instantiation
   size_t (*smem_bytes)(int D, int U, int threads);
 };
 
-// defined once per (cell, direction) in frnn_inst_*.cu; returns fn == nullptr when not instantiated
-LoopKernel get_fwd_kernel(int cell, int kt, int nt);
-LoopKernel get_bwd_kernel(int cell, int kt, int nt, int mpw);  // mpw = 0: all-gather exchange, > 0: reduce-scatter
-LoopKernel get_fwd_kernel_lstm(int kt, int nt);
-LoopKernel get_fwd_kernel_gru(int kt, int nt);
-LoopKernel get_fwd_kernel_elman(int kt, int nt);
-LoopKernel get_fwd_kernel_slstm(int kt, int nt);
-LoopKernel get_fwd_kernel_elmanc(int kt, int nt);
-LoopKernel get_bwd_kernel_elmanc(int kt, int nt, int mpw);
-LoopKernel get_bwd_kernel_lstm(int kt, int nt, int mpw);
-LoopKernel get_bwd_kernel_gru(int kt, int nt, int mpw);
-LoopKernel get_bwd_kernel_elman(int kt, int nt, int mpw);
-LoopKernel get_bwd_kernel_slstm(int kt, int nt, int mpw);
+// defined once per (cell, direction) in frnn_inst_*.cu
+#define FRNN_DECLARE(cell)                              \
+  LaneKernel lane_fwd_##cell(int kt, int u, int nt);    \
+  LaneKernel lane_bwd_##cell(int kt, int u, int nt);    \
+  LoopKernel stream_fwd_##cell(int nt);                 \
+  LoopKernel stream_bwd_##cell(int nt);
+FRNN_DECLARE(lstm) FRNN_DECLARE(gru) FRNN_DECLARE(elman) FRNN_DECLARE(elmanc) FRNN_DECLARE(slstm)
+#undef FRNN_DECLARE
 
 // chain-floor variants (frnn_inst_floor.cu); fn == nullptr for any tile but the benchmark configurations
-LoopKernel get_fwd_kernel_floor(int cell, int kt, int nt);
-LoopKernel get_bwd_kernel_floor(int cell, int kt, int nt, int mpw);
+LaneKernel lane_fwd_floor(int cell, int kt, int u, int nt);
+LaneKernel lane_bwd_floor(int cell, int kt, int u, int nt);
 
+// in front of a reverse lane loop: R^T as the fragments of its CTAs (U units each), fp32 gradients and status block zeroed
+size_t rt_pack_bytes(int Gr, int N, int D, int U);
+cudaError_t launch_bwd_prepare(const void* R, void* out, int Gr, int N, int D, int U, float* grads, size_t ngrads, unsigned* status,
+                               cudaStream_t stream);
 cudaError_t launch_pack_recurrent(const void* R, void* out, int Gr, int N, int D, int transpose, cudaStream_t stream);
 cudaError_t launch_recurrent_grad(int cell, int B, int T, int N, int D, int Gr, int Gw, int state_f32, const void* dWx,
                                   const void* dg0, const void* states, const void* s0, float* dR, int sm_count,

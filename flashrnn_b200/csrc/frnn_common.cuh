@@ -52,6 +52,7 @@ constexpr int kStages = 4;
 // Arguments of both time-loop kernels (forward uses the first block, backward all of it).
 struct LoopParams {
   const elem_t* Wx;   // [B,T,Gw,N,D]
+  const elem_t* R;           // [Gr,N,D,D] (lane loops, forward)
   const uint4* Rpack;        // recurrent matrix repacked into warp-MMA A fragments
   const elem_t* bias; // [Gt,N,D]
   const void* s0;            // [S,B,1,N,D]
@@ -62,7 +63,9 @@ struct LoopParams {
   elem_t* dg0;        // [B,T,N,D]   GRU only: delta of the recurrent-only gate
   void* ds0;                 // [S,B,1,N,D]
   float* dbias;              // fp32 [Gt,N,D] accumulated with atomics
+  void* last;                // [S,B,1,N,D] forward: the states after the last step, or null
   unsigned* status;
+  int clear_status;          // forward: CTA 0 zeroes the status block first
   int B, T, N, D;
   int U;                     // hidden units owned by one CTA (multiple of 16)
   int CS;                    // CTAs per cluster = D / U
@@ -93,8 +96,59 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint4& a, uint32_
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
+// the same with C = 0
+__device__ __forceinline__ void mma_16816_zero(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32." FRNN_MMA_TYPE "." FRNN_MMA_TYPE ".f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async4_u32(uint32_t smem_dst, const void* gsrc) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_dst), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async8_u32(uint32_t smem_dst, const void* gsrc) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_dst), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async16_u32(uint32_t smem_dst, const void* gsrc) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts64(uint32_t addr, uint2 v) {
+  asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(addr), "r"(v.x), "r"(v.y) : "memory");
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+// stores into another CTA's shared memory (shared::cluster addresses) that count their bytes on that CTA's mbarrier
+__device__ __forceinline__ void st_async_b32(uint32_t dst, uint32_t v, uint32_t mbar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(v), "r"(mbar) : "memory");
+}
+__device__ __forceinline__ void st_async_v2(uint32_t dst, uint2 v, uint32_t mbar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(mbar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async_v4(uint32_t dst, float a, float b, float c, float d, uint32_t mbar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "f"(a), "f"(b),
+               "f"(c), "f"(d), "r"(mbar) : "memory");
 }
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
@@ -112,6 +166,7 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   return r;
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // shared::cluster address of `local_addr` (a shared::cta address of this CTA) inside CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t rank) {
@@ -131,6 +186,9 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -138,6 +196,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
+// named CTA barriers: `bar_arrive` does not wait.  `threads` counts those of both sides.
+template <int THREADS> __device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(THREADS) : "memory"); }
+template <int THREADS> __device__ __forceinline__ void bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(THREADS) : "memory"); }
 __device__ __forceinline__ uint64_t global_timer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -228,6 +289,60 @@ __device__ __forceinline__ float2 unpack_x2(uint32_t w) {
   elem2_t v = *reinterpret_cast<elem2_t*>(&w);
   return elem2_to_floats(v);
 }
+
+// Two fp32 values, for the loops whose lanes own two units: S2 with scalar instructions, P2 in a register pair with the packed ones
+// (two multiplications or additions per issue slot, each rounded as the scalar ones are; but values that are not produced in
+// pairs have to be moved together, so which is faster depends on the loop).  The v_* functions exist for float, S2 and P2: the
+// cells are written once.
+struct S2 { float x, y; };
+struct P2 { unsigned long long v; };
+template <class V> __device__ __forceinline__ V v_pair(float lo, float hi) {
+  V r;
+  if constexpr (sizeof(r) == sizeof(S2) && alignof(V) == alignof(S2)) { r.x = lo; r.y = hi; }
+  else asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 v_get(S2 a) { return make_float2(a.x, a.y); }
+__device__ __forceinline__ float2 v_get(P2 a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v)); return r; }
+__device__ __forceinline__ P2 v_fma(P2 a, P2 b, P2 c) { P2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+__device__ __forceinline__ P2 v_mul(P2 a, P2 b) { P2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ P2 v_add(P2 a, P2 b) { P2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ S2 v_fma(S2 a, S2 b, S2 c) { return S2{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
+__device__ __forceinline__ S2 v_mul(S2 a, S2 b) { return S2{a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ S2 v_add(S2 a, S2 b) { return S2{a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ float v_fma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float v_mul(float a, float b) { return a * b; }
+__device__ __forceinline__ float v_add(float a, float b) { return a + b; }
+template <class V> __device__ __forceinline__ V v_const(float c) {
+  if constexpr (sizeof(V) == 8) return v_pair<V>(c, c);
+  else return c;
+}
+template <class F> __device__ __forceinline__ float v_map(float a, F f) { return f(a); }
+template <class F> __device__ __forceinline__ float v_map(float a, float b, F f) { return f(a, b); }
+template <class F> __device__ __forceinline__ float v_map(float a, float b, float c, F f) { return f(a, b, c); }
+template <class V, class F> __device__ __forceinline__ V v_map(V a, F f) { const float2 x = v_get(a); return v_pair<V>(f(x.x), f(x.y)); }
+template <class V, class F> __device__ __forceinline__ V v_map(V a, V b, F f) {
+  const float2 x = v_get(a), y = v_get(b);
+  return v_pair<V>(f(x.x, y.x), f(x.y, y.y));
+}
+template <class V, class F> __device__ __forceinline__ V v_map(V a, V b, V c, F f) {
+  const float2 x = v_get(a), y = v_get(b), z = v_get(c);
+  return v_pair<V>(f(x.x, y.x, z.x), f(x.y, y.y, z.y));
+}
+template <class V> __device__ __forceinline__ V v_neg(V a) { return v_mul(a, v_const<V>(-1.f)); }
+template <class V> __device__ __forceinline__ V v_sub(V a, V b) { return v_fma(b, v_const<V>(-1.f), a); }
+template <class V> __device__ __forceinline__ V v_one_minus(V a) { return v_fma(a, v_const<V>(-1.f), v_const<V>(1.f)); }
+template <class V> __device__ __forceinline__ V v_tanh(V a) { return v_map(a, [](float x) { return fast_tanh(x); }); }
+template <class V> __device__ __forceinline__ V v_sigmoid(V a) {
+#ifndef FRNN_EXACT_ACT
+  return v_fma(v_tanh(v_mul(a, v_const<V>(0.5f))), v_const<V>(0.5f), v_const<V>(0.5f));
+#else
+  return v_map(a, [](float x) { return fast_sigmoid(x); });
+#endif
+}
+template <class V> __device__ __forceinline__ V v_clamp(V a, float lim) { return v_map(a, [lim](float x) { return clampf(x, lim); }); }
+template <class V> __device__ __forceinline__ uint32_t v_pack(V a) { const float2 x = v_get(a); return pack_x2(x.x, x.y); }
+template <class V> __device__ __forceinline__ V v_unpack(uint32_t w) { const float2 x = unpack_x2(w); return v_pair<V>(x.x, x.y); }
 
 // Loads / stores of a pair of adjacent state values in the run-time state dtype.
 __device__ __forceinline__ float2 load_state2(const void* base, size_t elem_off, int f32) {

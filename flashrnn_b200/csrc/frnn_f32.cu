@@ -23,8 +23,7 @@
 #include <type_traits>
 
 #include "../../include/frnn.h"
-#include "frnn_bwd.cuh"
-#include "frnn_fwd.cuh"
+#include "frnn_cell.cuh"
 
 namespace FRNN_NS {
 
@@ -118,7 +117,9 @@ __global__ void __launch_bounds__(XTHREADS) x32_fwd_kernel(const XParams p) {
 #pragma unroll
       for (int s = 0; s < S; ++s)
         st[s] = t > 0 ? p.states[(((size_t)s * B + b) * T + (t - 1)) * ND + nd] : p.s0[((size_t)s * B + b) * ND + nd];
-      cell_forward<CELL>(prv, wx, bv, st, cv);
+      float gx[Gt];
+      gate_sums<CELL>(prv, wx, bv, gx);
+      cell_forward<CELL>(gx, st, cv);
       if (p.fclip > 0.f) st[0] = clampf(st[0], p.fclip);
 #pragma unroll
       for (int s = 0; s < S; ++s) p.states[(((size_t)s * B + b) * T + t) * ND + nd] = st[s];
@@ -376,7 +377,9 @@ __global__ void __launch_bounds__(XTHREADS, 1) x32c_fwd_kernel(const XParams p) 
 #pragma unroll
         for (int g = 0; g < Gr; ++g) prv[g] += pp[g * U];
       }
-      cell_forward<CELL>(prv, wxc[i], bias[i], st[i], cch[i]);
+      float gx[Gt];
+      gate_sums<CELL>(prv, wxc[i], bias[i], gx);
+      cell_forward<CELL>(gx, st[i], cch[i]);
       if (p.fclip > 0.f) st[i][0] = clampf(st[i][0], p.fclip);
       if (!it_ok[i]) {  // rows beyond B: keep everything zero
 #pragma unroll

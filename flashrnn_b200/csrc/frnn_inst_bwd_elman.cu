@@ -1,5 +1,6 @@
-// Instantiates the bwd time-loop kernel of the elman cell for every supported head dim and batch tile.
+// Instantiates the bwd time loops of the elman cell.
 #define FRNN_INST_CELL CELL_ELMAN
 #define FRNN_INST_BWD 1
-#define FRNN_INST_NAME get_bwd_kernel_elman
+#define FRNN_INST_LANE lane_bwd_elman
+#define FRNN_INST_STREAM stream_bwd_elman
 #include "frnn_inst.cuh"

@@ -1,5 +1,6 @@
-// Instantiates the bwd time-loop kernel of the Elman cell with forward clamp (caches the tanh output).
+// Instantiates the bwd time loops of the elmanc cell.
 #define FRNN_INST_CELL CELL_ELMAN_CLIP
 #define FRNN_INST_BWD 1
-#define FRNN_INST_NAME get_bwd_kernel_elmanc
+#define FRNN_INST_LANE lane_bwd_elmanc
+#define FRNN_INST_STREAM stream_bwd_elmanc
 #include "frnn_inst.cuh"

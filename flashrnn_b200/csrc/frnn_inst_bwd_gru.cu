@@ -1,5 +1,6 @@
-// Instantiates the bwd time-loop kernel of the gru cell for every supported head dim and batch tile.
+// Instantiates the bwd time loops of the gru cell.
 #define FRNN_INST_CELL CELL_GRU
 #define FRNN_INST_BWD 1
-#define FRNN_INST_NAME get_bwd_kernel_gru
+#define FRNN_INST_LANE lane_bwd_gru
+#define FRNN_INST_STREAM stream_bwd_gru
 #include "frnn_inst.cuh"

@@ -1,5 +1,6 @@
-// Instantiates the bwd time-loop kernel of the lstm cell for every supported head dim and batch tile.
+// Instantiates the bwd time loops of the lstm cell.
 #define FRNN_INST_CELL CELL_LSTM
 #define FRNN_INST_BWD 1
-#define FRNN_INST_NAME get_bwd_kernel_lstm
+#define FRNN_INST_LANE lane_bwd_lstm
+#define FRNN_INST_STREAM stream_bwd_lstm
 #include "frnn_inst.cuh"

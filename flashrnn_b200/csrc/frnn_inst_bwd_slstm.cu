@@ -1,5 +1,6 @@
-// Instantiates the bwd time-loop kernel of the slstm cell for every supported head dim and batch tile.
+// Instantiates the bwd time loops of the slstm cell.
 #define FRNN_INST_CELL CELL_SLSTM
 #define FRNN_INST_BWD 1
-#define FRNN_INST_NAME get_bwd_kernel_slstm
+#define FRNN_INST_LANE lane_bwd_slstm
+#define FRNN_INST_STREAM stream_bwd_slstm
 #include "frnn_inst.cuh"

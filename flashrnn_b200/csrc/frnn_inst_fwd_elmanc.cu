@@ -1,5 +1,6 @@
-// Instantiates the fwd time-loop kernel of the Elman cell with forward clamp (caches the tanh output).
+// Instantiates the fwd time loops of the elmanc cell.
 #define FRNN_INST_CELL CELL_ELMAN_CLIP
 #define FRNN_INST_BWD 0
-#define FRNN_INST_NAME get_fwd_kernel_elmanc
+#define FRNN_INST_LANE lane_fwd_elmanc
+#define FRNN_INST_STREAM stream_fwd_elmanc
 #include "frnn_inst.cuh"

@@ -1,5 +1,6 @@
-// Instantiates the fwd time-loop kernel of the lstm cell for every supported head dim and batch tile.
+// Instantiates the fwd time loops of the lstm cell.
 #define FRNN_INST_CELL CELL_LSTM
 #define FRNN_INST_BWD 0
-#define FRNN_INST_NAME get_fwd_kernel_lstm
+#define FRNN_INST_LANE lane_fwd_lstm
+#define FRNN_INST_STREAM stream_fwd_lstm
 #include "frnn_inst.cuh"

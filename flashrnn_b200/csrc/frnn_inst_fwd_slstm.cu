@@ -1,5 +1,6 @@
-// Instantiates the fwd time-loop kernel of the slstm cell for every supported head dim and batch tile.
+// Instantiates the fwd time loops of the slstm cell.
 #define FRNN_INST_CELL CELL_SLSTM
 #define FRNN_INST_BWD 0
-#define FRNN_INST_NAME get_fwd_kernel_slstm
+#define FRNN_INST_LANE lane_fwd_slstm
+#define FRNN_INST_STREAM stream_fwd_slstm
 #include "frnn_inst.cuh"

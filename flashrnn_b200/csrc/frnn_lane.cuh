@@ -1,0 +1,134 @@
+// What the forward and the reverse lane loop share (frnn_lane_fwd.cuh, frnn_lane_bwd.cuh): operand tiles in shared memory,
+// the register-resident product, and the exchange between the CTAs of a cluster.
+#pragma once
+#include "frnn_cell.cuh"
+
+namespace FRNN_NS {
+
+// Operand tile of 8 batch rows x K 16-bit values: blocks of 8 k, each [8 rows][16 bytes] = 128 contiguous bytes, the rows of
+// block i permuted by opnd_swz(i).  The 8 units (or gate rows) a warp produces for the 8 rows are ONE 128-byte block: what it
+// sends to another CTA, or stores, is one line instead of eight pieces (the exchange is charged per piece: with rows of a
+// plain [row][k] tile the C2 forward step took 1592 clk).  The permutation keeps the reads -- 16 bytes per lane, two rows of
+// four blocks per wavefront -- and the stores of pairs of blocks free of bank conflicts.
+__host__ __device__ constexpr uint32_t opnd_swz(uint32_t blk) { return (blk & 1) * 3 | ((blk & 2) << 1); }
+__host__ __device__ constexpr uint32_t opnd_off(uint32_t row, uint32_t k) { return (k >> 3) * 128 + ((row ^ opnd_swz(k >> 3)) << 4) + (k & 7) * 2; }
+__host__ __device__ constexpr int opnd_bytes(int k) { return k * 16; }
+
+// A fragments (16 rows x 32 k) of one lane: its rows gid and gid + 8, eight consecutive k each (k = 8 tig .. 8 tig + 7).
+// Which k an MMA calls its k-th is free as long as both operands agree, so a pair of k-steps takes contiguous 16 bytes
+// per lane from either operand -- R in its own layout in global memory, h or the deltas in shared memory -- and neither a
+// repacking pass nor ldmatrix is needed.  An odd last k-step uses four k per lane (.x, .y).
+struct AFrag { uint4 lo, hi; };
+
+// acc[m][nt][.] (+)= sum over k of A[m][.] (rows of this lane's MT tiles) times the operand tile: KS k-steps of 16, NT tiles of 8
+// batch rows (`nt_bytes` apart).  INIT: acc holds the start value, else it starts from zero.  NS independent accumulator sets (see
+// acc_sets).  The loads run PF k-pairs ahead of the products: without it every pair waited for its own 36 clk load.
+template <int MT, int KS, int NT, int NS, bool INIT, class L>
+__device__ __forceinline__ void lane_mma(const AFrag (&A)[MT][(KS + 1) / 2], uint32_t tile, int nt_bytes, int gid, int tig, float (&acc)[MT][NT][4],
+                                         L late) {
+  constexpr int KP = KS / 2, PF = KP < 4 ? (KP < 1 ? 1 : KP) : (NT > 1 ? 3 : 4);
+  static_assert(NS <= KS, "every set gets a product");
+  float part[NS][MT][NT][4];
+  const uint32_t base = tile + (uint32_t)tig * 128u + ((uint32_t)(gid ^ (int)opnd_swz((uint32_t)tig)) << 4);
+  uint4 b[PF][NT];
+#pragma unroll
+  for (int i = 0; i < PF && i < KP; ++i)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) b[i][nt] = lds128(base + (uint32_t)(i * 512 + nt * nt_bytes));
+  uint2 bo[NT];
+  if constexpr ((KS & 1) != 0) {  // odd last k-step: four k per lane, in blocks 4 KP + (tig >> 1)
+    const uint32_t blk = (uint32_t)(tig >> 1);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+      bo[nt] = lds64(tile + (uint32_t)(KP * 512 + nt * nt_bytes) + blk * 128u + (((uint32_t)gid ^ opnd_swz(blk)) << 4) + (uint32_t)(tig & 1) * 8u);
+  }
+  if constexpr (INIT) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) part[0][m][nt][c] = acc[m][nt][c];
+  }
+  auto step = [&](int k, const uint4& a, int m, int nt, uint32_t b0, uint32_t b1) {
+    if (k < NS && !(INIT && k == 0)) mma_16816_zero(part[k % NS][m][nt], a, b0, b1);
+    else mma_16816(part[k % NS][m][nt], a, b0, b1);
+  };
+#pragma unroll
+  for (int kp = 0; kp < KP; ++kp) {
+    uint4 cur[NT];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      cur[nt] = b[kp % PF][nt];
+      if (kp + PF < KP) b[kp % PF][nt] = lds128(base + (uint32_t)((kp + PF) * 512 + nt * nt_bytes));
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+        step(2 * kp, make_uint4(A[m][kp].lo.x, A[m][kp].hi.x, A[m][kp].lo.y, A[m][kp].hi.y), m, nt, cur[nt].x, cur[nt].y);
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+        step(2 * kp + 1, make_uint4(A[m][kp].lo.z, A[m][kp].hi.z, A[m][kp].lo.w, A[m][kp].hi.w), m, nt, cur[nt].z, cur[nt].w);
+  }
+  if constexpr ((KS & 1) != 0) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+        step(2 * KP, make_uint4(A[m][KP].lo.x, A[m][KP].hi.x, A[m][KP].lo.y, A[m][KP].hi.y), m, nt, bo[nt].x, bo[nt].y);
+  }
+  late();  // (work the products do not depend on, while the last of them complete)
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if constexpr (NS == 4) acc[m][nt][c] = (part[0][m][nt][c] + part[1][m][nt][c]) + (part[2][m][nt][c] + part[3][m][nt][c]);
+        else if constexpr (NS == 2) acc[m][nt][c] = part[0][m][nt][c] + part[1][m][nt][c];
+        else acc[m][nt][c] = part[0][m][nt][c];
+      }
+}
+// Accumulator sets for `tiles` 16x8 tiles per warp, `warps` warps per CTA and `ks` k-steps, at least `want` independent chains per
+// quadrant (see the uses).  An m16n8k16 occupies the tensor pipe of its quadrant for 8 clk and its result takes about 30.
+__host__ __device__ constexpr int acc_sets(int tiles, int warps, int ks, int want) {
+  const int chains = tiles * (warps > 4 ? warps / 4 : 1);
+  const int sets = chains >= want ? 1 : (2 * chains >= want ? 2 : 4);
+  return sets <= ks ? sets : (ks >= 2 ? 2 : 1);
+}
+template <bool PACKED> struct PairOf { using type = S2; };
+template <> struct PairOf<true> { using type = P2; };
+
+// Words of two 16-bit values in the activation cache: [t][n][b][D/2 unit pairs][slots]; four slots of a pair side by side (one
+// 16-byte access), a fifth (sLSTM) in a plane of its own behind all of them.  The layout knows nothing of tiles, so the
+// forward and the reverse loop choose theirs independently.
+template <int GC> struct CacheGeom {
+  static constexpr int MAIN = GC >= 4 ? 4 : GC;  // words per pair in the main plane (0: nothing cached)
+  static constexpr bool EXTRA = GC > 4;
+};
+
+constexpr int kLaneStages = 6;  // time steps of inputs in the lane loops' shared-memory ring
+
+// ---- IO warps.  A lane's values belong to 8 batch rows per warp instruction (the MMA's accumulator layout), and the L1 charges
+// a global access per row touched: with the compute lanes loading Wx and storing states and cache themselves the LSTM D = 64 forward
+// step spent ~700 of 1380 clk on it.  So one or two extra warps move everything between global memory and padded tiles in shared
+// memory, 16 bytes per lane along the rows, and the compute lanes touch shared memory only.
+__host__ __device__ constexpr int io_warps(int bytes_per_step) { return bytes_per_step > 6144 ? 2 : 1; }
+// row pitch of such a tile: 16 bytes of padding make the compute lanes' accesses (4 to 16 bytes, 8 rows) conflict-free
+__host__ __device__ constexpr int io_pitch(int row_bytes) { return row_bytes + 16; }
+
+// One lane's share of a tile of ROWS rows x CPR 16-byte chunks, moved by IOT lanes.  Chunk i of the lane is row row(i), chunk col().
+template <int ROWS, int CPR, int IOT>
+struct IoTile {
+  static constexpr int N = (ROWS * CPR + IOT - 1) / IOT;  // chunks per lane
+  static constexpr bool COLS_FIT = IOT % CPR == 0;
+  static_assert(COLS_FIT || CPR % IOT == 0, "chunks per row and lanes divide one another");
+  static __device__ __forceinline__ int row(int lane, int i) { return COLS_FIT ? lane / CPR + i * (IOT / CPR) : i / (CPR / IOT); }
+  static __device__ __forceinline__ int col(int lane, int i) { return COLS_FIT ? lane % CPR : lane + (i % (CPR / IOT > 0 ? CPR / IOT : 1)) * IOT; }
+  static __device__ __forceinline__ bool in(int lane, int i) { return ROWS * CPR % IOT == 0 || row(lane, i) < ROWS; }
+};
+
+}  // namespace FRNN_NS

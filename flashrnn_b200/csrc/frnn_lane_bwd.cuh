@@ -1,0 +1,448 @@
+// Reverse time loop, counterpart of the forward lane loop (frnn_lane_fwd.cuh): the lane that receives the recurrent
+// cotangent of a (unit, batch row) runs the closed-form backward of the cell for it.
+//
+// Work split.  A cluster of CS = D / U CTAs owns one head and 8 * NT batch rows; CTA c owns units [c*U, (c+1)*U) and keeps the
+// columns of R^T that belong to its units' gates (all D rows p) in registers.  Per step t = T-1 .. 0
+//   inputs   activations, states and cotangents of the step (shared memory, put there by the IO warps) and everything of the
+//            cell's backward that does not depend on dh: computed before the wait, in the shadow of the exchange;
+//   wait     for the partial sums of dh from every CTA of the cluster (CS > 1);
+//   cell     dh = external + sum of partials; gate deltas -> 16-bit operand tile in shared memory;
+//   barrier  of the CTA, IO warps included (the only one in the step);
+//   product  partial dh_{t-1}[all p] = R^T x deltas of this CTA's units; a warp owns whole 16-row tiles of p;
+//   push     CS > 1: every lane sends its four sums of a tile straight from the accumulators to the CTA that owns those p
+//            (one 16-byte st.async, counted on that CTA's mbarrier).  CS == 1: the sums already sit in the lanes that own the units.
+//   The IO warps store dWx from the delta tile itself and refill the input ring behind the barrier; db, the carried cotangents and
+//   the current states stay in registers.
+// Rows of a p tile: rows gid and gid + 8 of a lane are the adjacent units 2 gid, 2 gid + 1, so states, activations and
+// deltas move as pairs.
+// The delta tile is double-buffered: a warp may write the next step's deltas while another still multiplies; the one after
+// that lies behind the next barrier.
+//
+// Replaces FLASHRNNCellFusedBackward (reference flashrnn/flashrnn/fused/flashrnn_fused_backward.cu:129-624),
+// the FLASHRNNPointwiseBackward functions (fused/*_fused_pointwise.cuh; GRU: alternating/gru_pointwise.cu:120-193)
+// and gradientBiasAggregationKernel (flashrnn_fused_backward.cu:626-665).
+#pragma once
+#include "frnn_lane.cuh"
+
+namespace FRNN_NS {
+
+template <int CELL, int KT, int U, int NT>
+struct LaneBwdGeom {
+  using C = Cell<CELL>;
+  static constexpr int D = KT * 16, CS = D / U, BT = 8 * NT;
+  static constexpr bool CL = CS > 1;
+  static constexpr int W = CL ? U / 8 : KT;       // compute warps
+  static constexpr int NB = CL ? NT : 2 * NT;     // batch rows per lane (2 adjacent units each)
+  static constexpr int K = C::Gr * U, KS = K / 16, KP = (KS + 1) / 2;  // this CTA's gate rows
+  static constexpr int MT = (KT + W - 1) / W;     // p tiles per warp (the last warps may have one less)
+  static constexpr int GCM = CacheGeom<C::GC>::MAIN;
+  static constexpr bool GCX = CacheGeom<C::GC>::EXTRA;
+  static constexpr int NSS = C::NNEED + C::NEXT;  // state-typed rows per batch row
+  static constexpr int IOW = io_warps(BT * U * 2 * (C::Gw + C::GC + NSS)), IOT = 32 * IOW;
+  static constexpr int TH = 32 * W + IOT;
+  // columns of the delta tile: the R gates in order; the GRU's input-only gate n, which no product reads, behind them
+  static constexpr int DCOLS = C::Gr == 3 ? 4 * U : K, DT = opnd_bytes(DCOLS), DB = NT * DT;
+  static constexpr int RB = CL ? CS * (U / 16) * 32 * NT * 16 : 0;  // bytes of received partial sums of one step
+  // input ring: [kLaneStages] x { activations [BT] | fifth ones [BT] | states and cotangents [NSS][BT] }
+  static constexpr int CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2), SP = io_pitch(U * 4);
+  static constexpr int IN_E = GCM ? BT * CP : 0, IN_S = IN_E + (GCX ? BT * EP : 0), IN_B = IN_S + NSS * BT * SP;
+  static constexpr int OFF_R = 2 * DB, OFF_I = OFF_R + 2 * RB, OFF_BAR = OFF_I + kLaneStages * IN_B;
+  static constexpr size_t smem = OFF_BAR + 2 * 8;
+  static constexpr bool valid = D % U == 0 && (!CL || U % 8 == 0) && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget && (NT == 1 || CL);  // (16 rows: see lane_nt)
+};
+
+// Index of the first of the two 16-byte fragments (rows gid, gid + 8) of lane 0 in the packed R^T of head n, CTA c: see
+// bwd_prepare_kernel, which writes it.
+__host__ __device__ constexpr size_t rt_frag(int n, int CS, int c, int KT, int mt, int KP, int kp) {
+  return ((((size_t)n * CS + c) * KT + mt) * KP + kp) * 64;
+}
+
+// The IO warps' part: ES = bytes of a state element.
+template <int CELL, int KT, int U, int NT, int ES>
+__device__ __forceinline__ void lane_bwd_io(const LoopParams& p, unsigned char* smem_raw, int io, uint32_t crank) {
+  using G = LaneBwdGeom<CELL, KT, U, NT>;
+  using C = Cell<CELL>;
+  constexpr int Gw = C::Gw, NNEED = C::NNEED, NEXT = C::NEXT, BT = G::BT, IOT = G::IOT, D = G::D;
+  using TC = IoTile<BT, U * 2 * (G::GCM ? G::GCM : 1) / 16, IOT>;  // activations
+  using TE = IoTile<BT, U / 8, IOT>;                               // fifth activations
+  using TP = IoTile<NNEED * BT, U * ES / 16, IOT>;                 // states at t-1
+  using TQ = IoTile<NEXT * BT, U * ES / 16, IOT>;                  // cotangents at t
+  using TW = IoTile<Gw * BT, U / 8, IOT>;                          // dWx
+  const int T = p.T, N = p.N, B = p.B, n = blockIdx.z, bt0 = blockIdx.y * BT;
+  const size_t ND = (size_t)N * D;
+  const int unit0 = (int)crank * U;
+  const uint32_t sm = smem_u32(smem_raw), in = sm + G::OFF_I;
+
+  // ---- input pointers, first step T-1.  Rows beyond B: zero activations and cotangents make their deltas zero; their states only
+  // have to be finite divisors (0x3f80 twice is about 1 as fp32, and 1 or 1.9 twice as a 16-bit pair)
+  for (uint32_t i = io; i < kLaneStages * G::IN_B / 16; i += IOT) {
+    const uint32_t o = i * 16 % G::IN_B, w = o >= (uint32_t)G::IN_S && o < (uint32_t)(G::IN_S + NNEED * BT * G::SP) ? 0x3f803f80u : 0u;
+    sts128(in + i * 16, make_uint4(w, w, w, w));
+  }
+  if constexpr (G::IOW > 1) asm volatile("bar.sync 1, %0;" ::"n"(IOT) : "memory");
+  else __syncwarp();
+  const size_t st_sb = (size_t)T * ND * ES;
+  const unsigned char* pp[TP::N];
+  const unsigned char* p0[TP::N];  // the initial state, which takes the place of states[-1]
+#pragma unroll
+  for (int i = 0; i < TP::N; ++i) {
+    const int r = TP::row(io, i), k = r / BT, b = bt0 + r - k * BT;
+    int need = 0;
+#pragma unroll
+    for (int q = 0; q < NNEED; ++q) need = k == q ? C::need(q) : need;
+    const bool live = TP::in(io, i) && b < B;
+    const size_t col = ((size_t)n * D + unit0) * ES + TP::col(io, i) * 16;
+    pp[i] = live ? static_cast<const unsigned char*>(p.states) + ((size_t)need * B + b) * st_sb + (size_t)(T - 1) * ND * ES - ND * ES + col : nullptr;
+    p0[i] = static_cast<const unsigned char*>(p.s0) + ((size_t)need * B + (live ? b : 0)) * ND * ES + col;
+  }
+  const unsigned char* qp[TQ::N];
+#pragma unroll
+  for (int i = 0; i < TQ::N; ++i) {
+    const int r = TQ::row(io, i), k = r / BT, b = bt0 + r - k * BT;
+    qp[i] = (TQ::in(io, i) && b < B) ? static_cast<const unsigned char*>(p.dstates) +
+                                           ((size_t)k * p.ds_ss + (size_t)b * p.ds_sb + (size_t)(T - 1) * p.ds_st + (size_t)n * p.ds_sn + unit0) * ES +
+                                           TQ::col(io, i) * 16
+                                     : nullptr;
+  }
+  constexpr int CW = 2 * (G::GCM ? G::GCM : 1);  // bytes of activations per unit
+  const unsigned char* cbase = static_cast<const unsigned char*>(static_cast<const void*>(p.cache)) + ((((size_t)(T - 1) * N + n) * B) * D + unit0) * CW;
+  const unsigned char* ebase = static_cast<const unsigned char*>(static_cast<const void*>(p.cache)) + (size_t)T * N * B * D * 8 +
+                               ((((size_t)(T - 1) * N + n) * B) * D + unit0) * 2;
+  auto load = [&](int t, int stage) {  // in step order T-1, T-2, ...
+    if (t >= 0) {
+      const uint32_t o = in + stage * G::IN_B;
+      if constexpr (G::GCM > 0) {
+#pragma unroll
+        for (int i = 0; i < TC::N; ++i) {
+          const int r = TC::row(io, i);
+          if (TC::in(io, i) && bt0 + r < B) cp_async16_u32(o + r * G::CP + TC::col(io, i) * 16, cbase + (size_t)(bt0 + r) * D * CW + TC::col(io, i) * 16);
+        }
+        cbase -= (size_t)N * B * D * CW;
+      }
+      if constexpr (G::GCX) {
+#pragma unroll
+        for (int i = 0; i < TE::N; ++i) {
+          const int r = TE::row(io, i);
+          if (TE::in(io, i) && bt0 + r < B)
+            cp_async16_u32(o + G::IN_E + r * G::EP + TE::col(io, i) * 16, ebase + (size_t)(bt0 + r) * D * 2 + TE::col(io, i) * 16);
+        }
+        ebase -= (size_t)N * B * D * 2;
+      }
+#pragma unroll
+      for (int i = 0; i < TP::N; ++i)
+        if (pp[i] != nullptr) {
+          cp_async16_u32(o + G::IN_S + TP::row(io, i) * G::SP + TP::col(io, i) * 16, t > 0 ? pp[i] : p0[i]);
+          pp[i] -= ND * ES;
+        }
+#pragma unroll
+      for (int i = 0; i < TQ::N; ++i)
+        if (qp[i] != nullptr) {
+          cp_async16_u32(o + G::IN_S + (NNEED * BT + TQ::row(io, i)) * G::SP + TQ::col(io, i) * 16, qp[i]);
+          qp[i] -= (size_t)p.ds_st * ES;
+        }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < kLaneStages; ++s) load(T - 1 - s, s);
+
+  // ---- dWx[b][t][g][n][unit0 ..] from delta columns (g + first) * U
+  constexpr int GSH = C::Gr == 3 ? 1 : 0;  // GRU: column block 0 is the recurrent-only gate, which goes to dg0
+  elem_t* wp[TW::N];
+  uint32_t ws[TW::N];
+#pragma unroll
+  for (int i = 0; i < TW::N; ++i) {
+    const int r = TW::row(io, i), g = r / BT, bl = r - g * BT, b = bt0 + bl, c = TW::col(io, i);
+    ws[i] = sm + (bl >> 3) * G::DT + opnd_off(bl & 7, (g + GSH) * U + c * 8);
+    wp[i] = (TW::in(io, i) && b < B) ? p.dWx + (((size_t)b * T + (T - 1)) * Gw + g) * ND + (size_t)n * D + unit0 + c * 8 : nullptr;
+  }
+  elem_t* gp[TE::N];
+#pragma unroll
+  for (int i = 0; i < TE::N; ++i) {
+    const int b = bt0 + TE::row(io, i);
+    gp[i] = (GSH && TE::in(io, i) && b < B) ? p.dg0 + ((size_t)b * T + (T - 1)) * ND + (size_t)n * D + unit0 + TE::col(io, i) * 8 : nullptr;
+  }
+  // barrier j of the CTA: the deltas of step j are complete, its inputs consumed, the inputs of step j + 1 have landed
+  cp_async_wait<kLaneStages - 1>();
+  __syncthreads();  // (in front of step 0)
+  int stage = 0;
+  for (int j = 0; j < T; ++j) {
+    cp_async_wait<kLaneStages - 2>();
+    __syncthreads();
+    load(T - 1 - j - kLaneStages, stage);
+#pragma unroll
+    for (int i = 0; i < TW::N; ++i)
+      if (wp[i] != nullptr) {
+        *reinterpret_cast<uint4*>(wp[i]) = lds128(ws[i] + (j & 1) * G::DB);
+        wp[i] -= (size_t)Gw * ND;
+      }
+    if constexpr (GSH) {
+#pragma unroll
+      for (int i = 0; i < TE::N; ++i)
+        if (gp[i] != nullptr) {
+          const int bl = TE::row(io, i);
+          *reinterpret_cast<uint4*>(gp[i]) = lds128(sm + (j & 1) * G::DB + (bl >> 3) * G::DT + opnd_off(bl & 7, TE::col(io, i) * 8));
+          gp[i] -= ND;
+        }
+    }
+    stage = stage + 1 == kLaneStages ? 0 : stage + 1;
+  }
+  cp_async_wait<0>();
+}
+
+template <int CELL, int KT, int U, int NT>
+__global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT>::TH) lane_bwd_kernel(const __grid_constant__ LoopParams p) {
+  using G = LaneBwdGeom<CELL, KT, U, NT>;
+  using C = Cell<CELL>;
+  // packed arithmetic where it measured faster (LSTM D = 64, one CTA per head: B1024 N16, 11551 -> 9881 clk per step of all CTAs)
+  using F2 = typename PairOf<CELL == CELL_LSTM && !G::CL>::type;
+  constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, NNEED = C::NNEED, NEXT = C::NEXT;
+  constexpr int CS = G::CS, D = G::D, MT = G::MT, NB = G::NB, W = G::W, DB = G::DB, DT = G::DT, KP = G::KP, BT = G::BT;
+  constexpr int GCM = G::GCM;
+  constexpr bool CL = G::CL;
+  constexpr int NS = acc_sets(MT * NT, W, G::KS, 4);
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gid = lane >> 2, tig = lane & 3, a = gid & 1;
+  const int T = p.T, N = p.N, B = p.B;
+  const int n = blockIdx.z, bt0 = blockIdx.y * BT;
+  const uint32_t crank = CL ? cluster_ctarank() : 0u;
+  const size_t ND = (size_t)N * D;
+  const int f32 = p.state_f32;
+
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const uint32_t sm = smem_u32(smem_raw), recv = sm + G::OFF_R;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + G::OFF_BAR);  // [2] bytes of partial sums have arrived
+
+  if (CL) {
+    if (tid == 0) {
+      mbar_init(&full[0], 1);
+      mbar_init(&full[1], 1);
+      fence_mbar_init();
+      mbar_arrive_expect_tx(&full[0], G::RB);             // partial sums of step index 0 (t = T-1)
+      if (T > 1) mbar_arrive_expect_tx(&full[1], G::RB);  // step index 1
+    }
+    __syncthreads();
+    cluster_arrive();  // waited for before the first push
+  }
+
+  if (warp >= W) {
+    const int io = tid - 32 * W;
+    if (f32) lane_bwd_io<CELL, KT, U, NT, 4>(p, smem_raw, io, crank);
+    else lane_bwd_io<CELL, KT, U, NT, 2>(p, smem_raw, io, crank);
+    if (CL) {
+      __syncwarp();
+      cluster_wait();
+      cluster_arrive_relaxed();
+      cluster_wait();
+    }
+    return;
+  }
+
+  const int ul = CL ? warp * 8 + (gid >> 1) * 2 : warp * 16 + 2 * gid;  // this lane's units within the CTA: ul, ul + 1
+  const int unit = (int)crank * U + ul;
+  const size_t nd = (size_t)n * D + unit;
+  auto row_of = [&](int nb) { return CL ? nb * 8 + 2 * tig + a : (nb >> 1) * 8 + 2 * tig + (nb & 1); };
+
+  bool ok[NB];
+  uint32_t cw[NB], sw[NB], dloc[NB];  // activation and state words of row nb in the input ring, delta words in the tile
+  F2 car[NB][S], cur[NB][NNEED], dbacc[Gt];  // this lane's two units of row nb
+#pragma unroll
+  for (int g = 0; g < Gt; ++g) dbacc[g] = v_pair<F2>(0.f, 0.f);
+#pragma unroll
+  for (int nb = 0; nb < NB; ++nb) {
+    const int r = row_of(nb), b = bt0 + r;
+    ok[nb] = b < B;
+    cw[nb] = sm + G::OFF_I + r * G::CP + ul * 2 * GCM;
+    sw[nb] = sm + G::OFF_I + G::IN_S + r * G::SP + ul * (f32 ? 4 : 2);
+    dloc[nb] = sm + (r >> 3) * DT + opnd_off(r & 7, ul);
+#pragma unroll
+    for (int s = 0; s < S; ++s) car[nb][s] = v_pair<F2>(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < NNEED; ++k) {
+      float2 v = make_float2(1.f, 1.f);
+      if (ok[nb]) v = load_state2(p.states, (((size_t)C::need(k) * B + b) * T + (T - 1)) * ND + nd, f32);
+      cur[nb][k] = v_pair<F2>(v.x, v.y);
+    }
+  }
+  // gate g's word of a lane lies g * U columns on: a constant distance when U / 8 blocks leave the permutation unchanged
+  auto dgate = [&](int nb, int g) -> uint32_t {
+    if constexpr (U % 32 == 0) return dloc[nb] + g * (U * 16);
+    else return sm + (row_of(nb) >> 3) * DT + opnd_off(row_of(nb) & 7, g * U + ul);
+  };
+
+  // ---- this warp's fragments of R^T
+  AFrag A[MT][KP];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    const int mt = warp + m * W < KT ? warp + m * W : KT - 1;  // (a warp without an m-th tile repeats another's, and sends nothing)
+#pragma unroll
+    for (int kp = 0; kp < KP; ++kp) {
+      const uint4* src = p.Rpack + rt_frag(n, CS, (int)crank, KT, mt, KP, kp) + lane;
+      A[m][kp].lo = __ldg(src);
+      A[m][kp].hi = __ldg(src + 32);
+    }
+  }
+
+  uint32_t dst[MT], dbar[MT];  // shared::cluster address of this lane's slot for tile m in the CTA that owns the tile, and of its barrier
+  if constexpr (CL) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const int mt = warp + m * W < KT ? warp + m * W : KT - 1, owner = mt * 16 / U, tl = mt - owner * (U / 16);
+      dst[m] = map_to_cta(recv + (uint32_t)((((int)crank * (U / 16) + tl) * NT * 32 + lane) * 16), (uint32_t)owner);
+      dbar[m] = map_to_cta(smem_u32(&full[0]), (uint32_t)owner);
+    }
+  }
+  // where this lane's partial sums arrive: source c at + c * (U/16) * NT * 512, batch tile nt at + nt * 512
+  const uint32_t rsrc = recv + (uint32_t)((ul >> 4) * NT * 512 + (((ul & 15) >> 1) * 4 + tig) * 16 + a * 8);
+  const bool drop = p.test_drop && crank == 0;  // test hook: CTA 0 withholds its first message
+  bool poisoned = false;  // a wait of this thread expired: it neither waits nor sends any more and the loop runs out
+  F2 rec[NB];             // matrix part of dh of the step about to run (CS == 1: handed over in registers)
+#pragma unroll
+  for (int nb = 0; nb < NB; ++nb) rec[nb] = v_pair<F2>(0.f, 0.f);
+
+  auto wait_partials = [&](int j, int t) {  // sums produced in step index j
+    if (!poisoned) {
+      if (!mbar_wait_bounded(&full[j & 1], (uint32_t)((j >> 1) & 1))) {
+        poisoned = true;
+        report_timeout(p.status, t);
+      }
+      // re-arm for step index j + 2; never after an expired wait: that phase is still open, no arrival left to give
+      else if (tid == 0 && j + 2 < T) mbar_arrive_expect_tx(&full[j & 1], G::RB);
+    }
+  };
+  auto sum_partials = [&](int j) {
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      F2 v[CS];
+#pragma unroll
+      for (int c = 0; c < CS; ++c) {
+        const uint2 w = lds64(rsrc + (uint32_t)((j & 1) * G::RB + (c * (U / 16) * NT + nb) * 512));
+        v[c] = v_pair<F2>(__uint_as_float(w.x), __uint_as_float(w.y));
+      }
+      // all loads first, then two short addition chains
+      F2 x = v[0], y = v[CS > 1 ? 1 : 0];
+#pragma unroll
+      for (int c = 2; c < CS; ++c) {
+        F2& r = (c & 1) ? y : x;
+        r = v_add(r, v[c]);
+      }
+      rec[nb] = v_add(x, y);
+    }
+  };
+
+  // ---- a step's inputs and what follows from them alone
+  uint4 in_c[NB];
+  uint32_t in_x[NB];
+  uint2 in_s[NB][G::NSS];
+  F2 co[NB][BwdCoef<CELL>::N], dext0[NB];
+  auto load_inputs = [&](int stage) {
+    const uint32_t so = stage * G::IN_B;
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      if constexpr (GCM == 4) in_c[nb] = lds128(cw[nb] + so);
+      else if constexpr (GCM == 1) in_c[nb].x = lds32(cw[nb] + so);
+      if constexpr (GC > 4) in_x[nb] = lds32(sm + G::OFF_I + G::IN_E + row_of(nb) * G::EP + ul * 2 + so);
+#pragma unroll
+      for (int k = 0; k < G::NSS; ++k) {
+        if (f32) in_s[nb][k] = lds64(sw[nb] + so + k * (BT * G::SP));
+        else in_s[nb][k].x = lds32(sw[nb] + so + k * (BT * G::SP));
+      }
+    }
+  };
+  auto form_coefs = [&]() {
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      F2 chv[GCA], ss[G::NSS];
+      if constexpr (GCM > 0) {
+        const uint32_t ww[4] = {in_c[nb].x, in_c[nb].y, in_c[nb].z, in_c[nb].w};
+#pragma unroll
+        for (int k = 0; k < GCM; ++k) chv[k] = v_unpack<F2>(ww[k]);
+        if constexpr (GC > 4) chv[GC - 1] = v_unpack<F2>(in_x[nb]);
+      }
+#pragma unroll
+      for (int k = 0; k < G::NSS; ++k)
+        ss[k] = f32 ? v_pair<F2>(__uint_as_float(in_s[nb][k].x), __uint_as_float(in_s[nb][k].y)) : v_unpack<F2>(in_s[nb][k].x);
+      cell_backward_coef<CELL>(ss + NNEED, car[nb], chv, cur[nb], ss, co[nb]);
+      dext0[nb] = ss[NNEED];
+#pragma unroll
+      for (int k = 0; k < NNEED; ++k) cur[nb][k] = ss[k];
+    }
+  };
+
+  __syncthreads();  // the inputs of the first step have landed
+  int stage = 0;
+  for (int j = 0; j < T; ++j) {  // j-th step of the reverse loop, time index t = T-1-j
+    const int t = T - 1 - j, buf = j & 1;
+    load_inputs(stage);
+    form_coefs();
+    if constexpr (CL) {
+      if (j > 0) {
+        wait_partials(j - 1, t);
+        sum_partials(j - 1);
+      }
+    }
+    // ---- gate deltas
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      F2 dR_[Gr], dW_[Gw], dB_[Gt];
+      F2 r = car[nb][0];
+      if (!p.grad_cut) r = v_add(r, rec[nb]);
+      if (p.gclip > 0.f) r = v_clamp(r, p.gclip);
+      cell_backward_apply<CELL>(v_add(dext0[nb], r), co[nb], car[nb], dR_, dW_, dB_);
+#pragma unroll
+      for (int g = 0; g < Gr; ++g) sts32(dgate(nb, g) + buf * DB, v_pack(dR_[g]));
+      if constexpr (Gr == 3) sts32(dgate(nb, 3) + buf * DB, v_pack(dW_[2]));
+#pragma unroll
+      for (int g = 0; g < Gt; ++g) dbacc[g] = v_add(dbacc[g], dB_[g]);
+    }
+    __syncthreads();
+    // ---- partial dh_{t-1}
+    float acc[MT][NT][4];
+    lane_mma<MT, G::KS, NT, NS, false>(A, sm + buf * DB, DT, gid, tig, acc, []() {});
+    if constexpr (CL) {
+      if (j == 0) cluster_wait();
+      if (!poisoned && !(drop && j == 0)) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+          if (KT % W == 0 || warp + m * W < KT) {
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+              st_async_v4(dst[m] + buf * G::RB + nt * 512, acc[m][nt][0], acc[m][nt][2], acc[m][nt][1], acc[m][nt][3], dbar[m] + buf * 8);
+          }
+      }
+    } else {
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) rec[nb] = v_pair<F2>(acc[0][nb >> 1][nb & 1], acc[0][nb >> 1][2 + (nb & 1)]);
+    }
+    stage = stage + 1 == kLaneStages ? 0 : stage + 1;
+  }
+  if constexpr (CL) {
+    wait_partials(T - 1, -1);
+    sum_partials(T - 1);
+  }
+
+  // ---- cotangent of the initial states, bias gradient
+#pragma unroll
+  for (int nb = 0; nb < NB; ++nb) {
+    if (!ok[nb]) continue;
+    const size_t off = (size_t)(bt0 + row_of(nb)) * ND + nd;
+    if (!p.grad_cut) car[nb][0] = v_add(car[nb][0], rec[nb]);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const float2 v = v_get(car[nb][s]);
+      store_state2(p.ds0, off + (size_t)s * B * ND, f32, v.x, v.y);
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < Gt; ++g) {
+    const float2 v = v_get(dbacc[g]);
+    atomicAdd(p.dbias + (size_t)g * ND + nd, v.x);
+    atomicAdd(p.dbias + (size_t)g * ND + nd + 1, v.y);
+  }
+  // every message to this CTA has been waited for; only after an expired wait can one still be in flight, and then the barrier
+  // covers it
+  if (CL) { __syncwarp(); cluster_arrive_relaxed(); cluster_wait(); }
+}
+
+}  // namespace FRNN_NS

@@ -29,73 +29,9 @@
 // the FLASHRNNPointwiseBackward functions (fused/*_fused_pointwise.cuh; GRU: alternating/gru_pointwise.cu:120-193)
 // and gradientBiasAggregationKernel (flashrnn_fused_backward.cu:626-665).
 #pragma once
-#include "frnn_common.cuh"
+#include "frnn_cell.cuh"
 
 namespace FRNN_NS {
-
-// Closed-form backward of one cell update, fp32.
-//   dh        total cotangent of h_t (external + recurrent)
-//   dext[k]   external cotangents of the states 1..NEXT-1 (dext[0] unused)
-//   car[s]    in: cotangent carried from step t+1 for state s (s >= 1); out: carried to step t-1.
-//             car[0] out = the direct (non-matrix) part of dh_{t-1} (GRU: z * dh), else 0.
-//   cur[k]/prv[k]  needed states (Cell::need(k)) at t and t-1
-//   dR_[g]    deltas of the R-connected gates (order of R), dW_[g] of the Wx gates, dB_[g] of the bias gates
-template <int CELL>
-__device__ __forceinline__ void cell_backward(float dh, const float* dext, float* car, const float* cache,
-                                              const float* cur, const float* prv, float* dR_, float* dW_,
-                                              float* dB_) {
-  if constexpr ((CELL & kNoopCell) != 0) {  // chain-floor probe: no gate math
-    using C = Cell<CELL>;
-    const float dg = 0.25f * dh + cache[0] * 0.f;
-#pragma unroll
-    for (int g = 0; g < C::Gr; ++g) dR_[g] = dg;
-#pragma unroll
-    for (int g = 0; g < C::Gw; ++g) dW_[g] = dg;
-#pragma unroll
-    for (int g = 0; g < C::Gt; ++g) dB_[g] = dg;
-#pragma unroll
-    for (int s = 0; s < C::S; ++s) car[s] = 0.f;
-  } else if constexpr (CELL == CELL_LSTM) {  // vanilla_fwbw/bw.py:100-133
-    const float ig = cache[0], fg = cache[1], zv = cache[2], og = cache[3];
-    const float tc = fast_tanh(cur[0]);
-    const float dc = dext[1] + car[1] + dh * og * (1.f - tc * tc);
-    dR_[0] = dc * zv * ig * (1.f - ig);
-    dR_[1] = dc * prv[0] * fg * (1.f - fg);
-    dR_[2] = dc * ig * (1.f - zv * zv);
-    dR_[3] = dh * tc * og * (1.f - og);
-#pragma unroll
-    for (int g = 0; g < 4; ++g) { dW_[g] = dR_[g]; dB_[g] = dR_[g]; }
-    car[0] = 0.f; car[1] = dc * fg;
-  } else if constexpr (CELL == CELL_GRU) {  // alternating/gru_pointwise.cu:120-193
-    const float gr = cache[0], rg = cache[1], zg = cache[2], nv = cache[3];
-    const float dz = dh * (prv[0] - nv) * zg * (1.f - zg);
-    const float dn = dh * (1.f - zg) * (1.f - nv * nv);
-    const float dr = dn * gr * rg * (1.f - rg);
-    const float dg = dn * rg;
-    dR_[0] = dg; dR_[1] = dr; dR_[2] = dz;
-    dW_[0] = dr; dW_[1] = dz; dW_[2] = dn;
-    dB_[0] = dg; dB_[1] = dr; dB_[2] = dz; dB_[3] = dn;
-    car[0] = zg * dh;
-  } else if constexpr (CELL == CELL_ELMAN || CELL == CELL_ELMAN_CLIP) {  // fused/elman_fused_pointwise.cuh:62-93
-    const float hv = (CELL == CELL_ELMAN_CLIP) ? cache[0] : cur[0];  // the tanh output (before any forward clamp)
-    const float dg = dh * (1.f - hv * hv);
-    dR_[0] = dg; dW_[0] = dg; dB_[0] = dg;
-    car[0] = 0.f;
-  } else {  // sLSTM, vanilla_fwbw/bw.py:136-189 (stabiliser m treated as a constant)
-    const float ig = cache[0], fg = cache[1], zv = cache[2], og = cache[3], omsf = cache[4];
-    const float cn = cur[0], n2 = cur[1];
-    const float inv_n = __fdividef(1.f, n2);
-    const float dc = dext[1] + car[1] + dh * og * inv_n;
-    const float dn = dext[2] + car[2] - dh * og * cn * inv_n * inv_n;
-    dR_[0] = ig * (zv * dc + dn);
-    dR_[1] = fg * (dc * prv[0] + dn * prv[1]) * omsf;
-    dR_[2] = dc * ig * (1.f - zv * zv);
-    dR_[3] = dh * cn * inv_n * og * (1.f - og);
-#pragma unroll
-    for (int g = 0; g < 4; ++g) { dW_[g] = dR_[g]; dB_[g] = dR_[g]; }
-    car[0] = 0.f; car[1] = fg * dc; car[2] = fg * dn; car[3] = 0.f;
-  }
-}
 
 // U and CS implied by a reduce-scatter instantiation: all Gr*U/16 local k-steps per warp, MPW row tiles per warp
 template <int CELL, int KT, int MPW> struct RsGeom {

@@ -17,56 +17,9 @@
 // Replaces FLASHRNNCellFusedForward (reference flashrnn/flashrnn/fused/flashrnn_fused_forward.cu:146-659)
 // and the per-cell FLASHRNNPointwiseForward functions (fused/{lstm,gru,elman,slstm}_fused_pointwise.cuh).
 #pragma once
-#include "frnn_common.cuh"
+#include "frnn_cell.cuh"
 
 namespace FRNN_NS {
-
-// One cell update in fp32.  pre[g] = (R h)[g];  wx[g], bias[g] as laid out by the reference's gate orders
-// (vanilla/lstm.py:19, vanilla/gru.py:16-20, vanilla/elman.py:16-20, vanilla/slstm.py:16-18).
-// st[]: previous states in, new states out.  cache[]: values kept for the backward pass.
-template <int CELL>
-__device__ __forceinline__ void cell_forward(const float* pre, const float* wx, const float* bias, float* st,
-                                             float* cache) {
-  if constexpr ((CELL & kNoopCell) != 0) {  // chain-floor probe: no gate math, values stay bounded
-    using C = Cell<CELL>;
-    st[0] = 0.25f * (pre[0] + wx[0] + bias[0]);
-#pragma unroll
-    for (int k = 0; k < C::GC; ++k) cache[k] = st[0];
-  } else if constexpr (CELL == CELL_LSTM) {
-    const float ig = fast_sigmoid(pre[0] + wx[0] + bias[0]);
-    const float fg = fast_sigmoid(pre[1] + wx[1] + bias[1]);
-    const float zv = fast_tanh(pre[2] + wx[2] + bias[2]);
-    const float og = fast_sigmoid(pre[3] + wx[3] + bias[3]);
-    const float c = fg * st[1] + ig * zv;
-    st[0] = og * fast_tanh(c);
-    st[1] = c;
-    cache[0] = ig; cache[1] = fg; cache[2] = zv; cache[3] = og;
-  } else if constexpr (CELL == CELL_GRU) {
-    const float gr = pre[0] + bias[0];                       // recurrent-only gate
-    const float rg = fast_sigmoid(wx[0] + pre[1] + bias[1]);
-    const float zg = fast_sigmoid(wx[1] + pre[2] + bias[2]);
-    const float nv = fast_tanh(wx[2] + bias[3] + rg * gr);   // input-only gate n
-    st[0] = zg * st[0] + (1.f - zg) * nv;
-    cache[0] = gr; cache[1] = rg; cache[2] = zg; cache[3] = nv;
-  } else if constexpr (CELL == CELL_ELMAN || CELL == CELL_ELMAN_CLIP) {
-    st[0] = fast_tanh(pre[0] + wx[0] + bias[0]);
-    if constexpr (CELL == CELL_ELMAN_CLIP) cache[0] = st[0];  // h is clamped afterwards: keep the tanh output
-  } else {  // sLSTM; "m' = i~ when n == 0" is applied per element (fused/slstm_fused_pointwise.cuh:53-62)
-    const float ir = pre[0] + wx[0] + bias[0];
-    const float fr = pre[1] + wx[1] + bias[1];
-    const float zv = fast_tanh(pre[2] + wx[2] + bias[2]);
-    const float og = fast_sigmoid(pre[3] + wx[3] + bias[3]);
-    const float lfm = log_sigmoid(fr) + st[3];
-    const float mn = (st[2] == 0.f) ? ir : fmaxf(ir, lfm);
-    const float ig = fminf(1.f, __expf(ir - mn));
-    const float fg = fminf(1.f, __expf(lfm - mn));
-    const float c = fg * st[1] + ig * zv;
-    const float n = fmaxf(fg * st[2] + ig, 1.f);
-    st[0] = og * __fdividef(c, n);
-    st[1] = c; st[2] = n; st[3] = mn;
-    cache[0] = ig; cache[1] = fg; cache[2] = zv; cache[3] = og; cache[4] = 1.f - fast_sigmoid(fr);
-  }
-}
 
 // dynamic shared memory of the forward kernel, in bytes
 template <int CELL, int NT>
@@ -289,7 +242,9 @@ __global__ void __launch_bounds__(LaunchBounds<CELL, KT>::threads, LaunchBounds<
         for (int s = 0; s < S; ++s) sv[s] = st[i][s][e];
 #pragma unroll
         for (int g = 0; g < Gt; ++g) bv[g] = bias[i][g][e];
-        cell_forward<CELL>(prv[e], wxv[e], bv, sv, cv);
+        float gx[Gt];
+        gate_sums<CELL>(prv[e], wxv[e], bv, gx);
+        cell_forward<CELL>(gx, sv, cv);
         if (p.fclip > 0.f) sv[0] = clampf(sv[0], p.fclip);
         if (!it_ok[i]) {  // rows beyond B: keep everything zero
 #pragma unroll

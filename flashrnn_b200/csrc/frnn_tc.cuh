@@ -84,11 +84,6 @@ __host__ __device__ constexpr uint32_t instr_desc_16(int M, int N, int a_mn, int
          ((uint32_t)(M >> 4) << 24);
 }
 
-// ---- mbarrier extras
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // ---- tensor-map bulk copies (5-d tiles; coordinates innermost first; the innermost one must keep 16-byte alignment)
 __device__ __forceinline__ void tma_load_5d(uint32_t dst_smem, const void* tmap, int c0, int c1, int c2, int c3, int c4,
                                             uint64_t* bar) {

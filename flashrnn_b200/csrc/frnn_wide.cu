@@ -312,10 +312,8 @@ wide_fwd_elman_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
 // warps w and w + 4 share 32 rows and split the 64 units) read the accumulator 16 units at a time (4 gates x 16 columns),
 // keep the cell state c of their 32 units in registers (fp32) and write h_t into the shared-memory tile that the next
 // step multiplies and a bulk store sends to `states[0]`.  After the arrival that hands h_t on, c_t and the four cached
-// activations go straight to global memory: a thread owns 64 contiguous bytes per value kind, neighbouring lanes swap
-// halves, and each 32-byte store instruction covers 16 rows x 64 bytes.  The activation cache is written in the layout of
-// the REVERSE loop's own tile (one CTA per head, 16 batch rows: frnn_bwd_kernel reads it as it reads its forward
-// kernel's), so only the forward loop changes.
+// activations go straight to global memory with 32-byte stores, c with neighbouring lanes swapping halves.  The activation
+// cache has the one layout every 16-bit loop uses ([t][head][b][unit pair][4]), so lane_bwd_kernel runs the reverse loop.
 // Wx_t arrives as one tensor-map copy of [4 gates][128 rows][64] per step into a ring of two 64 KB stages; the stage of
 // step t is refilled with step t+2 as soon as the step's MMAs are known to have completed.
 struct WideGatesParams {
@@ -323,7 +321,7 @@ struct WideGatesParams {
   const elem_t* bias;  // [4,N,64]
   const elem_t* s0;    // [2,B,1,N,64]
   elem_t* states;      // [2,B,T,N,64]; h leaves through the tensor map, c through plain stores
-  uint32_t* cache;     // reverse loop's layout (16-row tiles): [t][head][tile][slot][row in tile][unit pair]; or null
+  uint32_t* cache;     // [t][head][b][unit pair][4 slots]; or null
   unsigned* status;
   int B, T, N;
   int test_drop;  // test hook: the copy of one Wx box (step index 2) is announced to its barrier but never issued
@@ -530,11 +528,8 @@ wide_fwd_gates_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
     const bool ok_e = be < B, ok_o = be + 1 < B;
     elem_t* c_e = p.states + (((size_t)B + (ok_e ? be : 0)) * T) * ND + (size_t)n * WD + 32 * half + (odd ? 16 : 0);
     elem_t* c_o = c_e + (size_t)T * ND;
-    const size_t tiles16 = (size_t)((B + 15) / 16);
-    uint32_t* ch_e = p.cache ? p.cache + (((size_t)n * tiles16 + (size_t)(be >> 4)) * WL_G) * 512 + (size_t)(be & 15) * 32 + 16 * half + (odd ? 8 : 0)
-                             : nullptr;
-    uint32_t* ch_o = ch_e ? ch_e + 32 : nullptr;
-    const size_t ch_step = (size_t)N * tiles16 * WL_G * 512;
+    uint4* ch = p.cache ? reinterpret_cast<uint4*>(p.cache) + ((size_t)n * B + (row_ok ? b : 0)) * 32 + 16 * half : nullptr;
+    const size_t ch_step = (size_t)N * B * 32;
     for (int t = 0; t < T; ++t) {
       if (!mbar_wait_bounded(&acc_full[t & 1], (uint32_t)((t >> 1) & 1))) { report_timeout(p.status, t); break; }
       tc_fence_after();
@@ -602,26 +597,29 @@ wide_fwd_gates_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
       fence_proxy_async_smem();  // the tile is read by the tensor core and by the bulk store
       tc_fence_before();
       mbar_arrive(h_ready);
-      // A thread owns 64 contiguous bytes per value kind.  Neighbouring lanes (rows 2m, 2m+1) swap halves so that each of
-      // the two store instructions covers 16 rows x 64 contiguous bytes instead of 32 rows x 32: the memory system is
-      // charged per piece of a 128-byte line, and this halves the pieces.
-#pragma unroll
-      for (int k = GRU ? 1 : 0; k < 1 + WL_G; ++k) {  // (the GRU has no second state)
-        if (k > 0 && ch_e == nullptr) break;
-        const uint4 s0 = odd ? out[k][0] : out[k][2], s1 = odd ? out[k][1] : out[k][3];
+      if constexpr (!GRU) {
+        // c: a thread owns 64 contiguous bytes.  Neighbouring lanes (rows 2m, 2m+1) swap halves so that each of the two store
+        // instructions covers 16 rows x 64 contiguous bytes instead of 32 rows x 32: the memory system is charged per piece of
+        // a 128-byte line, and this halves the pieces.
+        const uint4 s0 = odd ? out[0][0] : out[0][2], s1 = odd ? out[0][1] : out[0][3];
         uint4 r0, r1;
         r0.x = __shfl_xor_sync(0xffffffffu, s0.x, 1); r0.y = __shfl_xor_sync(0xffffffffu, s0.y, 1);
         r0.z = __shfl_xor_sync(0xffffffffu, s0.z, 1); r0.w = __shfl_xor_sync(0xffffffffu, s0.w, 1);
         r1.x = __shfl_xor_sync(0xffffffffu, s1.x, 1); r1.y = __shfl_xor_sync(0xffffffffu, s1.y, 1);
         r1.z = __shfl_xor_sync(0xffffffffu, s1.z, 1); r1.w = __shfl_xor_sync(0xffffffffu, s1.w, 1);
-        void* de = k == 0 ? static_cast<void*>(c_e) : static_cast<void*>(ch_e + 512 * (k - 1));
-        void* dn = k == 0 ? static_cast<void*>(c_o) : static_cast<void*>(ch_o + 512 * (k - 1));
-        if (ok_e) st_global_32B(de, odd ? r0 : out[k][0], odd ? r1 : out[k][1]);
-        if (ok_o) st_global_32B(dn, odd ? out[k][2] : r0, odd ? out[k][3] : r1);
+        if (ok_e) st_global_32B(c_e, odd ? r0 : out[0][0], odd ? r1 : out[0][1]);
+        if (ok_o) st_global_32B(c_o, odd ? out[0][2] : r0, odd ? out[0][3] : r1);
+      }
+      if (ch != nullptr && row_ok) {  // 256 contiguous bytes per thread: the four values of a unit pair side by side
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint4 &i4 = out[1][q], &f4 = out[2][q], &z4 = out[3][q], &o4 = out[4][q];
+          st_global_32B(ch + 4 * q, make_uint4(i4.x, f4.x, z4.x, o4.x), make_uint4(i4.y, f4.y, z4.y, o4.y));
+          st_global_32B(ch + 4 * q + 2, make_uint4(i4.z, f4.z, z4.z, o4.z), make_uint4(i4.w, f4.w, z4.w, o4.w));
+        }
       }
       c_e += ND; c_o += ND;
-      if (ch_e != nullptr) { ch_e += ch_step; ch_o += ch_step; }
-
+      if (ch != nullptr) ch += ch_step;
     }
   }
   tc_fence_before();

@@ -76,8 +76,9 @@ typedef struct frnn_plan {
   frnn_problem prob;
   int32_t cluster_size;    /* CTAs that share one (head, batch tile); exchange h through DSMEM */
   int32_t units_per_cta;   /* hidden units of the head owned by one CTA                      */
-  int32_t batch_tile;      /* batch rows per CTA (8, 16, 32 or 128; float32 loops: 8, 4 or 2) */
-  int32_t threads;         /* threads per CTA of the time-loop kernels                       */
+  int32_t batch_tile;      /* batch rows per CTA (8, 16, 32 or 128; float32 loops: 8, 4 or 2); head dims up to 256 run 16 and
+                              32 as 8- or 16-row tiles, whichever is faster for the cell and direction */
+  int32_t threads;         /* thread class of the tile (2 x gates x units); the lane loops launch their own number */
   int32_t wx_stages;       /* time steps of Wx prefetched ahead into shared memory           */
   int32_t cache_slots;     /* activation values cached per (b,t,n,d) in training             */
   int32_t test_drop_exchange; /* TEST HOOK, leave 0.  1: CTA 0 of every cluster withholds one exchange message
@@ -86,7 +87,8 @@ typedef struct frnn_plan {
                                  status block (float32 cluster loops: the message of step 1 in both loops).  With the 128-row loops (batch_tile 128, or wide_forward): one tile copy (step
                                  index 2) is announced to its barrier and never issued.  Exercises the failure-detection path
                                  without faulting the GPU.                                                          */
-  int32_t keep_packed_r;      /* 0: frnn_forward clears the status block and repacks R into the workspace (default).
+  int32_t keep_packed_r;      /* 0: frnn_forward clears the status block and, where its loop needs it, repacks R into the
+                                 workspace (default).
                                  1: the workspace is as an earlier frnn_forward with this plan left it and R has not
                                  changed since: skip both launches (step-by-step decoding calls frnn_forward once per
                                  token); a device status recorded by an earlier step stays until the caller reads it */
@@ -118,8 +120,8 @@ typedef struct frnn_fwd_args {
   void* states;        /* [S,B,T,N,D]  dtype_state (output)          */
   void* cache;         /* cache_bytes, output; may be NULL when training == 0 or plan.cache_bytes == 0 */
   void* workspace;     /* workspace_bytes                            */
-  void* last;          /* optional (NULL: off) [S,B,1,N,D] dtype_state (output): the states after step T-1 (one strided
-                          device copy behind the time loop).  May be the very buffer `s0` points to: chunked or
+  void* last;          /* optional (NULL: off) [S,B,1,N,D] dtype_state (output): the states after step T-1 (stored by the
+                          time loop, or by one strided device copy behind it).  May be the very buffer `s0` points to: chunked or
                           token-by-token calls then carry their states in place                              */
   int64_t wx_stride[4]; /* element strides of the B, T, G, N dimensions of Wx (the D dimension is contiguous).  All
                            four 0: dense [B,T,Gw,N,D].  Each must be a non-negative multiple of 8 (16 bytes), else
@@ -164,7 +166,7 @@ int frnn_query(const frnn_problem* problem, frnn_plan* out);
  * memory; cluster_size 1 otherwise selects the loops that stream R from L2), batch_tile 8, 4 or 2, wx_stages 0. */
 int frnn_query_tile(const frnn_problem* problem, int cluster_size, int batch_tile, int wx_stages, frnn_plan* out);
 
-/* Whole-sequence forward: one persistent launch (plus a small weight-repack launch).
+/* Whole-sequence forward: one persistent launch (head dims above 256: plus a small weight-repack launch).
  * Replaces ForwardPass::Run (flashrnn/flashrnn/fused/flashrnn_fused_forward.cu:772-975). */
 int frnn_forward(const frnn_plan* plan, const frnn_fwd_args* args, void* stream);
 

@@ -1,0 +1,27 @@
+"""GPU: the lane loops (head dims up to 256) at the sizes where they can go wrong: every head dim they are instantiated for, one
+step, as many steps as and one more than their input ring holds (6), and batches around the 8-row tile; one CTA per head and
+clusters, 8- and 16-row tiles."""
+import pytest
+import torch
+
+from tests.util import assert_parity, make_inputs, run_native, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("function", ["lstm", "gru", "elman", "slstm"])
+@pytest.mark.parametrize("D,cs,bt", [(16, 1, 8), (32, 1, 16), (32, 2, 8), (64, 1, 8), (64, 1, 16), (64, 4, 16), (96, 3, 8), (96, 6, 16),
+                                     (128, 2, 16), (128, 4, 8), (192, 6, 16), (256, 8, 8)])
+@pytest.mark.parametrize("B,T,state_f32", [(1, 1, False), (7, 6, True), (9, 7, False), (17, 2, True)])
+def test_lane_loops_edges(cuda_device, function, D, cs, bt, B, T, state_f32):
+    N = 2
+    Wx, R, b, s0 = make_inputs(function, B, T, N, D, seed=D + T, random_init=True, state_f32=state_f32)
+    S = s0.shape[0]
+    cot = torch.randn(S, B, T, N, D, generator=torch.Generator().manual_seed(T), dtype=torch.float64).to(torch.bfloat16).to(torch.float64)
+    if function == "slstm":
+        cot[1:] = 0
+    opts = dict(gradient_recurrent_clipval=0.05) if B == 9 else (dict(forward_clipval=0.5) if B == 7 else {})
+    got = run_native(function, Wx, R, b, s0, cot=cot, state_f32=state_f32, cluster_size=cs, batch_tile=bt, **opts)
+    ref = run_oracle(function, Wx, R, b, s0, cot=cot, clip=opts.get("gradient_recurrent_clipval", 0.0),
+                     forward_clip=opts.get("forward_clipval", 0.0))
+    assert_parity(function, got, ref, tag=f"{function} D{D} cs{cs} bt{bt} B{B} T{T}", zero_init=False)
