@@ -1,14 +1,16 @@
-"""ctypes binding of libfrnn_b200.so (the C ABI declared in include/frnn.h).
+"""ctypes binding of libfrnn_b200.so (the C ABI declared in include/frnn.h), and the loader of the native front end
+(csrc/host/frnn_torch.cpp) that the public calls go through.
 
-The library is loaded from the package directory (built in-tree by ``flashrnn_b200.build``).  There is no
+Both are loaded from the package directory (built in-tree by ``flashrnn_b200.build``).  There is no
 fallback of any kind: a missing library or a failing call raises.
 """
 from __future__ import annotations
 
 import ctypes
-from pathlib import Path
-
 import os
+import re
+from pathlib import Path
+from typing import NoReturn
 
 PKG = Path(__file__).resolve().parent
 # FRNN_B200_LIB points the binding at another build of the same library (development variants)
@@ -117,6 +119,36 @@ def lib() -> ctypes.CDLL:
             raise RuntimeError(f"libfrnn_b200.so has ABI {L.frnn_abi_version()}, the binding expects {ABI_VERSION}")
         _lib = L
     return _lib
+
+
+_bridge = None
+
+
+def bridge():
+    """The native front end, bound to the loaded library.  Raises if either has not been built."""
+    global _bridge
+    if _bridge is None:
+        L = lib()
+        try:
+            from . import _torch_bridge
+        except ImportError as e:
+            raise RuntimeError("flashrnn_b200/_torch_bridge.so is missing or was built for another torch: build it with "
+                               "`python -m flashrnn_b200.build`.  flashrnn_b200 has no CPU or PyTorch fallback.") from e
+        _torch_bridge.init(*(ctypes.cast(getattr(L, fn), ctypes.c_void_p).value for fn in (
+            "frnn_query", "frnn_query_tile", "frnn_forward", "frnn_backward", "frnn_finalize_grads", "frnn_status_string")))
+        _bridge = _torch_bridge
+    return _bridge
+
+
+_STATUS = re.compile(r"(frnn_\w+) failed with status (-?\d+): (.*)")
+
+
+def reraise(error: RuntimeError) -> NoReturn:
+    """``error`` of the native front end as FrnnError where a library call returned a status, else as it is."""
+    m = _STATUS.match(str(error))
+    if m:
+        raise FrnnError(m[1], int(m[2]), m[3]) from None
+    raise error
 
 
 def status_string(code: int) -> str:

@@ -13,12 +13,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "_build"
 LIB = PKG / "libfrnn_b200.so"
+BRIDGE_SRC = CSRC / "host" / "frnn_torch.cpp"
+BRIDGE = PKG / "_torch_bridge.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -54,6 +57,24 @@ def _compile(src: Path, headers: list[Path], force: bool, f16: bool = False) -> 
     return obj
 
 
+def build_bridge(force: bool = False) -> Path:
+    """Compile the native front end (a Python extension module) against the installed torch."""
+    if force or _stale(BRIDGE, [BRIDGE_SRC, PKG.parent / "include" / "frnn.h"]):
+        import torch
+        from torch.utils.cpp_extension import include_paths, library_paths
+
+        cuda = Path(_nvcc()).resolve().parent.parent
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *(f"-I{p}" for p in [*include_paths(), cuda / "include", sysconfig.get_paths()["include"]]),
+               str(BRIDGE_SRC), "-o", str(BRIDGE), *(f"-L{p}" for p in [*library_paths(), cuda / "lib64"]),
+               "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-lcudart"]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"g++ failed for {BRIDGE_SRC.name}:\n{res.stderr[-4000:]}")
+    return BRIDGE
+
+
 def build(force: bool = False, jobs: int | None = None, extra_flags: tuple[str, ...] = (), lib: Path | None = None,
           obj_dir: Path | None = None) -> Path:
     """Compile every .cu under csrc/ for sm_100a and link the shared library next to the package.
@@ -72,7 +93,9 @@ def build(force: bool = False, jobs: int | None = None, extra_flags: tuple[str, 
     units = [(s, f16) for f16 in (False, True) for s in srcs]
     jobs = jobs or min(len(units), os.cpu_count() or 4)
     with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
+        bridge = ex.submit(build_bridge, force)
         objs = list(ex.map(lambda u: _compile(u[0], headers, force, u[1]), units))
+        bridge.result()
     if force or _stale(LIB, objs):
         cmd = [_nvcc(), "-shared", "-o", str(LIB), *map(str, objs), "-cudart", "static"]
         res = subprocess.run(cmd, capture_output=True, text=True)

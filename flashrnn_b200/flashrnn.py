@@ -174,8 +174,9 @@ def _raise_on_device_status(ws: torch.Tensor, device, what: str) -> None:
 
 
 class _FrnnFunction(torch.autograd.Function):
-    """autograd bridge: one frnn_forward, one frnn_backward (+ optional all-reduce) + frnn_finalize_grads.
-    Takes the place of FlashRNNFunctionFused (reference flashrnn.py:688-801)."""
+    """autograd bridge of the calls with something between or behind the launches (an all-reduce of the gradients, a status
+    check): one frnn_forward, one frnn_backward (+ all-reduce) + frnn_finalize_grads.  All other calls take the native node of
+    csrc/host/frnn_torch.cpp.  Takes the place of FlashRNNFunctionFused (reference flashrnn.py:688-801)."""
 
     @staticmethod
     def forward(ctx, Wx, R, b, s0, cfg: FlashRNNConfig, training: bool, grad_group):
@@ -257,6 +258,14 @@ def flashrnn(
     addition: a ``torch.distributed`` process group (or ``True`` for the default group) over which dR/db are
     summed in backward when the batch is sharded across GPUs.
     """
+    if config is None and grad_allreduce_group is None and backend in _NATIVE_BACKENDS:
+        # the plain call: checked and run natively.  None: something is unusual, the code below takes it or says what is wrong
+        try:
+            out = (_native._bridge or _native.bridge()).call(Wx, R, b, states, function, dtype)
+        except RuntimeError as e:
+            _native.reraise(e)
+        if out is not None:
+            return out
     if config is None:
         config = _get_config(Wx, R, b, function, backend, dtype=dtype)
         if states is not None and states.dtype == torch.float32 and Wx.dtype != torch.float32:
@@ -292,14 +301,24 @@ def flashrnn(
     B, T, Gw, N, D = Wx.shape
     if Gw != config.num_gates_w or tuple(R.shape) != (config.num_gates_r, N, D, D) or tuple(b.shape) != (config.num_gates_t, N, D):
         raise ValueError(f"shape mismatch for function '{config.function}': Wx{tuple(Wx.shape)} R{tuple(R.shape)} b{tuple(b.shape)}")
-    if states is None:
+    if states is None and (T == 0 or config.initial_val != 0.0):
         states = _to_layout(_zero_state(config, Wx, batch=B), config.output_shape, "SBTHD").to(config.torch_dtype_s)
-    if tuple(states.shape) != (config.num_states, B, 1, N, D):
+    if states is not None and tuple(states.shape) != (config.num_states, B, 1, N, D):
         raise ValueError(f"states must be [S,B,1,N,D] = {(config.num_states, B, 1, N, D)}, got {tuple(states.shape)}")
     if T == 0:
         out = torch.empty((config.num_states, B, 0, N, D), dtype=config.torch_dtype_s, device=Wx.device)
         return (_to_layout(out, "SBTHD", config.output_shape),
                 _to_layout(states.to(config.torch_dtype_s), "SBTHD", config.output_shape))
+    if grad_allreduce_group is None and not config.check_device_status and not config._test_drop_exchange:
+        try:
+            all_states, last = _native.bridge().run(
+                Wx, R, b, states, config.function, config.dtype, config.dtype_s, config.forward_clipval or 0.0,
+                config.gradient_recurrent_clipval or 0.0, config.gradient_recurrent_cut, config.cluster_size, config.batch_tile)
+        except RuntimeError as e:
+            _native.reraise(e)
+        return _to_layout(all_states, "SBTHD", config.output_shape), _to_layout(last, "SBTHD", config.output_shape)
+    if states is None:
+        states = _to_layout(_zero_state(config, Wx, batch=B), config.output_shape, "SBTHD").to(config.torch_dtype_s)
     training = torch.is_grad_enabled() and any(t.requires_grad for t in (Wx, R, b, states))
     all_states = _FrnnFunction.apply(Wx, R, b, states, config, training, grad_allreduce_group)
     return (_to_layout(all_states, "SBTHD", config.output_shape),

@@ -1,24 +1,19 @@
 """Step-by-step (decoding) use of the forward loop.
 
 ``FlashRNNStepper`` keeps R, b, the carried states and every scratch buffer on the device and advances the recurrence
-by one chunk of time steps (default: one) per call: no allocation and no repacking of R per call -- the time loop and
-one strided copy that carries the last states in place, on the caller's current stream, so a step can be captured in a CUDA graph.  It is the
+by one chunk of time steps (default: one) per call: no allocation and no repacking of R per call -- one launch of the time loop,
+which also carries the last states in place, on the caller's current stream, so a step can be captured in a CUDA graph.  It is the
 counterpart of the reference's per-step kernel selection (``_get_kernel_step``, flashrnn/flashrnn/flashrnn.py:957-983;
 ``flashrnn_forward_step``, flashrnn/flashrnn/vanilla/__init__.py:73-121): same cells, same state layout, forward only.
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional
 
 import torch
 
 from . import _native
 from .flashrnn import DTYPE_DICT, rnn_function_registry
-
-
-def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
 
 
 class FlashRNNStepper:
@@ -51,7 +46,10 @@ class FlashRNNStepper:
         self._s0 = torch.zeros((S, batch_size, 1, N, D), dtype=sdt, device=dev)
         self._out = torch.empty((S, batch_size, chunk, N, D), dtype=sdt, device=dev)
         self._ws = torch.empty(int(self._plan.workspace_bytes), dtype=torch.uint8, device=dev)
-        self._packed = False
+        native = _native.bridge()
+        self._step = native.step
+        self._handle = native.stepper(self._R, self._b, self._s0, self._out, self._ws, bytes(self._plan),
+                                      (batch_size, chunk, Gw, N, D))
         if states is not None:
             self.reset(states)
 
@@ -68,15 +66,10 @@ class FlashRNNStepper:
         return self._s0
 
     def step(self, Wx: torch.Tensor) -> torch.Tensor:
-        if tuple(Wx.shape) != (self.B, self.chunk, self.Gw, self.N, self.D) or Wx.dtype != self._kdt or not Wx.is_contiguous():
-            raise ValueError(f"expected contiguous {self._kdt} Wx{(self.B, self.chunk, self.Gw, self.N, self.D)}")
-        dev = Wx.device
-        self._plan.keep_packed_r = 1 if self._packed else 0
-        # `last` = the s0 buffer itself: the carried states are updated in place by the library call
-        args = _native.FrnnFwdArgs(_ptr(Wx), _ptr(self._R), _ptr(self._b), _ptr(self._s0), _ptr(self._out), None, _ptr(self._ws),
-                                   _ptr(self._s0))
-        stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        with torch.cuda.device(dev):
-            _native.check("frnn_forward", _native.lib().frnn_forward(ctypes.byref(self._plan), ctypes.byref(args), stream))
-        self._packed = True
+        try:
+            ok = self._step(self._handle, Wx)
+        except RuntimeError as e:
+            _native.reraise(e)
+        if not ok:
+            raise ValueError(f"expected contiguous {self._kdt} Wx{(self.B, self.chunk, self.Gw, self.N, self.D)} on {self._R.device}")
         return self._out
