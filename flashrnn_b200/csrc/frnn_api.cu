@@ -20,7 +20,7 @@ static bool cell_dims(int cell, CellDims* d) {
   return false;
 }
 
-// The lane loops (head dims up to 256) and the streamed loops of a kernel family (kernel_cell) and direction.
+// The lane loops (head dims up to 256) and those for larger head dims of a kernel family (kernel_cell) and direction.
 static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt) {
   switch (cell) {
     case CELL_LSTM: return bwd ? lane_bwd_lstm(kt, u, nt) : lane_fwd_lstm(kt, u, nt);
@@ -31,15 +31,23 @@ static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt) {
   }
   return LaneKernel{nullptr, 0, 0};
 }
-static LoopKernel stream_kernel(int cell, bool bwd, int nt) {
+static BigKernel big_kernel(int cell, bool bwd, int u, int nt) {
   switch (cell) {
-    case CELL_LSTM: return bwd ? stream_bwd_lstm(nt) : stream_fwd_lstm(nt);
-    case CELL_GRU: return bwd ? stream_bwd_gru(nt) : stream_fwd_gru(nt);
-    case CELL_ELMAN: return bwd ? stream_bwd_elman(nt) : stream_fwd_elman(nt);
-    case CELL_ELMAN_CLIP: return bwd ? stream_bwd_elmanc(nt) : stream_fwd_elmanc(nt);
-    case CELL_SLSTM: return bwd ? stream_bwd_slstm(nt) : stream_fwd_slstm(nt);
+    case CELL_LSTM: return bwd ? big_bwd_lstm(u, nt) : big_fwd_lstm(u, nt);
+    case CELL_GRU: return bwd ? big_bwd_gru(u, nt) : big_fwd_gru(u, nt);
+    case CELL_ELMAN: return bwd ? big_bwd_elman(u, nt) : big_fwd_elman(u, nt);
+    case CELL_ELMAN_CLIP: return bwd ? big_bwd_elmanc(u, nt) : big_fwd_elmanc(u, nt);
+    case CELL_SLSTM: return bwd ? big_bwd_slstm(u, nt) : big_fwd_slstm(u, nt);
   }
-  return LoopKernel{nullptr, 0, nullptr};
+  return BigKernel{nullptr, 0, nullptr};
+}
+static cudaError_t big_pack(int cell, const void* R, void* out, int N, int D, cudaStream_t stream) {
+  switch (cell) {
+    case CELL_LSTM: return big_pack_lstm(R, out, N, D, stream);
+    case CELL_GRU: return big_pack_gru(R, out, N, D, stream);
+    case CELL_SLSTM: return big_pack_slstm(R, out, N, D, stream);
+    default: return big_pack_elman(R, out, N, D, stream);
+  }
 }
 
 // kernel family of a problem: the public cell id, except Elman with a forward clamp (caches its tanh output)
@@ -57,17 +65,18 @@ static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 constexpr size_t kMaxDynSmem = 227 * 1024;
 constexpr size_t kStatusBytes = 256;
 
-// head dims above 256 take the streamed kernels
-static bool streamed(const frnn_problem& pr) { return pr.D > 256; }
+// Head dims above 256 have kernels of their own (frnn_big_*.cuh).  Their plan names 64 units per CTA and clusters of D / 64; the
+// loops split the head further where they can (big_units).
+static bool is_big(const frnn_problem& pr) { return pr.D > 256; }
+constexpr int kBigPlanUnits = 64;
 
-// Scratch of a plan: status block, then what the plan's kernels need.  Only the streamed loops repack R for the forward pass.
+// Scratch of a plan: status block, then what the plan's kernels need.  Only head dims above 256 repack R for the forward pass.
 struct WsLayout { size_t rpack_fwd, rpack_bwd, grads, dg0, total; };
 static WsLayout workspace_layout(const frnn_problem& pr, const CellDims& cd, int units) {
   WsLayout w;
-  const size_t rbytes = (size_t)cd.Gr * pr.N * pr.D * pr.D * 2;
   size_t off = kStatusBytes;
-  w.rpack_fwd = off; if (streamed(pr)) off = align_up(off + rbytes, 256);
-  w.rpack_bwd = off; if (pr.training) off = align_up(off + (streamed(pr) ? rbytes : rt_pack_bytes(cd.Gr, pr.N, pr.D, units)), 256);
+  w.rpack_fwd = off; if (is_big(pr)) off = align_up(off + (size_t)(cd.Gr > 1 ? 4 : 1) * pr.N * pr.D * pr.D * 2, 256);
+  w.rpack_bwd = off; if (pr.training) off = align_up(off + rt_pack_bytes(cd.Gr, pr.N, pr.D, is_big(pr) ? big_units(pr.D) : units), 256);
   w.grads = off; if (pr.training) off = align_up(off + ((size_t)cd.Gr * pr.N * pr.D * pr.D + (size_t)cd.Gt * pr.N * pr.D) * 4, 256);
   w.dg0 = off;
   if (pr.training && pr.cell == CELL_GRU) off = align_up(off + (size_t)pr.B * pr.T * pr.N * pr.D * 2, 256);
@@ -97,20 +106,17 @@ static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) 
   const int D = pr.D;
   if (bt == kWideBatchTile) return cs == 1 && wide_problem(pr);  // 128-row tensor-core loops: one CTA per head and tile
   if (cs < 1 || D % cs) return false;
-  // clusters above 8 CTAs (a non-portable size): the streamed kernels, and 16 CTAs of 16 units for head dim 256
-  if (streamed(pr) ? (cs > 16 || D / cs != kStreamU) : (cs > 8 && !(cs == 16 && D == 256))) return false;
+  if (is_big(pr)) return D / cs == kBigPlanUnits && (bt == 8 || bt == 16);
+  // clusters above 8 CTAs (a non-portable size): 16 CTAs of 16 units for head dim 256
+  if (cs > 8 && !(cs == 16 && D == 256)) return false;
   const int U = D / cs;
   if (U % 16 || ((U / 16) & (U / 16 - 1))) return false;  // 16 * power of two
   if (bt != 8 && bt != 16 && bt != 32) return false;
   // a CTA owns at most 512 gate-row halves (256 from head dim 256, 384 from 192 up: the registers that hold R), and with
   // 32-row tiles at most 192 gate rows
   const int threads = 2 * cd.Gr * U;
-  if (threads > (streamed(pr) || D < 192 ? 512 : D < 256 ? 384 : 256)) return false;
-  if (bt == 32 && (streamed(pr) || cd.Gr * U > 192)) return false;
-  if (streamed(pr)) {
-    const LoopKernel f = stream_kernel(kernel_cell(pr), false, bt / 8), b = stream_kernel(kernel_cell(pr), true, bt / 8);
-    return f.smem_bytes(D, U, threads) <= kMaxDynSmem && b.smem_bytes(D, U, threads) <= kMaxDynSmem;
-  }
+  if (threads > (D < 192 ? 512 : D < 256 ? 384 : 256)) return false;
+  if (bt == 32 && cd.Gr * U > 192) return false;
   return lane_kernel(kernel_cell(pr), false, D / 16, U, lane_nt(pr, false, cs, bt)).fn &&
          lane_kernel(kernel_cell(pr), true, D / 16, U, lane_nt(pr, true, cs, bt)).fn;
 }
@@ -160,13 +166,13 @@ static bool choose_tile(const frnn_problem& pr, const CellDims& cd, int want_cs,
       for (int ci = -1; ci < 8; ++ci) {
         // (large batches of the single-gate cell do best without any cluster: Elman B1024 D=128, one CTA per head 100 M
         // tokens/s, clusters of 2 x 64 units 70)
-        if (ci < 0 && (want_cs || streamed(pr) || !cs32 || (fill && cd.Gr < 3))) continue;
+        if (ci < 0 && (want_cs || is_big(pr) || !cs32 || (fill && cd.Gr < 3))) continue;
         int cs = ci < 0 ? cs32 : (want_cs ? want_cs : (fill ? order_large[ci] : order_small[ci]));
         if (ci >= 0 && !fill && !want_cs && cs32 && cs > cs32) continue;  // fewer than 32 units per CTA
-        if (streamed(pr) && !want_cs) cs = pr.D / kStreamU;  // the streamed kernels have one geometry
-        const bool crowded = !fill && !want_cs && !streamed(pr) && pairs * cs > sms;
+        if (is_big(pr) && !want_cs) cs = pr.D / kBigPlanUnits;
+        const bool crowded = !fill && !want_cs && !is_big(pr) && pairs * cs > sms;
         if (!(pass == 0 && crowded) && tile_ok(pr, cd, cs, bt)) { *cs_out = cs; *bt_out = bt; return true; }
-        if (want_cs || streamed(pr)) break;
+        if (want_cs || is_big(pr)) break;
       }
     if (want_bt) break;
   }
@@ -182,7 +188,7 @@ static int validate_problem(const frnn_problem* pr, CellDims* cd) {
   if (pr->B < 1 || pr->T < 1 || pr->N < 1 || pr->D < 1) return FRNN_ERR_SHAPE;
   if (pr->N > 65535) return FRNN_ERR_SHAPE;
   if (pr->D % 16) return FRNN_ERR_SHAPE;
-  bool kt_ok = pr->D > 256 && pr->D <= kStreamMaxD && pr->D % kStreamU == 0;  // streamed kernels
+  bool kt_ok = pr->D > 256 && pr->D <= kBigMaxD && pr->D % kBigPlanUnits == 0;
   for (int i = 0; i < kNumKT; ++i) kt_ok = kt_ok || (kKTs[i] * 16 == pr->D);
   if (!kt_ok) return FRNN_ERR_SHAPE;
   return FRNN_OK;
@@ -252,32 +258,41 @@ static bool resolve_strides(const int64_t (&in)[4], const long long (&dense)[4],
   return true;
 }
 
-static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int rows, const frnn_plan& pl, const LoopParams& lp, cudaStream_t stream) {
+static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int cs, int rows, const frnn_plan& pl, const LoopParams& lp, cudaStream_t stream) {
   // always the fixed maximum, never this plan's own size: the attribute belongs to the kernel, not to the launch, and a
   // second host thread launching the same instantiation with a larger tile must not find it lowered in between
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
   if (e != cudaSuccess) return e;
-  if (pl.cluster_size > 8) {  // clusters of more than 8 CTAs are a non-portable size: opt in
+  if (cs > 8) {  // clusters of more than 8 CTAs are a non-portable size: opt in
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)pl.cluster_size, (unsigned)((pl.prob.B + rows - 1) / rows), (unsigned)pl.prob.N);
+  cfg.gridDim = dim3((unsigned)cs, (unsigned)((pl.prob.B + rows - 1) / rows), (unsigned)pl.prob.N);
   cfg.blockDim = dim3((unsigned)threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)pl.cluster_size;
+  attr[0].val.clusterDim.x = (unsigned)cs;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pl.cluster_size > 1 ? 1 : 0;
+  cfg.numAttrs = cs > 1 ? 1 : 0;
   void* args[1] = {const_cast<LoopParams*>(&lp)};
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
-static cudaError_t launch_stream(const LoopKernel& k, const frnn_plan& pl, const LoopParams& lp, cudaStream_t stream) {
-  return launch_loop(k.fn, pl.threads, k.smem_bytes(pl.prob.D, pl.units_per_cta, pl.threads), pl.batch_tile, pl, lp, stream);
+// 16-row tiles when 8-row ones would be more clusters than run at once (a B200 holds seven clusters of 16 CTAs)
+static int big_nt(const frnn_problem& pr) { return pr.B > 8 && (long long)((pr.B + 7) / 8) * pr.N * (pr.D / big_units(pr.D)) > 112 ? 2 : 1; }
+static int launch_big(const frnn_plan& pl, bool bwd, LoopParams lp, cudaStream_t stream) {
+  const frnn_problem& pr = pl.prob;
+  const int u = big_units(pr.D);
+  int nt = big_nt(pr);
+  BigKernel k = big_kernel(kernel_cell(pr), bwd, u, nt);
+  if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(kernel_cell(pr), bwd, u, nt = 1);  // (sLSTM reverse from head dim 896 up)
+  if (!k.fn || pl.probe_noop_cell) return FRNN_ERR_PLAN;
+  lp.CS = pr.D / u;
+  return (int)launch_loop(k.fn, k.threads, k.smem(pr.D), lp.CS, 8 * nt, pl, lp, stream);
 }
 static int launch_lane(const frnn_plan& pl, bool bwd, const LoopParams& lp, cudaStream_t stream) {
   const frnn_problem& pr = pl.prob;
@@ -285,7 +300,7 @@ static int launch_lane(const frnn_plan& pl, bool bwd, const LoopParams& lp, cuda
   const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(kernel_cell(pr), bwd, kt, pl.units_per_cta, nt)
                        : bwd              ? lane_bwd_floor(pr.cell, kt, pl.units_per_cta, nt)
                                           : lane_fwd_floor(pr.cell, kt, pl.units_per_cta, nt);
-  return k.fn ? (int)launch_loop(k.fn, k.threads, k.smem, 8 * nt, pl, lp, stream) : FRNN_ERR_PLAN;
+  return k.fn ? (int)launch_loop(k.fn, k.threads, k.smem, pl.cluster_size, 8 * nt, pl, lp, stream) : FRNN_ERR_PLAN;
 }
 
 static int sm_count_cached() {
@@ -379,13 +394,13 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
   long long wxs[4];
   if (!resolve_strides(a->wx_stride, wx_dense, wxs)) return FRNN_ERR_ALIGN;
 
-  const bool lane = !streamed(pr) && !is_wide(*plan) && !plan->wide_forward;
+  const bool wide = is_wide(*plan) || plan->wide_forward;
   // keep_packed_r: the workspace is left as the previous call left it (R fragments kept, status block not cleared, so
-  // an expired wait of an earlier step stays on record until the caller reads it).  The lane loops clear the block themselves.
-  cudaError_t e = plan->keep_packed_r || lane ? cudaSuccess : cudaMemsetAsync(ws, 0, kStatusBytes, stream);
+  // an expired wait of an earlier step stays on record until the caller reads it).  The other loops clear the block themselves.
+  cudaError_t e = plan->keep_packed_r || !wide ? cudaSuccess : cudaMemsetAsync(ws, 0, kStatusBytes, stream);
   if (e != cudaSuccess) return (int)e;
   if (a->last && !aligned16(a->last)) return FRNN_ERR_ALIGN;
-  // `last`: the lane loops store it; behind the others one strided device copy of states[:, :, T-1]
+  // `last`: one strided device copy of states[:, :, T-1] behind the 128-row loops; the others store it
   auto copy_last = [&]() -> cudaError_t {
     if (!a->last) return cudaSuccess;
     const size_t row = (size_t)pr.N * pr.D * (pr.dtype_state == FRNN_DTYPE_F32 ? 4 : 2);
@@ -404,7 +419,7 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
                                  reinterpret_cast<unsigned*>(ws), pr.B, pr.T, pr.N, pr.forward_clip, plan->test_drop_exchange, stream);
     return (int)(e == cudaSuccess ? copy_last() : e);
   }
-  if (!lane && !plan->keep_packed_r) e = launch_pack_recurrent(a->R, ws + w.rpack_fwd, cd.Gr, pr.N, pr.D, 0, stream);
+  if (is_big(pr) && !plan->keep_packed_r) e = big_pack(kernel_cell(pr), a->R, ws + w.rpack_fwd, pr.N, pr.D, stream);
   if (e != cudaSuccess) return (int)e;
 
   LoopParams lp = {};
@@ -424,10 +439,7 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
   lp.fclip = pr.forward_clip; lp.gclip = pr.grad_clip; lp.grad_cut = pr.grad_cut;
   lp.test_drop = plan->test_drop_exchange;
   lp.wx_sb = wxs[0]; lp.wx_st = wxs[1]; lp.wx_sg = wxs[2]; lp.wx_sn = wxs[3];
-  if (lane) return launch_lane(*plan, false, lp, stream);
-  if (plan->probe_noop_cell) return FRNN_ERR_PLAN;
-  e = launch_stream(stream_kernel(kernel_cell(pr), false, plan->batch_tile / 8), *plan, lp, stream);
-  return (int)(e == cudaSuccess ? copy_last() : e);
+  return is_big(pr) ? launch_big(*plan, false, lp, stream) : launch_lane(*plan, false, lp, stream);
 }
 
 #ifndef FRNN_F16
@@ -460,15 +472,15 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   if (!resolve_strides(a->dstates_stride, ds_dense, dss)) return FRNN_ERR_ALIGN;
 
   cudaError_t e = cudaSuccess;
-  if ((parts & FRNN_PART_LOOP) && !is_wide(*plan) && !streamed(pr)) {
-    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, plan->units_per_cta, grads, nR + nb, reinterpret_cast<unsigned*>(ws), stream);
+  if ((parts & FRNN_PART_LOOP) && !is_wide(*plan)) {
+    const bool big = is_big(pr);
+    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, big ? big_units(pr.D) : plan->units_per_cta, big, grads, nR + nb,
+                           reinterpret_cast<unsigned*>(ws), stream);
     if (e != cudaSuccess) return (int)e;
   } else if (parts & FRNN_PART_LOOP) {
     e = cudaMemsetAsync(ws, 0, kStatusBytes, stream);
     if (e != cudaSuccess) return (int)e;
     e = cudaMemsetAsync(grads, 0, (nR + nb) * sizeof(float), stream);
-    if (e != cudaSuccess) return (int)e;
-    if (!is_wide(*plan)) e = launch_pack_recurrent(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, 1, stream);
     if (e != cudaSuccess) return (int)e;
   }
   if (is_wide(*plan)) {  // one kernel: reverse loop with dR and db accumulated inside; the dR part has nothing left to do
@@ -497,14 +509,8 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   lp.test_drop = plan->test_drop_exchange;
   lp.ds_ss = dss[0]; lp.ds_sb = dss[1]; lp.ds_st = dss[2]; lp.ds_sn = dss[3];
   if (parts & FRNN_PART_LOOP) {
-    if (!streamed(pr)) {
-      rc = launch_lane(*plan, true, lp, stream);
-      if (rc) return rc;
-    } else {
-      if (plan->probe_noop_cell) return FRNN_ERR_PLAN;
-      e = launch_stream(stream_kernel(kernel_cell(pr), true, plan->batch_tile / 8), *plan, lp, stream);
-    }
-    if (e != cudaSuccess) return (int)e;
+    rc = is_big(pr) ? launch_big(*plan, true, lp, stream) : launch_lane(*plan, true, lp, stream);
+    if (rc) return rc;
   }
   // measured on B200: the tcgen05 kernel wins from head_dim 128 up (C2 0.167 vs 0.212 ms, C3 0.263 vs 0.304 ms) and at
   // head_dim 64 when the gates fill two 128-row tiles (LSTM B1024 T512 N16 D64: 1.43 vs 1.60 ms; the GRU's 192 rows, one

@@ -1,48 +1,17 @@
 // Helper kernels around the time loops:
-//   pack_recurrent_kernel  R[Gr,N,D,D] -> warp-MMA A fragments (forward: R, backward: R^T)
+//   bwd_prepare_kernel     R^T as warp-MMA A fragments of the reverse loops; gradients and status zeroed
 //   recurrent_grad_kernel  dR[g,n,d,p] = sum_{b,t} delta_g[b,t,n,d] * h_{t-1}[b,n,p]   (split-K tensor-core GEMM)
 //   cast_grads_kernel      fp32 dR || db -> parameter dtype
 #include "frnn_aux.cuh"
 
 namespace FRNN_NS {
 
-// One thread builds one 16-byte fragment (what one lane holds of one 16x16 A tile of mma.m16n8k16):
-//   out[((n*Gr + g)*(D/16) + ut)*(D/16) + k][lane] ;  A[row][kk], row/kk in 0..15
-//   forward : A[row][kk] = R[g][n][ut*16 + row][k*16 + kk]
-//   backward: A[row][kk] = R[g][n][k*16 + kk][ut*16 + row]      (rows = input unit p)
-__global__ void pack_recurrent_kernel(const elem_t* __restrict__ R, uint4* __restrict__ out, int Gr, int N, int D,
-                                      int transpose) {
-  const int KT = D / 16;
-  const size_t total = (size_t)N * Gr * KT * KT * 32;
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= total) return;
-  const int lane = (int)(idx & 31);
-  size_t r = idx >> 5;
-  const int k = (int)(r % KT); r /= KT;
-  const int ut = (int)(r % KT); r /= KT;
-  const int g = (int)(r % Gr);
-  const int n = (int)(r / Gr);
-  const int gid = lane >> 2, tig = lane & 3;
-  const elem_t* Rg = R + (((size_t)g * N + n) * D) * D;
-  auto at = [&](int row, int kk) -> unsigned short {
-    const int a = ut * 16 + row, c = k * 16 + kk;
-    const elem_t v = transpose ? Rg[(size_t)c * D + a] : Rg[(size_t)a * D + c];
-    return *reinterpret_cast<const unsigned short*>(&v);
-  };
-  auto pair = [&](int row, int kk) -> uint32_t { return (uint32_t)at(row, kk) | ((uint32_t)at(row, kk + 1) << 16); };
-  uint4 v;
-  v.x = pair(gid, 2 * tig);
-  v.y = pair(gid + 8, 2 * tig);
-  v.z = pair(gid, 2 * tig + 8);
-  v.w = pair(gid + 8, 2 * tig + 8);
-  out[idx] = v;
-}
-
 // In front of a reverse lane loop, one launch: R^T as the 16-byte fragments its warps keep in registers, the fp32 gradients
 // and the status block zeroed.  One thread builds the two fragments (rows 2 gid and 2 gid + 1 of a 16-row tile of p) of one
-// lane: eight consecutive gate rows k = 8 tig .. of the CTA's K = Gr * U (an odd last k-step: four).
+// lane: eight consecutive gate rows k = 8 tig .. of the CTA's K = Gr * U.  When K is an odd number of k-steps the last one takes four,
+// or (`pad`) eight of which those beyond K are zero.
 //   out[((((n * CS + c) * D/16 + mt) * KP + kp) * 2 + row parity) * 32 + lane], KP = ceil(K / 32)
-__global__ void bwd_prepare_kernel(const elem_t* __restrict__ R, uint4* __restrict__ out, int Gr, int N, int D, int U, int KP,
+__global__ void bwd_prepare_kernel(const elem_t* __restrict__ R, uint4* __restrict__ out, int Gr, int N, int D, int U, int KP, int pad,
                                    size_t nfrag, float4* __restrict__ grads, size_t ngrads4, unsigned* __restrict__ status) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < 64) status[idx] = 0u;
@@ -53,8 +22,8 @@ __global__ void bwd_prepare_kernel(const elem_t* __restrict__ R, uint4* __restri
   const int kp = (int)(r % KP); r /= KP;
   const int mt = (int)(r % (D / 16)); r /= (D / 16);
   const int c = (int)(r % CS), n = (int)(r / CS);
-  const bool pair = kp * 32 + 32 <= K;
-  const int k0 = kp * 32 + tig * (pair ? 8 : 4), ne = pair ? 8 : 4, g = k0 / U, u0 = k0 - g * U;
+  const bool pair = pad || kp * 32 + 32 <= K;
+  const int k0 = kp * 32 + tig * (pair ? 8 : 4), ne = k0 < K ? (pair ? 8 : 4) : 0, g = k0 < K ? k0 / U : 0, u0 = k0 - g * U;
   const unsigned* src = reinterpret_cast<const unsigned*>(R + ((((size_t)g * N + n) * D + (size_t)c * U + u0) * D + mt * 16 + 2 * gid));
   unsigned w[8];
 #pragma unroll
@@ -216,23 +185,14 @@ __global__ void cast_grads_kernel(const float* __restrict__ src, elem_t* __restr
 }
 
 // ---------------------------------------------------------------------------------------------------------
-cudaError_t launch_pack_recurrent(const void* R, void* out, int Gr, int N, int D, int transpose, cudaStream_t stream) {
-  const int KT = D / 16;
-  const size_t total = (size_t)N * Gr * KT * KT * 32;
-  const int threads = 256;
-  pack_recurrent_kernel<<<(unsigned)((total + threads - 1) / threads), threads, 0, stream>>>(
-      static_cast<const elem_t*>(R), static_cast<uint4*>(out), Gr, N, D, transpose);
-  return cudaGetLastError();
-}
-
 size_t rt_pack_bytes(int Gr, int N, int D, int U) { return (size_t)N * (D / U) * (D / 16) * ((Gr * U + 31) / 32) * 64 * 16; }
 
-cudaError_t launch_bwd_prepare(const void* R, void* out, int Gr, int N, int D, int U, float* grads, size_t ngrads, unsigned* status,
+cudaError_t launch_bwd_prepare(const void* R, void* out, int Gr, int N, int D, int U, int pad, float* grads, size_t ngrads, unsigned* status,
                                cudaStream_t stream) {
   const size_t nfrag = rt_pack_bytes(Gr, N, D, U) / 32;
   const int threads = 128;
   bwd_prepare_kernel<<<(unsigned)((nfrag + threads - 1) / threads), threads, 0, stream>>>(
-      static_cast<const elem_t*>(R), static_cast<uint4*>(out), Gr, N, D, U, (Gr * U + 31) / 32, nfrag, reinterpret_cast<float4*>(grads),
+      static_cast<const elem_t*>(R), static_cast<uint4*>(out), Gr, N, D, U, (Gr * U + 31) / 32, pad, nfrag, reinterpret_cast<float4*>(grads),
       ngrads / 4, status);
   return cudaGetLastError();
 }

@@ -12,27 +12,24 @@ namespace FRNN_NS {
 constexpr int kNumKT = 7;
 constexpr int kKTs[kNumKT] = {1, 2, 4, 6, 8, 12, 16};
 
-// head dims above 256 (multiples of 64 up to kStreamMaxD) run the streamed kernels: kStreamKT k-steps of R per warp
-// in registers, U = kStreamU units per CTA, cluster size D / kStreamU (up to 16, non-portable above 8)
-// (kStreamKT, kStreamU, kStreamMaxD: frnn_common.cuh)
-
 struct LaneKernel {
   const void* fn;  // kernel entry; null: no such instantiation
   int threads;
   size_t smem;
 };
-struct LoopKernel {
-  const void* fn;      // kernel entry
-  int max_threads;     // __launch_bounds__ of the instantiation
-  size_t (*smem_bytes)(int D, int U, int threads);
+struct BigKernel {
+  const void* fn;
+  int threads;
+  size_t (*smem)(int D);
 };
 
 // defined once per (cell, direction) in frnn_inst_*.cu
 #define FRNN_DECLARE(cell)                              \
   LaneKernel lane_fwd_##cell(int kt, int u, int nt);    \
   LaneKernel lane_bwd_##cell(int kt, int u, int nt);    \
-  LoopKernel stream_fwd_##cell(int nt);                 \
-  LoopKernel stream_bwd_##cell(int nt);
+  BigKernel big_fwd_##cell(int u, int nt);              \
+  BigKernel big_bwd_##cell(int u, int nt);              \
+  cudaError_t big_pack_##cell(const void* R, void* out, int N, int D, cudaStream_t stream);
 FRNN_DECLARE(lstm) FRNN_DECLARE(gru) FRNN_DECLARE(elman) FRNN_DECLARE(elmanc) FRNN_DECLARE(slstm)
 #undef FRNN_DECLARE
 
@@ -40,11 +37,10 @@ FRNN_DECLARE(lstm) FRNN_DECLARE(gru) FRNN_DECLARE(elman) FRNN_DECLARE(elmanc) FR
 LaneKernel lane_fwd_floor(int cell, int kt, int u, int nt);
 LaneKernel lane_bwd_floor(int cell, int kt, int u, int nt);
 
-// in front of a reverse lane loop: R^T as the fragments of its CTAs (U units each), fp32 gradients and status block zeroed
+// in front of a reverse loop: R^T as the fragments of its CTAs (U units each), fp32 gradients and status block zeroed
 size_t rt_pack_bytes(int Gr, int N, int D, int U);
-cudaError_t launch_bwd_prepare(const void* R, void* out, int Gr, int N, int D, int U, float* grads, size_t ngrads, unsigned* status,
+cudaError_t launch_bwd_prepare(const void* R, void* out, int Gr, int N, int D, int U, int pad, float* grads, size_t ngrads, unsigned* status,
                                cudaStream_t stream);
-cudaError_t launch_pack_recurrent(const void* R, void* out, int Gr, int N, int D, int transpose, cudaStream_t stream);
 cudaError_t launch_recurrent_grad(int cell, int B, int T, int N, int D, int Gr, int Gw, int state_f32, const void* dWx,
                                   const void* dg0, const void* states, const void* s0, float* dR, int sm_count,
                                   cudaStream_t stream);

@@ -82,10 +82,6 @@ struct LoopParams {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
-}
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
@@ -354,199 +350,11 @@ __device__ __forceinline__ void store_state2(void* base, size_t elem_off, int f3
   else *reinterpret_cast<uint32_t*>(static_cast<elem_t*>(base) + elem_off) = pack_x2(lo, hi);
 }
 
-// ------------------------------------------------------------------------------------------------ warp MMA
-// acc[nt][.] (16 rows x 8*NT batch columns, fp32) = Areg (16 x 16*KT, fragments in registers) times the
-// operand tile held in shared memory as `opnd[batch row][k]` (k contiguous, `stride` elements per row),
-// columns kofs .. kofs+16*KT.  Independent accumulator sets keep the dependent-MMA chains short.
-//
-// The operand is stored as one slice per producing CTA: slice c holds, for every batch row, the `1 << ushift`
-// * 16 k-columns that CTA c produces: element (b, k) sits at  (k16 >> ushift) * slice_elems + b * stride +
-// kofs + (k & (16 << ushift) - 1)  where k16 = k / 16.
-template <int KT, int NT>
-__device__ __forceinline__ void warp_mma_rows(const uint4 (&Areg)[KT], const elem_t* opnd, int stride, int kofs,
-                                              int ushift, int slice_elems, int lane, float (&out)[NT][4]) {
-  // independent accumulator sets: 4 chains, 8 for the longest rows (16 k-steps: C2 forward loop 0.780 -> 0.764 ms; with
-  // 8 or 12 k-steps the extra additions cost more than the shorter chains save)
-  constexpr int NSETS = (KT >= 16) ? 8 : 4;
-  constexpr int NACC = (NT >= NSETS) ? 1 : (NSETS / NT);
-  float acc[NACC][NT][4];
-#pragma unroll
-  for (int a = 0; a < NACC; ++a)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[a][nt][c] = 0.f;
-  const int j = lane >> 3, r = lane & 7;
-  if constexpr (NT == 1) {
-    // one ldmatrix.x4 covers two k-steps of the single 8-row batch tile
-    const uint32_t base = smem_u32(opnd + r * stride + kofs + (j & 1) * 8);
-    const int kmask = (1 << ushift) - 1;
-#pragma unroll
-    for (int k = 0; k < KT; k += 2) {
-      uint32_t b0, b1, b2, b3;
-      const int kk = k + (j >> 1);
-      ldmatrix_x4(base + (uint32_t)(((kk >> ushift) * slice_elems + (kk & kmask) * 16) * 2), b0, b1, b2, b3);
-      mma_16816(acc[k % NACC][0], Areg[k], b0, b1);
-      if (k + 1 < KT) mma_16816(acc[(k + 1) % NACC][0], Areg[k + 1], b2, b3);  // odd KT: second half unused
-    }
-  } else {
-    // one ldmatrix.x4 covers one k-step of two 8-row batch tiles
-    const uint32_t base = smem_u32(opnd + ((j >> 1) * 8 + r) * stride + kofs + (j & 1) * 8);
-    const int kmask = (1 << ushift) - 1;
-#pragma unroll
-    for (int k = 0; k < KT; ++k) {
-      const uint32_t koff = (uint32_t)(((k >> ushift) * slice_elems + (k & kmask) * 16) * 2);
-#pragma unroll
-      for (int np = 0; np < NT / 2; ++np) {
-        uint32_t b0, b1, b2, b3;
-        ldmatrix_x4(base + koff + (uint32_t)(np * 16 * stride * 2), b0, b1, b2, b3);
-        mma_16816(acc[k % NACC][2 * np], Areg[k], b0, b1);
-        mma_16816(acc[k % NACC][2 * np + 1], Areg[k], b2, b3);
-      }
-    }
-  }
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float s = acc[0][nt][c];
-#pragma unroll
-      for (int a = 1; a < NACC; ++a) s += acc[a][nt][c];
-      out[nt][c] = s;
-    }
-}
-
-// Continues such a product over the k-steps [k0, k1) whose A fragments do not fit the register file and are streamed
-// from global memory every time step (head dims above 256): fragment k of this warp's row tile sits at asrc[k * 32]
-// (lane offset already applied).  Accumulates into `acc`.  k1 - k0 must be even.
-// SMEM: the fragments are a copy of that range kept in shared memory (plain loads) instead of global memory.
-template <int NT, bool SMEM = false>
-__device__ __forceinline__ void warp_mma_stream(const uint4* asrc, int k0, int k1, const elem_t* opnd, int stride,
-                                                int kofs, int ushift, int slice_elems, int lane, float (&acc)[NT][4]) {
-  auto frag = [&](int k) -> uint4 {
-    if constexpr (SMEM) return asrc[(size_t)k * 32];
-    else return __ldg(asrc + (size_t)k * 32);
-  };
-  const int j = lane >> 3, r = lane & 7;
-  const int kmask = (1 << ushift) - 1;
-  // (one accumulator chain: four independent chains were measured and lost -- head dim 768 forward loop 3.64 -> 3.89 ms,
-  // reverse loop 5.00 -> 6.47 ms)
-  if constexpr (NT == 1) {
-    const uint32_t base = smem_u32(opnd + r * stride + kofs + (j & 1) * 8);
-#pragma unroll 2
-    for (int k = k0; k < k1; k += 2) {
-      const uint4 a0 = frag(k), a1 = frag(k + 1);
-      uint32_t b0, b1, b2, b3;
-      const int kk = k + (j >> 1);
-      ldmatrix_x4(base + (uint32_t)(((kk >> ushift) * slice_elems + (kk & kmask) * 16) * 2), b0, b1, b2, b3);
-      mma_16816(acc[0], a0, b0, b1);
-      mma_16816(acc[0], a1, b2, b3);
-    }
-  } else {
-    const uint32_t base = smem_u32(opnd + ((j >> 1) * 8 + r) * stride + kofs + (j & 1) * 8);
-#pragma unroll 2
-    for (int k = k0; k < k1; ++k) {
-      const uint4 a = frag(k);
-      const uint32_t koff = (uint32_t)(((k >> ushift) * slice_elems + (k & kmask) * 16) * 2);
-#pragma unroll
-      for (int np = 0; np < NT / 2; ++np) {
-        uint32_t b0, b1, b2, b3;
-        ldmatrix_x4(base + koff + (uint32_t)(np * 16 * stride * 2), b0, b1, b2, b3);
-        mma_16816(acc[2 * np], a, b0, b1);
-        mma_16816(acc[2 * np + 1], a, b2, b3);
-      }
-    }
-  }
-}
-
-// Same product for MT row tiles that share the operand: out[m] = A_m (16 x 16*KP, fragments Areg[m*KP + k]) times the
-// contiguous tile `opnd[batch row][k]`.  The operand fragments are loaded once per k-step and reused by all MT tiles.
-template <int MT, int KP, int NT>
-__device__ __forceinline__ void warp_mma_tiles(const uint4* Areg, const elem_t* opnd, int stride, int lane,
-                                               float (&out)[MT][NT][4]) {
-  constexpr int NACC = (MT * NT >= 4) ? 1 : (4 / (MT * NT));
-  float acc[NACC][MT][NT][4];
-#pragma unroll
-  for (int a = 0; a < NACC; ++a)
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[a][m][nt][c] = 0.f;
-  const int j = lane >> 3, r = lane & 7;
-  if constexpr (NT == 1) {
-    const uint32_t base = smem_u32(opnd + r * stride + (j >> 1) * 16 + (j & 1) * 8);
-#pragma unroll
-    for (int k = 0; k < KP; k += 2) {
-      uint32_t b0, b1, b2, b3;
-      ldmatrix_x4(base + (uint32_t)(k * 32), b0, b1, b2, b3);  // k-steps k and k+1 (the latter unused when KP is odd)
-#pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        mma_16816(acc[k % NACC][m][0], Areg[m * KP + k], b0, b1);
-        if (k + 1 < KP) mma_16816(acc[(k + 1) % NACC][m][0], Areg[m * KP + k + 1], b2, b3);
-      }
-    }
-  } else {
-    const uint32_t base = smem_u32(opnd + ((j >> 1) * 8 + r) * stride + (j & 1) * 8);
-#pragma unroll
-    for (int k = 0; k < KP; ++k) {
-#pragma unroll
-      for (int np = 0; np < NT / 2; ++np) {
-        uint32_t b0, b1, b2, b3;
-        ldmatrix_x4(base + (uint32_t)((np * 16 * stride + k * 16) * 2), b0, b1, b2, b3);
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-          mma_16816(acc[k % NACC][m][2 * np], Areg[m * KP + k], b0, b1);
-          mma_16816(acc[k % NACC][m][2 * np + 1], Areg[m * KP + k], b2, b3);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float s = acc[0][m][nt][c];
-#pragma unroll
-        for (int a = 1; a < NACC; ++a) s += acc[a][m][nt][c];
-        out[m][nt][c] = s;
-      }
-}
-
-// Threads per CTA the kernels are compiled for, by k-steps held in registers per warp.
-// Slot rows of the per-thread prefetch rings: threads beyond the item count of the CTA own no items and no slots
-// (8-row batch tiles of the 4-gate cells keep only every second thread busy in the pointwise phase).
-__host__ __device__ constexpr int ring_row_len(int U, int BT, int threads) {
-  return (U / 2) * BT < threads ? (U / 2) * BT : threads;
-}
-
-// Streamed kernels (head dims above 256): of the k-steps of R that do not fit a warp's registers, as many as the rest of
-// the shared-memory budget holds stay there for all T steps (one 512-byte fragment set per warp and k-step, an even
-// number of them); only what is left is re-read from L2 in every step.  `base_bytes` = the kernel's other shared memory.
-constexpr int kStreamKT = 8;      // k-steps of R a warp of the streamed kernels keeps in registers
-constexpr int kStreamU = 64;      // units per CTA of the streamed kernels (cluster size D / 64, up to 16)
-constexpr int kStreamMaxD = 1024;
+// ------------------------------------------------------------------------------------------------ geometry
 constexpr size_t kSmemBudget = 227 * 1024;
-__host__ __device__ constexpr int stream_ksm(int D, int kt_regs, int threads, size_t base_bytes) {
-  const int want = D / 16 - kt_regs;
-  const size_t per = (size_t)(threads / 32) * 512;
-  if (want <= 0 || base_bytes + 64 >= kSmemBudget) return 0;
-  const int fit = (int)((kSmemBudget - base_bytes - 64) / per) & ~1;
-  return fit < want ? fit : want;
-}
-
-template <int KT> struct MaxThreads { static constexpr int v = (KT >= 16) ? 256 : (KT >= 12) ? 384 : 512; };
-// Launch bounds per (cell, KT): a CTA never has more than 2*Gr*D threads (U <= D).  No minimum-blocks hint: capping
-// the registers of the small-head kernels to raise occupancy (6 instead of 4 CTAs per SM) made the Elman D=64
-// backward 70 % slower on B200 (measured), so the compiler is left free.
-template <int CELL, int KT> struct LaunchBounds {
-  static constexpr int cap = MaxThreads<KT>::v;
-  static constexpr int full = 32 * Cell<CELL>::Gr * KT;
-  static constexpr int threads = full < cap ? full : cap;
-  static constexpr int min_blocks = 1;
-};
+// Head dims above 256 (multiples of 64 up to kBigMaxD).  Units per CTA: the smallest of 32, 48, 64 that divides the head dim into at
+// most 16 CTAs.
+constexpr int kBigMaxD = 1024;
+__host__ __device__ constexpr int big_units(int D) { return D % 32 == 0 && D / 32 <= 16 ? 32 : (D % 48 == 0 && D / 48 <= 16 ? 48 : 64); }
 
 }  // namespace FRNN_NS

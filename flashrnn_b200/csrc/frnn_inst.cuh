@@ -1,10 +1,7 @@
 // Instantiation helper: each frnn_inst_<dir>_<cell>.cu defines FRNN_INST_CELL / FRNN_INST_BWD / FRNN_INST_LANE /
-// FRNN_INST_STREAM and includes this file, which emits the kernels of one cell and direction and their lookup functions.
+// FRNN_INST_BIG (/ FRNN_INST_PACK) and includes this file, which emits the kernels of one cell and direction and their lookup functions.
 #include "frnn_aux.cuh"
-#include "frnn_lane_bwd.cuh"
-#include "frnn_lane_fwd.cuh"
-#include "frnn_stream_bwd.cuh"
-#include "frnn_stream_fwd.cuh"
+#include "frnn_big_bwd.cuh"
 
 namespace FRNN_NS {
 
@@ -41,28 +38,24 @@ LaneKernel FRNN_INST_LANE(int kt, int u, int nt) {
   return LaneKernel{nullptr, 0, 0};
 }
 
-// ---- streamed loops (larger head dims): kStreamKT k-steps in registers, the rest of R from shared memory and L2
-LoopKernel FRNN_INST_STREAM(int nt) {
-  LoopKernel k{nullptr, 0, nullptr};
-  k.max_threads = LaunchBounds<FRNN_INST_CELL, kStreamKT>::threads;
+// ---- head dims above 256: units per CTA, batch tile / 8
 #if FRNN_INST_BWD
-  if (nt == 1) {
-    k.fn = reinterpret_cast<const void*>(&frnn_bwd_kernel<FRNN_INST_CELL, kStreamKT, 1, 0, true>);
-    k.smem_bytes = [](int D, int U, int threads) -> size_t { return bwd_smem_bytes<FRNN_INST_CELL, 1, 0>(D, U, threads); };
-  } else if (nt == 2) {
-    k.fn = reinterpret_cast<const void*>(&frnn_bwd_kernel<FRNN_INST_CELL, kStreamKT, 2, 0, true>);
-    k.smem_bytes = [](int D, int U, int threads) -> size_t { return bwd_smem_bytes<FRNN_INST_CELL, 2, 0>(D, U, threads); };
-  }
+#define FRNN_BIG(U, NT) \
+  if (u == U && nt == NT) return BigKernel{reinterpret_cast<const void*>(&big_bwd_kernel<FRNN_INST_CELL, U, NT>), BigBwdGeom<FRNN_INST_CELL, U, NT>::TH, \
+                                           [](int D) { return BigBwdGeom<FRNN_INST_CELL, U, NT>::smem(D); }};
 #else
-  if (nt == 1) {
-    k.fn = reinterpret_cast<const void*>(&frnn_fwd_kernel<FRNN_INST_CELL, kStreamKT, 1, true>);
-    k.smem_bytes = [](int D, int U, int threads) -> size_t { return fwd_smem_bytes<FRNN_INST_CELL, 1>(D, U, threads); };
-  } else if (nt == 2) {
-    k.fn = reinterpret_cast<const void*>(&frnn_fwd_kernel<FRNN_INST_CELL, kStreamKT, 2, true>);
-    k.smem_bytes = [](int D, int U, int threads) -> size_t { return fwd_smem_bytes<FRNN_INST_CELL, 2>(D, U, threads); };
-  }
+#define FRNN_BIG(U, NT) \
+  if (u == U && nt == NT) return BigKernel{reinterpret_cast<const void*>(&big_fwd_kernel<FRNN_INST_CELL, U, NT>), BigFwdGeom<FRNN_INST_CELL, U, NT>::TH, \
+                                           [](int D) { return BigFwdGeom<FRNN_INST_CELL, U, NT>::smem(D); }};
+cudaError_t FRNN_INST_PACK(const void* R, void* out, int N, int D, cudaStream_t stream) {
+  const size_t frags = (size_t)N * D * D * (Cell<FRNN_INST_CELL>::Gr > 1 ? 4 : 1) / 8;
+  big_pack_kernel<FRNN_INST_CELL><<<(unsigned)((frags + 255) / 256), 256, 0, stream>>>(static_cast<const elem_t*>(R), static_cast<uint4*>(out), N, D);
+  return cudaGetLastError();
+}
 #endif
-  return k;
+BigKernel FRNN_INST_BIG(int u, int nt) {
+  FRNN_BIG(32, 1) FRNN_BIG(48, 1) FRNN_BIG(64, 1) FRNN_BIG(32, 2) FRNN_BIG(48, 2) FRNN_BIG(64, 2)
+  return BigKernel{nullptr, 0, nullptr};
 }
 
 }  // namespace FRNN_NS

@@ -2,5 +2,5 @@
 #define FRNN_INST_CELL CELL_LSTM
 #define FRNN_INST_BWD 1
 #define FRNN_INST_LANE lane_bwd_lstm
-#define FRNN_INST_STREAM stream_bwd_lstm
+#define FRNN_INST_BIG big_bwd_lstm
 #include "frnn_inst.cuh"

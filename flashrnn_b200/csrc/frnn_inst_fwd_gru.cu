@@ -2,5 +2,6 @@
 #define FRNN_INST_CELL CELL_GRU
 #define FRNN_INST_BWD 0
 #define FRNN_INST_LANE lane_fwd_gru
-#define FRNN_INST_STREAM stream_fwd_gru
+#define FRNN_INST_BIG big_fwd_gru
+#define FRNN_INST_PACK big_pack_gru
 #include "frnn_inst.cuh"

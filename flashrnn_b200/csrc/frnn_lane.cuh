@@ -120,15 +120,24 @@ __host__ __device__ constexpr int io_warps(int bytes_per_step) { return bytes_pe
 // row pitch of such a tile: 16 bytes of padding make the compute lanes' accesses (4 to 16 bytes, 8 rows) conflict-free
 __host__ __device__ constexpr int io_pitch(int row_bytes) { return row_bytes + 16; }
 
-// One lane's share of a tile of ROWS rows x CPR 16-byte chunks, moved by IOT lanes.  Chunk i of the lane is row row(i), chunk col().
+// One lane's share of a tile of ROWS rows x CPR 16-byte chunks, moved by IOT lanes: chunk i of the lane is row row(i), column col(i).
+// `cpr`: the actual number of chunks per row where CPR is only the most there can be.
 template <int ROWS, int CPR, int IOT>
 struct IoTile {
   static constexpr int N = (ROWS * CPR + IOT - 1) / IOT;  // chunks per lane
-  static constexpr bool COLS_FIT = IOT % CPR == 0;
-  static_assert(COLS_FIT || CPR % IOT == 0, "chunks per row and lanes divide one another");
-  static __device__ __forceinline__ int row(int lane, int i) { return COLS_FIT ? lane / CPR + i * (IOT / CPR) : i / (CPR / IOT); }
-  static __device__ __forceinline__ int col(int lane, int i) { return COLS_FIT ? lane % CPR : lane + (i % (CPR / IOT > 0 ? CPR / IOT : 1)) * IOT; }
-  static __device__ __forceinline__ bool in(int lane, int i) { return ROWS * CPR % IOT == 0 || row(lane, i) < ROWS; }
+  // where chunks per row and lanes divide one another, a chunk's place is its lane's plus a constant (one address register for all i)
+  static constexpr bool COLS_FIT = IOT % CPR == 0, ROWS_FIT = CPR % IOT == 0;
+  static __device__ __forceinline__ int row(int lane, int i, int cpr = CPR) {
+    if (COLS_FIT && cpr == CPR) return lane / CPR + i * (IOT / CPR);
+    if (ROWS_FIT && cpr == CPR) return i / (ROWS_FIT ? CPR / IOT : 1);
+    return (int)((unsigned)(lane + i * IOT) / (unsigned)cpr);
+  }
+  static __device__ __forceinline__ int col(int lane, int i, int cpr = CPR) {
+    if (COLS_FIT && cpr == CPR) return lane % CPR;
+    if (ROWS_FIT && cpr == CPR) return lane + (i % (ROWS_FIT ? CPR / IOT : 1)) * IOT;
+    return (int)((unsigned)(lane + i * IOT) % (unsigned)cpr);
+  }
+  static __device__ __forceinline__ bool in(int lane, int i, int cpr = CPR) { return (ROWS * CPR % IOT == 0 && cpr == CPR) || lane + i * IOT < ROWS * cpr; }
 };
 
 }  // namespace FRNN_NS

@@ -40,6 +40,7 @@ struct LaneBwdGeom {
   static constexpr int NSS = C::NNEED + C::NEXT;  // state-typed rows per batch row
   static constexpr int IOW = io_warps(BT * U * 2 * (C::Gw + C::GC + NSS)), IOT = 32 * IOW;
   static constexpr int TH = 32 * W + IOT;
+  static constexpr int UNITS = U, STAGES = kLaneStages, NT8 = NT;
   // columns of the delta tile: the R gates in order; the GRU's input-only gate n, which no product reads, behind them
   static constexpr int DCOLS = C::Gr == 3 ? 4 * U : K, DT = opnd_bytes(DCOLS), DB = NT * DT;
   static constexpr int RB = CL ? CS * (U / 16) * 32 * NT * 16 : 0;  // bytes of received partial sums of one step
@@ -57,103 +58,102 @@ __host__ __device__ constexpr size_t rt_frag(int n, int CS, int c, int KT, int m
   return ((((size_t)n * CS + c) * KT + mt) * KP + kp) * 64;
 }
 
-// The IO warps' part: ES = bytes of a state element.
-template <int CELL, int KT, int U, int NT, int ES>
-__device__ __forceinline__ void lane_bwd_io(const LoopParams& p, unsigned char* smem_raw, int io, uint32_t crank) {
-  using G = LaneBwdGeom<CELL, KT, U, NT>;
+// The lanes that move data between global and shared memory.  ES: bytes of a state element (0: known at run time only); d0, in: the
+// delta tiles and the input ring in shared memory.  `drive(load, store)` runs them through the sequence: load(t, stage) starts the
+// copies of the inputs of time t (in step order T-1, T-2, ...), store(x) sends the deltas in tile x to dWx (in step order).
+template <int CELL, class G, int ES, class F>
+__device__ __forceinline__ void bwd_io(const LoopParams& p, uint32_t d0, uint32_t in, int io, uint32_t crank, F drive) {
   using C = Cell<CELL>;
-  constexpr int Gw = C::Gw, NNEED = C::NNEED, NEXT = C::NEXT, BT = G::BT, IOT = G::IOT, D = G::D;
+  constexpr int Gw = C::Gw, NNEED = C::NNEED, NEXT = C::NEXT, BT = G::BT, IOT = G::IOT, U = G::UNITS, STAGES = G::STAGES;
+  constexpr int CPR = U * (ES ? ES : 4) / 16;
   using TC = IoTile<BT, U * 2 * (G::GCM ? G::GCM : 1) / 16, IOT>;  // activations
-  using TE = IoTile<BT, U / 8, IOT>;                               // fifth activations
-  using TP = IoTile<NNEED * BT, U * ES / 16, IOT>;                 // states at t-1
-  using TQ = IoTile<NEXT * BT, U * ES / 16, IOT>;                  // cotangents at t
+  using TE = IoTile<BT, U / 8, IOT>;                               // fifth activations; GRU: delta of the recurrent-only gate
+  using TP = IoTile<NNEED * BT, CPR, IOT>;                         // states at t-1
+  using TQ = IoTile<NEXT * BT, CPR, IOT>;                          // cotangents at t
   using TW = IoTile<Gw * BT, U / 8, IOT>;                          // dWx
-  const int T = p.T, N = p.N, B = p.B, n = blockIdx.z, bt0 = blockIdx.y * BT;
+  const int T = p.T, N = p.N, B = p.B, D = p.D, n = blockIdx.z, bt0 = blockIdx.y * BT, unit0 = (int)crank * U;
+  const int es = ES ? ES : (p.state_f32 ? 4 : 2), cpr = U * es / 16;
   const size_t ND = (size_t)N * D;
-  const int unit0 = (int)crank * U;
-  const uint32_t sm = smem_u32(smem_raw), in = sm + G::OFF_I;
 
-  // ---- input pointers, first step T-1.  Rows beyond B: zero activations and cotangents make their deltas zero; their states only
-  // have to be finite divisors (0x3f80 twice is about 1 as fp32, and 1 or 1.9 twice as a 16-bit pair)
-  for (uint32_t i = io; i < kLaneStages * G::IN_B / 16; i += IOT) {
+  // Rows beyond B: zero activations and cotangents make their deltas zero; their states only have to be finite divisors (0x3f80
+  // twice is about 1 as fp32, and 1 or 1.9 twice as a 16-bit pair)
+  for (uint32_t i = io; i < STAGES * G::IN_B / 16; i += IOT) {
     const uint32_t o = i * 16 % G::IN_B, w = o >= (uint32_t)G::IN_S && o < (uint32_t)(G::IN_S + NNEED * BT * G::SP) ? 0x3f803f80u : 0u;
     sts128(in + i * 16, make_uint4(w, w, w, w));
   }
-  if constexpr (G::IOW > 1) asm volatile("bar.sync 1, %0;" ::"n"(IOT) : "memory");
+  if constexpr (IOT > 32) asm volatile("bar.sync 1, %0;" ::"n"(IOT) : "memory");
   else __syncwarp();
-  const size_t st_sb = (size_t)T * ND * ES;
+  // ---- input pointers, first step T-1
   const unsigned char* pp[TP::N];
   const unsigned char* p0[TP::N];  // the initial state, which takes the place of states[-1]
 #pragma unroll
   for (int i = 0; i < TP::N; ++i) {
-    const int r = TP::row(io, i), k = r / BT, b = bt0 + r - k * BT;
+    const int r = TP::row(io, i, cpr), k = r / BT, b = bt0 + r - k * BT;
     int need = 0;
 #pragma unroll
     for (int q = 0; q < NNEED; ++q) need = k == q ? C::need(q) : need;
-    const bool live = TP::in(io, i) && b < B;
-    const size_t col = ((size_t)n * D + unit0) * ES + TP::col(io, i) * 16;
-    pp[i] = live ? static_cast<const unsigned char*>(p.states) + ((size_t)need * B + b) * st_sb + (size_t)(T - 1) * ND * ES - ND * ES + col : nullptr;
-    p0[i] = static_cast<const unsigned char*>(p.s0) + ((size_t)need * B + (live ? b : 0)) * ND * ES + col;
+    const bool live = TP::in(io, i, cpr) && b < B;
+    const size_t col = ((size_t)n * D + unit0) * es + TP::col(io, i, cpr) * 16;
+    pp[i] = live ? static_cast<const unsigned char*>(p.states) + (((size_t)need * B + b) * T + (T - 1)) * ND * es - ND * es + col : nullptr;
+    p0[i] = static_cast<const unsigned char*>(p.s0) + ((size_t)need * B + (live ? b : 0)) * ND * es + col;
   }
   const unsigned char* qp[TQ::N];
 #pragma unroll
   for (int i = 0; i < TQ::N; ++i) {
-    const int r = TQ::row(io, i), k = r / BT, b = bt0 + r - k * BT;
-    qp[i] = (TQ::in(io, i) && b < B) ? static_cast<const unsigned char*>(p.dstates) +
-                                           ((size_t)k * p.ds_ss + (size_t)b * p.ds_sb + (size_t)(T - 1) * p.ds_st + (size_t)n * p.ds_sn + unit0) * ES +
-                                           TQ::col(io, i) * 16
-                                     : nullptr;
+    const int r = TQ::row(io, i, cpr), k = r / BT, b = bt0 + r - k * BT;
+    qp[i] = (TQ::in(io, i, cpr) && b < B) ? static_cast<const unsigned char*>(p.dstates) +
+                                                ((size_t)k * p.ds_ss + (size_t)b * p.ds_sb + (size_t)(T - 1) * p.ds_st + (size_t)n * p.ds_sn + unit0) * es +
+                                                TQ::col(io, i, cpr) * 16
+                                          : nullptr;
   }
   constexpr int CW = 2 * (G::GCM ? G::GCM : 1);  // bytes of activations per unit
-  const unsigned char* cbase = static_cast<const unsigned char*>(static_cast<const void*>(p.cache)) + ((((size_t)(T - 1) * N + n) * B) * D + unit0) * CW;
-  const unsigned char* ebase = static_cast<const unsigned char*>(static_cast<const void*>(p.cache)) + (size_t)T * N * B * D * 8 +
-                               ((((size_t)(T - 1) * N + n) * B) * D + unit0) * 2;
-  auto load = [&](int t, int stage) {  // in step order T-1, T-2, ...
+  const unsigned char* cbase = reinterpret_cast<const unsigned char*>(p.cache) + ((((size_t)(T - 1) * N + n) * B) * D + unit0) * CW;
+  const unsigned char* ebase = reinterpret_cast<const unsigned char*>(p.cache) + (size_t)T * N * B * D * 8 + ((((size_t)(T - 1) * N + n) * B) * D + unit0) * 2;
+  auto load = [&](int t, int stage) {
     if (t >= 0) {
       const uint32_t o = in + stage * G::IN_B;
       if constexpr (G::GCM > 0) {
 #pragma unroll
         for (int i = 0; i < TC::N; ++i) {
-          const int r = TC::row(io, i);
-          if (TC::in(io, i) && bt0 + r < B) cp_async16_u32(o + r * G::CP + TC::col(io, i) * 16, cbase + (size_t)(bt0 + r) * D * CW + TC::col(io, i) * 16);
+          const int r = TC::row(io, i), c = TC::col(io, i);
+          if (TC::in(io, i) && bt0 + r < B) cp_async16_u32(o + r * G::CP + c * 16, cbase + (size_t)(bt0 + r) * D * CW + c * 16);
         }
         cbase -= (size_t)N * B * D * CW;
       }
       if constexpr (G::GCX) {
 #pragma unroll
         for (int i = 0; i < TE::N; ++i) {
-          const int r = TE::row(io, i);
-          if (TE::in(io, i) && bt0 + r < B)
-            cp_async16_u32(o + G::IN_E + r * G::EP + TE::col(io, i) * 16, ebase + (size_t)(bt0 + r) * D * 2 + TE::col(io, i) * 16);
+          const int r = TE::row(io, i), c = TE::col(io, i);
+          if (TE::in(io, i) && bt0 + r < B) cp_async16_u32(o + G::IN_E + r * G::EP + c * 16, ebase + (size_t)(bt0 + r) * D * 2 + c * 16);
         }
         ebase -= (size_t)N * B * D * 2;
       }
 #pragma unroll
       for (int i = 0; i < TP::N; ++i)
         if (pp[i] != nullptr) {
-          cp_async16_u32(o + G::IN_S + TP::row(io, i) * G::SP + TP::col(io, i) * 16, t > 0 ? pp[i] : p0[i]);
-          pp[i] -= ND * ES;
+          cp_async16_u32(o + G::IN_S + TP::row(io, i, cpr) * G::SP + TP::col(io, i, cpr) * 16, t > 0 ? pp[i] : p0[i]);
+          pp[i] -= ND * es;
         }
 #pragma unroll
       for (int i = 0; i < TQ::N; ++i)
         if (qp[i] != nullptr) {
-          cp_async16_u32(o + G::IN_S + (NNEED * BT + TQ::row(io, i)) * G::SP + TQ::col(io, i) * 16, qp[i]);
-          qp[i] -= (size_t)p.ds_st * ES;
+          cp_async16_u32(o + G::IN_S + (NNEED * BT + TQ::row(io, i, cpr)) * G::SP + TQ::col(io, i, cpr) * 16, qp[i]);
+          qp[i] -= (size_t)p.ds_st * es;
         }
     }
     cp_async_commit();
   };
 #pragma unroll
-  for (int s = 0; s < kLaneStages; ++s) load(T - 1 - s, s);
+  for (int s = 0; s < STAGES; ++s) load(T - 1 - s, s);
 
-  // ---- dWx[b][t][g][n][unit0 ..] from delta columns (g + first) * U
+  // ---- dWx[b][t][g][n][unit0 ..] from delta columns (g + GSH) * U
   constexpr int GSH = C::Gr == 3 ? 1 : 0;  // GRU: column block 0 is the recurrent-only gate, which goes to dg0
   elem_t* wp[TW::N];
   uint32_t ws[TW::N];
 #pragma unroll
   for (int i = 0; i < TW::N; ++i) {
     const int r = TW::row(io, i), g = r / BT, bl = r - g * BT, b = bt0 + bl, c = TW::col(io, i);
-    ws[i] = sm + (bl >> 3) * G::DT + opnd_off(bl & 7, (g + GSH) * U + c * 8);
+    ws[i] = d0 + (bl >> 3) * G::DT + opnd_off(bl & 7, (g + GSH) * U + c * 8);
     wp[i] = (TW::in(io, i) && b < B) ? p.dWx + (((size_t)b * T + (T - 1)) * Gw + g) * ND + (size_t)n * D + unit0 + c * 8 : nullptr;
   }
   elem_t* gp[TE::N];
@@ -162,18 +162,11 @@ __device__ __forceinline__ void lane_bwd_io(const LoopParams& p, unsigned char* 
     const int b = bt0 + TE::row(io, i);
     gp[i] = (GSH && TE::in(io, i) && b < B) ? p.dg0 + ((size_t)b * T + (T - 1)) * ND + (size_t)n * D + unit0 + TE::col(io, i) * 8 : nullptr;
   }
-  // barrier j of the CTA: the deltas of step j are complete, its inputs consumed, the inputs of step j + 1 have landed
-  cp_async_wait<kLaneStages - 1>();
-  __syncthreads();  // (in front of step 0)
-  int stage = 0;
-  for (int j = 0; j < T; ++j) {
-    cp_async_wait<kLaneStages - 2>();
-    __syncthreads();
-    load(T - 1 - j - kLaneStages, stage);
+  auto store = [&](int x) {
 #pragma unroll
     for (int i = 0; i < TW::N; ++i)
       if (wp[i] != nullptr) {
-        *reinterpret_cast<uint4*>(wp[i]) = lds128(ws[i] + (j & 1) * G::DB);
+        *reinterpret_cast<uint4*>(wp[i]) = lds128(ws[i] + x * G::DB);
         wp[i] -= (size_t)Gw * ND;
       }
     if constexpr (GSH) {
@@ -181,13 +174,33 @@ __device__ __forceinline__ void lane_bwd_io(const LoopParams& p, unsigned char* 
       for (int i = 0; i < TE::N; ++i)
         if (gp[i] != nullptr) {
           const int bl = TE::row(io, i);
-          *reinterpret_cast<uint4*>(gp[i]) = lds128(sm + (j & 1) * G::DB + (bl >> 3) * G::DT + opnd_off(bl & 7, TE::col(io, i) * 8));
+          *reinterpret_cast<uint4*>(gp[i]) = lds128(d0 + x * G::DB + (bl >> 3) * G::DT + opnd_off(bl & 7, TE::col(io, i) * 8));
           gp[i] -= ND;
         }
     }
-    stage = stage + 1 == kLaneStages ? 0 : stage + 1;
-  }
+  };
+  drive(load, store);
   cp_async_wait<0>();
+}
+
+// The IO warps of the lane loop.
+template <int CELL, class G, int ES>
+__device__ __forceinline__ void lane_bwd_io(const LoopParams& p, uint32_t d0, uint32_t in, int io, uint32_t crank) {
+  constexpr int STAGES = G::STAGES;
+  const int T = p.T;
+  bwd_io<CELL, G, ES>(p, d0, in, io, crank, [&](auto& load, auto& store) {
+    // barrier j of the CTA: the deltas of step j are complete, its inputs consumed, the inputs of step j + 1 have landed
+    cp_async_wait<STAGES - 1>();
+    __syncthreads();  // (in front of step 0)
+    int stage = 0;
+    for (int j = 0; j < T; ++j) {
+      cp_async_wait<STAGES - 2>();
+      __syncthreads();
+      load(T - 1 - j - STAGES, stage);
+      store(j & 1);
+      stage = stage + 1 == STAGES ? 0 : stage + 1;
+    }
+  });
 }
 
 template <int CELL, int KT, int U, int NT>
@@ -228,8 +241,8 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT>::TH) lane_bwd_ker
 
   if (warp >= W) {
     const int io = tid - 32 * W;
-    if (f32) lane_bwd_io<CELL, KT, U, NT, 4>(p, smem_raw, io, crank);
-    else lane_bwd_io<CELL, KT, U, NT, 2>(p, smem_raw, io, crank);
+    if (f32) lane_bwd_io<CELL, G, 4>(p, sm, sm + G::OFF_I, io, crank);
+    else lane_bwd_io<CELL, G, 2>(p, sm, sm + G::OFF_I, io, crank);
     if (CL) {
       __syncwarp();
       cluster_wait();

@@ -13,7 +13,8 @@
 #include <mutex>
 
 // The scratch itself.  Every GPU that loads the library holds these bytes until the process exits.
-static __device__ __align__(256) unsigned char g_noalloc_scratch[FRNN_NOALLOC_MAX_SCRATCH_BYTES];
+// (A third more than the limit: the fragments of a GRU's three gates are padded to four.)
+static __device__ __align__(256) unsigned char g_noalloc_scratch[FRNN_NOALLOC_MAX_SCRATCH_BYTES / 3 * 4 + 1024];
 
 namespace {
 

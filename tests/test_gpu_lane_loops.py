@@ -1,6 +1,6 @@
 """GPU: the lane loops (head dims up to 256) at the sizes where they can go wrong: every head dim they are instantiated for, one
 step, as many steps as and one more than their input ring holds (6), and batches around the 8-row tile; one CTA per head and
-clusters, 8- and 16-row tiles."""
+clusters, 8- and 16-row tiles.  The same for their forms for head dims above 256."""
 import pytest
 import torch
 
@@ -14,14 +14,25 @@ pytestmark = pytest.mark.gpu
                                      (128, 2, 16), (128, 4, 8), (192, 6, 16), (256, 8, 8)])
 @pytest.mark.parametrize("B,T,state_f32", [(1, 1, False), (7, 6, True), (9, 7, False), (17, 2, True)])
 def test_lane_loops_edges(cuda_device, function, D, cs, bt, B, T, state_f32):
-    N = 2
+    _check(function, 2, D, B, T, state_f32, cluster_size=cs, batch_tile=bt)
+
+
+# 32, 48 and 64 units per CTA; R in registers alone, in shared memory too, and partly read from L2; with four heads the 16-row tiles
+@pytest.mark.parametrize("function", ["lstm", "gru", "elman", "slstm"])
+@pytest.mark.parametrize("N,D", [(1, 320), (4, 384), (1, 512), (4, 576), (1, 640), (1, 704), (1, 768), (4, 768), (1, 1024), (4, 1024)])
+@pytest.mark.parametrize("B,T,state_f32", [(1, 1, False), (7, 6, True), (9, 5, False), (17, 2, True)])
+def test_head_dims_above_256_edges(cuda_device, function, N, D, B, T, state_f32):
+    _check(function, N, D, B, T, state_f32)
+
+
+def _check(function, N, D, B, T, state_f32, **tile):
     Wx, R, b, s0 = make_inputs(function, B, T, N, D, seed=D + T, random_init=True, state_f32=state_f32)
     S = s0.shape[0]
     cot = torch.randn(S, B, T, N, D, generator=torch.Generator().manual_seed(T), dtype=torch.float64).to(torch.bfloat16).to(torch.float64)
     if function == "slstm":
         cot[1:] = 0
     opts = dict(gradient_recurrent_clipval=0.05) if B == 9 else (dict(forward_clipval=0.5) if B == 7 else {})
-    got = run_native(function, Wx, R, b, s0, cot=cot, state_f32=state_f32, cluster_size=cs, batch_tile=bt, **opts)
+    got = run_native(function, Wx, R, b, s0, cot=cot, state_f32=state_f32, **tile, **opts)
     ref = run_oracle(function, Wx, R, b, s0, cot=cot, clip=opts.get("gradient_recurrent_clipval", 0.0),
                      forward_clip=opts.get("forward_clipval", 0.0))
-    assert_parity(function, got, ref, tag=f"{function} D{D} cs{cs} bt{bt} B{B} T{T}", zero_init=False)
+    assert_parity(function, got, ref, tag=f"{function} N{N} D{D} {tile} B{B} T{T}", zero_init=False)
