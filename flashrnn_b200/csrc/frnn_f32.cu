@@ -18,12 +18,9 @@
 // Replaces, for float32, FLASHRNNCellFusedForward / FLASHRNNCellFusedBackward / the cuBLAS dR GEMM of the reference
 // (fused/flashrnn_fused_forward.cu:146-659, fused/flashrnn_fused_backward.cu:129-624, 1049-1058).
 #ifndef FRNN_F16  // compiled once, into the bfloat16 build, which owns the public entry points
-#define FRNN_NS_OVERRIDE frnn_x32
-#define FRNN_EXACT_ACT 1
 #include <type_traits>
 
-#include "../../include/frnn.h"
-#include "frnn_cell.cuh"
+#include "frnn_f32.cuh"
 
 namespace FRNN_NS {
 
@@ -33,20 +30,6 @@ constexpr int XBT = 8;        // batch rows per CTA
 constexpr int XTHREADS = 256;
 constexpr size_t kStatus = 256;
 constexpr size_t kSmemMax = 227 * 1024;
-
-struct XParams {
-  const float* Wx; const float* R; const float* RT; const float* bias; const float* s0;
-  float* states; float* cache;
-  const float* dstates; float* dWx; float* dg0; float* ds0; float* dbias;
-  unsigned* status;
-  int B, T, N, D;
-  int U, CS, KS;  // cluster loops: units per CTA, CTAs per cluster, k-splits of the matrix phase
-  int test_drop;  // test hook: CTA 0 of every cluster withholds its message of step 1
-  int r_in_smem;
-  float fclip, gclip;
-  int grad_cut;
-  long long wx_sb, wx_st, wx_sg, wx_sn, ds_ss, ds_sb, ds_st, ds_sn;
-};
 
 // RT[n][p][g*D + d] = R[g][n][d][p]
 __global__ void transpose_recurrent_kernel(const float* __restrict__ R, float* __restrict__ RT, int Gr, int N, int D) {
@@ -867,6 +850,24 @@ bool pick_tile(const frnn_problem& pr, const Dims& d, int cs, int bt, Tile* t) {
   *t = Tile{1, pr.D, XBT, 0, 0, 0, false, fwd_smem(pr, d, false), bwd_smem(pr, d)};
   return t->smem_f <= kSmemMax && t->smem_b <= kSmemMax;
 }
+// The lane loops (frnn_f32_lane.cuh): head dims up to 256 that split into CTAs of at most 32 units (64 with one CTA), a multiple of 4.  Their
+// tiles follow from the problem alone; the plan's tile is that of the loops below, which run every other head dim.
+bool lane_tile(const frnn_problem& pr, bool bwd, int* cs_out, XLane* k) {
+  int cs = 1;
+  if (pr.D > 64) {
+    for (cs = 2; cs <= 8 && (pr.D % cs || pr.D / cs % 4 || pr.D / cs > 32); ++cs) {}
+    if (cs > 8) return false;
+  }
+  // rows per CTA: as few as leave every CTA an SM of its own (a cluster its place)
+  const int fit = cs == 1 ? 148 : kResidentClusters[cs];
+  int bt = cs == 1 ? 1 : 2;
+  while (bt < 4 && (long long)((pr.B + bt - 1) / bt) * pr.N > fit) bt *= 2;
+  if (const char* e = getenv("XBT")) bt = atoi(e);
+  const int cell = pr.cell == CELL_ELMAN && pr.forward_clip > 0.f ? (int)CELL_ELMAN_CLIP : pr.cell;
+  *k = (bwd ? x32_lane_bwd : x32_lane_fwd)(cell, pr.D, pr.D / cs, bt);
+  *cs_out = cs;
+  return k->fn != nullptr && (pr.B + k->bt - 1) / k->bt <= 65535;
+}
 int validate(const frnn_problem* pr, Dims* d) {
   if (!pr) return FRNN_ERR_NULL;
   if (!dims_of(pr->cell, pr->forward_clip, d)) return FRNN_ERR_CELL;
@@ -904,6 +905,26 @@ cudaError_t launch_cluster(K kern, const frnn_problem& pr, const Tile& t, size_t
   cfg.attrs = attr;
   cfg.numAttrs = t.cs > 1 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, p);
+}
+cudaError_t launch_lane(const XLane& k, int cs, const frnn_problem& pr, XParams p, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);  // fixed maximum
+  if (e != cudaSuccess) return e;
+  p.CS = cs;
+  p.U = pr.D / cs;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cs, (unsigned)((pr.B + k.bt - 1) / k.bt), (unsigned)pr.N);
+  cfg.blockDim = dim3((unsigned)k.threads, 1, 1);
+  cfg.dynamicSmemBytes = k.smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cs > 1 ? 1 : 0;
+  void* args[1] = {&p};
+  return cudaLaunchKernelExC(&cfg, k.fn, args);
 }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 bool strides_ok(const int64_t (&in)[4], const long long (&dense)[4], long long (&out)[4]) {
@@ -970,7 +991,10 @@ __attribute__((visibility("hidden"))) int frnn_forward_f32(const frnn_plan* plan
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   const Ws w = ws_layout(pr, d);
   cudaError_t e = cudaSuccess;
-  if (!plan->keep_packed_r) {
+  XLane lane;
+  int lane_cs;
+  const bool is_lane = lane_tile(pr, false, &lane_cs, &lane);
+  if (!plan->keep_packed_r && !is_lane) {
     e = cudaMemsetAsync(ws, 0, kStatus, stream);
     if (e != cudaSuccess) return (int)e;
     const size_t total = (size_t)d.Gr * pr.N * pr.D * pr.D;
@@ -987,6 +1011,11 @@ __attribute__((visibility("hidden"))) int frnn_forward_f32(const frnn_plan* plan
   p.status = reinterpret_cast<unsigned*>(ws);
   p.fclip = pr.forward_clip; p.gclip = pr.grad_clip; p.grad_cut = pr.grad_cut;
   p.wx_sb = wxs[0]; p.wx_st = wxs[1]; p.wx_sg = wxs[2]; p.wx_sn = wxs[3];
+  if (is_lane) {
+    p.last = static_cast<float*>(a->last);
+    p.clear_status = !plan->keep_packed_r; p.test_drop = plan->test_drop_exchange;
+    return (int)launch_lane(lane, lane_cs, pr, p, stream);
+  }
   if (tl.cluster) {
     p.U = tl.u; p.CS = tl.cs; p.KS = tl.ksf; p.test_drop = plan->test_drop_exchange;
     auto launch = [&](auto cell) {
@@ -1067,7 +1096,12 @@ __attribute__((visibility("hidden"))) int frnn_backward_parts_f32(const frnn_pla
     p.fclip = pr.forward_clip; p.gclip = pr.grad_clip; p.grad_cut = pr.grad_cut;
     p.ds_ss = dss[0]; p.ds_sb = dss[1]; p.ds_st = dss[2]; p.ds_sn = dss[3];
     p.status = reinterpret_cast<unsigned*>(ws);
-    if (tl.cluster) {
+    XLane lane;
+    int lane_cs;
+    if (lane_tile(pr, true, &lane_cs, &lane)) {
+      p.test_drop = plan->test_drop_exchange;
+      e = launch_lane(lane, lane_cs, pr, p, stream);
+    } else if (tl.cluster) {
       p.U = tl.u; p.CS = tl.cs; p.KS = tl.ksb; p.test_drop = plan->test_drop_exchange;
       auto launch = [&](auto cell) {
       constexpr int CL = decltype(cell)::value;
