@@ -861,10 +861,11 @@ bool lane_tile(const frnn_problem& pr, bool bwd, int* cs_out, XLane* k) {
   // rows per CTA: as few as leave every CTA an SM of its own (a cluster its place)
   const int fit = cs == 1 ? 148 : kResidentClusters[cs];
   int bt = cs == 1 ? 1 : 2;
-  while (bt < 4 && (long long)((pr.B + bt - 1) / bt) * pr.N > fit) bt *= 2;
+  while (bt < (cs == 1 ? 4 : 8) && (long long)((pr.B + bt - 1) / bt) * pr.N > fit) bt *= 2;
   if (const char* e = getenv("XBT")) bt = atoi(e);
   const int cell = pr.cell == CELL_ELMAN && pr.forward_clip > 0.f ? (int)CELL_ELMAN_CLIP : pr.cell;
   *k = (bwd ? x32_lane_bwd : x32_lane_fwd)(cell, pr.D, pr.D / cs, bt);
+  if (!k->fn) *k = (bwd ? x32_lane_bwd : x32_lane_fwd)(cell, pr.D, pr.D / cs, bt / 2);
   *cs_out = cs;
   return k->fn != nullptr && (pr.B + k->bt - 1) / k->bt <= 65535;
 }

@@ -1,13 +1,16 @@
 // float32 lane loops (head dims up to 256): one persistent launch runs all T steps; the lane that ends up with a unit's gate sums runs
 // its cell.  All products and sums are FFMA in fp32.
 //
-// Work split.  A cluster of CS = D / U CTAs owns one head and BT = 1, 2 or 4 batch rows; CTA c owns the hidden units [c*U, (c+1)*U), a
-// warp four of them.  Up to head dim 64 CS is 1.
-//   Forward: the 8 lanes of a unit split k in interleaved quads; a lane keeps its part of the unit's Gr rows of R in registers (KQ quads:
-//   16 KQ values), so one 16-byte read of h feeds 4 Gr products.  The sums meet through shuffles that scatter the batch rows over the lanes.
-//   Reverse: a lane keeps a part of four columns of R.  CS == 1: a warp's own four columns, k = (gate, unit) split over its 32 lanes, so
+// Work split.  A cluster of CS = D / U CTAs owns one head and BT = 1, 2, 4 or 8 batch rows; CTA c owns the hidden units [c*U, (c+1)*U), LPU
+// lanes each.  Up to head dim 64 CS is 1.
+//   Forward: the lanes of a unit split k in interleaved quads; a lane keeps its part of the unit's Gr rows of R in registers (Elman: of
+//   the rows of four units, k split over their 4 LPU lanes), so one 16-byte read of h, which costs four wavefronts of shared memory
+//   whatever its lanes share, feeds 16 products.  The sums meet through shuffles that scatter the batch rows over the lanes.
+//   Reverse: a lane keeps a part of four columns of R.  CS == 1: a warp's own columns, k = (gate, unit) split over 4 LPU lanes, so
 //   that dh ends up in the lane that needs it; CS > 1: 16 columns per task, k split over 8 lanes, and the sums go to the CTA that
 //   owns the columns.
+// LPU is as small as the registers for R allow: the cell is issued once per warp whatever its lanes are worth (LSTM D = 64, one row, 8 lanes
+// per unit 1048 clk per step).
 // Operand tiles (h, deltas): quads of four consecutive k, [quad][row][4 floats], rows XOR-permuted so that the 8 lanes of a read hit
 // different banks; a warp's four units of a row are one quad, so its results and messages are blocks of BT * 16 bytes.
 // Exchange: st.async counted on the destination's mbarrier, as in frnn_lane_fwd.cuh.  Four IO warps move everything between global
@@ -30,8 +33,8 @@ __device__ __forceinline__ void x_unpack(uint4 v, P2& lo, P2& hi) {
   lo = v_pair<P2>(__uint_as_float(v.x), __uint_as_float(v.y));
   hi = v_pair<P2>(__uint_as_float(v.z), __uint_as_float(v.w));
 }
-// v[i][b], b < BT: sums over the lanes that differ in the bits 1, 2, 4; lane l ends up with row l & (BT - 1) in v[i][0]
-template <int BT, int NV> __device__ __forceinline__ void x_reduce8(float (&v)[NV][BT], int lane) {
+// v[i][b], b < BT: sums over the lanes that differ in the bits below LANES; lane l ends up with row l & (BT - 1) in v[i][0]
+template <int LANES, int BT, int NV> __device__ __forceinline__ void x_reduce(float (&v)[NV][BT], int lane) {
 #pragma unroll
   for (int m = BT / 2; m > 0; m /= 2) {
     const bool hi = (lane & m) != 0;
@@ -44,9 +47,22 @@ template <int BT, int NV> __device__ __forceinline__ void x_reduce8(float (&v)[N
       }
   }
 #pragma unroll
-  for (int m = BT; m < 8; m *= 2)
+  for (int m = BT; m < LANES; m *= 2)
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i][0] += __shfl_xor_sync(0xffffffffu, v[i][0], m);
+}
+// v[c][b]: unit c of four, row b; sums over the lanes that differ in the bits below 4 LPU.  Lane bits 2 LPU, LPU <- unit, those below <- row
+template <int LPU, int BT> __device__ __forceinline__ float x_reduce_units(const float (&v)[4][BT], int lane) {
+  float h[2][BT], o[1][BT];
+  const bool hi2 = (lane & (2 * LPU)) != 0, hi1 = (lane & LPU) != 0;
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int e = 0; e < BT; ++e) h[c][e] = (hi2 ? v[c + 2][e] : v[c][e]) + __shfl_xor_sync(0xffffffffu, hi2 ? v[c][e] : v[c + 2][e], 2 * LPU);
+#pragma unroll
+  for (int e = 0; e < BT; ++e) o[0][e] = (hi1 ? h[1][e] : h[0][e]) + __shfl_xor_sync(0xffffffffu, hi1 ? h[0][e] : h[1][e], LPU);
+  x_reduce<LPU, BT, 1>(o, lane);
+  return o[0][0];
 }
 // chunk idx of a [plane][row][quad] walk, quads fastest: idx = (plane * BT + b) * Q + q (inv = 65536 / Q + 1; idx < 65536 / Q)
 template <int BT> __device__ __forceinline__ void x_chunk(int idx, int Q, int inv, int& pl, int& b, int& q) {
@@ -56,11 +72,15 @@ template <int BT> __device__ __forceinline__ void x_chunk(int idx, int Q, int in
   pl = r / BT;
 }
 
-template <int CELL, int KQ, int BT>
+// LPU lanes per unit, KQ quads of k per lane
+template <int CELL, bool CL, int LPU, int KQ, int BT>
 struct XFwdGeom {
   using C = Cell<CELL>;
-  static constexpr int HB = KQ * 8 * BT * 16;  // bytes of an h tile
-  static constexpr int MAXQ = KQ <= 2 ? 8 * KQ : 8, MAXTH = 32 * MAXQ + kXIo;  // unit quads = compute warps per CTA, at most
+  static constexpr int KS = C::Gr == 1 ? 4 * LPU : LPU;  // lanes that split k for the same rows of R
+  static constexpr int HB = KQ * KS * BT * 16;           // bytes of an h tile
+  static constexpr int MAXQ = CL ? 8 : 16, MAXTH = 4 * LPU * MAXQ + kXIo;  // unit quads per CTA, threads, at most
+  static constexpr int NR = C::Gr == 1 ? 4 : C::Gr;  // rows of R per lane: a unit's gates, Elman: four units
+  static constexpr int GP = NR * KQ * BT > 128 ? 1 : NR * KQ * BT > 64 && KQ == 8 ? 2 : NR;  // of them, those multiplied in one pass over h (registers)
   static constexpr int NL = (C::Gw * BT * MAXQ + kXIo - 1) / kXIo, NS = ((C::S + C::GC) * BT * MAXQ + kXIo - 1) / kXIo;  // chunks per IO lane
   static __host__ __device__ constexpr int plane(int U) { return U / 4 * BT * 16; }
   static __host__ __device__ constexpr int off_x() { return 128 + 2 * HB; }
@@ -68,18 +88,16 @@ struct XFwdGeom {
   static __host__ __device__ constexpr size_t smem(int U) { return (size_t)off_o(U) + 2 * (size_t)(C::S + C::GC) * plane(U); }
 };
 
-// KQ = ceil(D / 32); up to KQ == 2 one CTA per head
-template <int CELL, int KQ, int BT>
-__global__ void __launch_bounds__(XFwdGeom<CELL, KQ, BT>::MAXTH, 1) x32l_fwd_kernel(const __grid_constant__ XParams p) {
-  using G = XFwdGeom<CELL, KQ, BT>;
+template <int CELL, bool CL, int LPU, int KQ, int BT>
+__global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32l_fwd_kernel(const __grid_constant__ XParams p) {
+  using G = XFwdGeom<CELL, CL, LPU, KQ, BT>;
   using C = Cell<CELL>;
-  constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, HB = G::HB;
-  constexpr bool CL = KQ > 2;
+  constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, HB = G::HB, UW = 32 / LPU, GP = G::GP, NR = G::NR, KS = G::KS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int D = p.D, U = p.U, Q = U >> 2, CS = p.CS, T = p.T, B = p.B, N = p.N;
   const int n = blockIdx.z, b0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
-  const int unit0 = (int)crank * U, TH = blockDim.x;
+  const int unit0 = (int)crank * U, TH = blockDim.x, W = (TH - kXIo) >> 5;  // W compute warps
   const size_t ND = (size_t)N * D;
   const uint32_t step_bytes = (uint32_t)(D * BT * 4);
 
@@ -98,8 +116,8 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, KQ, BT>::MAXTH, 1) x32l_fwd_ker
     p.status[0] = 0u; p.status[1] = 0u; p.status[2] = 0u; p.status[3] = 0u;
   }
   // h_{-1} -> tile 1 (step t reads tile (t + 1) & 1 and writes tile t & 1); quads beyond D stay zero in both
-  for (int i = tid; i < KQ * 8 * BT; i += TH) {
-    const int b = i / (KQ * 8), q = i - b * (KQ * 8);
+  for (int i = tid; i < KQ * KS * BT; i += TH) {
+    const int b = i / (KQ * KS), q = i - b * (KQ * KS);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     sts128(ht + xq_off<BT>(q, b), v);
     if (4 * q < D && b0 + b < B) v = *reinterpret_cast<const uint4*>(p.s0 + (size_t)(b0 + b) * ND + (size_t)n * D + 4 * q);
@@ -108,8 +126,8 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, KQ, BT>::MAXTH, 1) x32l_fwd_ker
   __syncthreads();
   if (CL) cluster_arrive();  // barriers initialised, h_{-1} read; waited for before the first push, or before `last` may overwrite s0
 
-  if (warp >= Q) {
-    const int io = tid - 32 * Q, inv = 65536 / Q + 1;
+  if (warp >= W) {
+    const int io = tid - 32 * W, inv = 65536 / Q + 1;
     const bool cache = GC > 0 && p.cache != nullptr;
     for (int i = io; i < kXStages * xs / 16; i += kXIo) sts128(ring + i * 16, make_uint4(0u, 0u, 0u, 0u));  // rows beyond B read as zero
     asm volatile("bar.sync 1, %0;" ::"n"(kXIo) : "memory");
@@ -180,26 +198,31 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, KQ, BT>::MAXTH, 1) x32l_fwd_ker
     return;
   }
 
-  const int kk = lane & 7, uq = lane >> 3, b = lane & (BT - 1), unit = unit0 + 4 * warp + uq;
-  const bool own = kk < BT, live = b0 + b < B;  // (the other lanes of a unit run the same rows and store nothing)
-  P2 w[Gr][KQ][2];
+  const int kk = lane & (KS - 1), b = lane & (BT - 1), ul = warp * UW + lane / LPU;  // this lane's unit within the CTA
+  const int unit = unit0 + (ul < U ? ul : U - 1);
+  // (the other lanes of a unit run the same rows, lanes beyond the last unit run it, and neither stores anything)
+  const bool own = (lane & (LPU - 1)) < BT && ul < U, live = b0 + b < B;
+  P2 w[NR][KQ][2];
 #pragma unroll
-  for (int g = 0; g < Gr; ++g)
+  for (int g = 0; g < NR; ++g) {
+    const int first = warp * UW + lane / KS * 4 + g, row = Gr == 1 ? unit0 + (first < U ? first : U - 1) : unit;
 #pragma unroll
     for (int i = 0; i < KQ; ++i) {
-      const int q = i * 8 + kk;
+      const int q = i * KS + kk;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (4 * q < D) v = __ldg(reinterpret_cast<const uint4*>(p.R + (((size_t)g * N + n) * D + unit) * D + 4 * q));
+      if (4 * q < D) v = __ldg(reinterpret_cast<const uint4*>(p.R + (((size_t)(Gr == 1 ? 0 : g) * N + n) * D + row) * D + 4 * q));
       x_unpack(v, w[g][i][0], w[g][i][1]);
     }
+  }
   const size_t nd = (size_t)n * D + unit;
   float bias[Gt], st[S], cch[GCA];
 #pragma unroll
   for (int g = 0; g < Gt; ++g) bias[g] = p.bias[(size_t)g * ND + nd];
 #pragma unroll
   for (int s = 0; s < S; ++s) st[s] = live ? p.s0[((size_t)s * B + b0 + b) * ND + nd] : 0.f;
-  const uint32_t word = (uint32_t)(warp * BT + b) * 16u + (uint32_t)uq * 4u;       // this lane's word in a plane of the ring, of the results
-  const uint32_t hw = xq_off<BT>((unit0 >> 2) + warp, b) + (uint32_t)uq * 4u;      // ... in an h tile
+  const int uc = unit - unit0;
+  const uint32_t word = (uint32_t)((uc >> 2) * BT + b) * 16u + (uint32_t)(uc & 3) * 4u;  // this lane's word in a plane of the ring, of the results
+  const uint32_t hw = xq_off<BT>(unit >> 2, b) + (uint32_t)(unit & 3) * 4u;              // ... in an h tile
   const uint32_t hr = ht + (uint32_t)(kk * BT) * 16u, sw = (uint32_t)(kk * BT >> 3) & (BT - 1);
   const int drop_t = (p.test_drop && crank == 0) ? 1 : -1;  // test hook: CTA 0 withholds its message of step 1
   const bool cache = GC > 0 && p.cache != nullptr;
@@ -218,29 +241,41 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, KQ, BT>::MAXTH, 1) x32l_fwd_ker
       }
       else if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(&full[prv], step_bytes);
     }
-    P2 acc[Gr][BT];
+    float v[NR][BT], pre[Gr], gx[Gt];
 #pragma unroll
-    for (int i = 0; i < KQ; ++i) {
-      P2 lo[BT], hi[BT];
+    for (int g0 = 0; g0 < NR; g0 += GP) {
+      P2 acc[GP][BT];
 #pragma unroll
-      for (int r = 0; r < BT; ++r) x_unpack(lds128(hr + prv * HB + (uint32_t)(i * 8 * BT) * 16u + (((uint32_t)r ^ sw) << 4)), lo[r], hi[r]);
+      for (int i = 0; i < KQ; ++i) {
+        P2 lo[BT], hi[BT];
+        constexpr int kRow = KS * BT;
 #pragma unroll
-      for (int g = 0; g < Gr; ++g)
+        for (int r = 0; r < BT; ++r)  // quad i * KS + kk; the row's place splits into a part of i and one of kk
+          x_unpack(lds128(hr + prv * HB + (uint32_t)(i * kRow) * 16u + (((uint32_t)(r ^ ((i * kRow >> 3) & (BT - 1))) ^ sw) << 4)), lo[r], hi[r]);
 #pragma unroll
-        for (int r = 0; r < BT; ++r) acc[g][r] = i == 0 ? v_mul(w[g][i][0], lo[r]) : v_fma(w[g][i][0], lo[r], acc[g][r]);
+        for (int g = 0; g < GP; ++g)
+          if (g0 + g < NR)
 #pragma unroll
-      for (int g = 0; g < Gr; ++g)
+            for (int r = 0; r < BT; ++r) acc[g][r] = i == 0 ? v_mul(w[g0 + g][i][0], lo[r]) : v_fma(w[g0 + g][i][0], lo[r], acc[g][r]);
 #pragma unroll
-        for (int r = 0; r < BT; ++r) acc[g][r] = v_fma(w[g][i][1], hi[r], acc[g][r]);
+        for (int g = 0; g < GP; ++g)
+          if (g0 + g < NR)
+#pragma unroll
+            for (int r = 0; r < BT; ++r) acc[g][r] = v_fma(w[g0 + g][i][1], hi[r], acc[g][r]);
+      }
+#pragma unroll
+      for (int g = 0; g < GP; ++g)
+        if (g0 + g < NR)
+#pragma unroll
+          for (int r = 0; r < BT; ++r) { const float2 s = v_get(acc[g][r]); v[g0 + g][r] = s.x + s.y; }
     }
-    float v[Gr][BT], pre[Gr], gx[Gt];
+    if constexpr (Gr == 1) {
+      pre[0] = x_reduce_units<LPU, BT>(v, lane);
+    } else {
+      x_reduce<LPU, BT, Gr>(v, lane);
 #pragma unroll
-    for (int g = 0; g < Gr; ++g)
-#pragma unroll
-      for (int r = 0; r < BT; ++r) { const float2 s = v_get(acc[g][r]); v[g][r] = s.x + s.y; }
-    x_reduce8<BT, Gr>(v, lane);
-#pragma unroll
-    for (int g = 0; g < Gr; ++g) pre[g] = v[g][0];
+      for (int g = 0; g < Gr; ++g) pre[g] = v[g][0];
+    }
     gate_sums<CELL>(pre, wx, bias, gx);
     cell_forward<CELL>(gx, st, cch);
     if (p.fclip > 0.f) st[0] = clampf(st[0], p.fclip);
@@ -275,13 +310,15 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, KQ, BT>::MAXTH, 1) x32l_fwd_ker
   if (CL) { __syncwarp(); cluster_arrive_relaxed(); cluster_wait(); }
 }
 
-// KS lanes over k: 32 with one CTA per head, 8 in clusters; KQ quads of k per lane, TB tasks of 128 / KS columns per warp
-template <int CELL, int KS, int KQ, int TB, int BT>
+// LPU lanes per unit.  k is split over KS = 4 LPU lanes with one CTA per head (a warp's own columns, so that dh ends up in the lane that runs
+// the unit), over 8 in clusters; KQ quads of k per lane, TB tasks of 128 / KS columns per warp
+template <int CELL, bool CL, int LPU, int KQ, int TB, int BT>
 struct XBwdGeom {
   using C = Cell<CELL>;
   static constexpr int PL = C::Gr == 3 ? 4 : C::Gr;  // planes of the delta tile: the R gates; the GRU's input-only gate behind them
   static constexpr int NIN = C::GC + C::NNEED + C::NEXT;
-  static constexpr int MAXQ = KS == 32 ? 16 : 8, MAXTH = 32 * MAXQ + kXIo;
+  static constexpr int KS = CL ? 8 : 4 * LPU;
+  static constexpr int MAXQ = CL ? 8 : 16, MAXTH = 4 * LPU * MAXQ + kXIo;
   static constexpr int NL = (NIN * BT * MAXQ + kXIo - 1) / kXIo, NS = ((C::Gw + (C::Gr == 3 ? 1 : 0)) * BT * MAXQ + kXIo - 1) / kXIo;
   static __host__ __device__ constexpr int plane(int U) { return U / 4 * BT * 16; }
   static __host__ __device__ constexpr int db(int U) { return PL * plane(U) > KS * KQ * BT * 16 ? PL * plane(U) : KS * KQ * BT * 16; }
@@ -290,18 +327,17 @@ struct XBwdGeom {
   static __host__ __device__ constexpr size_t smem(int U, int CS) { return (size_t)off_r(U) + (CS > 1 ? 2 * (size_t)CS * plane(U) : 0); }
 };
 
-template <int CELL, int KS, int KQ, int TB, int BT>
-__global__ void __launch_bounds__(XBwdGeom<CELL, KS, KQ, TB, BT>::MAXTH, 1) x32l_bwd_kernel(const __grid_constant__ XParams p) {
-  using G = XBwdGeom<CELL, KS, KQ, TB, BT>;
+template <int CELL, bool CL, int LPU, int KQ, int TB, int BT>
+__global__ void __launch_bounds__(XBwdGeom<CELL, CL, LPU, KQ, TB, BT>::MAXTH, 1) x32l_bwd_kernel(const __grid_constant__ XParams p) {
+  using G = XBwdGeom<CELL, CL, LPU, KQ, TB, BT>;
   using C = Cell<CELL>;
-  constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, NNEED = C::NNEED, NEXT = C::NEXT, NIN = G::NIN;
-  constexpr bool CL = KS == 8;
+  constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, NNEED = C::NNEED, NEXT = C::NEXT, NIN = G::NIN, KS = G::KS, UW = 32 / LPU;
   constexpr int GSH = Gr == 3 ? 1 : 0;  // GRU: plane 0 is the recurrent-only gate, which goes to dg0
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int D = p.D, U = p.U, Q = U >> 2, CS = p.CS, T = p.T, B = p.B, N = p.N;
   const int n = blockIdx.z, b0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
-  const int unit0 = (int)crank * U, TH = blockDim.x;
+  const int unit0 = (int)crank * U, TH = blockDim.x, W = (TH - kXIo) >> 5;
   const size_t ND = (size_t)N * D, col = (size_t)n * D + unit0;
   const bool exch = !p.grad_cut;  // with the recurrent gradient cut no dh crosses a step: no products, no exchange
 
@@ -322,8 +358,8 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, KS, KQ, TB, BT>::MAXTH, 1) x32l
   __syncthreads();
   if (CL) cluster_arrive();  // waited for before the first push
 
-  if (warp >= Q) {
-    const int io = tid - 32 * Q, inv = 65536 / Q + 1;
+  if (warp >= W) {
+    const int io = tid - 32 * W, inv = 65536 / Q + 1;
     // rows beyond B: zero activations and cotangents make their deltas zero; their states only have to be finite divisors
     for (int i = io; i < kXStages * xs / 16; i += kXIo) {
       const int pl = i * 16 % xs / plane;
@@ -415,14 +451,14 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, KS, KQ, TB, BT>::MAXTH, 1) x32l
     return;
   }
 
-  const int kk = lane & (KS - 1), uq = lane >> 3, b = lane & (BT - 1), unit = unit0 + 4 * warp + uq;
-  const bool own = (lane & 7) < BT, live = b0 + b < B;
+  const int kk = lane & (KS - 1), b = lane & (BT - 1), ul = warp * UW + lane / LPU, uc = ul < U ? ul : U - 1, unit = unit0 + uc;
+  const bool own = (lane & (LPU - 1)) < BT && ul < U, live = b0 + b < B;
   const size_t nd = (size_t)n * D + unit;
-  // columns c0[i] .. +3 of task i; k quad (gate, unit quad) number q of this CTA
-  P2 w[TB][4][KQ][2];
+  auto column0 = [&](int i) { return CL ? (warp + i * W) * 16 + (lane >> 3) * 4 : warp * UW + lane / KS * 4; };  // of task i
+  P2 w[TB][4][KQ][2];  // column, k quad (gate, unit quad)
 #pragma unroll
   for (int i = 0; i < TB; ++i) {
-    const int c0 = CL ? (warp + i * Q) * 16 + uq * 4 : 4 * warp;
+    const int c0 = column0(i);
 #pragma unroll
     for (int k = 0; k < KQ; ++k) {
       const int q = k * KS + kk, g = q / Q, u = unit0 + 4 * (q - g * Q);
@@ -445,7 +481,7 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, KS, KQ, TB, BT>::MAXTH, 1) x32l
   for (int g = 0; g < Gt; ++g) dbacc[g] = 0.f;
 #pragma unroll
   for (int k = 0; k < NNEED; ++k) cur[k] = live ? p.states[(((size_t)C::need(k) * B + b0 + b) * T + (T - 1)) * ND + nd] : 1.f;
-  const uint32_t word = (uint32_t)(warp * BT + b) * 16u + (uint32_t)uq * 4u;
+  const uint32_t word = (uint32_t)((uc >> 2) * BT + b) * 16u + (uint32_t)(uc & 3) * 4u;
   const uint32_t dr = dt + (uint32_t)(kk * BT) * 16u, sw = (uint32_t)(kk * BT >> 3) & (BT - 1);
   const bool drop = p.test_drop && crank == 0;  // test hook: CTA 0 withholds its message of the second step
   bool poisoned = false;
@@ -483,8 +519,8 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, KS, KQ, TB, BT>::MAXTH, 1) x32l
     cell_backward_apply<CELL>(ext[0] + r, co, car, dR_, dW_, dB_);
     if (own) {
 #pragma unroll
-      for (int g = 0; g < Gr; ++g) sts32(dt + (j & 1) * db + xq_off<BT>(g * Q + warp, b) + uq * 4u, __float_as_uint(dR_[g]));
-      if constexpr (GSH) sts32(dt + (j & 1) * db + xq_off<BT>(3 * Q + warp, b) + uq * 4u, __float_as_uint(dW_[2]));
+      for (int g = 0; g < Gr; ++g) sts32(dt + (j & 1) * db + xq_off<BT>(g * Q + (uc >> 2), b) + (uc & 3) * 4u, __float_as_uint(dR_[g]));
+      if constexpr (GSH) sts32(dt + (j & 1) * db + xq_off<BT>(3 * Q + (uc >> 2), b) + (uc & 3) * 4u, __float_as_uint(dW_[2]));
     }
 #pragma unroll
     for (int g = 0; g < Gt; ++g) dbacc[g] += dB_[g];
@@ -517,21 +553,12 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, KS, KQ, TB, BT>::MAXTH, 1) x32l
       for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int e = 0; e < BT; ++e) { const float2 s = v_get(acc[c][e]); v[c][e] = s.x + s.y; }
-      if constexpr (!CL) {  // lane bits 4, 3 <- column, the others <- row
-        float h[2][BT], o[1][BT];
-        const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int e = 0; e < BT; ++e) h[c][e] = (b4 ? v[c + 2][e] : v[c][e]) + __shfl_xor_sync(0xffffffffu, b4 ? v[c][e] : v[c + 2][e], 16);
-#pragma unroll
-        for (int e = 0; e < BT; ++e) o[0][e] = (b3 ? h[1][e] : h[0][e]) + __shfl_xor_sync(0xffffffffu, b3 ? h[0][e] : h[1][e], 8);
-        x_reduce8<BT, 1>(o, lane);
-        rec = o[0][0];
+      if constexpr (!CL) {
+        rec = x_reduce_units<LPU, BT>(v, lane);
       } else {
-        x_reduce8<BT, 4>(v, lane);
-        const int cq = (warp + i * Q) * 4 + uq, owner = cq / Q;  // the quad of columns
-        if (own && owner < CS && !poisoned && !(drop && j == 1)) {
+        x_reduce<8, BT, 4>(v, lane);
+        const int cq = column0(i) >> 2, owner = cq / Q;  // the quad of columns
+        if ((lane & 7) < BT && owner < CS && !poisoned && !(drop && j == 1)) {
           const uint32_t peer = map_to_cta(sm, (uint32_t)owner);
           st_async_v4(peer + (recv - sm) + (uint32_t)((j & 1) * rb + (int)crank * plane + ((cq - owner * Q) * BT + b) * 16), v[0][0], v[1][0], v[2][0],
                       v[3][0], peer + (j & 1) * 8);
@@ -550,7 +577,7 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, KS, KQ, TB, BT>::MAXTH, 1) x32l
   for (int g = 0; g < Gt; ++g) {
 #pragma unroll
     for (int m = 1; m < BT; m *= 2) dbacc[g] += __shfl_xor_sync(0xffffffffu, dbacc[g], m);
-    if ((lane & 7) == 0) atomicAdd(p.dbias + (size_t)g * ND + nd, dbacc[g]);
+    if ((lane & (LPU - 1)) == 0 && ul < U) atomicAdd(p.dbias + (size_t)g * ND + nd, dbacc[g]);
   }
   if (CL) { __syncwarp(); cluster_arrive_relaxed(); cluster_wait(); }
 }

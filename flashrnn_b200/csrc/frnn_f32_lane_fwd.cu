@@ -4,16 +4,17 @@
 
 namespace FRNN_NS {
 namespace {
-template <int CELL, int KQ, int BT> XLane make(int U) {
-  return XLane{reinterpret_cast<const void*>(&x32l_fwd_kernel<CELL, KQ, BT>), 8 * U + kXIo, BT, XFwdGeom<CELL, KQ, BT>::smem(U)};
+template <int CELL, bool CL, int LPU, int KQ, int BT> XLane make(int U) {
+  const int warps = (U * LPU + 31) / 32;
+  return XLane{reinterpret_cast<const void*>(&x32l_fwd_kernel<CELL, CL, LPU, KQ, BT>), 32 * warps + kXIo, BT, XFwdGeom<CELL, CL, LPU, KQ, BT>::smem(U)};
 }
-// k quads per lane: D / 32, rounded up to a power of two (padded with zeros).  Clusters take 2 rows at least, and no more from KQ = 8
-// on, whose part of R leaves no registers for them.
+// k quads per lane, from 4 * KQ * LPU units up (of which Elman's four-unit groups need a quarter)
+template <int CELL, bool CL, int LPU, int KQ, int BT> XLane quads(int U) { return make<CELL, CL, LPU, (Cell<CELL>::Gr > 1 ? KQ : KQ > 4 ? KQ / 4 : 1), BT>(U); }
 template <int CELL> XLane pick(int D, int U, int bt) {
-  if (D <= 32) return bt == 1 ? make<CELL, 1, 1>(U) : bt == 2 ? make<CELL, 1, 2>(U) : make<CELL, 1, 4>(U);
-  if (D <= 64) return bt == 1 ? make<CELL, 2, 1>(U) : bt == 2 ? make<CELL, 2, 2>(U) : make<CELL, 2, 4>(U);
-  if (D <= 128) return bt <= 2 ? make<CELL, 4, 2>(U) : make<CELL, 4, 4>(U);
-  return make<CELL, 8, 2>(U);
+  if (D <= 32) return bt == 1 ? quads<CELL, false, 2, 4, 1>(U) : bt == 2 ? quads<CELL, false, 2, 4, 2>(U) : quads<CELL, false, 4, 2, 4>(U);
+  if (D <= 64) return bt == 1 ? quads<CELL, false, 2, 8, 1>(U) : bt == 2 ? quads<CELL, false, 2, 8, 2>(U) : quads<CELL, false, 4, 4, 4>(U);
+  if (D <= 128) return bt <= 2 ? quads<CELL, true, 4, 8, 2>(U) : bt == 4 ? quads<CELL, true, 4, 8, 4>(U) : quads<CELL, true, 8, 4, 8>(U);
+  return bt <= 2 ? quads<CELL, true, 8, 8, 2>(U) : bt == 4 || Cell<CELL>::Gr > 1 ? quads<CELL, true, 8, 8, 4>(U) : quads<CELL, true, 8, 8, (Cell<CELL>::Gr > 1 ? 4 : 8)>(U);
 }
 }  // namespace
 
