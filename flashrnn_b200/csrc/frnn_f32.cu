@@ -5,13 +5,17 @@
 // the CUDA cores, gate nonlinearities from exp (error ~1e-6), so that it agrees with the fp32 `vanilla` loop to ~1e-5 --
 // the 16-bit tensor-core loops are the fast path, this one is for callers that need float32 results (reference checks,
 // gradient checks, small models).
+//   * lane loops (x32l_*, frnn_f32_lane.cuh): R in registers, head dims up to 256.  Against the cluster loops, clk per step:
+//     LSTM D = 64, 16 rows x 4 heads: forward 2360 -> 620, reverse 2810 -> 740; 64 x 8: 3030 -> 1570, 4360 -> 1550; D = 128, 16 x 2: 2500 -> 1310,
+//     3770 -> 1750; D = 256, 64 x 4: 17920 -> 15600, 23220 -> 18190.
 //   * cluster loops (x32c_*): a cluster of CS CTAs owns one head and 8 batch rows for all T steps; CTA c owns U = D / CS
 //     units, keeps its slice of R in shared memory as fp32 (Gr*U*D*4 bytes) and exchanges per step only what the others
 //     need -- its slice of h_t (forward, all-gather) or its partial sums of dh_{t-1} (reverse, reduce-scatter) -- with
-//     one bulk copy per peer that completes on the peer's mbarrier, the protocol of the 16-bit loops.  A thread's items
+//     one bulk copy per peer that completes on the peer's mbarrier.  A thread's items
 //     (batch row, unit) are fixed, so states, carried cotangents and bias stay in registers and the next step's global
 //     inputs are loaded one step ahead.  The matrix phase is FFMA from shared memory: a thread keeps 16 (forward: two
-//     gate rows x 8 batch rows) or 8 (reverse: one column x 8 batch rows) sums over its share of k.
+//     gate rows x 8 batch rows) or 8 (reverse: one column x 8 batch rows) sums over its share of k.  For head dims that the
+//     lane loops do not split, and Elman forward passes of many clusters.
 //   * streamed loops (x32_*): one CTA per (head, 8 batch rows), R read from L2 in every step; for head dims whose slices
 //     do not fit the shared memory of a portable cluster (e.g. four-gate cells above 256) or are no multiple of 4 units.
 //   * dR: a tiled fp32 GEMM over all (b, t) with split-K and fp32 atomics.
@@ -858,14 +862,23 @@ bool lane_tile(const frnn_problem& pr, bool bwd, int* cs_out, XLane* k) {
     for (cs = 2; cs <= 8 && (pr.D % cs || pr.D / cs % 4 || pr.D / cs > 32); ++cs) {}
     if (cs > 8) return false;
   }
-  // rows per CTA: as few as leave every CTA an SM of its own (a cluster its place)
-  const int fit = cs == 1 ? 148 : kResidentClusters[cs];
-  int bt = cs == 1 ? 1 : 2;
-  while (bt < (cs == 1 ? 4 : 8) && (long long)((pr.B + bt - 1) / bt) * pr.N > fit) bt *= 2;
-  if (const char* e = getenv("XBT")) bt = atoi(e);
+  // Rows per CTA: the fewest turns of all CTAs through the GPU, weighed with what a step takes (LSTM D = 64, 1, 2, 4 rows: 620, 830, 1590 clk;
+  // D = 20: 520, 640, 740; D = 128, 2, 4, 8 rows: 1310, 1750, 3140; a batch of 64 in two heads of D = 128 2560, 1750, 3140 for all of it)
+  const int weight[3][4] = {{6, 7, 9, 0}, {6, 8, 15, 0}, {0, 10, 14, 24}};
+  const int kind = cs > 1 ? 2 : pr.D > 32 ? 1 : 0, resident = cs > 1 ? kResidentClusters[cs] : kind ? 148 : 296;
+  int bt = 0;
+  long long best = 0;
+  for (int i = 0; i < 4; ++i) {
+    const long long tiles = (long long)((pr.B + (1 << i) - 1) >> i) * pr.N, cost = (tiles + resident - 1) / resident * weight[kind][i];
+    if (weight[kind][i] && (!bt || cost < best)) { bt = 1 << i; best = cost; }
+  }
+  // Elman's forward step has one row of R per unit to set against the reads of h: in clusters that queue up, the loop below with its
+  // 4 x 8 sums per thread is ahead (B64 N4 D256 7640 against 4070 clk for all clusters; B512 N8 D128 25060 against 23580)
+  if (!bwd && pr.cell == CELL_ELMAN && pr.D >= 128 && (long long)((pr.B + 1) / 2) * pr.N > 2 * resident) return false;
   const int cell = pr.cell == CELL_ELMAN && pr.forward_clip > 0.f ? (int)CELL_ELMAN_CLIP : pr.cell;
-  *k = (bwd ? x32_lane_bwd : x32_lane_fwd)(cell, pr.D, pr.D / cs, bt);
-  if (!k->fn) *k = (bwd ? x32_lane_bwd : x32_lane_fwd)(cell, pr.D, pr.D / cs, bt / 2);
+  XLane (*const loop)(int, int, int, int) = bwd ? x32_lane_bwd : x32_lane_fwd;
+  *k = loop(cell, pr.D, pr.D / cs, bt);
+  if (!k->fn) *k = loop(cell, pr.D, pr.D / cs, bt / 2);
   *cs_out = cs;
   return k->fn != nullptr && (pr.B + k->bt - 1) / k->bt <= 65535;
 }
