@@ -517,7 +517,10 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   // and a half tiles, lose: 1.43 vs 1.25 ms); for the one-gate Elman
   // cell at head_dim 64 (half a tile) the warp-MMA kernel with its many small CTAs streams faster (C5 1.55 vs 3.1 ms)
   // (the tcgen05 kernel keeps a whole row tile of dR, N = D <= 256 columns, in one TMEM allocation)
-  if ((parts & FRNN_PART_DR) && (pr.D >= 128 || cd.Gr * pr.D >= 256) && recurrent_grad_tma_supported(pr.D, lp.state_f32))
+  if ((parts & FRNN_PART_DR) && recurrent_grad_small_supported(pr.D))
+    e = launch_recurrent_grad_small(pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, lp.state_f32, a->dWx, ws + w.dg0, a->states, a->s0, grads,
+                                    sm_count_cached(), stream);
+  else if ((parts & FRNN_PART_DR) && (pr.D >= 128 || cd.Gr * pr.D >= 256) && recurrent_grad_tma_supported(pr.D, lp.state_f32))
     // bf16 states: both operands are [64 steps][64] tiles a tensor-map copy delivers ready for the MMA (C2: 0.087 ms
     // against 0.167 ms for the cp.async-fed kernel below)
     e = launch_recurrent_grad_tma(pr.cell, pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, a->dWx, ws + w.dg0, a->states, a->s0, grads,

@@ -69,6 +69,10 @@ bool recurrent_grad_tma_supported(int D, int state_f32);
 cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int Gr, int Gw, const void* dWx, const void* dg0,
                                       const void* states, const void* s0, float* dR, unsigned* status, int sm_count,
                                       cudaStream_t stream);
+// dR for head dims 16, 32, 64, 96 (frnn_dr_small.cu)
+bool recurrent_grad_small_supported(int D);
+cudaError_t launch_recurrent_grad_small(int B, int T, int N, int D, int Gr, int Gw, int state_f32, const void* dWx, const void* dg0,
+                                        const void* states, const void* s0, float* dR, int sm_count, cudaStream_t stream);
 cudaError_t launch_cast_grads(const float* src, void* dR, void* db, size_t nR, size_t nb, cudaStream_t stream);
 
 }  // namespace FRNN_NS
