@@ -394,7 +394,8 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
   long long wxs[4];
   if (!resolve_strides(a->wx_stride, wx_dense, wxs)) return FRNN_ERR_ALIGN;
 
-  const bool wide = is_wide(*plan) || plan->wide_forward;
+  // (a training pass stores activations, where the lane loop is ahead: see frnn_wide.cu)
+  const bool wide_gates = plan->wide_forward && !pr.training, wide = is_wide(*plan) || wide_gates;
   // keep_packed_r: the workspace is left as the previous call left it (R fragments kept, status block not cleared, so
   // an expired wait of an earlier step stays on record until the caller reads it).  The other loops clear the block themselves.
   cudaError_t e = plan->keep_packed_r || !wide ? cudaSuccess : cudaMemsetAsync(ws, 0, kStatusBytes, stream);
@@ -413,9 +414,9 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
                             pr.T, pr.N, plan->test_drop_exchange, stream);
     return (int)(e == cudaSuccess ? copy_last() : e);
   }
-  if (plan->wide_forward) {  // LSTM / GRU, head dim 64: 128-row forward loop; cache in the layout of the reverse loop's tile
+  if (wide_gates) {  // LSTM / GRU, head dim 64: 128-row forward loop
     if (plan->probe_noop_cell) return FRNN_ERR_PLAN;
-    e = launch_wide_gates_forward(pr.cell, a->Wx, wxs[0], wxs[1], wxs[2], wxs[3], a->R, a->b, a->s0, a->states, pr.training ? a->cache : nullptr,
+    e = launch_wide_gates_forward(pr.cell, a->Wx, wxs[0], wxs[1], wxs[2], wxs[3], a->R, a->b, a->s0, a->states,
                                  reinterpret_cast<unsigned*>(ws), pr.B, pr.T, pr.N, pr.forward_clip, plan->test_drop_exchange, stream);
     return (int)(e == cudaSuccess ? copy_last() : e);
   }

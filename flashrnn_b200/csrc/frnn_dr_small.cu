@@ -4,9 +4,11 @@
 // of heads whose elements lie side by side (HG * D of them: 128 to 512 bytes per gate and row), all their gates, and a contiguous range
 // of rows k = (b, t): every row's run goes through shared memory once, 16 bytes per cp.async along the rows, four stages deep, and
 // every warp keeps a 64 or 96 x 32 piece of the result in registers (mma.sync m16n8k16: the accumulators of a whole head, which
-// the tensor-map kernel holds in tensor memory, fit here too, and its 128-byte boxes were what limited it).  Two CTAs per SM.
+// the tensor-map kernel holds in tensor memory, fit here too).
 // The pieces of all CTAs meet in fp32 atomics on the gradient workspace.
-// Measured, LSTM: see launch_recurrent_grad_small.
+// Measured (before: one 64 x 64 tile of one gate per CTA, or the tensor-map kernel), us: LSTM B1024 T128 N24 D32 617 -> 175 (5.8 TB/s),
+// B1024 T256 N24 D16 1213 -> 248, B1024 T512 N16 D64 1437 -> 1232 (4.4 TB/s), B100 T500 N3 D96 135 -> 65; GRU B37 T333 N5 D96 52 -> 39;
+// sLSTM B256 T512 N16 D64 with fp32 states 772 -> 369.
 //
 // Replaces the post-loop cublasGemmStridedBatchedEx of the reference (flashrnn/flashrnn/fused/flashrnn_fused_backward.cu:
 // 1049-1058; util/blas.cu:199-219).
@@ -33,12 +35,13 @@ struct DrSmallGeom {
   static constexpr int HPU = D == 16 ? 2 : 1;                            // heads of it
   static constexpr int NT = D == 16 ? 2 : 4;                             // 8-column tiles of it
   static constexpr int UPH = (GR + GPU - 1) / GPU * (D / (8 * NT));      // pieces per head (D = 16: per two heads)
-  static constexpr int HG = D == 16 ? 8 : D == 32 ? 4 : GR > 1 ? 1 : D == 64 ? 4 : 3;
+  static constexpr int HG = D == 16 ? 8 : D == 32 ? 4 : D == 64 ? (GR > 1 ? 2 : 4) : (GR > 1 ? 1 : 3);
   static constexpr int W = HG * UPH / HPU, TH = 32 * W;
   static constexpr int ROW = HG * D;             // elements of a gate's run
   static constexpr int EH = F32 ? 4 : 2;
   static constexpr int PITCH = GR * ROW * 2 + ROW * EH + 16;  // an odd multiple of 16: ldmatrix reads 8 rows without conflicts
-  static constexpr int KC = PITCH <= 800 ? 32 : 16, STAGES = 4;
+  static constexpr int CTAS = D == 96 || (D == 64 && GR > 1) ? 1 : 2;  // per SM
+  static constexpr int KC = PITCH <= 800 ? 32 : 16, STAGES = CTAS == 1 ? 8 : 4;
   static constexpr int CA = GR * ROW / 8, CH = ROW * EH / 16, CPR = CA + CH, CHUNKS = KC * CPR, PT = (CHUNKS + TH - 1) / TH;
   static constexpr size_t smem = (size_t)STAGES * KC * PITCH;
 };
@@ -48,7 +51,7 @@ __device__ __forceinline__ void red_add_f32x2(float* addr, float a, float b) {
 }
 
 template <int D, int GR, bool F32>
-__global__ void __launch_bounds__(DrSmallGeom<D, GR, F32>::TH, D == 96 ? 1 : 2) recurrent_grad_small_kernel(const DrSmallParams p) {
+__global__ void __launch_bounds__(DrSmallGeom<D, GR, F32>::TH, DrSmallGeom<D, GR, F32>::CTAS) recurrent_grad_small_kernel(const DrSmallParams p) {
   using G = DrSmallGeom<D, GR, F32>;
   constexpr int GPU = G::GPU, HPU = G::HPU, NT = G::NT, MTG = D / 16, KC = G::KC, STAGES = G::STAGES, PITCH = G::PITCH, ROW = G::ROW;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -80,7 +83,7 @@ __global__ void __launch_bounds__(DrSmallGeom<D, GR, F32>::TH, D == 96 ? 1 : 2) 
     } else {
       const int e = (c - G::CA) * 16 / G::EH;
       if (n0 * D + e < N * D) src[i] = static_cast<const unsigned char*>(p.states) + ((size_t)k * ND + (size_t)n0 * D + e) * G::EH - ND * G::EH;
-      tt[i] = (int)(k % T);
+      tt[i] = (int)((uint32_t)k % (uint32_t)T);  // (2^32 rows do not fit the memory)
     }
     if (idx >= G::CHUNKS) src[i] = nullptr;
     if (idx < G::CHUNKS && src[i] == nullptr)  // columns beyond the last head
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(DrSmallGeom<D, GR, F32>::TH, D == 96 ? 1 : 2) 
           if (k < k1) {
             const unsigned char* s = src[i];
             if (tt[i] == 0)  // h_{t-1} of t = 0 is the initial state
-              s = static_cast<const unsigned char*>(p.s0) + ((size_t)(k / T) * ND + (size_t)n0 * D) * G::EH + (size_t)(c - G::CA) * 16;
+              s = static_cast<const unsigned char*>(p.s0) + ((size_t)((uint32_t)k / (uint32_t)T) * ND + (size_t)n0 * D) * G::EH + (size_t)(c - G::CA) * 16;
             cp_async16_u32(d, s);
           } else {
             sts128(d, make_uint4(0u, 0u, 0u, 0u));  // (delta is zero there; this only has to be finite)
@@ -195,8 +198,8 @@ cudaError_t launch(DrSmallParams p, int sm_count, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
   if (e != cudaSuccess) return e;
   const long long groups = (p.N + G::HG - 1) / G::HG, chunks = (p.K + G::KC - 1) / G::KC;
-  long long splits = (D == 96 ? 1 : 2) * (long long)sm_count / groups;  // one turn through the GPU
-  if (splits > (chunks + 7) / 8) splits = (chunks + 7) / 8;            // the atomics stay a small share
+  long long splits = G::CTAS * (long long)sm_count / groups;  // one turn through the GPU
+  if (splits > (chunks + 2) / 3) splits = (chunks + 2) / 3;            // the atomics stay a small share
   if (splits < 1) splits = 1;
   if (splits > 65535) splits = 65535;
   p.rows_per_split = (chunks + splits - 1) / splits * G::KC;

@@ -311,9 +311,10 @@ wide_fwd_elman_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
 // Two row threads per batch row (8 warps, two per scheduler; a warp reads the tensor-memory lanes of its quarter, so
 // warps w and w + 4 share 32 rows and split the 64 units) read the accumulator 16 units at a time (4 gates x 16 columns),
 // keep the cell state c of their 32 units in registers (fp32) and write h_t into the shared-memory tile that the next
-// step multiplies and a bulk store sends to `states[0]`.  After the arrival that hands h_t on, c_t and the four cached
-// activations go straight to global memory with 32-byte stores, c with neighbouring lanes swapping halves.  The activation
-// cache has the one layout every 16-bit loop uses ([t][head][b][unit pair][4]), so lane_bwd_kernel runs the reverse loop.
+// step multiplies and a bulk store sends to `states[0]`.  After the arrival that hands h_t on, c_t goes straight to global memory
+// with 32-byte stores, neighbouring lanes swapping halves.  For passes without gradients only: a training pass also has to store
+// the activations, 80 KB per step and CTA from 256 threads, and lane_fwd_kernel with its IO warps is ahead there (B1024 T512 N16:
+// LSTM 2.17 against 2.47 ms, GRU 1.86 against 2.22; without activations 2.05 against 1.47, 1.71 against 1.11).
 // Wx_t arrives as one tensor-map copy of [4 gates][128 rows][64] per step into a ring of two 64 KB stages; the stage of
 // step t is refilled with step t+2 as soon as the step's MMAs are known to have completed.
 struct WideGatesParams {
@@ -321,7 +322,6 @@ struct WideGatesParams {
   const elem_t* bias;  // [4,N,64]
   const elem_t* s0;    // [2,B,1,N,64]
   elem_t* states;      // [2,B,T,N,64]; h leaves through the tensor map, c through plain stores
-  uint32_t* cache;     // [t][head][b][unit pair][4 slots]; or null
   unsigned* status;
   int B, T, N;
   int test_drop;  // test hook: the copy of one Wx box (step index 2) is announced to its barrier but never issued
@@ -521,27 +521,25 @@ wide_fwd_gates_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
         }
       }
     }
-    // c_t -> states[1][b][t][n][:];  cache: 16-row tiles of the reverse loop, see WideGatesParams.  Pointers to this lane's
-    // 32-byte slot (units 32 half + 16 odd ..) in the even and in the odd row of its lane pair.
+    // c_t -> states[1][b][t][n][:].  Pointers to this lane's 32-byte slot (units 32 half + 16 odd ..) in the even and in the odd row of its
+    // lane pair.
     const bool odd = (lane & 1) != 0;
     const int be = b & ~1;
     const bool ok_e = be < B, ok_o = be + 1 < B;
     elem_t* c_e = p.states + (((size_t)B + (ok_e ? be : 0)) * T) * ND + (size_t)n * WD + 32 * half + (odd ? 16 : 0);
     elem_t* c_o = c_e + (size_t)T * ND;
-    uint4* ch = p.cache ? reinterpret_cast<uint4*>(p.cache) + ((size_t)n * B + (row_ok ? b : 0)) * 32 + 16 * half : nullptr;
-    const size_t ch_step = (size_t)N * B * 32;
     for (int t = 0; t < T; ++t) {
       if (!mbar_wait_bounded(&acc_full[t & 1], (uint32_t)((t >> 1) & 1))) { report_timeout(p.status, t); break; }
       tc_fence_after();
       unsigned char* hdst = sm + WL_OFF_H + (uint32_t)(t & 1) * WTILE;
       const uint32_t acc = trow + (uint32_t)(t & 1) * (WL_G * WD);
-      uint4 out[1 + WL_G][4];  // c_t and the four activations of this thread's 32 units, packed for the stores below
+      uint4 out[4];  // c_t of this thread's 32 units, packed for the stores below
 #pragma unroll
       for (int qq = 0; qq < 2; ++qq) {  // units 16 q .. 16 q + 15
         const int q = 2 * half + qq;
         uint32_t ri[16], rf[16], rz[16], ro[16];
         tmem_ld16x4(acc + 16 * q, acc + WD + 16 * q, acc + 2 * WD + 16 * q, acc + 3 * WD + 16 * q, ri, rf, rz, ro);
-        float hv[16], gi[16], gf[16], gz[16], go[16];  // h_t and the four cached values (LSTM: i, f, z, o; GRU: g~, r, z, n)
+        float hv[16], gi[16], gf[16], gz[16], go[16];  // h_t and the gates (LSTM: i, f, z, o; GRU: g~, r, z, n)
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           if constexpr (GRU) {
@@ -584,16 +582,10 @@ wide_fwd_gates_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
           float cv[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) cv[j] = cst[16 * qq + j];
-          pack16(cv, out[0][2 * qq], out[0][2 * qq + 1]);
+          pack16(cv, out[2 * qq], out[2 * qq + 1]);
         }
-        pack16(gi, out[1][2 * qq], out[1][2 * qq + 1]);
-        pack16(gf, out[2][2 * qq], out[2][2 * qq + 1]);
-        pack16(gz, out[3][2 * qq], out[3][2 * qq + 1]);
-        pack16(go, out[4][2 * qq], out[4][2 * qq + 1]);
       }
-      // h_t is complete: hand it to the next step first; the 20 global stores of this thread (c_t and the cache, 80 KB per
-      // step and CTA) come after the arrival, off the chain h_t -> MMA -> accumulator (LB forward loop 2.87 -> 2.63 ms
-      // together with the 32-byte stores).
+      // h_t is complete: hand it to the next step first; the stores of c_t come after the arrival, off the chain h_t -> MMA -> accumulator
       fence_proxy_async_smem();  // the tile is read by the tensor core and by the bulk store
       tc_fence_before();
       mbar_arrive(h_ready);
@@ -601,25 +593,16 @@ wide_fwd_gates_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
         // c: a thread owns 64 contiguous bytes.  Neighbouring lanes (rows 2m, 2m+1) swap halves so that each of the two store
         // instructions covers 16 rows x 64 contiguous bytes instead of 32 rows x 32: the memory system is charged per piece of
         // a 128-byte line, and this halves the pieces.
-        const uint4 s0 = odd ? out[0][0] : out[0][2], s1 = odd ? out[0][1] : out[0][3];
+        const uint4 s0 = odd ? out[0] : out[2], s1 = odd ? out[1] : out[3];
         uint4 r0, r1;
         r0.x = __shfl_xor_sync(0xffffffffu, s0.x, 1); r0.y = __shfl_xor_sync(0xffffffffu, s0.y, 1);
         r0.z = __shfl_xor_sync(0xffffffffu, s0.z, 1); r0.w = __shfl_xor_sync(0xffffffffu, s0.w, 1);
         r1.x = __shfl_xor_sync(0xffffffffu, s1.x, 1); r1.y = __shfl_xor_sync(0xffffffffu, s1.y, 1);
         r1.z = __shfl_xor_sync(0xffffffffu, s1.z, 1); r1.w = __shfl_xor_sync(0xffffffffu, s1.w, 1);
-        if (ok_e) st_global_32B(c_e, odd ? r0 : out[0][0], odd ? r1 : out[0][1]);
-        if (ok_o) st_global_32B(c_o, odd ? out[0][2] : r0, odd ? out[0][3] : r1);
-      }
-      if (ch != nullptr && row_ok) {  // 256 contiguous bytes per thread: the four values of a unit pair side by side
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint4 &i4 = out[1][q], &f4 = out[2][q], &z4 = out[3][q], &o4 = out[4][q];
-          st_global_32B(ch + 4 * q, make_uint4(i4.x, f4.x, z4.x, o4.x), make_uint4(i4.y, f4.y, z4.y, o4.y));
-          st_global_32B(ch + 4 * q + 2, make_uint4(i4.z, f4.z, z4.z, o4.z), make_uint4(i4.w, f4.w, z4.w, o4.w));
-        }
+        if (ok_e) st_global_32B(c_e, odd ? r0 : out[0], odd ? r1 : out[1]);
+        if (ok_o) st_global_32B(c_o, odd ? out[2] : r0, odd ? out[3] : r1);
       }
       c_e += ND; c_o += ND;
-      if (ch != nullptr) ch += ch_step;
     }
   }
   tc_fence_before();
@@ -1107,7 +1090,7 @@ bool wide_gates_forward_supported(int cell, int D, int state_f32) {
 }
 
 cudaError_t launch_wide_gates_forward(int cell, const void* Wx, long long wx_sb, long long wx_st, long long wx_sg, long long wx_sn, const void* R,
-                                     const void* bias, const void* s0, void* states, void* cache, unsigned* status, int B, int T,
+                                     const void* bias, const void* s0, void* states, unsigned* status, int B, int T,
                                      int N, float fclip, int test_drop, cudaStream_t stream) {
   CUtensorMap tm_wx, tm_st;
   if (!map_wx_gates(&tm_wx, Wx, cell == CELL_GRU ? 3 : 4, B, T, N, wx_sb, wx_st, wx_sg, wx_sn) ||
@@ -1118,7 +1101,6 @@ cudaError_t launch_wide_gates_forward(int cell, const void* Wx, long long wx_sb,
   p.bias = static_cast<const elem_t*>(bias);
   p.s0 = static_cast<const elem_t*>(s0);
   p.states = static_cast<elem_t*>(states);
-  p.cache = static_cast<uint32_t*>(cache);
   p.status = status;
   p.B = B; p.T = T; p.N = N;
   p.test_drop = test_drop;
