@@ -258,7 +258,10 @@ static bool resolve_strides(const int64_t (&in)[4], const long long (&dense)[4],
   return true;
 }
 
-static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int cs, int rows, const frnn_plan& pl, const LoopParams& lp, cudaStream_t stream) {
+// `overlap`: a decoding step behind another may start, and read R, while that one still runs (everything else waits for it on the device):
+// launch and prologue, about half of a one-token step, disappear behind the step before
+static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int cs, int rows, const frnn_plan& pl, const LoopParams& lp, bool overlap,
+                               cudaStream_t stream) {
   // always the fixed maximum, never this plan's own size: the attribute belongs to the kernel, not to the launch, and a
   // second host thread launching the same instantiation with a larger tile must not find it lowered in between
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
@@ -272,13 +275,20 @@ static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int cs,
   cfg.blockDim = dim3((unsigned)threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  unsigned na = 0;
+  if (cs > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = (unsigned)cs;
+    attr[na].val.clusterDim.y = 1;
+    attr[na++].val.clusterDim.z = 1;
+  }
+  if (overlap) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = cs > 1 ? 1 : 0;
+  cfg.numAttrs = na;
   void* args[1] = {const_cast<LoopParams*>(&lp)};
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
@@ -292,7 +302,7 @@ static int launch_big(const frnn_plan& pl, bool bwd, LoopParams lp, cudaStream_t
   if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(kernel_cell(pr), bwd, u, nt = 1);  // (sLSTM reverse from head dim 896 up)
   if (!k.fn || pl.probe_noop_cell) return FRNN_ERR_PLAN;
   lp.CS = pr.D / u;
-  return (int)launch_loop(k.fn, k.threads, k.smem(pr.D), lp.CS, 8 * nt, pl, lp, stream);
+  return (int)launch_loop(k.fn, k.threads, k.smem(pr.D), lp.CS, 8 * nt, pl, lp, !bwd && pl.keep_packed_r, stream);
 }
 static int launch_lane(const frnn_plan& pl, bool bwd, const LoopParams& lp, cudaStream_t stream) {
   const frnn_problem& pr = pl.prob;
@@ -300,7 +310,7 @@ static int launch_lane(const frnn_plan& pl, bool bwd, const LoopParams& lp, cuda
   const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(kernel_cell(pr), bwd, kt, pl.units_per_cta, nt)
                        : bwd              ? lane_bwd_floor(pr.cell, kt, pl.units_per_cta, nt)
                                           : lane_fwd_floor(pr.cell, kt, pl.units_per_cta, nt);
-  return k.fn ? (int)launch_loop(k.fn, k.threads, k.smem, pl.cluster_size, 8 * nt, pl, lp, stream) : FRNN_ERR_PLAN;
+  return k.fn ? (int)launch_loop(k.fn, k.threads, k.smem, pl.cluster_size, 8 * nt, pl, lp, !bwd && pl.keep_packed_r, stream) : FRNN_ERR_PLAN;
 }
 
 static int sm_count_cached() {

@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT>::TH, 1) big_fwd_kernel
   const uint32_t sm = smem_u32(smem_raw), hbuf = sm + G::OFF_H;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);  // [2] bytes of h tile x have arrived (and see lane_fwd_io)
 
+  grid_launch_next();
   if (tid == 0) {
     for (int x = 0; x < 2; ++x) mbar_init(&full[x], 1 + G::GROUPS);
     fence_mbar_init();
@@ -99,15 +100,6 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT>::TH, 1) big_fwd_kernel
   if (p.clear_status && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
     p.status[0] = 0u; p.status[1] = 0u; p.status[2] = 0u; p.status[3] = 0u;
   }
-  for (int idx = tid; idx < G::BT * (D / 2); idx += TH) {  // h_{-1} -> tile 1
-    const int bl = idx / (D / 2), k = 2 * (idx - bl * (D / 2));
-    float2 v = make_float2(0.f, 0.f);
-    if (bt0 + bl < B) v = load_state2(p.s0, (size_t)(bt0 + bl) * ND + (size_t)n * D + k, f32);
-    sts32(hbuf + HB + (bl >> 3) * HT + opnd_off(bl & 7, k), pack_x2(v.x, v.y));
-  }
-  __syncthreads();
-  cluster_arrive();  // barriers initialised, h_{-1} read; waited for before the first push, or before `last` may overwrite s0
-
   // ---- warp (grp, half): units [grp * UW, +UW), k-pairs [half * kph, +kph).  Its fragments: KRP pairs in registers, the next ksp
   // in shared memory (each lane reads back what it wrote itself), the rest in global memory
   const int half = warp >= G::GROUPS, grp = warp - half * G::GROUPS;
@@ -136,6 +128,16 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT>::TH, 1) big_fwd_kernel
   }
   const uint32_t rs = sm + G::off_r(D) + (uint32_t)(warp * ksp) * (MT * 1024) + lane * 16;
   for (int i = 0; i < ksp * MT * 2; ++i) sts128(rs + i * 512, __ldg(src + (size_t)KRP * (MT * 64) + i * 32));
+
+  grid_wait_previous();  // (R may be read before it: consecutive decoding steps overlap up to here)
+  for (int idx = tid; idx < G::BT * (D / 2); idx += TH) {  // h_{-1} -> tile 1
+    const int bl = idx / (D / 2), k = 2 * (idx - bl * (D / 2));
+    float2 v = make_float2(0.f, 0.f);
+    if (bt0 + bl < B) v = load_state2(p.s0, (size_t)(bt0 + bl) * ND + (size_t)n * D + k, f32);
+    sts32(hbuf + HB + (bl >> 3) * HT + opnd_off(bl & 7, k), pack_x2(v.x, v.y));
+  }
+  __syncthreads();
+  cluster_arrive();  // barriers initialised, h_{-1} read; waited for before the first push, or before `last` may overwrite s0
 
   const int ul = grp * G::UW + (QUAD ? (gid >> 1) * MT : 2 * gid), unit = (int)crank * U + ul;
   const uint32_t sums = sm + G::OFF_S + (uint32_t)(grp * MT * NT * 32 + lane) * 16;

@@ -920,7 +920,7 @@ cudaError_t launch_cluster(K kern, const frnn_problem& pr, const Tile& t, size_t
   cfg.numAttrs = t.cs > 1 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
-cudaError_t launch_lane(const XLane& k, int cs, const frnn_problem& pr, XParams p, cudaStream_t stream) {
+cudaError_t launch_lane(const XLane& k, int cs, const frnn_problem& pr, XParams p, bool overlap, cudaStream_t stream) {  // overlap: see launch_loop in frnn_api.cu
   cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);  // fixed maximum
   if (e != cudaSuccess) return e;
   p.CS = cs;
@@ -930,13 +930,20 @@ cudaError_t launch_lane(const XLane& k, int cs, const frnn_problem& pr, XParams 
   cfg.blockDim = dim3((unsigned)k.threads, 1, 1);
   cfg.dynamicSmemBytes = k.smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  unsigned na = 0;
+  if (cs > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = (unsigned)cs;
+    attr[na].val.clusterDim.y = 1;
+    attr[na++].val.clusterDim.z = 1;
+  }
+  if (overlap) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = cs > 1 ? 1 : 0;
+  cfg.numAttrs = na;
   void* args[1] = {&p};
   return cudaLaunchKernelExC(&cfg, k.fn, args);
 }
@@ -1028,7 +1035,7 @@ __attribute__((visibility("hidden"))) int frnn_forward_f32(const frnn_plan* plan
   if (is_lane) {
     p.last = static_cast<float*>(a->last);
     p.clear_status = !plan->keep_packed_r; p.test_drop = plan->test_drop_exchange;
-    return (int)launch_lane(lane, lane_cs, pr, p, stream);
+    return (int)launch_lane(lane, lane_cs, pr, p, plan->keep_packed_r != 0, stream);
   }
   if (tl.cluster) {
     p.U = tl.u; p.CS = tl.cs; p.KS = tl.ksf; p.test_drop = plan->test_drop_exchange;
@@ -1114,7 +1121,7 @@ __attribute__((visibility("hidden"))) int frnn_backward_parts_f32(const frnn_pla
     int lane_cs;
     if (lane_tile(pr, true, &lane_cs, &lane)) {
       p.test_drop = plan->test_drop_exchange;
-      e = launch_lane(lane, lane_cs, pr, p, stream);
+      e = launch_lane(lane, lane_cs, pr, p, false, stream);
     } else if (tl.cluster) {
       p.U = tl.u; p.CS = tl.cs; p.KS = tl.ksb; p.test_drop = plan->test_drop_exchange;
       auto launch = [&](auto cell) {

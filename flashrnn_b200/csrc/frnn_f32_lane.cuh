@@ -105,6 +105,26 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32
   const uint32_t sm = smem_u32(xsm), ht = sm + 128, ring = sm + G::off_x(), out = sm + G::off_o(U);
   const int plane = G::plane(U), xs = Gw * plane, ob = (S + GC) * plane;
   uint64_t* full = reinterpret_cast<uint64_t*>(xsm);  // [2] bytes of h tile x have arrived
+  grid_launch_next();
+  const int kk = lane & (KS - 1), b = lane & (BT - 1), ul = warp * UW + lane / LPU;  // this lane's unit within the CTA
+  const int unit = unit0 + (ul < U ? ul : U - 1);
+  // (the other lanes of a unit run the same rows, lanes beyond the last unit run it, and neither stores anything)
+  const bool own = (lane & (LPU - 1)) < BT && ul < U, live = b0 + b < B;
+  P2 w[NR][KQ][2];  // (nothing else is read before grid_wait_previous: consecutive decoding steps overlap up to there)
+  if (warp < W) {
+#pragma unroll
+    for (int g = 0; g < NR; ++g) {
+      const int first = warp * UW + lane / KS * 4 + g, row = Gr == 1 ? unit0 + (first < U ? first : U - 1) : unit;
+#pragma unroll
+      for (int i = 0; i < KQ; ++i) {
+        const int q = i * KS + kk;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (4 * q < D) v = __ldg(reinterpret_cast<const uint4*>(p.R + (((size_t)(Gr == 1 ? 0 : g) * N + n) * D + row) * D + 4 * q));
+        x_unpack(v, w[g][i][0], w[g][i][1]);
+      }
+    }
+  }
+  grid_wait_previous();
   if (CL && tid == 0) {
     mbar_init(&full[0], 1);
     mbar_init(&full[1], 1);
@@ -198,22 +218,6 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32
     return;
   }
 
-  const int kk = lane & (KS - 1), b = lane & (BT - 1), ul = warp * UW + lane / LPU;  // this lane's unit within the CTA
-  const int unit = unit0 + (ul < U ? ul : U - 1);
-  // (the other lanes of a unit run the same rows, lanes beyond the last unit run it, and neither stores anything)
-  const bool own = (lane & (LPU - 1)) < BT && ul < U, live = b0 + b < B;
-  P2 w[NR][KQ][2];
-#pragma unroll
-  for (int g = 0; g < NR; ++g) {
-    const int first = warp * UW + lane / KS * 4 + g, row = Gr == 1 ? unit0 + (first < U ? first : U - 1) : unit;
-#pragma unroll
-    for (int i = 0; i < KQ; ++i) {
-      const int q = i * KS + kk;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (4 * q < D) v = __ldg(reinterpret_cast<const uint4*>(p.R + (((size_t)(Gr == 1 ? 0 : g) * N + n) * D + row) * D + 4 * q));
-      x_unpack(v, w[g][i][0], w[g][i][1]);
-    }
-  }
   const size_t nd = (size_t)n * D + unit;
   float bias[Gt], st[S], cch[GCA];
 #pragma unroll

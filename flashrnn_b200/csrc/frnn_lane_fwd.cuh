@@ -359,6 +359,36 @@ __global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT>::TH, LaneFwdGeom<
   const uint32_t sm = smem_u32(smem_raw);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + G::OFF_BAR);  // [2] bytes of h tile x have arrived (and see lane_fwd_io)
 
+  grid_launch_next();
+  const int ul = warp * G::UW + (QUAD ? (gid >> 1) * MT : 2 * gid);  // this lane's units within the CTA: ul, ul + 1
+  const int unit = (int)crank * U + ul;
+
+  // ---- this lane's rows of R, all D inputs.  (Nothing else is read before grid_wait_previous: consecutive decoding steps overlap up to there.)
+  AFrag A[MT][KP];
+  if (warp < G::W) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int hi = 0; hi < 2; ++hi) {
+        const int g = QUAD ? hi * 2 + a : 0;
+        const elem_t* src = p.R + (((size_t)g * N + n) * D + (QUAD ? unit + m : unit + hi)) * D;
+#pragma unroll
+        for (int kp = 0; kp < KP; ++kp) {
+          uint4 v = make_uint4(0u, 0u, 0u, 0u);
+          if (g < Gr) {
+            if (2 * kp + 1 < KT) {
+              v = __ldg(reinterpret_cast<const uint4*>(src + kp * 32 + tig * 8));
+            } else {
+              const uint2 w = __ldg(reinterpret_cast<const uint2*>(src + kp * 32 + tig * 4));
+              v.x = w.x; v.y = w.y;
+            }
+          }
+          (hi ? A[m][kp].hi : A[m][kp].lo) = v;
+        }
+      }
+  }
+  grid_wait_previous();
+
   if (CL && tid == 0) {
     for (int x = 0; x < 2; ++x) {
       mbar_init(&full[x], 1 + G::IOW);
@@ -393,32 +423,6 @@ __global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT>::TH, LaneFwdGeom<
     }
     return;
   }
-
-  const int ul = warp * G::UW + (QUAD ? (gid >> 1) * MT : 2 * gid);  // this lane's units within the CTA: ul, ul + 1
-  const int unit = (int)crank * U + ul;
-
-  // ---- this lane's rows of R, all D inputs
-  AFrag A[MT][KP];
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int hi = 0; hi < 2; ++hi) {
-      const int g = QUAD ? hi * 2 + a : 0;
-      const elem_t* src = p.R + (((size_t)g * N + n) * D + (QUAD ? unit + m : unit + hi)) * D;
-#pragma unroll
-      for (int kp = 0; kp < KP; ++kp) {
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (g < Gr) {
-          if (2 * kp + 1 < KT) {
-            v = __ldg(reinterpret_cast<const uint4*>(src + kp * 32 + tig * 8));
-          } else {
-            const uint2 w = __ldg(reinterpret_cast<const uint2*>(src + kp * 32 + tig * 4));
-            v.x = w.x; v.y = w.y;
-          }
-        }
-        (hi ? A[m][kp].hi : A[m][kp].lo) = v;
-      }
-    }
 
   FwdLane<CELL, G, F2> lx;
   lx.init(p, sm + G::OFF_X, sm + G::OFF_O, HT, lane, ul, unit, n, bt0);

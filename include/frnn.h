@@ -91,7 +91,7 @@ typedef struct frnn_plan {
                                  workspace (default).
                                  1: the workspace is as an earlier frnn_forward with this plan left it and R has not
                                  changed since: skip both launches (step-by-step decoding calls frnn_forward once per
-                                 token); a device status recorded by an earlier step stays until the caller reads it */
+                                 token; a call may read R while the one queued before it still runs); a device status recorded by an earlier step stays until the caller reads it */
   int32_t probe_noop_cell;    /* MEASUREMENT HOOK, leave 0.  1: the time loops run with the gate arithmetic replaced by a
                                  pass-through (same exchange, matrix products, barriers and copies): their duration is
                                  the floor the serial chain of T dependent steps sets, which no cell math can undercut.
