@@ -98,9 +98,11 @@ static int plan_threads(const CellDims& cd, int units, int bt) { return bt == kW
 
 // Rows / 8 the lane loops run a plan's batch tile with (the activation cache and every result are the same whatever it is).
 // 16-row tiles reuse a fragment of R for two products but hold twice the items per lane.  Measured at batches that fill the GPU (clk per
-// step of all CTAs, 8 against 16 rows): forward LSTM D = 64 8887 / 11285, sLSTM 9283 / 12485, LSTM D = 128 8130 / 8214, but GRU D = 64
+// step of all CTAs, 8 against 16 rows): forward LSTM D = 64 8887 / 11285, sLSTM 9283 / 12485, LSTM D = 128 9790 / 8190, GRU D = 64
 // 8512 / 7320; reverse LSTM D = 64 9881 / 11400, GRU 8524 / 12100, sLSTM 7378 / 9263, but LSTM D = 128 (clusters) 10718 / 8900.
-static int lane_nt(const frnn_problem& pr, bool bwd, int cs, int bt) { return bt >= 16 && (bwd ? cs > 1 : pr.cell == CELL_GRU && cs == 1) ? 2 : 1; }
+static int lane_nt(const frnn_problem& pr, bool bwd, int cs, int bt) {
+  return bt >= 16 && (bwd ? cs > 1 : (pr.cell == CELL_GRU && cs == 1) || (pr.cell == CELL_LSTM && cs > 1 && pr.D == 128)) ? 2 : 1;
+}
 
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
   const int D = pr.D;

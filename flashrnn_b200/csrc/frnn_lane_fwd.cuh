@@ -47,7 +47,12 @@ struct LaneFwdGeom {
   static constexpr int OFF_X = 2 * HB, OFF_O = OFF_X + kLaneStages * XS, OFF_BAR = OFF_O + 2 * OUT_B;
   static constexpr size_t smem = OFF_BAR + 2 * 8;
   // 16-row tiles: only where some problem runs them (lane_nt in frnn_api.cu)
-  static constexpr bool valid = D % U == 0 && U % UW == 0 && CS <= 16 && TH <= 512 + 64 && (NT == 1 || (CELL == CELL_GRU && !CL));
+  static constexpr bool valid = D % U == 0 && U % UW == 0 && CS <= 16 && TH <= 512 + 64 && (NT == 1 || (CELL == CELL_GRU && !CL) || (CELL == CELL_LSTM && CL && KT == 8));
+  // CTAs per SM the registers are cut for (0: as the compiler sees fit), where it measured faster, clk per step, alone or of all CTAs of a large
+  // batch: clusters sLSTM D = 192 1134 -> 1100, Elman D = 128 835 -> 718, LSTM D = 128 1007 -> 925 (and 8-row tiles of a large
+  // batch 8070 -> 9790, so that takes 16 rows, 8190); single CTAs GRU D = 64 743 -> 690, 8680 -> 8310, with 16 rows 9390 -> 7510; sLSTM D = 64
+  // 9960 -> 9280.  Not LSTM D = 64 (813 -> 780, but 8940 -> 9290).
+  static constexpr int MINB = CL ? (KT >= 12 || !QUAD ? 1 : CELL == CELL_LSTM && KT == 8 ? 2 : 0) : (KT == 4 && (CELL == CELL_GRU || CELL == CELL_SLSTM)) || NT == 2 ? 2 : 0;
 };
 
 // The lanes that move data between global and shared memory.  ES: bytes of a state element (0: known at run time only); x0, o0: the Wx
@@ -329,10 +334,8 @@ struct FwdLane {
   }
 };
 
-// (16-row tiles run several CTAs per SM: without the bound the GRU D = 64 kernel takes 126 registers and one CTA less fits,
-// B1024 N16 7250 -> 9390 clk per step of all CTAs)
 template <int CELL, int KT, int U, int NT>
-__global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT>::TH, LaneFwdGeom<CELL, KT, U, NT>::CL || NT == 1 ? 0 : 2) lane_fwd_kernel(const __grid_constant__ LoopParams p) {
+__global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT>::TH, LaneFwdGeom<CELL, KT, U, NT>::MINB) lane_fwd_kernel(const __grid_constant__ LoopParams p) {
   using G = LaneFwdGeom<CELL, KT, U, NT>;
   using C = Cell<CELL>;
   // packed arithmetic where it measured faster (LSTM D = 128 step 1023 -> 975 clk; D = 64, one CTA, 847 -> 890)
