@@ -525,20 +525,17 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
     rc = is_big(pr) ? launch_big(*plan, true, lp, stream) : launch_lane(*plan, true, lp, stream);
     if (rc) return rc;
   }
-  // measured on B200: the tcgen05 kernel wins from head_dim 128 up (C2 0.167 vs 0.212 ms, C3 0.263 vs 0.304 ms) and at
-  // head_dim 64 when the gates fill two 128-row tiles (LSTM B1024 T512 N16 D64: 1.43 vs 1.60 ms; the GRU's 192 rows, one
-  // and a half tiles, lose: 1.43 vs 1.25 ms); for the one-gate Elman
-  // cell at head_dim 64 (half a tile) the warp-MMA kernel with its many small CTAs streams faster (C5 1.55 vs 3.1 ms)
-  // (the tcgen05 kernel keeps a whole row tile of dR, N = D <= 256 columns, in one TMEM allocation)
+  // dR.  Small heads: what counts is reading whole runs of neighbouring heads (frnn_dr_small.cu).  From head dim 128 up 16-bit states: both
+  // operands are [64 steps][64] tiles a tensor-map copy delivers ready for the MMA (C2: 0.087 ms against 0.167 ms for the cp.async-fed kernel;
+  // above 256, in column tiles, LSTM D = 768 0.445 -> 0.138 ms, D = 512 N2 0.350 -> 0.139 ms, against the warp-MMA kernel).  fp32 states: the
+  // cp.async-fed tcgen05 kernel while a row tile of dR, D columns, fits one TMEM allocation, the warp-MMA kernel above.
   if ((parts & FRNN_PART_DR) && recurrent_grad_small_supported(pr.D))
     e = launch_recurrent_grad_small(pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, lp.state_f32, a->dWx, ws + w.dg0, a->states, a->s0, grads,
                                     sm_count_cached(), stream);
-  else if ((parts & FRNN_PART_DR) && (pr.D >= 128 || cd.Gr * pr.D >= 256) && recurrent_grad_tma_supported(pr.D, lp.state_f32))
-    // bf16 states: both operands are [64 steps][64] tiles a tensor-map copy delivers ready for the MMA (C2: 0.087 ms
-    // against 0.167 ms for the cp.async-fed kernel below)
+  else if ((parts & FRNN_PART_DR) && recurrent_grad_tma_supported(pr.D, lp.state_f32))
     e = launch_recurrent_grad_tma(pr.cell, pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, a->dWx, ws + w.dg0, a->states, a->s0, grads,
                                   reinterpret_cast<unsigned*>(ws), sm_count_cached(), stream);
-  else if ((parts & FRNN_PART_DR) && pr.D >= 128 && pr.D <= 256)
+  else if ((parts & FRNN_PART_DR) && pr.D <= 256)
     e = launch_recurrent_grad_tc(pr.cell, pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, lp.state_f32, a->dWx, ws + w.dg0, a->states,
                                  a->s0, grads, reinterpret_cast<unsigned*>(ws), sm_count_cached(), stream);
   else if (parts & FRNN_PART_DR)

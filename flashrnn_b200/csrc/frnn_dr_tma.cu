@@ -3,10 +3,10 @@
 //   dR[g,n,d,p] = sum_{b,t} delta_g[b,t,n,d] * h_{t-1}[b,n,p]
 //
 // Same GEMM as frnn_dr_tc.cu (C[(g,d), p] = A^T B per head, both operands MN-major exactly as the time loops left them
-// in HBM), for bf16 states and head dims that are multiples of 64: a 64-step stretch of one batch row is, for every 64
+// in HBM), for 16-bit states and head dims that are multiples of 64: a 64-step stretch of one batch row is, for every 64
 // consecutive d (or p), one [64 t][64] tile with 128-byte rows -- the box of a tensor-map copy with 128-byte swizzle
 // and, unchanged, one block of a UMMA operand.  One CTA owns MT tiles of 128 rows of (g,d) (two such blocks each), all D
-// columns of p and a range of 64-step chunks (split-K over gridDim.z); the MT accumulators share every h block that is
+// columns of p (above 256: a column tile of up to 256) and a range of 64-step chunks (split-K over gridDim.z); the MT accumulators share every h block that is
 // fetched, so h crosses L2 -> shared memory once per MT * 128 rows (MT = 2 for D = 256, 3 for D = 128: the tensor
 // memory holds MT * D <= 512 fp32 columns):
 //   * warp 4, one lane: per chunk 2 MT + D/64 bulk loads into a 3- or 4-stage ring (mbarrier byte counts), then 4 MT
@@ -42,6 +42,7 @@ struct DrTmaParams {
   int chunks_per_split;
   int tmem_cols;             // power of two >= mt * D, >= 32
   int mt;                    // 128-row tiles of (g,d) per CTA
+  int ct, nbw;               // column tiles of p, 64-wide blocks of each (the last may repeat the head's last block: computed again, not stored)
   int stages;                // ring depth (<= DT_STAGES)
 };
 
@@ -53,8 +54,8 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* sm = smem_raw + (base - raw);
   const int D = p.D, N = p.N, T = p.T, nb = D >> 6;  // nb = 64-wide blocks per gate (rows) / of p (columns)
-  const int MT = p.mt, NS = p.stages;
-  const uint32_t stage_bytes = (uint32_t)(2 * MT + nb) * DT_BLK;
+  const int MT = p.mt, NS = p.stages, nbw = p.nbw, DW = nbw * 64, ctile = blockIdx.x % p.ct;
+  const uint32_t stage_bytes = (uint32_t)(2 * MT + nbw) * DT_BLK;
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + (size_t)NS * stage_bytes);          // [DT_STAGES] bytes have landed
   uint64_t* empty = full + DT_STAGES;                                                  // [DT_STAGES] MMAs have read the stage
   uint64_t* done = empty + DT_STAGES;
@@ -63,7 +64,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n = blockIdx.y;
   const int RB = p.Gr * nb;                            // 64-row blocks of (g,d)
-  const int rbase = 2 * MT * blockIdx.x;               // blocks rbase .. rbase + 2 MT - 1; those beyond RB repeat the last one
+  const int rbase = 2 * MT * (blockIdx.x / p.ct);      // blocks rbase .. rbase + 2 MT - 1; those beyond RB repeat the last one
                                                        // (computed again, not stored)
   const long long total_chunks = (long long)p.B * p.chunks_per_b;
   const long long c_begin = (long long)blockIdx.z * p.chunks_per_split;
@@ -85,7 +86,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
 
   if (warp == 4) {
     if (lane == 0) {
-      const uint32_t idesc = instr_desc_16(128, D, 1, 1);  // both operands MN-major
+      const uint32_t idesc = instr_desc_16(128, DW, 1, 1);  // both operands MN-major
       constexpr uint32_t HI = desc_hi(1024, true);
       constexpr uint32_t LBO = (DT_BLK >> 4) << 16;          // 64-wide blocks of m / n follow each other at 8 KB
       const void* tmw = &tm_dwx;
@@ -106,7 +107,10 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
           if (p.cell == CELL_GRU && g == 0) tma_load_5d(dst + i * DT_BLK, tmg, d0, n, t0, b, 0, &full[s]);
           else tma_load_5d(dst + i * DT_BLK, tmw, d0, n, (p.cell == CELL_GRU) ? g - 1 : g, t0, b, &full[s]);
         }
-        for (int pb = 0; pb < nb; ++pb) tma_load_5d(dst + (2 * MT + pb) * DT_BLK, tmh, pb * 64, n, t0 - 1, b, 0, &full[s]);
+        for (int pb = 0; pb < nbw; ++pb) {
+          const int cb = ctile * nbw + pb < nb ? ctile * nbw + pb : nb - 1;
+          tma_load_5d(dst + (2 * MT + pb) * DT_BLK, tmh, cb * 64, n, t0 - 1, b, 0, &full[s]);
+        }
         ++loads;
       };
       for (int ci = 0; ci < nchunks && ci < NS; ++ci) load(ci);
@@ -118,7 +122,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
         seen = ci + 1;
         const uint32_t s_lo = ((base + (uint32_t)s * stage_bytes) >> 4) | LBO, b_lo = s_lo + (uint32_t)MT * ((2 * DT_BLK) >> 4);
         for (int mt = 0; mt < MT; ++mt) {
-          const uint32_t a_lo = s_lo + (uint32_t)mt * ((2 * DT_BLK) >> 4), acc = tmem + (uint32_t)(mt * D);
+          const uint32_t a_lo = s_lo + (uint32_t)mt * ((2 * DT_BLK) >> 4), acc = tmem + (uint32_t)(mt * DW);
 #pragma unroll
           for (uint32_t ks = 0; ks < DT_KC / 16; ++ks)  // 16 rows of a block = 2048 bytes per k-step
             umma_parts(acc, a_lo + 128 * ks, HI, b_lo + 128 * ks, HI, idesc, (ci > 0 || ks > 0) ? 1u : 0u);
@@ -158,10 +162,11 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
     const elem_t* d0src = from_dg0 ? p.dg0 + (size_t)n * D + d
                                           : p.dWx + (size_t)((p.cell == CELL_GRU) ? g - 1 : g) * ND + (size_t)n * D + d;
     const size_t d0stride = (from_dg0 ? (size_t)1 : (size_t)p.Gw) * ND * T;  // elements between batch rows at t = 0
-    for (int col0 = 0; col0 < D; col0 += 32) {
+    for (int cw = 0; cw < DW; cw += 32) {
       uint32_t r[32];
-      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * D + col0), r);
-      if (!row_ok) continue;
+      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * DW + cw), r);
+      const int col0 = ctile * DW + cw;
+      if (!row_ok || col0 >= D) continue;
       float v[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
@@ -195,7 +200,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
 
 }  // namespace
 
-bool recurrent_grad_tma_supported(int D, int state_f32) { return !state_f32 && D >= 64 && D <= 256 && D % 64 == 0; }
+bool recurrent_grad_tma_supported(int D, int state_f32) { return !state_f32 && D >= 64 && D % 64 == 0; }
 
 cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int Gr, int Gw, const void* dWx, const void* dg0,
                                       const void* states, const void* s0, float* dR, unsigned* status, int sm_count,
@@ -226,34 +231,36 @@ cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int 
   p.chunks_per_b = (T + DT_KC - 1) / DT_KC;
   // tiles of 128 rows per CTA: as many as share one fetch of h, within 512 tensor-memory columns and a ring of at least
   // three stages in shared memory
-  const int nb = D / 64, tiles = (Gr * nb + 1) / 2;
-  int mt = 512 / D;
+  const int nb = D / 64, tiles = (Gr * nb + 1) / 2, ct = (nb + 3) / 4, nbw = (nb + ct - 1) / ct, DW = nbw * 64;
+  int mt = 512 / DW;
   if (mt > 3) mt = 3;
   if (mt > tiles) mt = tiles;
-  while (mt > 1 && 3 * (size_t)(2 * mt + nb) * DT_BLK > (size_t)200 * 1024) --mt;
+  while (mt > 1 && 3 * (size_t)(2 * mt + nbw) * DT_BLK > (size_t)200 * 1024) --mt;
   mt = (tiles + (tiles + mt - 1) / mt - 1) / ((tiles + mt - 1) / mt);  // same number of CTAs, evenly filled
 #ifdef FRNN_DR_ONE_TILE  // development aid: one tile per CTA
   mt = 1;
 #endif
   p.mt = mt;
-  int stages = (int)(((size_t)200 * 1024) / ((size_t)(2 * mt + nb) * DT_BLK));
+  p.ct = ct;
+  p.nbw = nbw;
+  int stages = (int)(((size_t)200 * 1024) / ((size_t)(2 * mt + nbw) * DT_BLK));
   p.stages = stages > DT_STAGES ? DT_STAGES : stages;
   int cols = 32;
-  while (cols < mt * D) cols *= 2;
+  while (cols < mt * DW) cols *= 2;
   p.tmem_cols = cols;
   const int mtiles = (tiles + mt - 1) / mt;
   const long long chunks = (long long)B * p.chunks_per_b;
-  const long long base_ctas = (long long)mtiles * N;
+  const long long base_ctas = (long long)mtiles * ct * N;
   long long splits = sm_count / base_ctas;  // one CTA per SM (shared memory): stay within a single wave
   if (splits > (chunks + 3) / 4) splits = (chunks + 3) / 4;  // at least 4 chunks per split
   if (splits < 1) splits = 1;
   if (splits > 65535) splits = 65535;
   p.chunks_per_split = (int)((chunks + splits - 1) / splits);
   splits = (chunks + p.chunks_per_split - 1) / p.chunks_per_split;
-  const size_t smem = (size_t)p.stages * (2 * mt + nb) * DT_BLK + 8 * (2 * DT_STAGES + 1) + 16 + 1024;
+  const size_t smem = (size_t)p.stages * (2 * mt + nbw) * DT_BLK + 8 * (2 * DT_STAGES + 1) + 16 + 1024;
   cudaError_t e = cudaFuncSetAttribute(recurrent_grad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);  // fixed maximum, so that concurrent host threads never lower each other's setting
   if (e != cudaSuccess) return e;
-  recurrent_grad_tma_kernel<<<dim3((unsigned)mtiles, (unsigned)N, (unsigned)splits), DT_THREADS, smem, stream>>>(tm_dwx, tm_dg0,
+  recurrent_grad_tma_kernel<<<dim3((unsigned)(mtiles * ct), (unsigned)N, (unsigned)splits), DT_THREADS, smem, stream>>>(tm_dwx, tm_dg0,
                                                                                                                  tm_st, p);
   return cudaGetLastError();
 }
