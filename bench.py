@@ -53,10 +53,10 @@ WORKLOADS = {
 }
 DIMS = {"lstm": (4, 4, 4, 2), "gru": (3, 3, 4, 1), "elman": (1, 1, 1, 1), "slstm": (4, 4, 4, 4)}
 METRIC = "fwd+bwd tokens/sec (B*T/s)"
-# DRAM bytes (read + write) of ONE launch of the reverse time loop, from an `ncu --set full` capture of
-# `python bench.py --steps 2 --warmup 1 --no-cpu` on a B200; reported with its provenance, for the kernel build named.
-NCU_TRAFFIC = {"C2": {"bytes": 237_750_016 + 105_541_632, "source": "ncu --set full capture of frnn_bwd_kernel<lstm,KT16,NT1,MPW2> on this "
-                      "command line with --steps 1 --min-seconds 0, 2026-11-25 (the kernel has not changed since)"}}
+# DRAM bytes (read + write) of ONE launch of the reverse time loop, from an ncu capture (SpeedOfLight, MemoryWorkloadAnalysis) of
+# `python bench.py --workload C2 --steps 1 --warmup 3 --min-seconds 0 --no-cpu` on a B200; reported with its provenance.
+NCU_TRAFFIC = {"C2": {"bytes": 344_170_000, "source": "ncu capture of lane_bwd_kernel<lstm,KT16,U32,NT1> on this command line with --steps 1 "
+                      "--min-seconds 0, 2026-12-02: 472.6 GB/s for 728.3 us"}}
 # fwd+bwd of the reference's own CUDA backend on a B200 of this pool, measured by `bench.py --impl reference_gpu`
 # (tokens/s; None: not measured).  The live arm is the source of truth; this record lets the default line carry the ratio.
 REFERENCE_GPU_RECORD = {
@@ -458,7 +458,7 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
         "tile": {"cluster_size": plan.cluster_size, "units_per_cta": plan.units_per_cta, "batch_tile": plan.batch_tile, "threads": plan.threads,
                  "wide_forward": int(plan.wide_forward)},  # 1: forward loop on the 128-row tcgen05 kernel (LSTM, head dim 64)
         "roofline": {
-            "bound": "hbm", "kernel": "wide_bwd_elman_kernel (reverse time loop, dR and db inside)" if wide else "frnn_bwd_kernel (reverse time loop)",
+            "bound": "hbm", "kernel": "wide_bwd_elman_kernel (reverse time loop, dR and db inside)" if wide else "x32l_bwd_kernel (reverse time loop)" if job.f32io else "lane_bwd_kernel (reverse time loop)",
             "achieved": achieved, "peak": job.hbm_peak, "unit": "GB/s", "frac": achieved / job.hbm_peak, "peak_source": job.peak_source,
             "traffic": None, "traffic_source": None, "algorithmic_bytes_per_launch": bwd_bytes,
             "forward_loop": {"achieved": fwd_bytes / (fwd_ms * 1e-3) / 1e9, "frac": fwd_bytes / (fwd_ms * 1e-3) / 1e9 / job.hbm_peak,
@@ -470,7 +470,7 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
             "chain_floor": chain,
             "note": "streams one 16 KB tile per operand, step and CTA; HBM-bound" if wide else
                     "the serial chain of 2T dependent steps (chain_floor), not HBM or the tensor pipe, bounds this workload"},
-        "clocks": clk.summary(), "launches_per_step": 3 if wide else 6,
+        "clocks": clk.summary(), "launches_per_step": 3 if wide or job.f32io else 6 if D > 256 else 5,  # pack of R (head dims above 256), loops, R^T, dR, cast
     }
     if keep is not None:
         keep.update(Wx=Wx, R=R, b=b, s0=s0, gcnt=gcnt)
