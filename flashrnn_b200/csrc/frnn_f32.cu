@@ -779,6 +779,13 @@ __global__ void __launch_bounds__(XTHREADS) x32_dr_kernel(const XDrParams p) {
   }
 }
 
+// dR and db, side by side in the workspace, to the caller's tensors in one launch
+__global__ void copy_grads_kernel(const float4* __restrict__ src, float4* __restrict__ dR, float4* __restrict__ db, size_t nR, size_t total) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nR) dR[i] = src[i];
+  else if (i < total) db[i - nR] = src[i];
+}
+
 struct Dims { int Gr, Gw, Gt, S, GC; };
 bool dims_of(int cell, float fclip, Dims* d) {
   switch (cell) {
@@ -790,17 +797,6 @@ bool dims_of(int cell, float fclip, Dims* d) {
   return false;
 }
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
-struct Ws { size_t rt, grads, dg0, total; };
-Ws ws_layout(const frnn_problem& pr, const Dims& d) {
-  Ws w;
-  size_t off = kStatus;
-  w.rt = off; off = up256(off + (size_t)d.Gr * pr.N * pr.D * pr.D * 4);
-  w.grads = off; off = up256(off + ((size_t)d.Gr * pr.N * pr.D * pr.D + (size_t)d.Gt * pr.N * pr.D) * 4);
-  w.dg0 = off;
-  if (pr.cell == CELL_GRU) off = up256(off + (size_t)pr.B * pr.T * pr.N * pr.D * 4);
-  w.total = off;
-  return w;
-}
 size_t fwd_smem(const frnn_problem& pr, const Dims& d, bool r_in) {
   return ((size_t)XBT * pr.D + (size_t)XBT * d.Gr * pr.D + (r_in ? (size_t)pr.D * d.Gr * pr.D : 0)) * 4;
 }
@@ -881,6 +877,20 @@ bool lane_tile(const frnn_problem& pr, bool bwd, int* cs_out, XLane* k) {
   if (!k->fn) *k = loop(cell, pr.D, pr.D / cs, bt / 2);
   *cs_out = cs;
   return k->fn != nullptr && (pr.B + k->bt - 1) / k->bt <= 65535;
+}
+struct Ws { size_t rt, grads, dg0, total; };
+Ws ws_layout(const frnn_problem& pr, const Dims& d) {
+  Ws w;
+  size_t off = kStatus;
+  int cs;
+  XLane lane;
+  w.rt = off;  // (the lane loops read R as it is)
+  if (!lane_tile(pr, false, &cs, &lane)) off = up256(off + (size_t)d.Gr * pr.N * pr.D * pr.D * 4);
+  w.grads = off; off = up256(off + ((size_t)d.Gr * pr.N * pr.D * pr.D + (size_t)d.Gt * pr.N * pr.D) * 4);
+  w.dg0 = off;
+  if (pr.cell == CELL_GRU) off = up256(off + (size_t)pr.B * pr.T * pr.N * pr.D * 4);
+  w.total = off;
+  return w;
 }
 int validate(const frnn_problem* pr, Dims* d) {
   if (!pr) return FRNN_ERR_NULL;
@@ -1104,9 +1114,12 @@ __attribute__((visibility("hidden"))) int frnn_backward_parts_f32(const frnn_pla
   const size_t nR = (size_t)d.Gr * pr.N * pr.D * pr.D, nb = (size_t)d.Gt * pr.N * pr.D;
   cudaError_t e = cudaSuccess;
   if (parts & FRNN_PART_LOOP) {
-    e = cudaMemsetAsync(ws, 0, kStatus, stream);
-    if (e != cudaSuccess) return (int)e;
-    e = cudaMemsetAsync(grads, 0, (nR + nb) * sizeof(float), stream);
+    if (w.grads == kStatus) {  // one stretch of memory
+      e = cudaMemsetAsync(ws, 0, kStatus + (nR + nb) * sizeof(float), stream);
+    } else {
+      e = cudaMemsetAsync(ws, 0, kStatus, stream);
+      if (e == cudaSuccess) e = cudaMemsetAsync(grads, 0, (nR + nb) * sizeof(float), stream);
+    }
     if (e != cudaSuccess) return (int)e;
     XParams p = {};
     p.R = static_cast<const float*>(a->R); p.s0 = static_cast<const float*>(a->s0);
@@ -1186,9 +1199,14 @@ __attribute__((visibility("hidden"))) int frnn_finalize_grads_f32(const frnn_pla
   const frnn_problem& pr = plan->prob;
   const size_t nR = (size_t)d.Gr * pr.N * pr.D * pr.D, nb = (size_t)d.Gt * pr.N * pr.D;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  cudaError_t e = cudaMemcpyAsync(dR, grads_f32, nR * 4, cudaMemcpyDeviceToDevice, stream);
-  if (e != cudaSuccess) return (int)e;
-  return (int)cudaMemcpyAsync(db, static_cast<const float*>(grads_f32) + nR, nb * 4, cudaMemcpyDeviceToDevice, stream);
+  if (!aligned16(grads_f32) || !aligned16(dR) || !aligned16(db)) {
+    const cudaError_t e = cudaMemcpyAsync(dR, grads_f32, nR * 4, cudaMemcpyDeviceToDevice, stream);
+    return (int)(e != cudaSuccess ? e : cudaMemcpyAsync(db, static_cast<const float*>(grads_f32) + nR, nb * 4, cudaMemcpyDeviceToDevice, stream));
+  }
+  const size_t quads = (nR + nb) / 4;  // (both are multiples of 4: head dims are)
+  copy_grads_kernel<<<(unsigned)((quads + 255) / 256), 256, 0, stream>>>(static_cast<const float4*>(grads_f32), static_cast<float4*>(dR), static_cast<float4*>(db),
+                                                                         nR / 4, quads);
+  return (int)cudaGetLastError();
 }
 
 }  // extern "C"
