@@ -66,9 +66,31 @@ constexpr size_t kMaxDynSmem = 227 * 1024;
 constexpr size_t kStatusBytes = 256;
 
 // Head dims above 256 have kernels of their own (frnn_big_*.cuh).  Their plan names 64 units per CTA and clusters of D / 64; the
-// loops split the head further where they can (big_units).
+// loops split the head as big_tile says.
 static bool is_big(const frnn_problem& pr) { return pr.D > 256; }
 constexpr int kBigPlanUnits = 64;
+
+// Units per CTA and rows / 8 of those loops: the fewest turns of all clusters through the GPU (as many as a B200 keeps resident, by size), weighed
+// with what a step of both loops takes.  Measured, 8 / 16 rows, clk: LSTM D = 384 with 32 units 3750 / 5850, 48 units 5120 / 9480, 64 units
+// 8000 / 15380; D = 512 32 units 4230 / 7080, 64 units 8950 / 17350; D = 768 48 units 8710 / 17820, 64 units 15330 / 25490; Elman D = 512 32 units
+// 3590 / 5960, 64 units 3890 / 6350.  (32 units whatever the batch: GRU B23 T227 N5 D384 1.37 ms against 1.07 with fewer CTAs per head.)
+struct BigTile { int u, nt; };
+static BigTile big_tile(const frnn_problem& pr) {
+  static const int resident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 12, 11, 10, 9, 8, 7, 7, 7};
+  BigTile best = {64, 1};
+  long long best_cost = -1;
+  const int units[3] = {32, 48, 64}, gates[3][2] = {{100, 160}, {140, 270}, {230, 400}}, elman[3][2] = {{90, 132}, {90, 146}, {100, 160}};
+  const auto& weight = pr.cell == CELL_ELMAN ? elman : gates;
+  for (int i = 0; i < 3; ++i) {
+    const int u = units[i], cs = pr.D / u;
+    if (pr.D % u || cs > 16 || pr.D / 16 > u) continue;
+    for (int nt = 1; nt <= (pr.B > 8 ? 2 : 1); ++nt) {
+      const long long tiles = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N, cost = (tiles + resident[cs] - 1) / resident[cs] * weight[i][nt - 1];
+      if (best_cost < 0 || cost < best_cost) { best = {u, nt}; best_cost = cost; }
+    }
+  }
+  return best;
+}
 
 // Scratch of a plan: status block, then what the plan's kernels need.  Only head dims above 256 repack R for the forward pass.
 struct WsLayout { size_t rpack_fwd, rpack_bwd, grads, dg0, total; };
@@ -76,7 +98,7 @@ static WsLayout workspace_layout(const frnn_problem& pr, const CellDims& cd, int
   WsLayout w;
   size_t off = kStatusBytes;
   w.rpack_fwd = off; if (is_big(pr)) off = align_up(off + (size_t)(cd.Gr > 1 ? 4 : 1) * pr.N * pr.D * pr.D * 2, 256);
-  w.rpack_bwd = off; if (pr.training) off = align_up(off + rt_pack_bytes(cd.Gr, pr.N, pr.D, is_big(pr) ? big_units(pr.D) : units), 256);
+  w.rpack_bwd = off; if (pr.training) off = align_up(off + rt_pack_bytes(cd.Gr, pr.N, pr.D, is_big(pr) ? big_tile(pr).u : units), 256);
   w.grads = off; if (pr.training) off = align_up(off + ((size_t)cd.Gr * pr.N * pr.D * pr.D + (size_t)cd.Gt * pr.N * pr.D) * 4, 256);
   w.dg0 = off;
   if (pr.training && pr.cell == CELL_GRU) off = align_up(off + (size_t)pr.B * pr.T * pr.N * pr.D * 2, 256);
@@ -294,12 +316,10 @@ static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int cs,
   void* args[1] = {const_cast<LoopParams*>(&lp)};
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
-// 16-row tiles when 8-row ones would be more clusters than run at once (a B200 holds seven clusters of 16 CTAs)
-static int big_nt(const frnn_problem& pr) { return pr.B > 8 && (long long)((pr.B + 7) / 8) * pr.N * (pr.D / big_units(pr.D)) > 112 ? 2 : 1; }
 static int launch_big(const frnn_plan& pl, bool bwd, LoopParams lp, cudaStream_t stream) {
   const frnn_problem& pr = pl.prob;
-  const int u = big_units(pr.D);
-  int nt = big_nt(pr);
+  const int u = big_tile(pr).u;
+  int nt = big_tile(pr).nt;
   BigKernel k = big_kernel(kernel_cell(pr), bwd, u, nt);
   if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(kernel_cell(pr), bwd, u, nt = 1);  // (sLSTM reverse from head dim 896 up)
   if (!k.fn || pl.probe_noop_cell) return FRNN_ERR_PLAN;
@@ -487,7 +507,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   cudaError_t e = cudaSuccess;
   if ((parts & FRNN_PART_LOOP) && !is_wide(*plan)) {
     const bool big = is_big(pr);
-    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, big ? big_units(pr.D) : plan->units_per_cta, big, grads, nR + nb,
+    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, big ? big_tile(pr).u : plan->units_per_cta, big, grads, nR + nb,
                            reinterpret_cast<unsigned*>(ws), stream);
     if (e != cudaSuccess) return (int)e;
   } else if (parts & FRNN_PART_LOOP) {

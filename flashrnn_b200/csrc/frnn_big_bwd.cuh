@@ -19,7 +19,7 @@ struct BigBwdGeom {
   static constexpr int WC = U / 8, W = 2 * WC, IOT = 32 * (W - WC), TH = 32 * W;  // warps of the cell, of the products; the others move the data
   static constexpr int NB = NT;
   static constexpr int K = C::Gr * U, KP = (K + 31) / 32;
-  static constexpr int MT = 4;  // p tiles per warp, at most: big_units keeps D / 16 <= 4 W
+  static constexpr int MT = 4;  // p tiles per warp, at most: D / 16 <= 4 W
   static constexpr int GCM = CacheGeom<C::GC>::MAIN;
   static constexpr bool GCX = CacheGeom<C::GC>::EXTRA;
   static constexpr int NSS = C::NNEED + C::NEXT;

@@ -1,6 +1,6 @@
 // Forward time loop for head dims above 256 (multiples of 64 up to kBigMaxD), where R does not fit the registers of a cluster:
 // the lane loop of frnn_lane_fwd.cuh with
-//   * up to 16 CTAs of U = 32, 48 or 64 units per head (big_units): as many SMs as a cluster can have, so that R -- 4.7 MB at
+//   * up to 16 CTAs of U = 32, 48 or 64 units per head (big_tile in frnn_api.cu): with few heads and rows as many SMs as a cluster can have, so that R -- 4.7 MB at
 //     head dim 768 -- lies in their registers (KRP k-pairs per warp) and shared memory (the rest of it) for all T steps; only what
 //     fits neither is re-read from L2 in every step (head dims 640 and 704, and 832 up, of the cells with three or four gates);
 //   * two warps per 8-unit group that split k; the second hands its sums to the first through shared memory (one named

@@ -357,9 +357,7 @@ __device__ __forceinline__ void store_state2(void* base, size_t elem_off, int f3
 
 // ------------------------------------------------------------------------------------------------ geometry
 constexpr size_t kSmemBudget = 227 * 1024;
-// Head dims above 256 (multiples of 64 up to kBigMaxD).  Units per CTA: the smallest of 32, 48, 64 that divides the head dim into at
-// most 16 CTAs.
+// Head dims above 256: multiples of 64 up to this
 constexpr int kBigMaxD = 1024;
-__host__ __device__ constexpr int big_units(int D) { return D % 32 == 0 && D / 32 <= 16 ? 32 : (D % 48 == 0 && D / 48 <= 16 ? 48 : 64); }
 
 }  // namespace FRNN_NS
