@@ -76,7 +76,7 @@ constexpr int kBigPlanUnits = 64;
 // 3590 / 5960, 64 units 3890 / 6350.  (32 units whatever the batch: GRU B23 T227 N5 D384 1.37 ms against 1.07 with fewer CTAs per head.)
 struct BigTile { int u, nt; };
 static BigTile big_tile(const frnn_problem& pr) {
-  static const int resident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 12, 11, 10, 9, 8, 7, 7, 7};
+  static const int resident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 12, 11, 8, 8, 8, 8, 7, 7};
   BigTile best = {64, 1};
   long long best_cost = -1;
   const int units[3] = {32, 48, 64}, gates[3][2] = {{100, 160}, {140, 270}, {230, 400}}, elman[3][2] = {{90, 132}, {90, 146}, {100, 160}};
