@@ -18,12 +18,13 @@ LIB_PATH = Path(os.environ.get("FRNN_B200_LIB") or PKG / "libfrnn_b200.so")
 
 ABI_VERSION = 3
 NOALLOC_MAX_SCRATCH_BYTES = 8 << 20  # FRNN_NOALLOC_MAX_SCRATCH_BYTES
+LOOPS = ("lane", "big", "wide", "f32_lane", "f32_cluster", "f32_stream")  # FRNN_LOOP_*
 CELL_IDS = {"lstm": 0, "gru": 1, "elman": 2, "slstm": 3}
 DTYPE_BF16, DTYPE_F32, DTYPE_F16 = 0, 1, 2
 
 # every symbol include/frnn.h declares
 EXPORTS = (
-    "frnn_abi_version", "frnn_query", "frnn_query_tile", "frnn_forward", "frnn_backward", "frnn_backward_parts",
+    "frnn_abi_version", "frnn_query", "frnn_query_tile", "frnn_query_loop", "frnn_forward", "frnn_backward", "frnn_backward_parts",
     "frnn_forward_noalloc",
     "frnn_finalize_grads", "frnn_read_device_status", "frnn_status_string",
 )
@@ -48,6 +49,11 @@ class FrnnPlan(ctypes.Structure):
         ("cache_bytes", ctypes.c_uint64), ("workspace_bytes", ctypes.c_uint64), ("grads_offset", ctypes.c_uint64),
         ("grads_count", ctypes.c_uint64),
     ]
+
+
+class FrnnLoopShape(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int32) for n in ("loop", "cluster_size", "units_per_cta", "batch_rows", "threads", "input_stages")] + \
+               [("grid", ctypes.c_uint32 * 3), ("launches", ctypes.c_int32)]
 
 
 class FrnnFwdArgs(ctypes.Structure):
@@ -101,6 +107,7 @@ def lib() -> ctypes.CDLL:
         L.frnn_query.argtypes = [ctypes.POINTER(FrnnProblem), ctypes.POINTER(FrnnPlan)]
         L.frnn_query_tile.argtypes = [ctypes.POINTER(FrnnProblem), ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                       ctypes.POINTER(FrnnPlan)]
+        L.frnn_query_loop.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.c_int, ctypes.POINTER(FrnnLoopShape)]
         L.frnn_forward.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.POINTER(FrnnFwdArgs), ctypes.c_void_p]
         L.frnn_backward.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.POINTER(FrnnBwdArgs), ctypes.c_void_p]
         L.frnn_backward_parts.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.POINTER(FrnnBwdArgs), ctypes.c_void_p, ctypes.c_int]
@@ -112,7 +119,7 @@ def lib() -> ctypes.CDLL:
         L.frnn_read_device_status.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(FrnnDevStatus)]
         L.frnn_status_string.argtypes = [ctypes.c_int]
         L.frnn_status_string.restype = ctypes.c_char_p
-        for fn in ("frnn_query", "frnn_query_tile", "frnn_forward", "frnn_backward", "frnn_finalize_grads",
+        for fn in ("frnn_query", "frnn_query_tile", "frnn_query_loop", "frnn_forward", "frnn_backward", "frnn_finalize_grads",
                    "frnn_read_device_status"):
             getattr(L, fn).restype = ctypes.c_int
         if L.frnn_abi_version() != ABI_VERSION:
@@ -180,3 +187,10 @@ def query(problem: FrnnProblem, cluster_size: int = 0, batch_tile: int = 0) -> F
     else:
         check("frnn_query", lib().frnn_query(ctypes.byref(problem), ctypes.byref(plan)))
     return plan
+
+
+def query_loop(plan: FrnnPlan, backward: bool) -> FrnnLoopShape:
+    """The launch of the plan's forward or reverse time loop."""
+    shape = FrnnLoopShape()
+    check("frnn_query_loop", lib().frnn_query_loop(ctypes.byref(plan), int(backward), ctypes.byref(shape)))
+    return shape

@@ -116,6 +116,8 @@ static bool is_wide(const frnn_plan& pl) { return pl.batch_tile == kWideBatchTil
 static bool wide_gates_problem(const frnn_problem& pr) {
   return wide_gates_forward_supported(pr.cell, pr.D, pr.dtype_state == FRNN_DTYPE_F32);
 }
+// (a training pass stores activations, where the lane loop is ahead: see frnn_wide.cu)
+static bool runs_wide_gates(const frnn_plan& pl) { return pl.wide_forward && !pl.prob.training; }
 static int plan_threads(const CellDims& cd, int units, int bt) { return bt == kWideBatchTile ? kWideThreads : 2 * cd.Gr * units; }
 
 // Rows / 8 the lane loops run a plan's batch tile with (the activation cache and every result are the same whatever it is).
@@ -282,28 +284,64 @@ static bool resolve_strides(const int64_t (&in)[4], const long long (&dense)[4],
   return true;
 }
 
+// The kernel a time loop of a plan runs, with its CTAs.  fn null: there is none (a measurement variant of another tile).
+struct LoopLaunch {
+  const void* fn;
+  int threads, stages;
+  size_t smem;
+  int cs, u, rows;
+};
+static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
+  const frnn_problem& pr = pl.prob;
+  const int cell = kernel_cell(pr);
+  if (is_big(pr)) {
+    const BigTile t = big_tile(pr);
+    int nt = t.nt;
+    BigKernel k = big_kernel(cell, bwd, t.u, nt);
+    if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(cell, bwd, t.u, nt = 1);  // (sLSTM reverse from head dim 896 up)
+    if (!k.fn || pl.probe_noop_cell) return LoopLaunch{};
+    return LoopLaunch{k.fn, k.threads, bwd ? kBigStages - 1 : kBigStages, k.smem(pr.D), pr.D / t.u, t.u, 8 * nt};
+  }
+  const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.cluster_size, pl.batch_tile);
+  const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(cell, bwd, kt, u, nt) : bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
+  return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt};
+}
+// One CTA per head and tile: x: tiles of the batch.  Clusters: x: the CTAs of one, y: tiles, which end at 65535 blocks; the 8-row tiles of a
+// batch that a plan of 16 or 32 rows takes can be more, and such a batch goes in several launches.  z: heads.  (All tiles in x, a cluster
+// after the other, or a first tile added to blockIdx.y for single CTAs too: the compiler then gives the loops other registers, sLSTM D = 192
+// training 5.03 -> 5.16 ms, LSTM D = 64 inference 427 -> 470 us.)
+constexpr int kMaxTiles = 65535;
+static int loop_tiles(const LoopLaunch& k, const frnn_problem& pr) { return (pr.B + k.rows - 1) / k.rows; }
+static dim3 loop_grid(const LoopLaunch& k, const frnn_problem& pr, int first_tile) {
+  const int left = loop_tiles(k, pr) - first_tile;
+  return k.cs == 1 ? dim3((unsigned)left, 1, (unsigned)pr.N) : dim3((unsigned)k.cs, (unsigned)(left < kMaxTiles ? left : kMaxTiles), (unsigned)pr.N);
+}
+static int loop_launches(const LoopLaunch& k, const frnn_problem& pr) { return k.cs == 1 ? 1 : (loop_tiles(k, pr) + kMaxTiles - 1) / kMaxTiles; }
+
 // `overlap`: a decoding step behind another may start, and read R, while that one still runs (everything else waits for it on the device):
 // launch and prologue, about half of a one-token step, disappear behind the step before
-static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int cs, int rows, const frnn_plan& pl, const LoopParams& lp, bool overlap,
-                               cudaStream_t stream) {
+static int launch_loop(const frnn_plan& pl, bool bwd, LoopParams lp, cudaStream_t stream) {
+  const LoopLaunch k = loop_of(pl, bwd);
+  if (!k.fn) return FRNN_ERR_PLAN;
+  const bool overlap = !bwd && pl.keep_packed_r;
+  lp.CS = k.cs;
   // always the fixed maximum, never this plan's own size: the attribute belongs to the kernel, not to the launch, and a
   // second host thread launching the same instantiation with a larger tile must not find it lowered in between
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
-  if (e != cudaSuccess) return e;
-  if (cs > 8) {  // clusters of more than 8 CTAs are a non-portable size: opt in
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
+  cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+  if (e != cudaSuccess) return (int)e;
+  if (k.cs > 8) {  // clusters of more than 8 CTAs are a non-portable size: opt in
+    e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return (int)e;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)cs, (unsigned)((pl.prob.B + rows - 1) / rows), (unsigned)pl.prob.N);
-  cfg.blockDim = dim3((unsigned)threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
+  cfg.blockDim = dim3((unsigned)k.threads, 1, 1);
+  cfg.dynamicSmemBytes = k.smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   unsigned na = 0;
-  if (cs > 1) {
+  if (k.cs > 1) {
     attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = (unsigned)cs;
+    attr[na].val.clusterDim.x = (unsigned)k.cs;
     attr[na].val.clusterDim.y = 1;
     attr[na++].val.clusterDim.z = 1;
   }
@@ -313,26 +351,14 @@ static cudaError_t launch_loop(const void* fn, int threads, size_t smem, int cs,
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  void* args[1] = {const_cast<LoopParams*>(&lp)};
-  return cudaLaunchKernelExC(&cfg, fn, args);
-}
-static int launch_big(const frnn_plan& pl, bool bwd, LoopParams lp, cudaStream_t stream) {
-  const frnn_problem& pr = pl.prob;
-  const int u = big_tile(pr).u;
-  int nt = big_tile(pr).nt;
-  BigKernel k = big_kernel(kernel_cell(pr), bwd, u, nt);
-  if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(kernel_cell(pr), bwd, u, nt = 1);  // (sLSTM reverse from head dim 896 up)
-  if (!k.fn || pl.probe_noop_cell) return FRNN_ERR_PLAN;
-  lp.CS = pr.D / u;
-  return (int)launch_loop(k.fn, k.threads, k.smem(pr.D), lp.CS, 8 * nt, pl, lp, !bwd && pl.keep_packed_r, stream);
-}
-static int launch_lane(const frnn_plan& pl, bool bwd, const LoopParams& lp, cudaStream_t stream) {
-  const frnn_problem& pr = pl.prob;
-  const int kt = pr.D / 16, nt = lane_nt(pr, bwd, pl.cluster_size, pl.batch_tile);
-  const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(kernel_cell(pr), bwd, kt, pl.units_per_cta, nt)
-                       : bwd              ? lane_bwd_floor(pr.cell, kt, pl.units_per_cta, nt)
-                                          : lane_fwd_floor(pr.cell, kt, pl.units_per_cta, nt);
-  return k.fn ? (int)launch_loop(k.fn, k.threads, k.smem, pl.cluster_size, 8 * nt, pl, lp, !bwd && pl.keep_packed_r, stream) : FRNN_ERR_PLAN;
+  void* args[1] = {&lp};
+  for (int i = 0; i < loop_launches(k, pl.prob) && e == cudaSuccess; ++i) {
+    cfg.gridDim = loop_grid(k, pl.prob, i * kMaxTiles);
+    lp.tile0 = (unsigned)(i * kMaxTiles);
+    e = cudaLaunchKernelExC(&cfg, k.fn, args);
+    lp.clear_status = 0;
+  }
+  return (int)e;
 }
 
 static int sm_count_cached() {
@@ -365,6 +391,7 @@ using namespace FRNN_NS;
 extern "C" {
 int frnn_query_f16(const frnn_problem*, frnn_plan*);
 int frnn_query_tile_f16(const frnn_problem*, int, int, int, frnn_plan*);
+int frnn_query_loop_f16(const frnn_plan*, int, frnn_loop_shape*);
 int frnn_forward_f16(const frnn_plan*, const frnn_fwd_args*, void*);
 int frnn_backward_parts_f16(const frnn_plan*, const frnn_bwd_args*, void*, int);
 int frnn_finalize_grads_f16(const frnn_plan*, const void*, void*, void*, void*);
@@ -378,6 +405,7 @@ int frnn_finalize_grads_f16(const frnn_plan*, const void*, void*, void*, void*);
   if (is_f32) return call
 extern "C" {
 int frnn_query_f32(const frnn_problem*, int, int, int, frnn_plan*);
+int frnn_query_loop_f32(const frnn_plan*, int, frnn_loop_shape*);
 int frnn_forward_f32(const frnn_plan*, const frnn_fwd_args*, void*);
 int frnn_backward_parts_f32(const frnn_plan*, const frnn_bwd_args*, void*, int);
 int frnn_finalize_grads_f32(const frnn_plan*, const void*, void*, void*, void*);
@@ -406,6 +434,28 @@ int FRNN_ENTRY(frnn_query_tile)(const frnn_problem* problem, int cluster_size, i
   return fill_plan(problem, cluster_size, batch_tile, wx_stages, out);
 }
 
+int FRNN_ENTRY(frnn_query_loop)(const frnn_plan* plan, int backward, frnn_loop_shape* out) {
+  FRNN_FORWARD_F32(wants_f32(plan), frnn_query_loop_f32(plan, backward, out));
+  FRNN_FORWARD_F16(wants_f16(plan), frnn_query_loop_f16(plan, backward, out));
+  CellDims cd;
+  const int rc = check_plan(plan, &cd);
+  if (rc) return rc;
+  if (!out) return FRNN_ERR_NULL;
+  const frnn_problem& pr = plan->prob;
+  if (backward && !pr.training) return FRNN_ERR_TRAINING;
+  if (is_wide(*plan) || (!backward && runs_wide_gates(*plan))) {
+    const uint32_t tiles = (uint32_t)((pr.B + kWideBatchTile - 1) / kWideBatchTile);
+    *out = {FRNN_LOOP_WIDE, 1, pr.D, kWideBatchTile, is_wide(*plan) ? kWideThreads : kWideGatesThreads,
+            !is_wide(*plan) ? kWideGatesStages : backward ? kWideBwdStages : kWideFwdStages, {tiles, (uint32_t)pr.N, 1}, 1};
+    return FRNN_OK;
+  }
+  const LoopLaunch k = loop_of(*plan, backward != 0);
+  if (!k.fn) return FRNN_ERR_PLAN;
+  const dim3 g = loop_grid(k, pr, 0);
+  *out = {is_big(pr) ? FRNN_LOOP_BIG : FRNN_LOOP_LANE, k.cs, k.u, k.rows, k.threads, k.stages, {g.x, g.y, g.z}, loop_launches(k, pr)};
+  return FRNN_OK;
+}
+
 int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void* stream_) {
   FRNN_FORWARD_F32(wants_f32(plan), frnn_forward_f32(plan, a, stream_));
   FRNN_FORWARD_F16(wants_f16(plan), frnn_forward_f16(plan, a, stream_));
@@ -426,8 +476,7 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
   long long wxs[4];
   if (!resolve_strides(a->wx_stride, wx_dense, wxs)) return FRNN_ERR_ALIGN;
 
-  // (a training pass stores activations, where the lane loop is ahead: see frnn_wide.cu)
-  const bool wide_gates = plan->wide_forward && !pr.training, wide = is_wide(*plan) || wide_gates;
+  const bool wide_gates = runs_wide_gates(*plan), wide = is_wide(*plan) || wide_gates;
   // keep_packed_r: the workspace is left as the previous call left it (R fragments kept, status block not cleared, so
   // an expired wait of an earlier step stays on record until the caller reads it).  The other loops clear the block themselves.
   cudaError_t e = plan->keep_packed_r || !wide ? cudaSuccess : cudaMemsetAsync(ws, 0, kStatusBytes, stream);
@@ -467,12 +516,11 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
   lp.cache = pr.training ? static_cast<elem_t*>(a->cache) : nullptr;
   lp.status = reinterpret_cast<unsigned*>(ws);
   lp.B = pr.B; lp.T = pr.T; lp.N = pr.N; lp.D = pr.D;
-  lp.U = plan->units_per_cta; lp.CS = plan->cluster_size;
   lp.state_f32 = pr.dtype_state == FRNN_DTYPE_F32;
   lp.fclip = pr.forward_clip; lp.gclip = pr.grad_clip; lp.grad_cut = pr.grad_cut;
   lp.test_drop = plan->test_drop_exchange;
   lp.wx_sb = wxs[0]; lp.wx_st = wxs[1]; lp.wx_sg = wxs[2]; lp.wx_sn = wxs[3];
-  return is_big(pr) ? launch_big(*plan, false, lp, stream) : launch_lane(*plan, false, lp, stream);
+  return launch_loop(*plan, false, lp, stream);
 }
 
 #ifndef FRNN_F16
@@ -536,13 +584,12 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   lp.dbias = grads + nR;
   lp.status = reinterpret_cast<unsigned*>(ws);
   lp.B = pr.B; lp.T = pr.T; lp.N = pr.N; lp.D = pr.D;
-  lp.U = plan->units_per_cta; lp.CS = plan->cluster_size;
   lp.state_f32 = pr.dtype_state == FRNN_DTYPE_F32;
   lp.fclip = pr.forward_clip; lp.gclip = pr.grad_clip; lp.grad_cut = pr.grad_cut;
   lp.test_drop = plan->test_drop_exchange;
   lp.ds_ss = dss[0]; lp.ds_sb = dss[1]; lp.ds_st = dss[2]; lp.ds_sn = dss[3];
   if (parts & FRNN_PART_LOOP) {
-    rc = is_big(pr) ? launch_big(*plan, true, lp, stream) : launch_lane(*plan, true, lp, stream);
+    rc = launch_loop(*plan, true, lp, stream);
     if (rc) return rc;
   }
   // dR.  Small heads: what counts is reading whole runs of neighbouring heads (frnn_dr_small.cu).  From head dim 128 up 16-bit states: both

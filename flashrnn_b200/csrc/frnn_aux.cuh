@@ -49,7 +49,7 @@ cudaError_t launch_recurrent_grad_tc(int cell, int B, int T, int N, int D, int G
                                      int sm_count, cudaStream_t stream);
 // 128-row tensor-core time loops (frnn_wide.cu): one CTA per (head, 128 batch rows); the backward also produces dR and db
 constexpr int kWideBatchTile = 128;
-constexpr int kWideThreads = 160;
+constexpr int kWideThreads = 160, kWideFwdStages = 8, kWideBwdStages = 4;  // time steps of inputs in flight
 bool wide_supported(int cell, int D, int state_f32, float fclip, float gclip, int grad_cut);
 // wx_s* / ds_s*: element strides of the batch, time and head dimensions of Wx / dstates (their head dim is contiguous)
 cudaError_t launch_wide_forward(const void* Wx, long long wx_sb, long long wx_st, long long wx_sn, const void* R,
@@ -59,6 +59,7 @@ cudaError_t launch_wide_backward(const void* R, const void* s0, const void* stat
                                  long long ds_st, long long ds_sn, void* dWx, void* ds0, float* dR, float* dbias,
                                  unsigned* status, int B, int T, int N, int test_drop, cudaStream_t stream);
 // 128-row forward loop of the LSTM and GRU cells at head dim 64 (frnn_wide.cu), without an activation cache
+constexpr int kWideGatesThreads = 288, kWideGatesStages = 2;
 bool wide_gates_forward_supported(int cell, int D, int state_f32);
 cudaError_t launch_wide_gates_forward(int cell, const void* Wx, long long wx_sb, long long wx_st, long long wx_sg, long long wx_sn, const void* R,
                                      const void* bias, const void* s0, void* states, unsigned* status, int B, int T,

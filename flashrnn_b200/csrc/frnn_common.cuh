@@ -67,8 +67,8 @@ struct LoopParams {
   unsigned* status;
   int clear_status;          // forward: CTA 0 zeroes the status block first
   int B, T, N, D;
-  int U;                     // hidden units owned by one CTA (multiple of 16)
-  int CS;                    // CTAs per cluster = D / U
+  unsigned tile0;            // first batch tile of the launch
+  int CS;                    // CTAs per cluster
   int state_f32;             // states / dstates / s0 / ds0 are fp32 (else bf16)
   float fclip, gclip;        // <= 0: off
   int grad_cut;              // backward: ignore the matrix part of the recurrent cotangent (truncated BPTT)
@@ -359,5 +359,7 @@ __device__ __forceinline__ void store_state2(void* base, size_t elem_off, int f3
 constexpr size_t kSmemBudget = 227 * 1024;
 // Head dims above 256: multiples of 64 up to this
 constexpr int kBigMaxD = 1024;
+// time steps of inputs in the shared-memory rings: lane loops, forward loop above head dim 256 (its reverse loop: one less)
+constexpr int kLaneStages = 6, kBigStages = 4;
 
 }  // namespace FRNN_NS

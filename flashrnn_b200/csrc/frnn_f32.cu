@@ -823,6 +823,7 @@ bool cluster_tile(const frnn_problem& pr, const Dims& d, int cs, int bt, Tile* t
     bt = 8;
     while (bt > 2 && (long long)((pr.B + bt / 2 - 1) / (bt / 2)) * pr.N <= kResidentClusters[cs]) bt /= 2;
   }
+  if ((pr.B + bt - 1) / bt > 65535) return false;  // batch tiles are blocks in y
   t->cs = cs; t->u = u; t->bt = bt; t->cluster = true;
   const int tm = bt == 8 ? 4 : 2;  // gate rows per thread in the forward matrix phase
   t->ksf = clampi((int)(XTHREADS * tm / gu), 1, clampi((int)(32768 / (bt * gu * 4)), 1, 16));  // partial sums within 32 KB
@@ -912,12 +913,14 @@ int check(const frnn_plan* pl, Dims* d, Tile* t) {
     return FRNN_ERR_PLAN;
   return FRNN_OK;
 }
+dim3 cluster_grid(const frnn_problem& pr, int cs, int bt) { return dim3((unsigned)cs, (unsigned)((pr.B + bt - 1) / bt), (unsigned)pr.N); }
+dim3 stream_grid(const frnn_problem& pr) { return dim3((unsigned)((pr.B + XBT - 1) / XBT), (unsigned)pr.N); }
 template <typename K>
 cudaError_t launch_cluster(K kern, const frnn_problem& pr, const Tile& t, size_t smem, const XParams& p, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);  // fixed maximum
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)t.cs, (unsigned)((pr.B + t.bt - 1) / t.bt), (unsigned)pr.N);
+  cfg.gridDim = cluster_grid(pr, t.cs, t.bt);
   cfg.blockDim = dim3(XTHREADS, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -936,7 +939,7 @@ cudaError_t launch_lane(const XLane& k, int cs, const frnn_problem& pr, XParams 
   p.CS = cs;
   p.U = pr.D / cs;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)cs, (unsigned)((pr.B + k.bt - 1) / k.bt), (unsigned)pr.N);
+  cfg.gridDim = cluster_grid(pr, cs, k.bt);
   cfg.blockDim = dim3((unsigned)k.threads, 1, 1);
   cfg.dynamicSmemBytes = k.smem;
   cfg.stream = stream;
@@ -1000,6 +1003,30 @@ __attribute__((visibility("hidden"))) int frnn_query_f32(const frnn_problem* pr,
   pl.grads_offset = w.grads;
   pl.grads_count = (uint64_t)d.Gr * pr->N * pr->D * pr->D + (uint64_t)d.Gt * pr->N * pr->D;
   *out = pl;
+  return FRNN_OK;
+}
+
+__attribute__((visibility("hidden"))) int frnn_query_loop_f32(const frnn_plan* plan, int backward, frnn_loop_shape* out) {
+  Dims d;
+  Tile tl;
+  const int rc = check(plan, &d, &tl);
+  if (rc) return rc;
+  if (!out) return FRNN_ERR_NULL;
+  const frnn_problem& pr = plan->prob;
+  if (backward && !pr.training) return FRNN_ERR_TRAINING;
+  XLane k;
+  int cs;
+  dim3 g;
+  if (lane_tile(pr, backward != 0, &cs, &k)) {
+    g = cluster_grid(pr, cs, k.bt);
+    *out = {FRNN_LOOP_F32_LANE, cs, pr.D / cs, k.bt, k.threads, kXStages, {g.x, g.y, g.z}, 1};
+  } else if (tl.cluster) {
+    g = cluster_grid(pr, tl.cs, tl.bt);
+    *out = {FRNN_LOOP_F32_CLUSTER, tl.cs, tl.u, tl.bt, XTHREADS, 0, {g.x, g.y, g.z}, 1};
+  } else {
+    g = stream_grid(pr);
+    *out = {FRNN_LOOP_F32_STREAM, 1, pr.D, XBT, XTHREADS, 0, {g.x, g.y, g.z}, 1};
+  }
   return FRNN_OK;
 }
 
@@ -1067,7 +1094,7 @@ __attribute__((visibility("hidden"))) int frnn_forward_f32(const frnn_plan* plan
     }
   } else {
     p.r_in_smem = fwd_smem(pr, d, true) <= kSmemMax;
-    const dim3 grid((unsigned)((pr.B + XBT - 1) / XBT), (unsigned)pr.N);
+    const dim3 grid = stream_grid(pr);
     const size_t smem = fwd_smem(pr, d, p.r_in_smem != 0);
     auto launch = [&](auto kern) -> cudaError_t {
       cudaError_t s = set_smem(kern);
@@ -1154,7 +1181,7 @@ __attribute__((visibility("hidden"))) int frnn_backward_parts_f32(const frnn_pla
         break;
     }
     } else {
-      const dim3 grid((unsigned)((pr.B + XBT - 1) / XBT), (unsigned)pr.N);
+      const dim3 grid = stream_grid(pr);
       const size_t smem = bwd_smem(pr, d);
       auto launch = [&](auto kern) -> cudaError_t {
         cudaError_t s = set_smem(kern);

@@ -21,6 +21,8 @@ struct XParams {
   long long wx_sb, wx_st, wx_sg, wx_sn, ds_ss, ds_sb, ds_st, ds_sn;
 };
 
+constexpr int kXStages = 4;  // time steps of inputs in the lane loops' shared-memory ring
+
 // The lane loop of a cell for head dim D in clusters of D / U CTAs, `bt` batch rows per cluster or the nearest there are; null when there
 // is none.
 struct XLane { const void* fn; int threads, bt; size_t smem; };

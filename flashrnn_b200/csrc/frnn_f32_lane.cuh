@@ -23,7 +23,7 @@
 
 namespace FRNN_NS {
 
-constexpr int kXStages = 4, kXIoWarps = 4, kXIo = 32 * kXIoWarps;
+constexpr int kXIoWarps = 4, kXIo = 32 * kXIoWarps;
 
 // byte offset of (quad q, row b) in an operand tile
 template <int BT> __host__ __device__ __forceinline__ constexpr uint32_t xq_off(int q, int b) {

@@ -110,8 +110,6 @@ template <int GC> struct CacheGeom {
   static constexpr bool EXTRA = GC > 4;
 };
 
-constexpr int kLaneStages = 6;  // time steps of inputs in the lane loops' shared-memory ring
-
 // ---- IO warps.  A lane's values belong to 8 batch rows per warp instruction (the MMA's accumulator layout), and the L1 charges
 // a global access per row touched: with the compute lanes loading Wx and storing states and cache themselves the LSTM D = 64 forward
 // step spent ~700 of 1380 clk on it.  So one or two extra warps move everything between global memory and padded tiles in shared

@@ -31,9 +31,9 @@ constexpr int WD = 64;                          // head dim
 constexpr int WM = 128;                         // batch rows per CTA = UMMA M
 constexpr uint32_t WTILE = WM * WD * 2;         // bytes of a [128][64] bf16 tile
 constexpr uint32_t WMAT = WD * WD * 2;          // bytes of a [64][64] bf16 operand
-constexpr int WF_STAGES = 8;                    // forward: Wx tiles in flight
-constexpr int WB_STAGES = 4;                    // backward: h tiles and cotangent tiles in flight (each)
-constexpr int W_THREADS = 160;
+constexpr int WF_STAGES = kWideFwdStages;       // forward: Wx tiles in flight
+constexpr int WB_STAGES = kWideBwdStages;       // backward: h tiles and cotangent tiles in flight (each)
+constexpr int W_THREADS = kWideThreads;
 
 // byte offset of 16-byte chunk `chunk` of row `row` inside a 128-byte-swizzled tile
 __device__ __forceinline__ uint32_t sw128(uint32_t row, uint32_t chunk) { return row * 128u + ((chunk ^ (row & 7u)) << 4); }
@@ -328,9 +328,9 @@ struct WideGatesParams {
   float fclip;    // > 0: the new h is clamped to [-fclip, fclip]
 };
 constexpr int WL_G = 4;
-constexpr int WL_THREADS = 288;  // warps 0-7: two row threads per batch row; warp 8, one lane: every bulk copy and MMA
+constexpr int WL_THREADS = kWideGatesThreads;  // warps 0-7: two row threads per batch row; warp 8, one lane: every bulk copy and MMA
 constexpr uint32_t WL_OFF_WX = 0;                                   // 2 stages x 4 gate tiles
-constexpr uint32_t WL_OFF_H = WL_OFF_WX + 2 * WL_G * WTILE;         // h_t in tile t & 1
+constexpr uint32_t WL_OFF_H = WL_OFF_WX + kWideGatesStages * WL_G * WTILE;         // h_t in tile t & 1
 constexpr uint32_t WL_OFF_R = WL_OFF_H + 2 * WTILE;                 // [256][64] K-major, 128-byte swizzle
 constexpr uint32_t WL_OFF_I = WL_OFF_R + WL_G * WMAT;
 constexpr uint32_t WL_OFF_ONES = WL_OFF_I + WMAT;                   // A operand [128 rows][16 k], k = 0 holds 1.0

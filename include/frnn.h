@@ -166,6 +166,30 @@ int frnn_query(const frnn_problem* problem, frnn_plan* out);
  * memory; cluster_size 1 otherwise selects the loops that stream R from L2), batch_tile 8, 4 or 2, wx_stages 0. */
 int frnn_query_tile(const frnn_problem* problem, int cluster_size, int batch_tile, int wx_stages, frnn_plan* out);
 
+/* The launch of one time loop of a plan, as frnn_query_loop reports it. */
+enum {
+  FRNN_LOOP_LANE = 0,        /* 16-bit, head dims up to 256                                            */
+  FRNN_LOOP_BIG = 1,         /* 16-bit, head dims above 256                                            */
+  FRNN_LOOP_WIDE = 2,        /* 16-bit, 128 batch rows per CTA                                         */
+  FRNN_LOOP_F32_LANE = 3,    /* float32, R in registers                                                */
+  FRNN_LOOP_F32_CLUSTER = 4, /* float32, R in the shared memory of a cluster                           */
+  FRNN_LOOP_F32_STREAM = 5   /* float32, R read from L2 in every step                                  */
+};
+typedef struct frnn_loop_shape {
+  int32_t loop;              /* FRNN_LOOP_*                                                            */
+  int32_t cluster_size;      /* CTAs that share one (head, batch tile)                                 */
+  int32_t units_per_cta;
+  int32_t batch_rows;        /* batch rows per CTA                                                     */
+  int32_t threads;           /* per CTA                                                                */
+  int32_t input_stages;      /* time steps of inputs in flight in shared memory (0: none kept there)   */
+  uint32_t grid[3];          /* CTAs of a launch                                                       */
+  int32_t launches;          /* more than 1: batches of more tiles than a grid holds (65535)           */
+} frnn_loop_shape;
+
+/* Pure host function: what the forward (backward = 0) or reverse time loop of a plan is launched with.  No counterpart in
+ * the reference. */
+int frnn_query_loop(const frnn_plan* plan, int backward, frnn_loop_shape* out);
+
 /* Whole-sequence forward: one persistent launch (head dims above 256: plus a small weight-repack launch).
  * Replaces ForwardPass::Run (flashrnn/flashrnn/fused/flashrnn_fused_forward.cu:772-975). */
 int frnn_forward(const frnn_plan* plan, const frnn_fwd_args* args, void* stream);

@@ -306,3 +306,32 @@ def test_float32_tile_table_covers_every_head_dim():
                 plan = _native.query(_native.make_problem(function, B, 3, 2, D, True, True, f32=True))
                 assert plan.cluster_size * plan.units_per_cta == D and plan.batch_tile in (2, 4, 8), (function, D, B)
                 assert plan.units_per_cta <= 64 or plan.cluster_size == 1
+
+
+@pytest.mark.parametrize("function", ["lstm", "gru", "elman", "slstm"])
+def test_time_loops_of_huge_batches_stay_inside_the_launch_limits(function):
+    """Whatever batch the planner takes, both time loops cover it with a grid a launch accepts (65535 blocks in y and z, 2^31 - 1 in x)."""
+    def loops(prob):
+        plan = _native.query(prob)
+        for backward in (False, True):
+            s = _native.query_loop(plan, backward)
+            x, y, z = s.grid
+            assert 1 <= x < 2 ** 31 and 1 <= y <= 65535 and 1 <= z <= 65535, (prob.D, prob.B, s.loop, tuple(s.grid))
+            ctas, tiles = s.cluster_size * prob.N, -(-prob.B // s.batch_rows)
+            assert s.cluster_size * s.units_per_cta == prob.D and x * y * z == ctas * min(tiles, x * y * z // ctas)
+            assert (s.launches - 1) * (x * y * z // ctas) < tiles <= s.launches * (x * y * z // ctas)
+    for D in (16, 32, 64, 96, 128, 192, 256, 320, 384, 512, 768, 1024):
+        taken = 524280 if function == "elman" else 1048560
+        for B in (1, 524280, 524281, 600000, 1048560):
+            prob = _native.make_problem(function, B, 1, 1, D, False, True)
+            if B <= taken or (function == "elman" and D == 64):
+                loops(prob)
+            else:
+                with pytest.raises(_native.FrnnError):
+                    _native.query(prob)
+    for D in (16, 64, 88, 128, 256, 512):
+        for B in (1, 131071, 262141, 524280):
+            loops(_native.make_problem(function, B, 1, 1, D, True, True, f32=True))
+    with pytest.raises(_native.FrnnError) as e:  # 150000 tiles of two rows
+        _native.query(_native.make_problem(function, 300000, 1, 1, 64, True, True, f32=True), 1, 2)
+    assert e.value.code == -6
