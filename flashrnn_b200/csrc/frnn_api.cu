@@ -65,8 +65,8 @@ static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 constexpr size_t kMaxDynSmem = 227 * 1024;
 constexpr size_t kStatusBytes = 256;
 
-// Head dims above 256 have kernels of their own (frnn_big_*.cuh).  Their plan names 64 units per CTA and clusters of D / 64; the
-// loops split the head as big_tile says.
+// Head dims above 256 have kernels of their own (frnn_big_*.cuh).  Their plan names 64 units per CTA and clusters of D / 64; unless the
+// caller asked for that, the loops split the head as big_tile says.
 static bool is_big(const frnn_problem& pr) { return pr.D > 256; }
 constexpr int kBigPlanUnits = 64;
 
@@ -75,7 +75,8 @@ constexpr int kBigPlanUnits = 64;
 // 8000 / 15380; D = 512 32 units 4230 / 7080, 64 units 8950 / 17350; D = 768 48 units 8710 / 17820, 64 units 15330 / 25490; Elman D = 512 32 units
 // 3590 / 5960, 64 units 3890 / 6350.  (32 units whatever the batch: GRU B23 T227 N5 D384 1.37 ms against 1.07 with fewer CTAs per head.)
 struct BigTile { int u, nt; };
-static BigTile big_tile(const frnn_problem& pr) {
+static BigTile big_tile(const frnn_problem& pr, int forced_bt) {
+  if (forced_bt) return {kBigPlanUnits, forced_bt / 8};
   static const int resident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 12, 11, 8, 8, 8, 8, 7, 7};
   BigTile best = {64, 1};
   long long best_cost = -1;
@@ -92,13 +93,17 @@ static BigTile big_tile(const frnn_problem& pr) {
   return best;
 }
 
+static BigTile big_tile(const frnn_plan& pl) { return big_tile(pl.prob, pl.forced_tile ? pl.batch_tile : 0); }
+static int loop_units(const frnn_plan& pl) { return is_big(pl.prob) ? big_tile(pl).u : pl.units_per_cta; }
+
 // Scratch of a plan: status block, then what the plan's kernels need.  Only head dims above 256 repack R for the forward pass.
 struct WsLayout { size_t rpack_fwd, rpack_bwd, grads, dg0, total; };
+// units: per CTA of the reverse loop
 static WsLayout workspace_layout(const frnn_problem& pr, const CellDims& cd, int units) {
   WsLayout w;
   size_t off = kStatusBytes;
   w.rpack_fwd = off; if (is_big(pr)) off = align_up(off + (size_t)(cd.Gr > 1 ? 4 : 1) * pr.N * pr.D * pr.D * 2, 256);
-  w.rpack_bwd = off; if (pr.training) off = align_up(off + rt_pack_bytes(cd.Gr, pr.N, pr.D, is_big(pr) ? big_tile(pr).u : units), 256);
+  w.rpack_bwd = off; if (pr.training) off = align_up(off + rt_pack_bytes(cd.Gr, pr.N, pr.D, units), 256);
   w.grads = off; if (pr.training) off = align_up(off + ((size_t)cd.Gr * pr.N * pr.D * pr.D + (size_t)cd.Gt * pr.N * pr.D) * 4, 256);
   w.dg0 = off;
   if (pr.training && pr.cell == CELL_GRU) off = align_up(off + (size_t)pr.B * pr.T * pr.N * pr.D * 2, 256);
@@ -246,7 +251,8 @@ static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_pl
   // one bf16 pair per (item, slot, step) in the time loops' own order; batch rows padded to whole tiles
   const uint64_t rows = (uint64_t)((pr->B + cbt - 1) / cbt) * cbt;
   pl.cache_bytes = rows * pr->T * pl.cache_slots * pr->N * pr->D * 2;
-  const WsLayout w = workspace_layout(*pr, cd, pl.units_per_cta);
+  pl.forced_tile = cs || bt;
+  const WsLayout w = workspace_layout(*pr, cd, loop_units(pl));
   pl.workspace_bytes = w.total;
   pl.grads_offset = w.grads;
   pl.grads_count = (uint64_t)cd.Gr * pr->N * pr->D * pr->D + (uint64_t)cd.Gt * pr->N * pr->D;
@@ -262,7 +268,8 @@ static int check_plan(const frnn_plan* pl, CellDims* cd) {
   if (!tile_ok(pl->prob, *cd, pl->cluster_size, pl->batch_tile)) return FRNN_ERR_PLAN;
   if (pl->units_per_cta * pl->cluster_size != pl->prob.D) return FRNN_ERR_PLAN;
   if (pl->threads != plan_threads(*cd, pl->units_per_cta, pl->batch_tile)) return FRNN_ERR_PLAN;
-  if (pl->workspace_bytes != workspace_layout(pl->prob, *cd, pl->units_per_cta).total) return FRNN_ERR_PLAN;
+  if (pl->forced_tile != 0 && pl->forced_tile != 1) return FRNN_ERR_PLAN;
+  if (pl->workspace_bytes != workspace_layout(pl->prob, *cd, loop_units(*pl)).total) return FRNN_ERR_PLAN;
   if (pl->wide_forward && !(pl->wide_forward == 1 && wide_gates_problem(pl->prob) && pl->cluster_size == 1 && pl->batch_tile == 16))
     return FRNN_ERR_PLAN;
   return FRNN_OK;
@@ -295,7 +302,7 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
   const frnn_problem& pr = pl.prob;
   const int cell = kernel_cell(pr);
   if (is_big(pr)) {
-    const BigTile t = big_tile(pr);
+    const BigTile t = big_tile(pl);
     int nt = t.nt;
     BigKernel k = big_kernel(cell, bwd, t.u, nt);
     if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(cell, bwd, t.u, nt = 1);  // (sLSTM reverse from head dim 896 up)
@@ -469,7 +476,7 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
       !aligned16(a->workspace) || (a->cache && !aligned16(a->cache)))
     return FRNN_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const WsLayout w = workspace_layout(pr, cd, plan->units_per_cta);
+  const WsLayout w = workspace_layout(pr, cd, loop_units(*plan));
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   const long long nd = (long long)pr.N * pr.D;
   const long long wx_dense[4] = {(long long)pr.T * cd.Gw * nd, cd.Gw * nd, nd, pr.D};
@@ -543,7 +550,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
       !aligned16(a->ds0) || !aligned16(a->workspace) || (a->cache && !aligned16(a->cache)))
     return FRNN_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const WsLayout w = workspace_layout(pr, cd, plan->units_per_cta);
+  const WsLayout w = workspace_layout(pr, cd, loop_units(*plan));
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   float* grads = reinterpret_cast<float*>(ws + w.grads);
   const size_t nR = (size_t)cd.Gr * pr.N * pr.D * pr.D, nb = (size_t)cd.Gt * pr.N * pr.D;
@@ -555,7 +562,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   cudaError_t e = cudaSuccess;
   if ((parts & FRNN_PART_LOOP) && !is_wide(*plan)) {
     const bool big = is_big(pr);
-    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, big ? big_tile(pr).u : plan->units_per_cta, big, grads, nR + nb,
+    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, loop_units(*plan), big, grads, nR + nb,
                            reinterpret_cast<unsigned*>(ws), stream);
     if (e != cudaSuccess) return (int)e;
   } else if (parts & FRNN_PART_LOOP) {

@@ -852,8 +852,9 @@ bool pick_tile(const frnn_problem& pr, const Dims& d, int cs, int bt, Tile* t) {
   return t->smem_f <= kSmemMax && t->smem_b <= kSmemMax;
 }
 // The lane loops (frnn_f32_lane.cuh): head dims up to 256 that split into CTAs of at most 32 units (64 with one CTA), a multiple of 4.  Their
-// tiles follow from the problem alone; the plan's tile is that of the loops below, which run every other head dim.
-bool lane_tile(const frnn_problem& pr, bool bwd, int* cs_out, XLane* k) {
+// tiles follow from the problem alone; the plan's tile is that of the other loops, which run every other head dim and what a caller asks for.
+bool lane_tile(const frnn_problem& pr, bool forced, bool bwd, int* cs_out, XLane* k) {
+  if (forced) return false;
   int cs = 1;
   if (pr.D > 64) {
     for (cs = 2; cs <= 8 && (pr.D % cs || pr.D / cs % 4 || pr.D / cs > 32); ++cs) {}
@@ -880,13 +881,13 @@ bool lane_tile(const frnn_problem& pr, bool bwd, int* cs_out, XLane* k) {
   return k->fn != nullptr && (pr.B + k->bt - 1) / k->bt <= 65535;
 }
 struct Ws { size_t rt, grads, dg0, total; };
-Ws ws_layout(const frnn_problem& pr, const Dims& d) {
+Ws ws_layout(const frnn_problem& pr, const Dims& d, bool forced) {
   Ws w;
   size_t off = kStatus;
   int cs;
   XLane lane;
   w.rt = off;  // (the lane loops read R as it is)
-  if (!lane_tile(pr, false, &cs, &lane)) off = up256(off + (size_t)d.Gr * pr.N * pr.D * pr.D * 4);
+  if (!lane_tile(pr, forced, false, &cs, &lane)) off = up256(off + (size_t)d.Gr * pr.N * pr.D * pr.D * 4);
   w.grads = off; off = up256(off + ((size_t)d.Gr * pr.N * pr.D * pr.D + (size_t)d.Gt * pr.N * pr.D) * 4);
   w.dg0 = off;
   if (pr.cell == CELL_GRU) off = up256(off + (size_t)pr.B * pr.T * pr.N * pr.D * 4);
@@ -909,7 +910,8 @@ int check(const frnn_plan* pl, Dims* d, Tile* t) {
   const int rc = validate(&pl->prob, d);
   if (rc) return rc;
   if (!pick_tile(pl->prob, *d, pl->cluster_size, pl->batch_tile, t) || pl->threads != XTHREADS ||
-      pl->units_per_cta != t->u || pl->workspace_bytes != ws_layout(pl->prob, *d).total || pl->probe_noop_cell)
+      pl->units_per_cta != t->u || (pl->forced_tile != 0 && pl->forced_tile != 1) ||
+      pl->workspace_bytes != ws_layout(pl->prob, *d, pl->forced_tile != 0).total || pl->probe_noop_cell)
     return FRNN_ERR_PLAN;
   return FRNN_OK;
 }
@@ -998,7 +1000,8 @@ __attribute__((visibility("hidden"))) int frnn_query_f32(const frnn_problem* pr,
   pl.wx_stages = 0;
   pl.cache_slots = d.GC;
   pl.cache_bytes = (uint64_t)pr->B * pr->T * d.GC * pr->N * pr->D * 4;
-  const Ws w = ws_layout(*pr, d);
+  pl.forced_tile = cs || bt;
+  const Ws w = ws_layout(*pr, d, pl.forced_tile != 0);
   pl.workspace_bytes = w.total;
   pl.grads_offset = w.grads;
   pl.grads_count = (uint64_t)d.Gr * pr->N * pr->D * pr->D + (uint64_t)d.Gt * pr->N * pr->D;
@@ -1017,7 +1020,7 @@ __attribute__((visibility("hidden"))) int frnn_query_loop_f32(const frnn_plan* p
   XLane k;
   int cs;
   dim3 g;
-  if (lane_tile(pr, backward != 0, &cs, &k)) {
+  if (lane_tile(pr, plan->forced_tile != 0, backward != 0, &cs, &k)) {
     g = cluster_grid(pr, cs, k.bt);
     *out = {FRNN_LOOP_F32_LANE, cs, pr.D / cs, k.bt, k.threads, kXStages, {g.x, g.y, g.z}, 1};
   } else if (tl.cluster) {
@@ -1047,11 +1050,11 @@ __attribute__((visibility("hidden"))) int frnn_forward_f32(const frnn_plan* plan
   if (!strides_ok(a->wx_stride, wx_dense, wxs)) return FRNN_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
-  const Ws w = ws_layout(pr, d);
+  const Ws w = ws_layout(pr, d, plan->forced_tile != 0);
   cudaError_t e = cudaSuccess;
   XLane lane;
   int lane_cs;
-  const bool is_lane = lane_tile(pr, false, &lane_cs, &lane);
+  const bool is_lane = lane_tile(pr, plan->forced_tile != 0, false, &lane_cs, &lane);
   if (!plan->keep_packed_r && !is_lane) {
     e = cudaMemsetAsync(ws, 0, kStatus, stream);
     if (e != cudaSuccess) return (int)e;
@@ -1136,7 +1139,7 @@ __attribute__((visibility("hidden"))) int frnn_backward_parts_f32(const frnn_pla
   if (!strides_ok(a->dstates_stride, ds_dense, dss)) return FRNN_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
-  const Ws w = ws_layout(pr, d);
+  const Ws w = ws_layout(pr, d, plan->forced_tile != 0);
   float* grads = reinterpret_cast<float*>(ws + w.grads);
   const size_t nR = (size_t)d.Gr * pr.N * pr.D * pr.D, nb = (size_t)d.Gt * pr.N * pr.D;
   cudaError_t e = cudaSuccess;
@@ -1159,7 +1162,7 @@ __attribute__((visibility("hidden"))) int frnn_backward_parts_f32(const frnn_pla
     p.status = reinterpret_cast<unsigned*>(ws);
     XLane lane;
     int lane_cs;
-    if (lane_tile(pr, true, &lane_cs, &lane)) {
+    if (lane_tile(pr, plan->forced_tile != 0, true, &lane_cs, &lane)) {
       p.test_drop = plan->test_drop_exchange;
       e = launch_lane(lane, lane_cs, pr, p, false, stream);
     } else if (tl.cluster) {

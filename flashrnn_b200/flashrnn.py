@@ -82,7 +82,7 @@ class FlashRNNConfig:
     dtype_a: Optional[str] = None
     enable_automatic_mixed_precision: bool = True
     initial_val: Union[float, Sequence[float]] = 0.0
-    # sm_100a tile override for measurements: 0 = take the library's table
+    # sm_100a tile override for measurements: 0 = take the library's table (see frnn_query_tile in include/frnn.h)
     cluster_size: int = 0
     batch_tile: int = 0
     # synchronise after each launch and raise if a bounded device-side wait expired (a CTA of a cluster never

@@ -102,7 +102,8 @@ typedef struct frnn_plan {
                                  forward loop writes.  Set by frnn_query for large-batch LSTM and GRU problems at
                                  head_dim 64 (16-bit states) on 16-row tiles; frnn_query_tile(cluster_size 1,
                                  batch_tile 128) asks for it, any other forced tile leaves it 0.                       */
-  int32_t reserved[2];
+  int32_t forced_tile;        /* 1: the tile was asked for (frnn_query_tile): the loops run it instead of what their own tables say */
+  int32_t reserved;
   uint64_t cache_bytes;     /* size of the activation cache (opaque layout, tied to this plan) */
   uint64_t workspace_bytes; /* size of the scratch workspace                                  */
   uint64_t grads_offset;    /* byte offset, inside the workspace, of the fp32 gradients dR || db */
@@ -162,7 +163,9 @@ int frnn_query(const frnn_problem* problem, frnn_plan* out);
 
 /* Same as frnn_query but with the tile forced by the caller (used to measure the tile table);
  * any of the three may be 0 = "use the table's value".  Invalid combinations return FRNN_ERR_PLAN.
- * float32 problems: cluster_size 1..8 (units per CTA a multiple of 4, at most 64, its fp32 slice of R within shared
+ * 16-bit problems: batch_tile is the most rows a CTA takes (there is no 32-row loop any more, and 16-row ones only where they were
+ * faster; above head dim 256 the loops take 8 or 16 rows as asked, with cluster_size = D / 64); frnn_query_loop says what runs.
+ * float32 problems: a forced tile runs the loops with R in shared memory: cluster_size 1..8 (units per CTA a multiple of 4, at most 64, its fp32 slice of R within shared
  * memory; cluster_size 1 otherwise selects the loops that stream R from L2), batch_tile 8, 4 or 2, wx_stages 0. */
 int frnn_query_tile(const frnn_problem* problem, int cluster_size, int batch_tile, int wx_stages, frnn_plan* out);
 

@@ -102,13 +102,15 @@ def test_wide_loops_report_a_copy_that_never_lands(cuda_device):
     assert st.code == 0 and torch.isfinite(dWx.float()).all()
 
 
-def test_float32_cluster_loops_report_a_withheld_message(cuda_device):
+@pytest.mark.parametrize("loop,tile", [("f32_lane", (0, 0)), ("f32_cluster", (4, 8))])
+def test_float32_cluster_loops_report_a_withheld_message(cuda_device, loop, tile):
     """The float32 cluster loops use the same exchange protocol: forward (h slices) and reverse loop (partial sums of dh)
     each report the message CTA 0 withholds, the kernels end, and a clean run follows in the same context."""
     Wx, R, b, s0 = [t.to(cuda_device, torch.float32) for t in make_inputs("lstm", 8, 6, 1, 128, seed=33, dtype=torch.float32)]
     B, T, _, N, D = Wx.shape
-    plan = nv.query(nv.make_problem("lstm", B, T, N, D, True, True, f32=True))
-    assert plan.cluster_size > 1
+    plan = nv.query(nv.make_problem("lstm", B, T, N, D, True, True, f32=True), *tile)
+    shapes = [nv.query_loop(plan, b) for b in (False, True)]
+    assert all(nv.LOOPS[s.loop] == loop and s.cluster_size > 1 for s in shapes)
     P = lambda t: ctypes.c_void_p(t.data_ptr())
     stream = ctypes.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)
     states = torch.zeros(2, B, T, N, D, device=cuda_device, dtype=torch.float32)
@@ -121,7 +123,7 @@ def test_float32_cluster_loops_report_a_withheld_message(cuda_device):
     plan.test_drop_exchange = 1
     nv.check("frnn_forward", L.frnn_forward(ctypes.byref(plan), ctypes.byref(fa), stream))
     nv.check("status", L.frnn_read_device_status(P(ws), stream, ctypes.byref(st)))
-    assert st.code == 1 and st.cta < plan.cluster_size * N * ((B + plan.batch_tile - 1) // plan.batch_tile)
+    assert st.code == 1 and st.cta < shapes[0].grid[0] * shapes[0].grid[1] * shapes[0].grid[2]
     plan.test_drop_exchange = 0
     nv.check("frnn_forward", L.frnn_forward(ctypes.byref(plan), ctypes.byref(fa), stream))
     nv.check("status", L.frnn_read_device_status(P(ws), stream, ctypes.byref(st)))

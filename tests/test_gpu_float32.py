@@ -114,6 +114,10 @@ def test_float32_cluster_sizes(cuda_device, function, D, cs, bt):
     B, T, N = 11, 10, 2
     plan = _native.query(_native.make_problem(function, B, T, N, D, True, True, f32=True), cs, bt)
     assert plan.cluster_size * plan.units_per_cta == D and (cs == 0 or plan.cluster_size == cs) and (bt == 0 or plan.batch_tile == bt)
+    if cs or bt:
+        for backward in (False, True):
+            loop = _native.query_loop(plan, backward)
+            assert _native.LOOPS[loop.loop] in ("f32_cluster", "f32_stream") and (loop.cluster_size, loop.batch_rows) == (plan.cluster_size, plan.batch_tile)
     Wx, R, b, s0 = make_inputs(function, B, T, N, D, seed=5 + D + cs, random_init=(function != "slstm"), dtype=torch.float32)
     g = torch.Generator().manual_seed(9)
     cot = torch.randn(s0.shape[0], B, T, N, D, generator=g, dtype=torch.float64).float().double()

@@ -25,6 +25,12 @@ def test_head_dims_above_256_edges(cuda_device, function, N, D, B, T, state_f32)
     _check(function, N, D, B, T, state_f32)
 
 
+# a tile the caller asks for: 64 units per CTA whatever the table says
+@pytest.mark.parametrize("function,D,bt", [("lstm", 512, 16), ("gru", 384, 8), ("elman", 512, 16), ("slstm", 384, 16)])
+def test_head_dims_above_256_forced_tile(cuda_device, function, D, bt):
+    _check(function, 2, D, 17, 3, False, cluster_size=D // 64, batch_tile=bt)
+
+
 def _check(function, N, D, B, T, state_f32, **tile):
     Wx, R, b, s0 = make_inputs(function, B, T, N, D, seed=D + T, random_init=True, state_f32=state_f32)
     S = s0.shape[0]

@@ -335,3 +335,27 @@ def test_time_loops_of_huge_batches_stay_inside_the_launch_limits(function):
     with pytest.raises(_native.FrnnError) as e:  # 150000 tiles of two rows
         _native.query(_native.make_problem(function, 300000, 1, 1, 64, True, True, f32=True), 1, 2)
     assert e.value.code == -6
+
+
+def test_a_forced_tile_is_what_the_loops_run():
+    mk, loops = _native.make_problem, lambda plan: [_native.query_loop(plan, b) for b in (False, True)]
+    # float32: the loops with R in shared memory; without a forced tile the ones with R in registers
+    for function, D, cs, bt in [("lstm", 64, 1, 8), ("lstm", 64, 2, 4), ("gru", 96, 3, 2), ("slstm", 192, 6, 4), ("elman", 256, 8, 8), ("lstm", 320, 8, 2)]:
+        plan = _native.query(mk(function, 11, 4, 2, D, True, True, f32=True), cs, bt)
+        assert plan.forced_tile == 1
+        for s in loops(plan):
+            assert (_native.LOOPS[s.loop], s.cluster_size, s.units_per_cta, s.batch_rows) == ("f32_cluster", cs, D // cs, bt), (function, D, cs, bt)
+        if D <= 256:
+            assert all(_native.LOOPS[s.loop] == "f32_lane" for s in loops(_native.query(mk(function, 11, 4, 2, D, True, True, f32=True))))
+    assert all(_native.LOOPS[s.loop] == "f32_stream" for s in loops(_native.query(mk("lstm", 11, 4, 2, 128, True, True, f32=True), 1, 8)))
+    # 16-bit, above head dim 256: 64 units and the rows asked for
+    for function in ("lstm", "gru", "elman", "slstm"):
+        for D in (320, 512, 768, 1024):
+            for bt in (8, 16):
+                for backward, s in enumerate(loops(_native.query(mk(function, 300, 4, 2, D, False, True), D // 64, bt))):
+                    rows = 8 if function == "slstm" and D == 1024 and backward else bt  # (16 do not fit its shared memory)
+                    assert (_native.LOOPS[s.loop], s.cluster_size, s.units_per_cta, s.batch_rows) == ("big", D // 64, 64, rows), (function, D, bt)
+    # 16-bit, up to 256: the cluster asked for, at most the rows
+    for function, D, cs, bt in [("lstm", 64, 1, 8), ("lstm", 64, 4, 16), ("gru", 128, 2, 16), ("elman", 128, 8, 32), ("slstm", 256, 16, 8)]:
+        for s in loops(_native.query(mk(function, 300, 4, 2, D, False, True), cs, bt)):
+            assert (_native.LOOPS[s.loop], s.cluster_size) == ("lane", cs) and s.batch_rows <= bt
