@@ -43,15 +43,17 @@ WORKLOADS = {
     "C4": ("slstm", 8, 4096, 4, 192, True),
     "C5": ("elman", 1024, 2048, 16, 64, False),
     "C5s": ("elman", 1024, 256, 16, 64, False),  # C5 with T cut to 256 (2.1 GB resident): the size ncu captures use
-    "LB": ("lstm", 1024, 512, 16, 64, False),    # large-batch LSTM (the reference's batch-size sweeps): 16-row tiles, HBM-side regime
-    "LBs": ("lstm", 512, 128, 16, 64, False),    # LB cut to 0.7 GB resident (512 CTAs, same tile): the size ncu captures use
-    "LBm": ("lstm", 1024, 64, 16, 64, False),    # LB with T cut to 64 (1.3 GB resident, 128 CTAs of 128 rows): ncu captures of the memory-bound case
+    "LB": ("lstm", 1024, 512, 16, 64, False),    # large-batch LSTM (the reference's batch-size sweeps): as many CTAs as fill the GPU several times
+    "LBs": ("lstm", 512, 128, 16, 64, False),    # LB cut to 0.7 GB resident, same loops: the size ncu captures use
+    "LBm": ("lstm", 1024, 64, 16, 64, False),    # LB with T cut to 64 (1.3 GB resident): ncu captures of the memory-bound case
     "GB": ("gru", 1024, 512, 16, 64, False),     # large-batch GRU, as LB
     # the head-dim sweep of the reference's README figure (LSTM bf16 B16 T1024, head_dim x heads = 768)
     "H16": ("lstm", 16, 1024, 48, 16, False), "H32": ("lstm", 16, 1024, 24, 32, False), "H64": ("lstm", 16, 1024, 12, 64, False),
     "H128": ("lstm", 16, 1024, 6, 128, False), "H256": ("lstm", 16, 1024, 3, 256, False), "H768": ("lstm", 16, 1024, 1, 768, False),
 }
 DIMS = {"lstm": (4, 4, 4, 2), "gru": (3, 3, 4, 1), "elman": (1, 1, 1, 1), "slstm": (4, 4, 4, 4)}
+REVERSE_KERNELS = {"lane": "lane_bwd_kernel", "big": "big_bwd_kernel", "wide": "wide_bwd_elman_kernel", "f32_lane": "x32l_bwd_kernel",
+                   "f32_cluster": "x32c_bwd_kernel", "f32_stream": "x32_bwd_kernel"}  # by what frnn_query_loop says
 METRIC = "fwd+bwd tokens/sec (B*T/s)"
 # DRAM bytes (read + write) of ONE launch of the reverse time loop, from an ncu capture (SpeedOfLight, MemoryWorkloadAnalysis) of
 # `python bench.py --workload C2 --steps 1 --warmup 3 --min-seconds 0 --no-cpu` on a B200; reported with its provenance.
@@ -421,7 +423,8 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
 
     # ---- floor of the serial chain: the same loops with the gate arithmetic taken out (frnn_plan.probe_noop_cell)
     chain = None
-    wide = plan.batch_tile == 128
+    loops = {name: nv.query_loop(plan, name == "reverse") for name in ("forward", "reverse")}
+    wide = nv.LOOPS[loops["reverse"].loop] == "wide"
     if floor and not wide:
         probe = nv.FrnnPlan.from_buffer_copy(plan)
         probe.probe_noop_cell = 1
@@ -455,10 +458,10 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
         "ms_per_step": ms, "ms_per_step_best": min(block_ms), "blocks": nblocks, "timed_seconds": sum(block_ms) * args.steps * 1e-3,
         "kernel_ms": {"forward_loop": fwd_ms, "backward_loop": bwd_ms, "recurrent_grad": dr_ms},
         "us_per_time_step": {"forward": 1e3 * fwd_ms / T, "backward": 1e3 * bwd_ms / T},
-        "tile": {"cluster_size": plan.cluster_size, "units_per_cta": plan.units_per_cta, "batch_tile": plan.batch_tile, "threads": plan.threads,
-                 "wide_forward": int(plan.wide_forward)},  # 1: forward loop on the 128-row tcgen05 kernel (LSTM, head dim 64)
+        "tile": {name: {"loop": nv.LOOPS[s.loop], "cluster_size": s.cluster_size, "units_per_cta": s.units_per_cta, "batch_rows": s.batch_rows,
+                        "threads": s.threads, "ctas": s.grid[0] * s.grid[1] * s.grid[2] * s.launches} for name, s in loops.items()},  # as launched
         "roofline": {
-            "bound": "hbm", "kernel": "wide_bwd_elman_kernel (reverse time loop, dR and db inside)" if wide else "x32l_bwd_kernel (reverse time loop)" if job.f32io else "lane_bwd_kernel (reverse time loop)",
+            "bound": "hbm", "kernel": REVERSE_KERNELS[nv.LOOPS[loops["reverse"].loop]] + (" (reverse time loop, dR and db inside)" if wide else " (reverse time loop)"),
             "achieved": achieved, "peak": job.hbm_peak, "unit": "GB/s", "frac": achieved / job.hbm_peak, "peak_source": job.peak_source,
             "traffic": None, "traffic_source": None, "algorithmic_bytes_per_launch": bwd_bytes,
             "forward_loop": {"achieved": fwd_bytes / (fwd_ms * 1e-3) / 1e9, "frac": fwd_bytes / (fwd_ms * 1e-3) / 1e9 / job.hbm_peak,
@@ -469,8 +472,10 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
                            "fp32_cuda_core_frac": (6.0 * E * Gr * D / (ms * 1e-3) / 1e12) / (148 * 128 * 2 * 1.965e-3) if job.f32io else None},
             "chain_floor": chain,
             "note": "streams one 16 KB tile per operand, step and CTA; HBM-bound" if wide else
+                    "more CTAs than SMs: issue slots of the cells and memory bound this workload" if min(s.grid[0] * s.grid[1] * s.grid[2] for s in loops.values()) > 148 else
                     "the serial chain of 2T dependent steps (chain_floor), not HBM or the tensor pipe, bounds this workload"},
-        "clocks": clk.summary(), "launches_per_step": 3 if wide or job.f32io else 6 if D > 256 else 5,  # pack of R (head dims above 256), loops, R^T, dR, cast
+        # loops, dR and cast; in front: fragments of R^T (16-bit), of R (head dims above 256), R^T (float32 but for the lane loop)
+        "clocks": clk.summary(), "launches_per_step": 3 if wide else 4 + (nv.LOOPS[loops["forward"].loop] != "f32_lane") if job.f32io else 6 if D > 256 else 5,
     }
     if keep is not None:
         keep.update(Wx=Wx, R=R, b=b, s0=s0, gcnt=gcnt)

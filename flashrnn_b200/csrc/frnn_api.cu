@@ -230,7 +230,7 @@ static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_pl
   const int rc = validate_problem(pr, &cd);
   if (rc) return rc;
   if (!out) return FRNN_ERR_NULL;
-  if (stages != 0 && stages != kStages) return FRNN_ERR_PLAN;
+  if (stages != 0 && stages != 4) return FRNN_ERR_PLAN;  // (the one depth there was before the loops had rings of their own)
   int ccs = 0, cbt = 0;
   if (!choose_tile(*pr, cd, cs, bt, &ccs, &cbt)) return (cs || bt) ? FRNN_ERR_PLAN : FRNN_ERR_SHAPE;
   if ((long long)((pr->B + cbt - 1) / cbt) > 65535) return FRNN_ERR_SHAPE;
@@ -241,12 +241,12 @@ static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_pl
   pl.units_per_cta = pr->D / ccs;
   pl.batch_tile = cbt;
   pl.threads = plan_threads(cd, pl.units_per_cta, cbt);
-  pl.wx_stages = kStages;
   // measured on B200: LSTM B1024 T512 N16 D64 (128 CTAs of 128 rows) forward loop 2.07 ms against 3.40 ms on the 16-row
   // tiles; B512 T128 N16 (64 CTAs) 0.49 against 0.51 ms -- a step of the 128-row loop takes ~3.8 us however few CTAs run,
   // so it pays once its CTAs occupy most of the SMs.  GRU B1024 T512 N16 D64: 1.74 against 3.25 ms.
   pl.wide_forward = wide_gates_problem(*pr) && ccs == 1 && cbt == 16 &&
                     (bt == kWideBatchTile || (!cs && !bt && (long long)(pr->B / kWideBatchTile) * pr->N >= 96));
+  pl.wx_stages = is_wide(pl) ? kWideFwdStages : runs_wide_gates(pl) ? kWideGatesStages : is_big(*pr) ? kBigStages : kLaneStages;
   pl.cache_slots = cache_slots_of(*pr, cd);
   // one bf16 pair per (item, slot, step) in the time loops' own order; batch rows padded to whole tiles
   const uint64_t rows = (uint64_t)((pr->B + cbt - 1) / cbt) * cbt;

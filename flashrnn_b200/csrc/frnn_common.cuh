@@ -46,9 +46,6 @@ template <> struct Cell<CELL_LSTM | kNoopCell> : Cell<CELL_LSTM> {};
 template <> struct Cell<CELL_GRU | kNoopCell> : Cell<CELL_GRU> {};
 template <> struct Cell<CELL_SLSTM | kNoopCell> : Cell<CELL_SLSTM> {};
 
-// Time steps of inputs kept in flight ahead of the step being computed (cp.async ring depth).
-constexpr int kStages = 4;
-
 // Arguments of both time-loop kernels (forward uses the first block, backward all of it).
 struct LoopParams {
   const elem_t* Wx;   // [B,T,Gw,N,D]

@@ -14,7 +14,7 @@
 // st.async, which also counts the bytes on the destination's mbarrier: no staging, no proxy fence, no elected thread.
 // h is double-buffered; a CTA can only write h_{t+1} after it has received h_t of every warp of the cluster, i.e. after
 // all of them have read h_{t-1}, so nothing else orders the buffers.  CS == 1: plain stores and one CTA barrier.
-// IO warps (frnn_lane.cuh) prefetch Wx kStages steps ahead and store states and activations; the compute lanes leave their
+// IO warps (frnn_lane.cuh) prefetch Wx kLaneStages steps ahead and store states and activations; the compute lanes leave their
 // results in a double-buffered shared-memory tile after the push, in the shadow of the exchange.
 //
 // Replaces FLASHRNNCellFusedForward (reference flashrnn/flashrnn/fused/flashrnn_fused_forward.cu:146-659)

@@ -70,16 +70,16 @@ typedef struct frnn_problem {
 
 /* Launch plan chosen by frnn_query from the measured sm_100a tile table.  Replaces the reference's
  * compile-time tiling macros solved by flashrnn/autotune/constrint.py and bisected in
- * flashrnn/flashrnn/cuda_init_parametric.py:92-358.  Treat as opaque; sizes are for the caller. */
+ * flashrnn/flashrnn/cuda_init_parametric.py:92-358.  Treat as opaque; sizes are for the caller.  The tile fields name the class the
+ * plan belongs to; rows, units, threads and CTAs of each loop follow from it by rules of the loops, and frnn_query_loop reports them. */
 typedef struct frnn_plan {
   int32_t abi_version;
   frnn_problem prob;
   int32_t cluster_size;    /* CTAs that share one (head, batch tile); exchange h through DSMEM */
   int32_t units_per_cta;   /* hidden units of the head owned by one CTA                      */
-  int32_t batch_tile;      /* batch rows per CTA (8, 16, 32 or 128; float32 loops: 8, 4 or 2); head dims up to 256 run 16 and
-                              32 as 8- or 16-row tiles, whichever is faster for the cell and direction */
-  int32_t threads;         /* thread class of the tile (2 x gates x units); the lane loops launch their own number */
-  int32_t wx_stages;       /* time steps of Wx prefetched ahead into shared memory           */
+  int32_t batch_tile;      /* batch rows (8, 16, 32 or 128; float32: 8, 4 or 2): the most a CTA takes */
+  int32_t threads;         /* thread class of the tile (2 x gates x units), not what a loop launches  */
+  int32_t wx_stages;       /* time steps of Wx the forward loop keeps in flight in shared memory      */
   int32_t cache_slots;     /* activation values cached per (b,t,n,d) in training             */
   int32_t test_drop_exchange; /* TEST HOOK, leave 0.  1: CTA 0 of every cluster withholds one exchange message
                                  (forward: its h of step 1; backward: its first message) so that its peers' bounded
@@ -97,9 +97,9 @@ typedef struct frnn_plan {
                                  the floor the serial chain of T dependent steps sets, which no cell math can undercut.
                                  Results are meaningless.  Exists for the tiles of the benchmark configurations only
                                  (lstm D=256, gru D=128, slstm D=192, 8-row batch tiles); elsewhere FRNN_ERR_PLAN.   */
-  int32_t wide_forward;       /* 1: the forward loop runs as the 128-row tensor-core loop (tcgen05, one CTA per head and
-                                 128 batch rows) while the reverse loop keeps the tile above, whose cache layout the
-                                 forward loop writes.  Set by frnn_query for large-batch LSTM and GRU problems at
+  int32_t wide_forward;       /* 1: without gradients (training == 0) the forward loop runs as the 128-row tensor-core loop (tcgen05, one
+                                 CTA per head and 128 batch rows); a training pass, which has to store activations, runs the loop
+                                 of the tile above all the same.  Set by frnn_query for large-batch LSTM and GRU problems at
                                  head_dim 64 (16-bit states) on 16-row tiles; frnn_query_tile(cluster_size 1,
                                  batch_tile 128) asks for it, any other forced tile leaves it 0.                       */
   int32_t forced_tile;        /* 1: the tile was asked for (frnn_query_tile): the loops run it instead of what their own tables say */
@@ -162,7 +162,8 @@ int frnn_abi_version(void);
 int frnn_query(const frnn_problem* problem, frnn_plan* out);
 
 /* Same as frnn_query but with the tile forced by the caller (used to measure the tile table);
- * any of the three may be 0 = "use the table's value".  Invalid combinations return FRNN_ERR_PLAN.
+ * any of the three may be 0 = "use the table's value".  Invalid combinations return FRNN_ERR_PLAN.  wx_stages: the depth of the
+ * input ring belongs to the loop; 4 (16-bit problems) is accepted and changes nothing.
  * 16-bit problems: batch_tile is the most rows a CTA takes (there is no 32-row loop any more, and 16-row ones only where they were
  * faster; above head dim 256 the loops take 8 or 16 rows as asked, with cluster_size = D / 64); frnn_query_loop says what runs.
  * float32 problems: a forced tile runs the loops with R in shared memory: cluster_size 1..8 (units per CTA a multiple of 4, at most 64, its fp32 slice of R within shared

@@ -359,3 +359,20 @@ def test_a_forced_tile_is_what_the_loops_run():
     for function, D, cs, bt in [("lstm", 64, 1, 8), ("lstm", 64, 4, 16), ("gru", 128, 2, 16), ("elman", 128, 8, 32), ("slstm", 256, 16, 8)]:
         for s in loops(_native.query(mk(function, 300, 4, 2, D, False, True), cs, bt)):
             assert (_native.LOOPS[s.loop], s.cluster_size) == ("lane", cs) and s.batch_rows <= bt
+
+
+def test_plans_report_the_loops_they_run():
+    mk = _native.make_problem
+    kind = lambda plan, b: (lambda s: (_native.LOOPS[s.loop], s.batch_rows, s.threads, s.input_stages))(_native.query_loop(plan, b))
+    train, infer = _native.query(mk("lstm", 1024, 512, 16, 64, False, True)), _native.query(mk("lstm", 1024, 512, 16, 64, False, False))
+    assert kind(train, False) == ("lane", 8, 320, 6) and kind(train, True) == ("lane", 8, 192, 6)
+    assert kind(infer, False) == ("wide", 128, 288, 2)
+    with pytest.raises(_native.FrnnError) as e:
+        _native.query_loop(infer, True)
+    assert e.value.code == -7
+    elman = _native.query(mk("elman", 1024, 2048, 16, 64, False, True))
+    assert kind(elman, False) == ("wide", 128, 160, 8) and kind(elman, True) == ("wide", 128, 160, 4)
+    for prob in (mk("lstm", 16, 8, 4, 256, False, True), mk("lstm", 8, 8, 1, 512, False, False), mk("elman", 1024, 8, 16, 64, False, True),
+                 mk("gru", 1024, 8, 16, 64, False, False), mk("gru", 1024, 8, 16, 64, False, True)):
+        plan = _native.query(prob)
+        assert plan.wx_stages == _native.query_loop(plan, False).input_stages
