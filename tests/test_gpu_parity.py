@@ -35,7 +35,7 @@ NO_SUCH_TILE = {("lstm", 1, 8), ("lstm", 1, 32), ("lstm", 2, 32), ("gru", 1, 8),
 @pytest.mark.parametrize("cs,bt", [(1, 8), (2, 16), (4, 8), (8, 16), (1, 32), (2, 32)])
 def test_parity_every_cluster_size(cuda_device, function, cs, bt):
     """Same answer whatever tile the plan uses (cluster exchange through DSMEM vs single CTA); a tile that cannot exist
-    is refused with FRNN_ERR_PLAN before anything is launched."""
+    is refused with FRNN_ERR_PLAN before anything is launched.  ``bt`` is the most rows a CTA takes: there is no 32-row loop."""
     B, T, N, D = 20, 12, 2, 128
     from flashrnn_b200 import _native
 
@@ -44,7 +44,10 @@ def test_parity_every_cluster_size(cuda_device, function, cs, bt):
             _native.query(_native.make_problem(function, B, T, N, D, False, True), cs, bt)
         assert e.value.code == -6
         return
-    _native.query(_native.make_problem(function, B, T, N, D, False, True), cs, bt)
+    plan = _native.query(_native.make_problem(function, B, T, N, D, False, True), cs, bt)
+    for backward in (False, True):
+        loop = _native.query_loop(plan, backward)
+        assert loop.cluster_size == cs and loop.batch_rows <= bt and loop.batch_rows in (8, 16)
     Wx, R, b, s0 = make_inputs(function, B, T, N, D, seed=7, random_init=True)
     got = run_native(function, Wx, R, b, s0, cluster_size=cs, batch_tile=bt)
     ref = run_oracle(function, Wx, R, b, s0)
@@ -66,8 +69,8 @@ def test_parity_32_unit_tiles(cuda_device, function, D, T, state_f32):
 
 @pytest.mark.parametrize("function,D", [("lstm", 64), ("gru", 64), ("slstm", 64), ("lstm", 128)])
 def test_parity_large_batch_16_row_tiles(cuda_device, function, D):
-    """Enough (head, batch tile) pairs to fill the GPU: the table switches the cells with three or four gates to 16-row
-    batch tiles (one CTA per head up to head dim 64, clusters of 32-unit CTAs above)."""
+    """Enough (head, batch tile) pairs to fill the GPU: the table switches the cells with three or four gates to plans of 16
+    rows (one CTA per head up to head dim 64, clusters of 32-unit CTAs above), of which a loop takes 8 or 16 at a time."""
     from flashrnn_b200 import _native
 
     B, T, N = 168, 5, 13  # ragged: 10.5 tiles of 16 rows
@@ -75,6 +78,8 @@ def test_parity_large_batch_16_row_tiles(cuda_device, function, D):
     assert plan.batch_tile == 16 and plan.units_per_cta == (64 if D == 64 else 32)
     Wx, R, b, s0 = make_inputs(function, B, T, N, D, seed=53, random_init=(function != "slstm"))
     got = run_native(function, Wx, R, b, s0)
+    assert {_native.query_loop(plan, b).batch_rows for b in (False, True)} == {("lstm", 64): {8}, ("gru", 64): {8, 16}, ("slstm", 64): {8},
+                                                                               ("lstm", 128): {16}}[function, D]
     ref = run_oracle(function, Wx, R, b, s0)
     assert_parity(function, got, ref, tag=f"{function} D{D} large batch", zero_init=(function == "slstm"))
 

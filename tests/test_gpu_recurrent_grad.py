@@ -17,3 +17,22 @@ def test_recurrent_grad_edges(cuda_device, function, D, N, B, T, state_f32):
     got = run_native(function, Wx, R, b, s0, cot=cot, state_f32=state_f32)
     ref = run_oracle(function, Wx, R, b, s0, cot=cot)
     assert_parity(function, got, ref, tag=f"{function} D{D} N{N} B{B} T{T}", zero_init=False)
+
+
+# the tensor-map kernel (16-bit states, head dims 128, 192, 256, and 768 as an example of three column tiles): sequences shorter than, equal to
+# and just beyond the 64 steps of its copies, initial states (the h_{-1} term that is added outside the MMA), batches that do not fill a
+# split evenly, and the GRU, whose first gate's deltas come from a buffer of their own
+@pytest.mark.parametrize("function,B,T,N,D", [
+    ("lstm", 3, 1, 2, 128), ("lstm", 5, 64, 1, 256), ("lstm", 2, 65, 2, 128), ("lstm", 9, 130, 1, 192),
+    ("gru", 4, 1, 3, 128), ("gru", 7, 63, 1, 192), ("gru", 3, 129, 2, 256),
+    ("slstm", 6, 66, 1, 128), ("elman", 5, 70, 2, 256), ("elman", 11, 2, 1, 128),
+    ("lstm", 3, 64, 1, 768), ("gru", 2, 129, 1, 768), ("elman", 3, 129, 2, 128),
+])
+def test_parameter_gradients_at_chunk_edges(cuda_device, function, B, T, N, D):
+    Wx, R, b, s0 = make_inputs(function, B, T, N, D, seed=B * T + D, random_init=True)
+    cot = torch.randn(s0.shape[0], B, T, N, D, generator=torch.Generator().manual_seed(11), dtype=torch.float64).to(torch.bfloat16).to(torch.float64)
+    if function == "slstm":
+        cot[3] = 0.0  # the stabiliser state has no cotangent in the closed-form backward
+    got = run_native(function, Wx, R, b, s0, cot=cot)
+    ref = run_oracle(function, Wx, R, b, s0, cot=cot)
+    assert_parity(function, got, ref, tag=f"{function} B{B} T{T} N{N} D{D}", zero_init=False)
