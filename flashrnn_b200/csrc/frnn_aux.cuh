@@ -64,7 +64,7 @@ bool wide_gates_forward_supported(int cell, int D, int state_f32);
 cudaError_t launch_wide_gates_forward(int cell, const void* Wx, long long wx_sb, long long wx_st, long long wx_sg, long long wx_sn, const void* R,
                                      const void* bias, const void* s0, void* states, unsigned* status, int B, int T,
                                      int N, float fclip, int test_drop, cudaStream_t stream);
-// dR fed by tensor-map bulk copies (frnn_dr_tma.cu): 16-bit states, head dims that are multiples of 64
+// dR fed by tensor-map bulk copies (frnn_dr_tma.cu): 16-bit states, head dims of 128 up that are multiples of 64
 bool recurrent_grad_tma_supported(int D, int state_f32);
 cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int Gr, int Gw, const void* dWx, const void* dg0,
                                       const void* states, const void* s0, float* dR, unsigned* status, int sm_count,

@@ -49,7 +49,6 @@ struct BwdLane {
   using C = Cell<CELL>;
   static constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, NNEED = C::NNEED, NEXT = C::NEXT;
   static constexpr int NB = G::NB, BT = G::BT, U = G::UNITS, GCM = G::GCM, NSS = G::NSS;
-  static constexpr bool CL = G::CL;
   F2 car[NB][S], cur[NB][NNEED], dbacc[Gt];
   F2 co[NB][BwdCoef<CELL>::N], dext0[NB];     // what the step's deltas need beside the recurrent part of dh
   uint32_t cw[NB], ew[NB], sw[NB], dloc[NB];  // activation and state words of row nb in the input ring, delta words in the tile
@@ -60,7 +59,7 @@ struct BwdLane {
   int a, tig, bt0, f32, ul, dt;
   uint32_t d0;
 
-  __device__ __forceinline__ int row_of(int nb) const { return CL ? nb * 8 + 2 * tig + a : (nb >> 1) * 8 + 2 * tig + (nb & 1); }
+  __device__ __forceinline__ int row_of(int nb) const { return nb * 8 + 2 * tig + a; }
   // d0: delta tiles (dt bytes per 8 rows), in: input ring; ul: first unit within the CTA, unit: within the head
   __device__ __forceinline__ void init(const LoopParams& p, uint32_t d0_, int dt_, uint32_t in, int lane, int ul_, int unit, int n, int bt0_) {
     const size_t ND = (size_t)p.N * p.D;

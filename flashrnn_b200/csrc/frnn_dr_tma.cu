@@ -3,7 +3,7 @@
 //   dR[g,n,d,p] = sum_{b,t} delta_g[b,t,n,d] * h_{t-1}[b,n,p]
 //
 // Same GEMM as frnn_dr_tc.cu (C[(g,d), p] = A^T B per head, both operands MN-major exactly as the time loops left them
-// in HBM), for 16-bit states and head dims that are multiples of 64: a 64-step stretch of one batch row is, for every 64
+// in HBM), for 16-bit states and head dims of 128 up that are multiples of 64: a 64-step stretch of one batch row is, for every 64
 // consecutive d (or p), one [64 t][64] tile with 128-byte rows -- the box of a tensor-map copy with 128-byte swizzle
 // and, unchanged, one block of a UMMA operand.  One CTA owns MT tiles of 128 rows of (g,d) (two such blocks each), all D
 // columns of p (above 256: a column tile of up to 256) and a range of 64-step chunks (split-K over gridDim.z); the MT accumulators share every h block that is
@@ -200,7 +200,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
 
 }  // namespace
 
-bool recurrent_grad_tma_supported(int D, int state_f32) { return !state_f32 && D >= 64 && D % 64 == 0; }
+bool recurrent_grad_tma_supported(int D, int state_f32) { return !state_f32 && D >= 128 && D % 64 == 0; }
 
 cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int Gr, int Gw, const void* dWx, const void* dg0,
                                       const void* states, const void* s0, float* dR, unsigned* status, int sm_count,
