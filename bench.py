@@ -459,7 +459,7 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
         "kernel_ms": {"forward_loop": fwd_ms, "backward_loop": bwd_ms, "recurrent_grad": dr_ms},
         "us_per_time_step": {"forward": 1e3 * fwd_ms / T, "backward": 1e3 * bwd_ms / T},
         "tile": {name: {"loop": nv.LOOPS[s.loop], "cluster_size": s.cluster_size, "units_per_cta": s.units_per_cta, "batch_rows": s.batch_rows,
-                        "threads": s.threads, "ctas": s.grid[0] * s.grid[1] * s.grid[2] * s.launches} for name, s in loops.items()},  # as launched
+                        "threads": s.threads, "ctas": s.grid[0] * s.grid[1] * s.grid[2]} for name, s in loops.items()},  # as launched
         "roofline": {
             "bound": "hbm", "kernel": REVERSE_KERNELS[nv.LOOPS[loops["reverse"].loop]] + (" (reverse time loop, dR and db inside)" if wide else " (reverse time loop)"),
             "achieved": achieved, "peak": job.hbm_peak, "unit": "GB/s", "frac": achieved / job.hbm_peak, "peak_source": job.peak_source,

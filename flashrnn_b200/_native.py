@@ -53,7 +53,7 @@ class FrnnPlan(ctypes.Structure):
 
 class FrnnLoopShape(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int32) for n in ("loop", "cluster_size", "units_per_cta", "batch_rows", "threads", "input_stages")] + \
-               [("grid", ctypes.c_uint32 * 3), ("launches", ctypes.c_int32)]
+               [("grid", ctypes.c_uint32 * 3)]
 
 
 class FrnnFwdArgs(ctypes.Structure):

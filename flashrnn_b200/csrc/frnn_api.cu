@@ -86,6 +86,7 @@ static BigTile big_tile(const frnn_problem& pr, int forced_bt) {
     const int u = units[i], cs = pr.D / u;
     if (pr.D % u || cs > 16 || pr.D / 16 > u) continue;
     for (int nt = 1; nt <= (pr.B > 8 ? 2 : 1); ++nt) {
+      if (nt == 1 && (pr.B + 7) / 8 > 65535) continue;  // blocks in y
       const long long tiles = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N, cost = (tiles + resident[cs] - 1) / resident[cs] * weight[i][nt - 1];
       if (best_cost < 0 || cost < best_cost) { best = {u, nt}; best_cost = cost; }
     }
@@ -125,12 +126,16 @@ static bool wide_gates_problem(const frnn_problem& pr) {
 static bool runs_wide_gates(const frnn_plan& pl) { return pl.wide_forward && !pl.prob.training; }
 static int plan_threads(const CellDims& cd, int units, int bt) { return bt == kWideBatchTile ? kWideThreads : 2 * cd.Gr * units; }
 
-// Rows / 8 the lane loops run a plan's batch tile with (the activation cache and every result are the same whatever it is).
+// Rows / 8 the lane loops run a plan's batch tile with (the activation cache and every result are the same whatever it is): 16 where the caller
+// asked for as many, or where 8-row tiles would be more than a grid holds in y; else what is faster.
 // 16-row tiles reuse a fragment of R for two products but hold twice the items per lane.  Measured at batches that fill the GPU (clk per
 // step of all CTAs, 8 against 16 rows): forward LSTM D = 64 8887 / 11285, sLSTM 9283 / 12485, LSTM D = 128 9790 / 8190, GRU D = 64
 // 8512 / 7320; reverse LSTM D = 64 9881 / 11400, GRU 8524 / 12100, sLSTM 7378 / 9263, but LSTM D = 128 (clusters) 10718 / 8900.
-static int lane_nt(const frnn_problem& pr, bool bwd, int cs, int bt) {
-  return bt >= 16 && (bwd ? cs > 1 : (pr.cell == CELL_GRU && cs == 1) || (pr.cell == CELL_LSTM && cs > 1 && pr.D == 128)) ? 2 : 1;
+constexpr int kMaxTiles = 65535;  // blocks in y
+static int lane_nt(const frnn_problem& pr, bool bwd, int cs, int bt, bool forced) {
+  if (bt < 16) return 1;
+  if (forced || (pr.B + 7) / 8 > kMaxTiles) return 2;
+  return (bwd ? cs > 1 : (pr.cell == CELL_GRU && cs == 1) || (pr.cell == CELL_LSTM && cs > 1 && pr.D == 128)) ? 2 : 1;
 }
 
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
@@ -148,8 +153,9 @@ static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) 
   const int threads = 2 * cd.Gr * U;
   if (threads > (D < 192 ? 512 : D < 256 ? 384 : 256)) return false;
   if (bt == 32 && cd.Gr * U > 192) return false;
-  return lane_kernel(kernel_cell(pr), false, D / 16, U, lane_nt(pr, false, cs, bt)).fn &&
-         lane_kernel(kernel_cell(pr), true, D / 16, U, lane_nt(pr, true, cs, bt)).fn;
+  for (int nt = 1; nt <= (bt < 16 ? 1 : 2); ++nt)
+    if (!lane_kernel(kernel_cell(pr), false, D / 16, U, nt).fn || !lane_kernel(kernel_cell(pr), true, D / 16, U, nt).fn) return false;
+  return true;
 }
 
 static int sm_count_cached();
@@ -225,6 +231,32 @@ static int validate_problem(const frnn_problem* pr, CellDims* cd) {
   return FRNN_OK;
 }
 
+// The kernel a time loop of a plan runs, with its CTAs.  fn null: there is none (a measurement variant of another tile).
+struct LoopLaunch {
+  const void* fn;
+  int threads, stages;
+  size_t smem;
+  int cs, u, rows;
+};
+static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
+  const frnn_problem& pr = pl.prob;
+  const int cell = kernel_cell(pr);
+  if (is_big(pr)) {
+    const BigTile t = big_tile(pl);
+    int nt = t.nt;
+    BigKernel k = big_kernel(cell, bwd, t.u, nt);
+    if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(cell, bwd, t.u, nt = 1);  // (sLSTM reverse from head dim 896 up)
+    if (!k.fn || pl.probe_noop_cell) return LoopLaunch{};
+    return LoopLaunch{k.fn, k.threads, bwd ? kBigStages - 1 : kBigStages, k.smem(pr.D), pr.D / t.u, t.u, 8 * nt};
+  }
+  const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.cluster_size, pl.batch_tile, pl.forced_tile);
+  const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(cell, bwd, kt, u, nt) : bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
+  return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt};
+}
+// x: the CTAs of a cluster, y: tiles of the batch, z: heads
+static int loop_tiles(const LoopLaunch& k, const frnn_problem& pr) { return (pr.B + k.rows - 1) / k.rows; }
+static dim3 loop_grid(const LoopLaunch& k, const frnn_problem& pr) { return dim3((unsigned)k.cs, (unsigned)loop_tiles(k, pr), (unsigned)pr.N); }
+
 static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_plan* out) {
   CellDims cd;
   const int rc = validate_problem(pr, &cd);
@@ -252,6 +284,9 @@ static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_pl
   const uint64_t rows = (uint64_t)((pr->B + cbt - 1) / cbt) * cbt;
   pl.cache_bytes = rows * pr->T * pl.cache_slots * pr->N * pr->D * 2;
   pl.forced_tile = cs || bt;
+  if (is_big(*pr))
+    for (int bwd = 0; bwd <= (pr->training ? 1 : 0); ++bwd)
+      if (loop_tiles(loop_of(pl, bwd), *pr) > kMaxTiles) return FRNN_ERR_SHAPE;  // (sLSTM from head dim 960 up has no 16-row reverse loop)
   const WsLayout w = workspace_layout(*pr, cd, loop_units(pl));
   pl.workspace_bytes = w.total;
   pl.grads_offset = w.grads;
@@ -291,40 +326,6 @@ static bool resolve_strides(const int64_t (&in)[4], const long long (&dense)[4],
   return true;
 }
 
-// The kernel a time loop of a plan runs, with its CTAs.  fn null: there is none (a measurement variant of another tile).
-struct LoopLaunch {
-  const void* fn;
-  int threads, stages;
-  size_t smem;
-  int cs, u, rows;
-};
-static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
-  const frnn_problem& pr = pl.prob;
-  const int cell = kernel_cell(pr);
-  if (is_big(pr)) {
-    const BigTile t = big_tile(pl);
-    int nt = t.nt;
-    BigKernel k = big_kernel(cell, bwd, t.u, nt);
-    if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(cell, bwd, t.u, nt = 1);  // (sLSTM reverse from head dim 896 up)
-    if (!k.fn || pl.probe_noop_cell) return LoopLaunch{};
-    return LoopLaunch{k.fn, k.threads, bwd ? kBigStages - 1 : kBigStages, k.smem(pr.D), pr.D / t.u, t.u, 8 * nt};
-  }
-  const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.cluster_size, pl.batch_tile);
-  const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(cell, bwd, kt, u, nt) : bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
-  return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt};
-}
-// One CTA per head and tile: x: tiles of the batch.  Clusters: x: the CTAs of one, y: tiles, which end at 65535 blocks; the 8-row tiles of a
-// batch that a plan of 16 or 32 rows takes can be more, and such a batch goes in several launches.  z: heads.  (All tiles in x, a cluster
-// after the other, or a first tile added to blockIdx.y for single CTAs too: the compiler then gives the loops other registers, sLSTM D = 192
-// training 5.03 -> 5.16 ms, LSTM D = 64 inference 427 -> 470 us.)
-constexpr int kMaxTiles = 65535;
-static int loop_tiles(const LoopLaunch& k, const frnn_problem& pr) { return (pr.B + k.rows - 1) / k.rows; }
-static dim3 loop_grid(const LoopLaunch& k, const frnn_problem& pr, int first_tile) {
-  const int left = loop_tiles(k, pr) - first_tile;
-  return k.cs == 1 ? dim3((unsigned)left, 1, (unsigned)pr.N) : dim3((unsigned)k.cs, (unsigned)(left < kMaxTiles ? left : kMaxTiles), (unsigned)pr.N);
-}
-static int loop_launches(const LoopLaunch& k, const frnn_problem& pr) { return k.cs == 1 ? 1 : (loop_tiles(k, pr) + kMaxTiles - 1) / kMaxTiles; }
-
 // `overlap`: a decoding step behind another may start, and read R, while that one still runs (everything else waits for it on the device):
 // launch and prologue, about half of a one-token step, disappear behind the step before
 static int launch_loop(const frnn_plan& pl, bool bwd, LoopParams lp, cudaStream_t stream) {
@@ -341,6 +342,7 @@ static int launch_loop(const frnn_plan& pl, bool bwd, LoopParams lp, cudaStream_
     if (e != cudaSuccess) return (int)e;
   }
   cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = loop_grid(k, pl.prob);
   cfg.blockDim = dim3((unsigned)k.threads, 1, 1);
   cfg.dynamicSmemBytes = k.smem;
   cfg.stream = stream;
@@ -359,13 +361,7 @@ static int launch_loop(const frnn_plan& pl, bool bwd, LoopParams lp, cudaStream_
   cfg.attrs = attr;
   cfg.numAttrs = na;
   void* args[1] = {&lp};
-  for (int i = 0; i < loop_launches(k, pl.prob) && e == cudaSuccess; ++i) {
-    cfg.gridDim = loop_grid(k, pl.prob, i * kMaxTiles);
-    lp.tile0 = (unsigned)(i * kMaxTiles);
-    e = cudaLaunchKernelExC(&cfg, k.fn, args);
-    lp.clear_status = 0;
-  }
-  return (int)e;
+  return (int)cudaLaunchKernelExC(&cfg, k.fn, args);
 }
 
 static int sm_count_cached() {
@@ -453,13 +449,13 @@ int FRNN_ENTRY(frnn_query_loop)(const frnn_plan* plan, int backward, frnn_loop_s
   if (is_wide(*plan) || (!backward && runs_wide_gates(*plan))) {
     const uint32_t tiles = (uint32_t)((pr.B + kWideBatchTile - 1) / kWideBatchTile);
     *out = {FRNN_LOOP_WIDE, 1, pr.D, kWideBatchTile, is_wide(*plan) ? kWideThreads : kWideGatesThreads,
-            !is_wide(*plan) ? kWideGatesStages : backward ? kWideBwdStages : kWideFwdStages, {tiles, (uint32_t)pr.N, 1}, 1};
+            !is_wide(*plan) ? kWideGatesStages : backward ? kWideBwdStages : kWideFwdStages, {tiles, (uint32_t)pr.N, 1}};
     return FRNN_OK;
   }
   const LoopLaunch k = loop_of(*plan, backward != 0);
   if (!k.fn) return FRNN_ERR_PLAN;
-  const dim3 g = loop_grid(k, pr, 0);
-  *out = {is_big(pr) ? FRNN_LOOP_BIG : FRNN_LOOP_LANE, k.cs, k.u, k.rows, k.threads, k.stages, {g.x, g.y, g.z}, loop_launches(k, pr)};
+  const dim3 g = loop_grid(k, pr);
+  *out = {is_big(pr) ? FRNN_LOOP_BIG : FRNN_LOOP_LANE, k.cs, k.u, k.rows, k.threads, k.stages, {g.x, g.y, g.z}};
   return FRNN_OK;
 }
 

@@ -15,7 +15,6 @@ template <int CELL, int U, int NT>
 struct BigBwdGeom {
   using C = Cell<CELL>;
   static constexpr int BT = 8 * NT, NT8 = NT, UNITS = U, STAGES = kBigStages - 1;
-  static __device__ __forceinline__ int row0(const LoopParams& p) { return (int)(p.tile0 + blockIdx.y) * BT; }
   static constexpr bool CL = true;
   static constexpr int WC = U / 8, W = 2 * WC, IOT = 32 * (W - WC), TH = 32 * W;  // warps of the cell, of the products; the others move the data
   static constexpr int NB = NT;
@@ -168,7 +167,7 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3, a = gid & 1;
   const int T = p.T, N = p.N, D = p.D, CS = p.CS;
-  const int n = blockIdx.z, bt0 = G::row0(p);
+  const int n = blockIdx.z, bt0 = blockIdx.y * G::BT;
   const uint32_t crank = cluster_ctarank();
   const int ptiles = D / 16, fsm = G::fsm(D), RB = G::recv_bytes(D);
 

@@ -21,7 +21,6 @@ template <int CELL, int U, int NT>
 struct BigFwdGeom {
   using C = Cell<CELL>;
   static constexpr int BT = 8 * NT, NT8 = NT, UNITS = U, STAGES = kBigStages;
-  static __device__ __forceinline__ int row0(const LoopParams& p) { return (int)(p.tile0 + blockIdx.y) * BT; }
   static constexpr bool QUAD = C::Gr > 1, CL = true;
   static constexpr int MT = QUAD ? 2 : 1, UW = QUAD ? 8 : 16;
   static constexpr int GROUPS = U / UW, W = 2 * GROUPS, IOT = 32 * GROUPS, TH = 32 * W;
@@ -78,7 +77,7 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT>::TH, 1) big_fwd_kernel
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
   const int T = p.T, N = p.N, B = p.B, D = p.D, CS = p.CS;
-  const int n = blockIdx.z, bt0 = G::row0(p);
+  const int n = blockIdx.z, bt0 = blockIdx.y * G::BT;
   const uint32_t crank = cluster_ctarank();
   const int f32 = p.state_f32;
   const size_t ND = (size_t)N * D;

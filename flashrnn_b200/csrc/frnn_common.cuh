@@ -64,12 +64,11 @@ struct LoopParams {
   unsigned* status;
   int clear_status;          // forward: CTA 0 zeroes the status block first
   int B, T, N, D;
-  unsigned tile0;            // first batch tile of the launch
+  int test_drop;             // test hook: CTA 0 of each cluster withholds one exchange message (see frnn_plan)
   int CS;                    // CTAs per cluster
   int state_f32;             // states / dstates / s0 / ds0 are fp32 (else bf16)
   float fclip, gclip;        // <= 0: off
   int grad_cut;              // backward: ignore the matrix part of the recurrent cotangent (truncated BPTT)
-  int test_drop;             // test hook: CTA 0 of each cluster withholds one exchange message (see frnn_plan)
   // element strides of the caller-produced tensors (D contiguous): Wx[b][t][g][n][.], dstates[s][b][t][n][.]
   long long wx_sb, wx_st, wx_sg, wx_sn;
   long long ds_ss, ds_sb, ds_st, ds_sn;

@@ -1022,13 +1022,13 @@ __attribute__((visibility("hidden"))) int frnn_query_loop_f32(const frnn_plan* p
   dim3 g;
   if (lane_tile(pr, plan->forced_tile != 0, backward != 0, &cs, &k)) {
     g = cluster_grid(pr, cs, k.bt);
-    *out = {FRNN_LOOP_F32_LANE, cs, pr.D / cs, k.bt, k.threads, kXStages, {g.x, g.y, g.z}, 1};
+    *out = {FRNN_LOOP_F32_LANE, cs, pr.D / cs, k.bt, k.threads, kXStages, {g.x, g.y, g.z}};
   } else if (tl.cluster) {
     g = cluster_grid(pr, tl.cs, tl.bt);
-    *out = {FRNN_LOOP_F32_CLUSTER, tl.cs, tl.u, tl.bt, XTHREADS, 0, {g.x, g.y, g.z}, 1};
+    *out = {FRNN_LOOP_F32_CLUSTER, tl.cs, tl.u, tl.bt, XTHREADS, 0, {g.x, g.y, g.z}};
   } else {
     g = stream_grid(pr);
-    *out = {FRNN_LOOP_F32_STREAM, 1, pr.D, XBT, XTHREADS, 0, {g.x, g.y, g.z}, 1};
+    *out = {FRNN_LOOP_F32_STREAM, 1, pr.D, XBT, XTHREADS, 0, {g.x, g.y, g.z}};
   }
   return FRNN_OK;
 }

@@ -30,8 +30,6 @@ template <int CELL, int KT, int U, int NT>
 struct LaneBwdGeom {
   using C = Cell<CELL>;
   static constexpr int D = KT * 16, CS = D / U, BT = 8 * NT;
-  // first batch row of the CTA (see loop_grid in frnn_api.cu)
-  static __device__ __forceinline__ int row0(const LoopParams& p) { return (int)(CS > 1 ? p.tile0 + blockIdx.y : blockIdx.x) * BT; }
   static constexpr bool CL = CS > 1;
   static constexpr int W = CL ? U / 8 : KT;       // compute warps
   static constexpr int NB = CL ? NT : 2 * NT;     // batch rows per lane (2 adjacent units each)
@@ -51,7 +49,7 @@ struct LaneBwdGeom {
   static constexpr int IN_E = GCM ? BT * CP : 0, IN_S = IN_E + (GCX ? BT * EP : 0), IN_B = IN_S + NSS * BT * SP;
   static constexpr int OFF_R = 2 * DB, OFF_I = OFF_R + 2 * RB, OFF_BAR = OFF_I + kLaneStages * IN_B;
   static constexpr size_t smem = OFF_BAR + 2 * 8;
-  static constexpr bool valid = D % U == 0 && (!CL || U % 8 == 0) && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget && (NT == 1 || CL);  // (16 rows: see lane_nt)
+  static constexpr bool valid = D % U == 0 && (!CL || U % 8 == 0) && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget;
 };
 
 // Index of the first of the two 16-byte fragments (rows gid, gid + 8) of lane 0 in the packed R^T of head n, CTA c: see
@@ -73,7 +71,7 @@ __device__ __forceinline__ void bwd_io(const LoopParams& p, uint32_t d0, uint32_
   using TP = IoTile<NNEED * BT, CPR, IOT>;                         // states at t-1
   using TQ = IoTile<NEXT * BT, CPR, IOT>;                          // cotangents at t
   using TW = IoTile<Gw * BT, U / 8, IOT>;                          // dWx
-  const int T = p.T, N = p.N, B = p.B, D = p.D, n = blockIdx.z, bt0 = G::row0(p), unit0 = (int)crank * U;
+  const int T = p.T, N = p.N, B = p.B, D = p.D, n = blockIdx.z, bt0 = blockIdx.y * BT, unit0 = (int)crank * U;
   const int es = ES ? ES : (p.state_f32 ? 4 : 2), cpr = U * es / 16;
   const size_t ND = (size_t)N * D;
 
@@ -220,7 +218,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT>::TH) lane_bwd_ker
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3, a = gid & 1;
   const int T = p.T, N = p.N, B = p.B;
-  const int n = blockIdx.z, bt0 = G::row0(p);
+  const int n = blockIdx.z, bt0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
   const size_t ND = (size_t)N * D;
   const int f32 = p.state_f32;

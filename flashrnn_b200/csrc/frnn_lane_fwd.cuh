@@ -28,8 +28,6 @@ template <int CELL, int KT, int U, int NT>
 struct LaneFwdGeom {
   using C = Cell<CELL>;
   static constexpr int D = KT * 16, CS = D / U, BT = 8 * NT;
-  // first batch row of the CTA (see loop_grid in frnn_api.cu)
-  static __device__ __forceinline__ int row0(const LoopParams& p) { return (int)(CS > 1 ? p.tile0 + blockIdx.y : blockIdx.x) * BT; }
   static constexpr bool QUAD = C::Gr > 1, CL = CS > 1;
   static constexpr int MT = QUAD ? 2 : 1;
   static constexpr int UW = QUAD ? 4 * MT : 16 * MT;  // units per warp
@@ -48,8 +46,7 @@ struct LaneFwdGeom {
   static constexpr int OUT_C = C::S * BT * SP, OUT_E = OUT_C + (GCM ? BT * CP : 0), OUT_B = OUT_E + (GCX ? BT * EP : 0);
   static constexpr int OFF_X = 2 * HB, OFF_O = OFF_X + kLaneStages * XS, OFF_BAR = OFF_O + 2 * OUT_B;
   static constexpr size_t smem = OFF_BAR + 2 * 8;
-  // 16-row tiles: only where some problem runs them (lane_nt in frnn_api.cu)
-  static constexpr bool valid = D % U == 0 && U % UW == 0 && CS <= 16 && TH <= 512 + 64 && (NT == 1 || (CELL == CELL_GRU && !CL) || (CELL == CELL_LSTM && CL && KT == 8));
+  static constexpr bool valid = D % U == 0 && U % UW == 0 && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget;
   // CTAs per SM the registers are cut for (0: as the compiler sees fit), where it measured faster, clk per step, alone or of all CTAs of a large
   // batch: clusters sLSTM D = 192 1134 -> 1100, Elman D = 128 835 -> 718, LSTM D = 128 1007 -> 925 (and 8-row tiles of a large
   // batch 8070 -> 9790, so that takes 16 rows, 8190); single CTAs GRU D = 64 743 -> 690, 8680 -> 8310, with 16 rows 9390 -> 7510; sLSTM D = 64
@@ -68,7 +65,7 @@ __device__ __forceinline__ void fwd_io(const LoopParams& p, uint32_t x0, uint32_
   using TS = IoTile<S * BT, U * (ES ? ES : 4) / 16, IOT>;          // states
   using TC = IoTile<BT, U * 2 * (G::GCM ? G::GCM : 1) / 16, IOT>;  // activations
   using TE = IoTile<BT, U / 8, IOT>;                               // fifth activations
-  const int T = p.T, N = p.N, B = p.B, D = p.D, n = blockIdx.z, bt0 = G::row0(p), unit0 = (int)crank * U;
+  const int T = p.T, N = p.N, B = p.B, D = p.D, n = blockIdx.z, bt0 = blockIdx.y * BT, unit0 = (int)crank * U;
   const int es = ES ? ES : (p.state_f32 ? 4 : 2), cpr = U * es / 16;
   const size_t ND = (size_t)N * D;
   const bool cache = GC > 0 && p.cache != nullptr;
@@ -355,7 +352,7 @@ __global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT>::TH, LaneFwdGeom<
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3, a = gid & 1;
   const int T = p.T, N = p.N, B = p.B;
-  const int n = blockIdx.z, bt0 = G::row0(p);
+  const int n = blockIdx.z, bt0 = blockIdx.y * G::BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
   const int f32 = p.state_f32;
   const size_t ND = (size_t)N * D;

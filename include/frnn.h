@@ -71,7 +71,7 @@ typedef struct frnn_problem {
 /* Launch plan chosen by frnn_query from the measured sm_100a tile table.  Replaces the reference's
  * compile-time tiling macros solved by flashrnn/autotune/constrint.py and bisected in
  * flashrnn/flashrnn/cuda_init_parametric.py:92-358.  Treat as opaque; sizes are for the caller.  The tile fields name the class the
- * plan belongs to; rows, units, threads and CTAs of each loop follow from it by rules of the loops, and frnn_query_loop reports them. */
+ * plan belongs to unless the caller asked for them; rows, units, threads and CTAs of each loop follow from it by rules of the loops, and frnn_query_loop reports them. */
 typedef struct frnn_plan {
   int32_t abi_version;
   frnn_problem prob;
@@ -164,8 +164,8 @@ int frnn_query(const frnn_problem* problem, frnn_plan* out);
 /* Same as frnn_query but with the tile forced by the caller (used to measure the tile table);
  * any of the three may be 0 = "use the table's value".  Invalid combinations return FRNN_ERR_PLAN.  wx_stages: the depth of the
  * input ring belongs to the loop; 4 (16-bit problems) is accepted and changes nothing.
- * 16-bit problems: batch_tile is the most rows a CTA takes (there is no 32-row loop any more, and 16-row ones only where they were
- * faster; above head dim 256 the loops take 8 or 16 rows as asked, with cluster_size = D / 64); frnn_query_loop says what runs.
+ * 16-bit problems: batch_tile 8 or 16 (32, accepted up to head dim 256, runs as 16: there is no 32-row loop any more), above head dim 256 with
+ * cluster_size = D / 64.
  * float32 problems: a forced tile runs the loops with R in shared memory: cluster_size 1..8 (units per CTA a multiple of 4, at most 64, its fp32 slice of R within shared
  * memory; cluster_size 1 otherwise selects the loops that stream R from L2), batch_tile 8, 4 or 2, wx_stages 0. */
 int frnn_query_tile(const frnn_problem* problem, int cluster_size, int batch_tile, int wx_stages, frnn_plan* out);
@@ -186,8 +186,7 @@ typedef struct frnn_loop_shape {
   int32_t batch_rows;        /* batch rows per CTA                                                     */
   int32_t threads;           /* per CTA                                                                */
   int32_t input_stages;      /* time steps of inputs in flight in shared memory (0: none kept there)   */
-  uint32_t grid[3];          /* CTAs of a launch                                                       */
-  int32_t launches;          /* more than 1: batches of more tiles than a grid holds (65535)           */
+  uint32_t grid[3];          /* CTAs                                                                   */
 } frnn_loop_shape;
 
 /* Pure host function: what the forward (backward = 0) or reverse time loop of a plan is launched with.  No counterpart in

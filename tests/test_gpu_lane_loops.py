@@ -10,8 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("function", ["lstm", "gru", "elman", "slstm"])
-@pytest.mark.parametrize("D,cs,bt", [(16, 1, 8), (32, 1, 16), (32, 2, 8), (64, 1, 8), (64, 1, 16), (64, 4, 16), (96, 3, 8), (96, 6, 16),
-                                     (128, 2, 16), (128, 4, 8), (192, 6, 16), (256, 8, 8)])
+@pytest.mark.parametrize("D,cs,bt", [(16, 1, 8), (16, 1, 16), (32, 1, 16), (32, 2, 8), (64, 1, 8), (64, 1, 16), (64, 4, 16), (96, 3, 8), (96, 6, 16),
+                                     (128, 2, 16), (128, 4, 8), (192, 6, 16), (256, 8, 8), (256, 8, 16)])
 @pytest.mark.parametrize("B,T,state_f32", [(1, 1, False), (7, 6, True), (9, 7, False), (17, 2, True)])
 def test_lane_loops_edges(cuda_device, function, D, cs, bt, B, T, state_f32):
     _check(function, 2, D, B, T, state_f32, cluster_size=cs, batch_tile=bt)

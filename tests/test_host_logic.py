@@ -317,14 +317,12 @@ def test_time_loops_of_huge_batches_stay_inside_the_launch_limits(function):
             s = _native.query_loop(plan, backward)
             x, y, z = s.grid
             assert 1 <= x < 2 ** 31 and 1 <= y <= 65535 and 1 <= z <= 65535, (prob.D, prob.B, s.loop, tuple(s.grid))
-            ctas, tiles = s.cluster_size * prob.N, -(-prob.B // s.batch_rows)
-            assert s.cluster_size * s.units_per_cta == prob.D and x * y * z == ctas * min(tiles, x * y * z // ctas)
-            assert (s.launches - 1) * (x * y * z // ctas) < tiles <= s.launches * (x * y * z // ctas)
+            assert s.cluster_size * s.units_per_cta == prob.D and x * y * z == s.cluster_size * prob.N * -(-prob.B // s.batch_rows)
     for D in (16, 32, 64, 96, 128, 192, 256, 320, 384, 512, 768, 1024):
         taken = 524280 if function == "elman" else 1048560
         for B in (1, 524280, 524281, 600000, 1048560):
             prob = _native.make_problem(function, B, 1, 1, D, False, True)
-            if B <= taken or (function == "elman" and D == 64):
+            if (B <= taken or (function == "elman" and D == 64)) and not (function == "slstm" and D == 1024 and B > 524280):
                 loops(prob)
             else:
                 with pytest.raises(_native.FrnnError):
@@ -355,10 +353,10 @@ def test_a_forced_tile_is_what_the_loops_run():
                 for backward, s in enumerate(loops(_native.query(mk(function, 300, 4, 2, D, False, True), D // 64, bt))):
                     rows = 8 if function == "slstm" and D == 1024 and backward else bt  # (16 do not fit its shared memory)
                     assert (_native.LOOPS[s.loop], s.cluster_size, s.units_per_cta, s.batch_rows) == ("big", D // 64, 64, rows), (function, D, bt)
-    # 16-bit, up to 256: the cluster asked for, at most the rows
+    # 16-bit, up to 256: the cluster and the rows asked for (32: 16)
     for function, D, cs, bt in [("lstm", 64, 1, 8), ("lstm", 64, 4, 16), ("gru", 128, 2, 16), ("elman", 128, 8, 32), ("slstm", 256, 16, 8)]:
         for s in loops(_native.query(mk(function, 300, 4, 2, D, False, True), cs, bt)):
-            assert (_native.LOOPS[s.loop], s.cluster_size) == ("lane", cs) and s.batch_rows <= bt
+            assert (_native.LOOPS[s.loop], s.cluster_size) == ("lane", cs) and s.batch_rows == min(bt, 16)
 
 
 def test_plans_report_the_loops_they_run():
