@@ -31,13 +31,13 @@ static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt) {
   }
   return LaneKernel{nullptr, 0, 0};
 }
-static BigKernel big_kernel(int cell, bool bwd, int u, int nt) {
+static BigKernel big_kernel(int cell, bool bwd, int u, int nt, bool dense) {
   switch (cell) {
-    case CELL_LSTM: return bwd ? big_bwd_lstm(u, nt) : big_fwd_lstm(u, nt);
-    case CELL_GRU: return bwd ? big_bwd_gru(u, nt) : big_fwd_gru(u, nt);
-    case CELL_ELMAN: return bwd ? big_bwd_elman(u, nt) : big_fwd_elman(u, nt);
-    case CELL_ELMAN_CLIP: return bwd ? big_bwd_elmanc(u, nt) : big_fwd_elmanc(u, nt);
-    case CELL_SLSTM: return bwd ? big_bwd_slstm(u, nt) : big_fwd_slstm(u, nt);
+    case CELL_LSTM: return bwd ? big_bwd_lstm(u, nt) : big_fwd_lstm(u, nt, dense);
+    case CELL_GRU: return bwd ? big_bwd_gru(u, nt) : big_fwd_gru(u, nt, dense);
+    case CELL_ELMAN: return bwd ? big_bwd_elman(u, nt) : big_fwd_elman(u, nt, dense);
+    case CELL_ELMAN_CLIP: return bwd ? big_bwd_elmanc(u, nt) : big_fwd_elmanc(u, nt, dense);
+    case CELL_SLSTM: return bwd ? big_bwd_slstm(u, nt) : big_fwd_slstm(u, nt, dense);
   }
   return BigKernel{nullptr, 0, nullptr};
 }
@@ -61,8 +61,10 @@ static int cache_slots_of(const frnn_problem& pr, const CellDims& cd) {
   return (pr.cell == CELL_ELMAN && !(pr.forward_clip > 0.f)) ? 0 : cd.GC;
 }
 
+constexpr int kMaxTiles = 65535;  // blocks in y of a launch
+
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-constexpr size_t kMaxDynSmem = 227 * 1024;
+constexpr size_t kMaxDynSmem = 227 * 1024, kSmemPerSm = 228 * 1024;
 constexpr size_t kStatusBytes = 256;
 
 // Head dims above 256 have kernels of their own (frnn_big_*.cuh).  Their plan names 64 units per CTA and clusters of D / 64; unless the
@@ -70,32 +72,56 @@ constexpr size_t kStatusBytes = 256;
 static bool is_big(const frnn_problem& pr) { return pr.D > 256; }
 constexpr int kBigPlanUnits = 64;
 
-// Units per CTA and rows / 8 of those loops: the fewest turns of all clusters through the GPU (as many as a B200 keeps resident, by size), weighed
-// with what a step of both loops takes.  Measured, 8 / 16 rows, clk: LSTM D = 384 with 32 units 3750 / 5850, 48 units 5120 / 9480, 64 units
-// 8000 / 15380; D = 512 32 units 4230 / 7080, 64 units 8950 / 17350; D = 768 48 units 8710 / 17820, 64 units 15330 / 25490; Elman D = 512 32 units
-// 3590 / 5960, 64 units 3890 / 6350.  (32 units whatever the batch: GRU B23 T227 N5 D384 1.37 ms against 1.07 with fewer CTAs per head.)
-struct BigTile { int u, nt; };
-static BigTile big_tile(const frnn_problem& pr, int forced_bt) {
-  if (forced_bt) return {kBigPlanUnits, forced_bt / 8};
-  static const int resident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 12, 11, 8, 8, 8, 8, 7, 7};
-  BigTile best = {64, 1};
+// Units per CTA and rows / 8 of one of those loops: the fewest turns of all clusters through the GPU, weighed with what a step takes.
+// `dense`: the form of Elman's 64-unit forward CTAs of which two fit an SM (frnn_big_fwd.cuh).
+struct BigTile { int u, nt; bool dense; };
+// A step alone, 8 / 16 rows, in hundredths of a 32-unit one of 8 rows: 32, 48 and 64 units up to head dim 576 (forward) and 512 (reverse), 48 and 64
+// above.  Measured, us per step: D = 384, 32, 48, 64 units: LSTM forward 1.06 / 1.54, 1.12 / 2.02, 1.68 / 2.53, reverse 1.00 / 1.63, 1.67 / 3.00, 2.60 / 5.58; GRU
+// forward 1.02 / 1.51, 1.12 / 1.95, 1.70 / 2.76, reverse 0.96 / 1.57, 1.54 / 2.63, 2.02 / 3.81; sLSTM forward 1.12 / 1.67, 1.38 / 2.38, 1.92 / 3.56, reverse
+// 1.05 / 1.73, 1.83 / 4.17, 2.98 / 6.09; Elman 0.80 / 1.25, 0.86 / 1.28, 0.82 / 1.28, reverse 0.96 / 1.44, 0.96 / 1.57, 1.03 / 1.76.  D = 768, 48, 64 units: LSTM
+// forward 2.15 / 3.86, 3.36 / 4.72, reverse 2.56 / 5.43, 4.59 / 8.45.
+constexpr int kBigWeight[4][2][5][2] = {
+    {{{100, 146}, {110, 190}, {160, 240}, {106, 186}, {160, 232}}, {{100, 163}, {168, 302}, {256, 560}, {168, 356}, {300, 540}}},   // LSTM: forward, reverse
+    {{{100, 146}, {110, 191}, {160, 260}, {106, 190}, {161, 240}}, {{100, 162}, {158, 272}, {205, 395}, {145, 290}, {250, 390}}},   // GRU
+    {{{100, 156}, {106, 160}, {102, 175}, {100, 172}, {102, 172}}, {{100, 155}, {104, 162}, {107, 178}, {104, 170}, {106, 182}}},   // Elman
+    {{{100, 146}, {123, 212}, {163, 320}, {126, 252}, {178, 300}}, {{100, 164}, {176, 405}, {286, 590}, {178, 401}, {310, 553}}}};  // sLSTM
+static BigTile big_tile(const frnn_problem& pr, bool bwd) {
+  // clusters of one CTA per SM that a B200 keeps resident, by their size (12: as if; the occupancy calculator says 8)
+  static const int resident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 14, 11, 8, 7, 8, 8, 7, 7};
+  const bool elman = pr.cell == CELL_ELMAN;
+  BigTile best = {64, 1, false};
   long long best_cost = -1;
-  const int units[3] = {32, 48, 64}, gates[3][2] = {{100, 160}, {140, 270}, {230, 400}}, elman[3][2] = {{90, 132}, {90, 146}, {100, 160}};
-  const auto& weight = pr.cell == CELL_ELMAN ? elman : gates;
+  auto offer = [&](int i, int nt, bool dense, int weight, int per_sm, int shared) {  // shared: a step beside another CTA's, in percent of one alone
+    const long long tiles = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N, alone = resident[pr.D / (32 + 16 * i)];
+    if (nt == 1 && (pr.B + 7) / 8 > kMaxTiles) return;
+    const long long turns = (tiles + alone * per_sm - 1) / (alone * per_sm), cost = tiles <= alone ? weight * 100LL : turns * weight * shared;
+    if (best_cost < 0 || cost < best_cost) { best = {32 + 16 * i, nt, dense}; best_cost = cost; }
+  };
   for (int i = 0; i < 3; ++i) {
-    const int u = units[i], cs = pr.D / u;
+    const int u = 32 + 16 * i, cs = pr.D / u;
     if (pr.D % u || cs > 16 || pr.D / 16 > u) continue;
     for (int nt = 1; nt <= (pr.B > 8 ? 2 : 1); ++nt) {
-      if (nt == 1 && (pr.B + 7) / 8 > 65535) continue;  // blocks in y
-      const long long tiles = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N, cost = (tiles + resident[cs] - 1) / resident[cs] * weight[i][nt - 1];
-      if (best_cost < 0 || cost < best_cost) { best = {u, nt}; best_cost = cost; }
+      const int weight = kBigWeight[pr.cell][bwd][pr.D > (bwd ? 512 : 576) ? 2 + i : i][nt - 1];
+      // Elman's CTAs are small: two of 32 units fit an SM (of clusters of 16 little more run at once than with one), and two of 64 units in the
+      // forward loop's dense form, beside each other 1.3 times slower.  That form has all of R in registers up to D = 512 and nearly all at 640, where it
+      // takes the place of the other; above, its step is longer, D = 1024 1.35 / 2.44 -> 1.64 / 2.89 us, and it pays where clusters queue up.  All clusters
+      // of B600, us per step, one per SM and two: N5 D320 11.1 -> 6.3, N5 D384 13.9 -> 8.5, N3 D640 22.3 -> 12.9, N2 D1024 32.4 -> 25.3.
+      const bool small = elman && u == 32 && cs <= 12;
+      if (!(elman && !bwd && u == 64 && pr.D <= 640)) offer(i, nt, false, weight, small ? 2 : 1, small ? 115 : 100);
+      if (elman && !bwd && u == 64) {
+        const bool two = big_kernel(CELL_ELMAN, false, u, nt, true).smem(pr.D) <= kSmemPerSm / 2 - 1024;
+        offer(i, nt, true, nt == 1 ? 106 + (pr.D > 640 ? (pr.D - 640) / 32 : 0) : 165 + (pr.D > 640 ? (pr.D - 640) / 8 : 0), two ? 2 : 1, two ? 130 : 100);
+      }
     }
   }
   return best;
 }
-
-static BigTile big_tile(const frnn_plan& pl) { return big_tile(pl.prob, pl.forced_tile ? pl.batch_tile : 0); }
-static int loop_units(const frnn_plan& pl) { return is_big(pl.prob) ? big_tile(pl).u : pl.units_per_cta; }
+static BigTile big_tile(const frnn_plan& pl, bool bwd) {
+  if (pl.forced_tile) return {kBigPlanUnits, pl.batch_tile / 8, pl.prob.cell == CELL_ELMAN && !bwd && pl.prob.D <= 640};
+  return big_tile(pl.prob, bwd);
+}
+// units per CTA of the reverse loop, by which R^T is packed
+static int reverse_units(const frnn_plan& pl) { return is_big(pl.prob) ? big_tile(pl, true).u : pl.units_per_cta; }
 
 // Scratch of a plan: status block, then what the plan's kernels need.  Only head dims above 256 repack R for the forward pass.
 struct WsLayout { size_t rpack_fwd, rpack_bwd, grads, dg0, total; };
@@ -131,7 +157,6 @@ static int plan_threads(const CellDims& cd, int units, int bt) { return bt == kW
 // 16-row tiles reuse a fragment of R for two products but hold twice the items per lane.  Measured at batches that fill the GPU (clk per
 // step of all CTAs, 8 against 16 rows): forward LSTM D = 64 8887 / 11285, sLSTM 9283 / 12485, LSTM D = 128 9790 / 8190, GRU D = 64
 // 8512 / 7320; reverse LSTM D = 64 9881 / 11400, GRU 8524 / 12100, sLSTM 7378 / 9263, but LSTM D = 128 (clusters) 10718 / 8900.
-constexpr int kMaxTiles = 65535;  // blocks in y
 static int lane_nt(const frnn_problem& pr, bool bwd, int cs, int bt, bool forced) {
   if (bt < 16) return 1;
   if (forced || (pr.B + 7) / 8 > kMaxTiles) return 2;
@@ -242,10 +267,10 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
   const frnn_problem& pr = pl.prob;
   const int cell = kernel_cell(pr);
   if (is_big(pr)) {
-    const BigTile t = big_tile(pl);
+    const BigTile t = big_tile(pl, bwd);
     int nt = t.nt;
-    BigKernel k = big_kernel(cell, bwd, t.u, nt);
-    if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(cell, bwd, t.u, nt = 1);  // (sLSTM reverse from head dim 896 up)
+    BigKernel k = big_kernel(cell, bwd, t.u, nt, t.dense);
+    if (k.fn && k.smem(pr.D) > kSmemBudget) k = big_kernel(cell, bwd, t.u, nt = 1, t.dense);  // (sLSTM reverse from head dim 960 up)
     if (!k.fn || pl.probe_noop_cell) return LoopLaunch{};
     return LoopLaunch{k.fn, k.threads, bwd ? kBigStages - 1 : kBigStages, k.smem(pr.D), pr.D / t.u, t.u, 8 * nt};
   }
@@ -287,7 +312,7 @@ static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_pl
   if (is_big(*pr))
     for (int bwd = 0; bwd <= (pr->training ? 1 : 0); ++bwd)
       if (loop_tiles(loop_of(pl, bwd), *pr) > kMaxTiles) return FRNN_ERR_SHAPE;  // (sLSTM from head dim 960 up has no 16-row reverse loop)
-  const WsLayout w = workspace_layout(*pr, cd, loop_units(pl));
+  const WsLayout w = workspace_layout(*pr, cd, reverse_units(pl));
   pl.workspace_bytes = w.total;
   pl.grads_offset = w.grads;
   pl.grads_count = (uint64_t)cd.Gr * pr->N * pr->D * pr->D + (uint64_t)cd.Gt * pr->N * pr->D;
@@ -304,7 +329,7 @@ static int check_plan(const frnn_plan* pl, CellDims* cd) {
   if (pl->units_per_cta * pl->cluster_size != pl->prob.D) return FRNN_ERR_PLAN;
   if (pl->threads != plan_threads(*cd, pl->units_per_cta, pl->batch_tile)) return FRNN_ERR_PLAN;
   if (pl->forced_tile != 0 && pl->forced_tile != 1) return FRNN_ERR_PLAN;
-  if (pl->workspace_bytes != workspace_layout(pl->prob, *cd, loop_units(*pl)).total) return FRNN_ERR_PLAN;
+  if (pl->workspace_bytes != workspace_layout(pl->prob, *cd, reverse_units(*pl)).total) return FRNN_ERR_PLAN;
   if (pl->wide_forward && !(pl->wide_forward == 1 && wide_gates_problem(pl->prob) && pl->cluster_size == 1 && pl->batch_tile == 16))
     return FRNN_ERR_PLAN;
   return FRNN_OK;
@@ -472,7 +497,7 @@ int FRNN_ENTRY(frnn_forward)(const frnn_plan* plan, const frnn_fwd_args* a, void
       !aligned16(a->workspace) || (a->cache && !aligned16(a->cache)))
     return FRNN_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const WsLayout w = workspace_layout(pr, cd, loop_units(*plan));
+  const WsLayout w = workspace_layout(pr, cd, reverse_units(*plan));
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   const long long nd = (long long)pr.N * pr.D;
   const long long wx_dense[4] = {(long long)pr.T * cd.Gw * nd, cd.Gw * nd, nd, pr.D};
@@ -546,7 +571,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
       !aligned16(a->ds0) || !aligned16(a->workspace) || (a->cache && !aligned16(a->cache)))
     return FRNN_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const WsLayout w = workspace_layout(pr, cd, loop_units(*plan));
+  const WsLayout w = workspace_layout(pr, cd, reverse_units(*plan));
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   float* grads = reinterpret_cast<float*>(ws + w.grads);
   const size_t nR = (size_t)cd.Gr * pr.N * pr.D * pr.D, nb = (size_t)cd.Gt * pr.N * pr.D;
@@ -558,7 +583,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   cudaError_t e = cudaSuccess;
   if ((parts & FRNN_PART_LOOP) && !is_wide(*plan)) {
     const bool big = is_big(pr);
-    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, loop_units(*plan), big, grads, nR + nb,
+    e = launch_bwd_prepare(a->R, ws + w.rpack_bwd, cd.Gr, pr.N, pr.D, reverse_units(*plan), big, grads, nR + nb,
                            reinterpret_cast<unsigned*>(ws), stream);
     if (e != cudaSuccess) return (int)e;
   } else if (parts & FRNN_PART_LOOP) {

@@ -17,7 +17,7 @@
 
 namespace FRNN_NS {
 
-template <int CELL, int U, int NT>
+template <int CELL, int U, int NT, bool DENSE>
 struct BigFwdGeom {
   using C = Cell<CELL>;
   static constexpr int BT = 8 * NT, NT8 = NT, UNITS = U, STAGES = kBigStages;
@@ -27,8 +27,10 @@ struct BigFwdGeom {
   static constexpr int NB = QUAD ? NT : 2 * NT;
   static constexpr int GCM = CacheGeom<C::GC>::MAIN;
   static constexpr bool GCX = CacheGeom<C::GC>::EXTRA;
-  // k-pairs of R per warp in registers: what the register file leaves beside the ~60 of everything else (U = 32: all there are)
-  static constexpr int KRP = QUAD ? (U == 32 ? 8 : U == 48 ? 6 : 2) : (U == 32 ? 8 : U == 48 ? 12 : 16);
+  // k-pairs of R per warp in registers: what the register file leaves beside the ~60 of everything else (U = 32: all there are).  DENSE (Elman, 64
+  // units): half of it, so that two CTAs fit an SM, 226 -> 128 registers (see big_tile in frnn_api.cu)
+  static_assert(!DENSE || (!QUAD && U == 64), "the dense form is Elman's of 64 units");
+  static constexpr int KRP = QUAD ? (U == 32 ? 8 : U == 48 ? 6 : 2) : (U == 32 || DENSE ? 8 : U == 48 ? 12 : 16);
   // Buffers for the k-pairs that fit neither registers nor shared memory: reloaded from L2 as soon as they are used, so two pairs per warp
   // are in flight all the time, the wait for h included (one at a time, loaded where it was used: D = 1024 LSTM step 10310 clk)
   static constexpr int PB = QUAD && U == 64 ? 2 : 0;
@@ -69,9 +71,9 @@ __global__ void big_pack_kernel(const elem_t* __restrict__ R, uint4* __restrict_
   out[idx] = g < C::Gr ? __ldg(reinterpret_cast<const uint4*>(R + (((size_t)g * N + n) * D + unit) * D + kp * 32 + tig * 8)) : make_uint4(0u, 0u, 0u, 0u);
 }
 
-template <int CELL, int U, int NT>
-__global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT>::TH, 1) big_fwd_kernel(const __grid_constant__ LoopParams p) {
-  using G = BigFwdGeom<CELL, U, NT>;
+template <int CELL, int U, int NT, bool DENSE>
+__global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 : 1) big_fwd_kernel(const __grid_constant__ LoopParams p) {
+  using G = BigFwdGeom<CELL, U, NT, DENSE>;
   constexpr int MT = G::MT, TH = G::TH, KRP = G::KRP, NS = G::QUAD ? 1 : 2;
   constexpr bool QUAD = G::QUAD;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -44,18 +44,31 @@ LaneKernel FRNN_INST_LANE(int kt, int u, int nt) {
   if (u == U && nt == NT) return BigKernel{reinterpret_cast<const void*>(&big_bwd_kernel<FRNN_INST_CELL, U, NT>), BigBwdGeom<FRNN_INST_CELL, U, NT>::TH, \
                                            [](int D) { return BigBwdGeom<FRNN_INST_CELL, U, NT>::smem(D); }};
 #else
-#define FRNN_BIG(U, NT) \
-  if (u == U && nt == NT) return BigKernel{reinterpret_cast<const void*>(&big_fwd_kernel<FRNN_INST_CELL, U, NT>), BigFwdGeom<FRNN_INST_CELL, U, NT>::TH, \
-                                           [](int D) { return BigFwdGeom<FRNN_INST_CELL, U, NT>::smem(D); }};
+template <int U, int NT, bool DENSE>
+static BigKernel big_entry() {
+  using G = BigFwdGeom<FRNN_INST_CELL, U, NT, DENSE>;
+  return BigKernel{reinterpret_cast<const void*>(&big_fwd_kernel<FRNN_INST_CELL, U, NT, DENSE>), G::TH, [](int D) { return G::smem(D); }};
+}
 cudaError_t FRNN_INST_PACK(const void* R, void* out, int N, int D, cudaStream_t stream) {
   const size_t frags = (size_t)N * D * D * (Cell<FRNN_INST_CELL>::Gr > 1 ? 4 : 1) / 8;
   big_pack_kernel<FRNN_INST_CELL><<<(unsigned)((frags + 255) / 256), 256, 0, stream>>>(static_cast<const elem_t*>(R), static_cast<uint4*>(out), N, D);
   return cudaGetLastError();
 }
 #endif
+#if FRNN_INST_BWD
 BigKernel FRNN_INST_BIG(int u, int nt) {
   FRNN_BIG(32, 1) FRNN_BIG(48, 1) FRNN_BIG(64, 1) FRNN_BIG(32, 2) FRNN_BIG(48, 2) FRNN_BIG(64, 2)
   return BigKernel{nullptr, 0, nullptr};
 }
+#else
+BigKernel FRNN_INST_BIG(int u, int nt, bool dense) {
+  if constexpr (Cell<FRNN_INST_CELL>::Gr == 1) {
+    if (dense) return u != 64 ? BigKernel{nullptr, 0, nullptr} : nt == 2 ? big_entry<64, 2, true>() : big_entry<64, 1, true>();
+  }
+  if (dense) return BigKernel{nullptr, 0, nullptr};
+  if (nt == 2) return u == 32 ? big_entry<32, 2, false>() : u == 48 ? big_entry<48, 2, false>() : big_entry<64, 2, false>();
+  return u == 32 ? big_entry<32, 1, false>() : u == 48 ? big_entry<48, 1, false>() : big_entry<64, 1, false>();
+}
+#endif
 
 }  // namespace FRNN_NS

@@ -25,6 +25,13 @@ def test_head_dims_above_256_edges(cuda_device, function, N, D, B, T, state_f32)
     _check(function, N, D, B, T, state_f32)
 
 
+# enough clusters that Elman's forward loop takes CTAs of which two share an SM (R in registers alone, in shared memory too), and that the
+# two loops split the head differently
+@pytest.mark.parametrize("function,N,D", [("elman", 4, 512), ("elman", 3, 704), ("elman", 2, 1024), ("lstm", 5, 320), ("slstm", 5, 384)])
+def test_head_dims_above_256_many_clusters(cuda_device, function, N, D):
+    _check(function, N, D, 147, 3, False)
+
+
 # a tile the caller asks for: 64 units per CTA whatever the table says
 @pytest.mark.parametrize("function,D,bt", [("lstm", 512, 16), ("gru", 384, 8), ("elman", 512, 16), ("slstm", 384, 16)])
 def test_head_dims_above_256_forced_tile(cuda_device, function, D, bt):
