@@ -620,16 +620,18 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
     rc = launch_loop(*plan, true, lp, stream);
     if (rc) return rc;
   }
-  // dR.  Small heads: what counts is reading whole runs of neighbouring heads (frnn_dr_small.cu).  From head dim 128 up 16-bit states: both
-  // operands are [64 steps][64] tiles a tensor-map copy delivers ready for the MMA (C2: 0.087 ms against 0.167 ms for the cp.async-fed kernel;
-  // above 256, in column tiles, LSTM D = 768 0.445 -> 0.138 ms, D = 512 N2 0.350 -> 0.139 ms, against the warp-MMA kernel).  A tile is 64 steps of one
-  // batch row: above 256, where less than half of the tiles would be used, the warp-MMA kernel is ahead (Elman B342 T26 N5 D384 0.082 against
-  // 0.179 ms).  fp32 states: the
-  // cp.async-fed tcgen05 kernel while a row tile of dR, D columns, fits one TMEM allocation, the warp-MMA kernel above.
+  // dR.  Small heads: what counts is reading whole runs of neighbouring heads (frnn_dr_small.cu).  From head dim 128 up, 16-bit states: both
+  // operands are [64 steps][64] tiles a tensor-map copy delivers ready for the MMA (LSTM B16 T1024 N4 D256 0.087 ms against 0.167 ms for the cp.async-fed
+  // kernel; above 256, in column tiles, LSTM B16 T1024 N1 D768 0.445 -> 0.138 ms, against the warp-MMA kernel).  Above 256 the warp-MMA kernel is ahead
+  //  * where less than half of a tile's 64 steps of one batch row would be used (Elman B342 T26 N5 D384 0.082 against 0.179 ms);
+  //  * on few products: the tensor-map kernel takes 18 to 31 us however few they are, the other 6 us and 16 more per 1e9 products (LSTM N1 D320, 512, 2048,
+  //    4096 rows 10, 16, 27 against 25, 21, 23 us; Elman N1 D512, 2048, 4096, 8000 rows 12, 19, 31 against 25, 23, 23; GRU N1 D768, 512, 1000 rows 16, 25 against 31, 23).
+  // fp32 states: the cp.async-fed tcgen05 kernel while a row tile of dR, D columns, fits one TMEM allocation, the warp-MMA kernel above.
+  const bool tma_pays = pr.D <= 256 || (2 * pr.T >= (pr.T + 63) / 64 * 64 && (double)nR * pr.B * pr.T >= 1.2e9);
   if ((parts & FRNN_PART_DR) && recurrent_grad_small_supported(pr.D))
     e = launch_recurrent_grad_small(pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, lp.state_f32, a->dWx, ws + w.dg0, a->states, a->s0, grads,
                                     sm_count_cached(), stream);
-  else if ((parts & FRNN_PART_DR) && recurrent_grad_tma_supported(pr.D, lp.state_f32) && (pr.D <= 256 || 2 * pr.T >= (pr.T + 63) / 64 * 64))
+  else if ((parts & FRNN_PART_DR) && recurrent_grad_tma_supported(pr.D, lp.state_f32) && tma_pays)
     e = launch_recurrent_grad_tma(pr.cell, pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, a->dWx, ws + w.dg0, a->states, a->s0, grads,
                                   reinterpret_cast<unsigned*>(ws), sm_count_cached(), stream);
   else if ((parts & FRNN_PART_DR) && pr.D <= 256)
