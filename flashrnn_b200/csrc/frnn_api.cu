@@ -154,13 +154,21 @@ static int plan_threads(const CellDims& cd, int units, int bt) { return bt == kW
 
 // Rows / 8 the lane loops run a plan's batch tile with (the activation cache and every result are the same whatever it is): 16 where the caller
 // asked for as many, or where 8-row tiles would be more than a grid holds in y; else what is faster.
-// 16-row tiles reuse a fragment of R for two products but hold twice the items per lane.  Measured at batches that fill the GPU (clk per
-// step of all CTAs, 8 against 16 rows): forward LSTM D = 64 8887 / 11285, sLSTM 9283 / 12485, LSTM D = 128 9790 / 8190, GRU D = 64
-// 8512 / 7320; reverse LSTM D = 64 9881 / 11400, GRU 8524 / 12100, sLSTM 7378 / 9263, but LSTM D = 128 (clusters) 10718 / 8900.
-static int lane_nt(const frnn_problem& pr, bool bwd, int cs, int bt, bool forced) {
+// 16-row tiles reuse a fragment of R for two products but hold twice the items per lane.  Measured at batches that fill the GPU, B1024 and N * D = 1024, T = 48,
+// us of 8 / 16 rows; forward: GRU D = 64 205 / 185, D = 32 162 / 181 (B256 N24 T128 96 / 92), D = 16 166 / 175 (B1024 N24 T128 192 / 169); LSTM D = 64 217 / 305, D = 96 356 / 324 (B200 118 / 137), D = 128 463 / 390, D = 192
+// 545 / 667, D = 256 1222 / 921; GRU D = 96 333 / 297 (B200 113 / 127), D = 128 361 / 378, D = 192 500 / 634, D = 256 1184 / 865; sLSTM D = 64 301 / 471, D = 96 493 / 419 (B256 N8
+// T128, three turns of 16-row clusters, 256 / 288),
+// D = 128 568 / 477, D = 192 624 / 754, D = 256 1280 / 1020.  Reverse: one CTA per head, D = 64, LSTM 248 / 287, GRU 218 / 299, sLSTM 304 / 369; clusters, LSTM D = 96 to
+// 256 493 / 395, 513 / 456, 1063 / 884, 1394 / 1082, GRU 381 / 386 (B200 130 / 158), 421 / 421 (B200 134 / 160), 558 / 499, 738 / 1002, sLSTM 565 / 662, 612 / 703, 1020 / 800,
+// 1442 / 1128.
+static int lane_nt(const frnn_problem& pr, bool bwd, int bt, bool forced) {
   if (bt < 16) return 1;
   if (forced || (pr.B + 7) / 8 > kMaxTiles) return 2;
-  return (bwd ? cs > 1 : (pr.cell == CELL_GRU && cs == 1) || (pr.cell == CELL_LSTM && cs > 1 && pr.D == 128)) ? 2 : 1;
+  const int D = pr.D;
+  const bool two = bwd ? D >= 96 && (pr.cell == CELL_LSTM || D == 192 || (pr.cell == CELL_SLSTM && D == 256))
+                       : D == 256 || (D <= 64 && pr.cell == CELL_GRU) || (D == 128 && pr.cell != CELL_GRU) ||
+                             (D == 96 && pr.cell == CELL_SLSTM && (pr.B + 15) / 16 * (long long)pr.N >= 180);
+  return two ? 2 : 1;
 }
 
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
@@ -274,7 +282,7 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
     if (!k.fn || pl.probe_noop_cell) return LoopLaunch{};
     return LoopLaunch{k.fn, k.threads, bwd ? kBigStages - 1 : kBigStages, k.smem(pr.D), pr.D / t.u, t.u, 8 * nt};
   }
-  const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.cluster_size, pl.batch_tile, pl.forced_tile);
+  const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.batch_tile, pl.forced_tile);
   const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(cell, bwd, kt, u, nt) : bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
   return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt};
 }
@@ -308,7 +316,7 @@ static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_pl
   // one bf16 pair per (item, slot, step) in the time loops' own order; batch rows padded to whole tiles
   const uint64_t rows = (uint64_t)((pr->B + cbt - 1) / cbt) * cbt;
   pl.cache_bytes = rows * pr->T * pl.cache_slots * pr->N * pr->D * 2;
-  pl.forced_tile = cs || bt;
+  pl.forced_tile = (cs || bt) && bt != kWideBatchTile;  // (128 rows: a loop of its own, the other loops as if nothing was asked for)
   if (is_big(*pr))
     for (int bwd = 0; bwd <= (pr->training ? 1 : 0); ++bwd)
       if (loop_tiles(loop_of(pl, bwd), *pr) > kMaxTiles) return FRNN_ERR_SHAPE;  // (sLSTM from head dim 960 up has no 16-row reverse loop)
