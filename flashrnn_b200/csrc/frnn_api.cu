@@ -206,11 +206,9 @@ static bool choose_tile(const frnn_problem& pr, const CellDims& cd, int want_cs,
     *bt_out = kWideBatchTile;
     return true;
   }
-  // Measured on B200.  Small batches (fewer than 128 (head, batch tile) pairs; every benchmark configuration but the large
-  // Elman one): 8-row batch tiles -- more CTAs, shorter steps; 16-row tiles double the step time of the serial chain.
-  // Large batches of the cells with three or four gates: 16-row tiles, whose CTAs reuse every fragment of R for two
-  // 8-row MMA columns (LSTM B1024 N16 D64: 55 -> 72 M tokens/s through the two loops; GRU 64 -> 75; sLSTM 82 -> 96; LSTM
-  // B512 N8 D128 37 -> 48; 32-row tiles spill in the reverse loop and lose).  Elman keeps 8 rows (D=128: 100 against 72).
+  // Large batches of the cells with three or four gates (128 or more (head, 16-row tile) pairs): plans of 16 rows, of which lane_nt and big_tile
+  // say what each loop takes at a time.  Small batches: 8 rows, more CTAs and shorter steps (one tile alone, 8 / 16 rows, T = 128, us of both loops:
+  // LSTM D = 64 119 / 211, D = 128 137 / 195, GRU D = 256 178 / 259), and Elman always (B1024 N6 D = 128, T = 32: 129 / 113, but B1024 N12 D = 64 84 / 88).
   const bool rows16 = cd.Gr >= 3 && (long long)((pr.B + 15) / 16) * pr.N >= 128;
   const int bt_pref[3] = {rows16 ? 16 : 8, rows16 ? 8 : 16, 32};
   for (int bi = 0; bi < 3; ++bi) {
@@ -221,23 +219,22 @@ static bool choose_tile(const frnn_problem& pr, const CellDims& cd, int want_cs,
     const int order_small[8] = {8, 4, 2, 1, 6, 3, 7, 5};
     const int order_large[8] = {1, 2, 4, 8, 3, 6, 5, 7};
     const int sms = sm_count_cached();
-    // The preferred cluster, small batch or large: 32 units per CTA from head dim 128 (clusters of D/32), the whole head in
-    // one CTA up to head dim 64.  16-unit CTAs (3-4 warps each) lose more in the exchange than they gain in the matrix
-    // phase (GRU head dim 128, 16 pairs: clusters of 8 x 16 units 3.54 ms, 4 x 32 units 3.03 ms, 2 x 64 3.37 ms; LSTM head dim
-    // 256: 16 x 16 units 1.07 ms per forward loop against 0.78 ms for 8 x 32; large batch LSTM D=128: 4 x 32 units 48, 2 x 64
-    // units 41 M tokens/s); up to head dim 64 one CTA per head, no exchange at all, wins (LSTM D=64, 2 pairs: fwd + bwd
-    // loops 0.33 ms against 0.35 / 0.36 ms for clusters of 2 / 4; Elman D=64: 0.46 against 0.65 / 0.81 ms; large batch LSTM
-    // D=64: 72 against 66 M tokens/s).
-    // Small batches fall back to smaller clusters when the preferred one would not give every CTA an SM of its own
-    // (C3 with clusters of 8: 256 CTAs on 148 SMs 3.64 ms, clusters of 4: 128 CTAs 3.05 ms); the second pass takes
+    // The preferred cluster, small batch or large: 32 units per CTA from head dim 96 (clusters of D / 32), the whole head in one CTA up to head
+    // dim 64, without any exchange.  us of both loops, one 8-row tile and T = 128 | B1024, N * D = 768 and T = 32 with the better of 8 and 16 rows:
+    // D = 64, 1, 2, 4 CTAs: LSTM 119, 129, 123 | 274, 354, 443; GRU 107, 119, 114 | 244, 301, 386; sLSTM 129, 125, 121 | 352, 468, 536; Elman 54, 92, 90 | 84,
+    // 153, 252.  D = 96, 3, 6 CTAs: LSTM 142, 125 | 436, 524.  D = 128, 2, 4, 8 CTAs: LSTM 205, 137, 135 | 534, 465, 593; GRU 175, 138, 135 | 425, 430, 543; sLSTM
+    // 206, 158, 156 | 610, 599, 762.  D = 192, 3, 6 CTAs: GRU 189, 148 | 543, 569.  D = 256, 8, 16 CTAs: LSTM 181, 190 | 1068, 1490.
+    // Small batches fall back to smaller clusters when the preferred one would not give every CTA an SM of its own; the second pass takes
     // whatever exists.
     const int cs32 = pr.D <= 64 ? 1 : ((pr.D % 32 == 0 && pr.D / 32 <= 8) ? pr.D / 32 : 0);
     for (int pass = 0; pass < 2; ++pass)
       for (int ci = -1; ci < 8; ++ci) {
-        // (large batches of the single-gate cell do best without any cluster: Elman B1024 D=128, one CTA per head 100 M
-        // tokens/s, clusters of 2 x 64 units 70)
-        if (ci < 0 && (want_cs || is_big(pr) || !cs32 || (fill && cd.Gr < 3))) continue;
-        int cs = ci < 0 ? cs32 : (want_cs ? want_cs : (fill ? order_large[ci] : order_small[ci]));
+        // Elman, where its CTAs fill the GPU or would not all get an SM: the whole head in one CTA up to head dim 128, 64 units per CTA above.  us of
+        // both loops, T = 48: B150 N10 D = 128, 1, 2, 4 CTAs 62, 74, 100; D = 192, 3, 6 CTAs, B150 N5 84, 125, N10 145, 196; D = 256, 2, 4, 8 CTAs, B150 N5
+        // 169, 119, 183, B300 N4 244, 190, 265.  (Forward alone, B1024 N4 D = 256 T64, 2, 4 CTAs 274, 307: without gradients the smallest cluster.)
+        const int first = cd.Gr > 1 || (!fill && (pass == 0 || pr.D < 192)) ? cs32 : pr.D >= 192 && (pr.training || !fill) ? pr.D / 64 : 0;
+        if (ci < 0 && (want_cs || is_big(pr) || !first)) continue;
+        int cs = ci < 0 ? first : (want_cs ? want_cs : (fill ? order_large[ci] : order_small[ci]));
         if (ci >= 0 && !fill && !want_cs && cs32 && cs > cs32) continue;  // fewer than 32 units per CTA
         if (is_big(pr) && !want_cs) cs = pr.D / kBigPlanUnits;
         const bool crowded = !fill && !want_cs && !is_big(pr) && pairs * cs > sms;
@@ -306,9 +303,9 @@ static int fill_plan(const frnn_problem* pr, int cs, int bt, int stages, frnn_pl
   pl.units_per_cta = pr->D / ccs;
   pl.batch_tile = cbt;
   pl.threads = plan_threads(cd, pl.units_per_cta, cbt);
-  // measured on B200: LSTM B1024 T512 N16 D64 (128 CTAs of 128 rows) forward loop 2.07 ms against 3.40 ms on the 16-row
-  // tiles; B512 T128 N16 (64 CTAs) 0.49 against 0.51 ms -- a step of the 128-row loop takes ~3.8 us however few CTAs run,
-  // so it pays once its CTAs occupy most of the SMs.  GRU B1024 T512 N16 D64: 1.74 against 3.25 ms.
+  // A step of the 128-row forward loop takes about 2.5 us however few CTAs run, so it pays once they occupy most of the SMs.  Inference, N16 T128, B = 512,
+  // 640, 768, 1024, 2048 (64, 80, 96, 128, 256 CTAs), us against the better of the lane loops: LSTM 299 / 255, 313 / 323, 325 / 392, 345 / 459, 696 / 901; GRU 245 /
+  // 213, 250 / 269, 255 / 326, 273 / 388, 536 / 762.
   pl.wide_forward = wide_gates_problem(*pr) && ccs == 1 && cbt == 16 &&
                     (bt == kWideBatchTile || (!cs && !bt && (long long)(pr->B / kWideBatchTile) * pr->N >= 96));
   pl.wx_stages = is_wide(pl) ? kWideFwdStages : runs_wide_gates(pl) ? kWideGatesStages : is_big(*pr) ? kBigStages : kLaneStages;
