@@ -160,14 +160,18 @@ static int plan_threads(const CellDims& cd, int units, int bt) { return bt == kW
 // T128, three turns of 16-row clusters, 256 / 288),
 // D = 128 568 / 477, D = 192 624 / 754, D = 256 1280 / 1020.  Reverse: one CTA per head, D = 64, LSTM 248 / 287, GRU 218 / 299, sLSTM 304 / 369; clusters, LSTM D = 96 to
 // 256 493 / 395, 513 / 456, 1063 / 884, 1394 / 1082, GRU 381 / 386 (B200 130 / 158), 421 / 421 (B200 134 / 160), 558 / 499, 738 / 1002, sLSTM 565 / 662, 612 / 703, 1020 / 800,
-// 1442 / 1128.
+// 1442 / 1128.  D = 16, B1024, N = 24, 40 (T = 96), 64, 96: forward sLSTM 332 / 292, 585 / 533, 369 / 328, 523 / 484, LSTM 210 / 189, 392 / 326, 248 / 229, 358 / 337 (without
+// gradients 134 / 139, 237 / 207, 149 / 166, 235 / 245), Elman 49 / 49, 138 / 81, 68 / 57, 142 / 89, reverse 131 / 82, 210 / 113, 151 / 92, 233 / 137, sLSTM 371 / 394, 648 / 586,
+// 347 / 491, 536 / 731; with a quarter of the tiles 8 rows are ahead everywhere, by 5 to 20 %.
+constexpr long long kManyTiles = 1500;
 static int lane_nt(const frnn_problem& pr, bool bwd, int bt, bool forced) {
   if (bt < 16) return 1;
   if (forced || (pr.B + 7) / 8 > kMaxTiles) return 2;
   const int D = pr.D;
+  const long long tiles = (long long)((pr.B + 15) / 16) * pr.N;
+  if (D == 16 && pr.cell != CELL_GRU) return tiles >= kManyTiles && (pr.cell == CELL_ELMAN || (!bwd && (pr.cell == CELL_SLSTM || pr.training))) ? 2 : 1;
   const bool two = bwd ? D >= 96 && (pr.cell == CELL_LSTM || D == 192 || (pr.cell == CELL_SLSTM && D == 256))
-                       : D == 256 || (D <= 64 && pr.cell == CELL_GRU) || (D == 128 && pr.cell != CELL_GRU) ||
-                             (D == 96 && pr.cell == CELL_SLSTM && (pr.B + 15) / 16 * (long long)pr.N >= 180);
+                       : D == 256 || (D <= 64 && pr.cell == CELL_GRU) || (D == 128 && pr.cell != CELL_GRU) || (D == 96 && pr.cell == CELL_SLSTM && tiles >= 180);
   return two ? 2 : 1;
 }
 
@@ -208,8 +212,9 @@ static bool choose_tile(const frnn_problem& pr, const CellDims& cd, int want_cs,
   }
   // Large batches of the cells with three or four gates (128 or more (head, 16-row tile) pairs): plans of 16 rows, of which lane_nt and big_tile
   // say what each loop takes at a time.  Small batches: 8 rows, more CTAs and shorter steps (one tile alone, 8 / 16 rows, T = 128, us of both loops:
-  // LSTM D = 64 119 / 211, D = 128 137 / 195, GRU D = 256 178 / 259), and Elman always (B1024 N6 D = 128, T = 32: 129 / 113, but B1024 N12 D = 64 84 / 88).
-  const bool rows16 = cd.Gr >= 3 && (long long)((pr.B + 15) / 16) * pr.N >= 128;
+  // LSTM D = 64 119 / 211, D = 128 137 / 195, GRU D = 256 178 / 259), and Elman above head dim 16 (B1024 N6 D = 128, T = 32: 129 / 113, but B1024 N12 D = 64 84 / 88).
+  const long long tiles16 = (long long)((pr.B + 15) / 16) * pr.N;
+  const bool rows16 = cd.Gr >= 3 ? tiles16 >= 128 : pr.D == 16 && tiles16 >= kManyTiles && (pr.B + 7) / 8 <= kMaxTiles;
   const int bt_pref[3] = {rows16 ? 16 : 8, rows16 ? 8 : 16, 32};
   for (int bi = 0; bi < 3; ++bi) {
     const int bt = want_bt ? want_bt : bt_pref[bi];

@@ -25,6 +25,17 @@ def test_head_dims_above_256_edges(cuda_device, function, N, D, B, T, state_f32)
     _check(function, N, D, B, T, state_f32)
 
 
+# head dim 16 with enough tiles for 16 rows in some of the loops
+@pytest.mark.parametrize("function", ["lstm", "elman", "slstm"])
+def test_head_dim_16_many_tiles(cuda_device, function):
+    from flashrnn_b200 import _native
+
+    N, B, T = 100, 233, 3
+    plan = _native.query(_native.make_problem(function, B, T, N, 16, False, True))
+    assert [_native.query_loop(plan, b).batch_rows for b in (False, True)] == [16, 16 if function == "elman" else 8]
+    _check(function, N, 16, B, T, False)
+
+
 # enough clusters that Elman's forward loop takes CTAs of which two share an SM (R in registers alone, in shared memory too), and that the
 # two loops split the head differently
 @pytest.mark.parametrize("function,N,D", [("elman", 4, 512), ("elman", 3, 704), ("elman", 2, 1024), ("lstm", 5, 320), ("slstm", 5, 384)])
