@@ -54,7 +54,7 @@ struct LoopParams {
   const elem_t* bias; // [Gt,N,D]
   const void* s0;            // [S,B,1,N,D]
   void* states;              // [S,B,T,N,D]  (forward: out, backward: in)
-  elem_t* cache;      // [B,T,GC,N,D] (forward: out or null, backward: in)
+  elem_t* cache;      // activations, see CacheGeom in frnn_lane.cuh (forward: out or null, backward: in)
   const void* dstates;       // [S,B,T,N,D]
   elem_t* dWx;        // [B,T,Gw,N,D]
   elem_t* dg0;        // [B,T,N,D]   GRU only: delta of the recurrent-only gate

@@ -2,7 +2,7 @@
 //
 // Per byte read there is little to compute here (D products per element of delta), so what counts is how memory is read.  A CTA owns a group
 // of heads whose elements lie side by side (HG * D of them: 128 to 512 bytes per gate and row), all their gates, and a contiguous range
-// of rows k = (b, t): every row's run goes through shared memory once, 16 bytes per cp.async along the rows, four stages deep, and
+// of rows k = (b, t): every row's run goes through shared memory once, 16 bytes per cp.async along the rows, four stages deep (eight where one CTA fills an SM), and
 // every warp keeps a 64 or 96 x 32 piece of the result in registers (mma.sync m16n8k16: the accumulators of a whole head, which
 // the tensor-map kernel holds in tensor memory, fit here too).
 // The pieces of all CTAs meet in fp32 atomics on the gradient workspace.

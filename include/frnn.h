@@ -213,7 +213,8 @@ int frnn_backward_parts(const frnn_plan* plan, const frnn_bwd_args* args, void* 
  * No counterpart in the reference.  Meant for callers that must not allocate device memory where they call the
  * library (a fixed arena handed out at start-up, a hot path on which cudaMalloc's device synchronisation is not
  * acceptable): the forward's scratch -- status block + R repacked into tensor-core fragments -- lives in a
- * file-scope device array of FRNN_NOALLOC_MAX_SCRATCH_BYTES inside the library, which every GPU that loads the
+ * file-scope device array inside the library (10.7 MiB: a third more than FRNN_NOALLOC_MAX_SCRATCH_BYTES, since the fragments of a
+ * GRU's three gates are padded to four), which every GPU that loads the
  * library holds until the process exits.  The entry point itself allocates and frees nothing, through the CUDA
  * runtime or any other library; what happens once per device is the driver loading this library's device code, see
  * "first call" below.
@@ -223,7 +224,7 @@ int frnn_backward_parts(const frnn_plan* plan, const frnn_bwd_args* args, void* 
  *     FRNN_ERR_TOO_LARGE is returned and nothing is launched.
  *   - First call on a device: it looks up the array's device address (cudaGetSymbolAddress, with that device
  *     current).  If nothing of the library has run on that device yet, this lookup makes the driver load the
- *     library's device code, which is when the 8 MiB are set aside and which may synchronise the device.  Make that
+ *     library's device code, which is when the array is set aside and which may synchronise the device.  Make that
  *     first call at start-up, before any stream capture and before the latency-critical phase.  To prime a device
  *     without launching work, call with a valid `problem` and an `args` whose tensor pointers are NULL: the address
  *     is looked up, then the call returns FRNN_ERR_NULL and nothing is enqueued.
