@@ -25,6 +25,12 @@ def test_head_dims_above_256_edges(cuda_device, function, N, D, B, T, state_f32)
     _check(function, N, D, B, T, state_f32)
 
 
+# the clusters that large batches run with 16 rows
+@pytest.mark.parametrize("function,D,cs", [("slstm", 96, 3), ("lstm", 96, 3), ("slstm", 128, 4), ("lstm", 128, 4), ("gru", 192, 6), ("gru", 256, 8)])
+def test_lane_loops_16_rows(cuda_device, function, D, cs):
+    _check(function, 2, D, 25, 8, function == "slstm", cluster_size=cs, batch_tile=16)
+
+
 # head dim 16 with enough tiles for 16 rows in some of the loops
 @pytest.mark.parametrize("function", ["lstm", "elman", "slstm"])
 def test_head_dim_16_many_tiles(cuda_device, function):
