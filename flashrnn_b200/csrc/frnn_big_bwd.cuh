@@ -42,7 +42,8 @@ struct BigBwdGeom {
   static __host__ __device__ constexpr size_t smem(int D) { return (size_t)off_r(D) + (size_t)fsm(D) * W * MG * 1024; }
 };
 
-// One compute lane: two adjacent units of NB batch rows.
+// One compute lane: two adjacent units of NB batch rows.  (lane_bwd_kernel has the same in local variables.  With this struct in its place
+// the compiler gives its loops other registers: LSTM D = 96 B1024 502 -> 646 us, D = 64 582 -> 621, GRU D = 128 536 -> 563, geometric mean of 182 problems 1.00.)
 template <int CELL, class G, class F2>
 struct BwdLane {
   using C = Cell<CELL>;
