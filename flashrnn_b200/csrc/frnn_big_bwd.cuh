@@ -165,7 +165,7 @@ template <int CELL, int U, int NT>
 __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel(const __grid_constant__ LoopParams p) {
   using G = BigBwdGeom<CELL, U, NT>;
   constexpr int MT = G::MT, NB = G::NB, W = G::W, DB = G::DB, DT = G::DT, KP = G::KP, KRP = G::KRP, TH = G::TH;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
   const int gid = lane >> 2, tig = lane & 3, a = gid & 1;
   const int T = p.T, N = p.N, D = p.D, CS = p.CS;
   const int n = blockIdx.z, bt0 = blockIdx.y * G::BT;
@@ -311,14 +311,12 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) rec[nb] = v_pair<S2>(0.f, 0.f);
     auto wait_partials = [&](int j, int t) {  // sums produced in step index j
-      if (!poisoned) {
-        if (!mbar_wait_bounded(&full[j & 1], (uint32_t)((j >> 1) & 1))) {
-          poisoned = true;
-          *gave_up = 1;
-          report_timeout(p.status, t);
-        }
-        else if (tid == 0 && j + 2 < T) mbar_arrive_expect_tx(&full[j & 1], RB);
+      if (!mbar_wait_warp(&full[j & 1], (uint32_t)((j >> 1) & 1), poisoned)) {
+        poisoned = true;
+        *gave_up = 1;
+        if (lane == 0) report_timeout(p.status, t);
       }
+      mbar_arrive_expect_tx_if(tid == 0 && j + 2 < T && !poisoned, &full[j & 1], RB);
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
         S2 x = v_pair<S2>(0.f, 0.f), y = x;

@@ -155,6 +155,9 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_addr, uint32_t ran
   return r;
 }
 
+// threadIdx.x / 32, known to the compiler to be the same in all lanes of a warp
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // ---- programmatic dependent launch (decoding steps, launched with the attribute): the next launch may start now / every launch in front of
 // this one has completed and its writes are visible
 __device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -197,6 +200,32 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
       if (mbar_try_wait(bar, parity)) return true;
     if (global_timer_ns() - t0 > 1000000000ull) return false;
   }
+}
+// The same for a converged warp of which every lane waits.  The branch depends on a vote, which the compiler knows to be the same in all lanes: a
+// phase that is complete costs 50 clk, with a branch on each lane's own result (mbar_wait_bounded) 125 -- in the time loops that is behind the
+// last arrival, in every step.  `skip`: an earlier wait of this warp expired, do not wait.  The result is the same in all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, bool skip = false) {
+  auto done = [&]() {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %3, 0;\n\tsetp.eq.u32 p, 0, 0;\n\t"
+        "@!q mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"((uint32_t)skip) : "memory");
+    return __all_sync(0xffffffffu, ok != 0) != 0;
+  };
+  if (done()) return true;
+  const uint64_t t0 = global_timer_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 256; ++i)
+      if (done()) return true;
+    if (__any_sync(0xffffffffu, global_timer_ns() - t0 > 1000000000ull)) return false;
+  }
+}
+// mbar_arrive_expect_tx where `on`, without a branch
+__device__ __forceinline__ void mbar_arrive_expect_tx_if(bool on, uint64_t* bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}"
+               ::"r"(smem_u32(bar)), "r"(bytes), "r"((uint32_t)on) : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // copies `bytes` (multiple of 16) from this CTA's shared memory to the same offset space of another CTA of the

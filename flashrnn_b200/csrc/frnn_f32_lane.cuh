@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32
   using G = XFwdGeom<CELL, CL, LPU, KQ, BT>;
   using C = Cell<CELL>;
   constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, HB = G::HB, UW = 32 / LPU, GP = G::GP, NR = G::NR, KS = G::KS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = CL ? warp_index() : tid >> 5;
   const int D = p.D, U = p.U, Q = U >> 2, CS = p.CS, T = p.T, B = p.B, N = p.N;
   const int n = blockIdx.z, b0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32
   const uint32_t hr = ht + (uint32_t)(kk * BT) * 16u, sw = (uint32_t)(kk * BT >> 3) & (BT - 1);
   const int drop_t = (p.test_drop && crank == 0) ? 1 : -1;  // test hook: CTA 0 withholds its message of step 1
   const bool cache = GC > 0 && p.cache != nullptr;
-  bool poisoned = false;  // a wait of this thread expired: it neither waits nor sends any more and the loop runs out
+  bool poisoned = false;  // a wait of this warp expired: it neither waits nor sends any more and the loop runs out
   __syncthreads();        // Wx of steps 0 and 1 has landed
   int stage = 0;
   for (int t = 0; t < T; ++t) {
@@ -238,12 +238,12 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32
     float wx[Gw];
 #pragma unroll
     for (int g = 0; g < Gw; ++g) wx[g] = __uint_as_float(lds32(ring + stage * xs + g * plane + word));
-    if (CL && t > 0 && !poisoned) {
-      if (!mbar_wait_bounded(&full[prv], (uint32_t)(((t - 1) >> 1) & 1))) {
+    if (CL && t > 0) {
+      if (!mbar_wait_warp(&full[prv], (uint32_t)(((t - 1) >> 1) & 1), poisoned)) {
         poisoned = true;
-        report_timeout(p.status, t);
+        if (lane == 0) report_timeout(p.status, t);
       }
-      else if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(&full[prv], step_bytes);
+      mbar_arrive_expect_tx_if(tid == 0 && t + 2 < T && !poisoned, &full[prv], step_bytes);
     }
     float v[NR][BT], pre[Gr], gx[Gt];
 #pragma unroll
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, CL, LPU, KQ, TB, BT>::MAXTH, 1)
   using C = Cell<CELL>;
   constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, NNEED = C::NNEED, NEXT = C::NEXT, NIN = G::NIN, KS = G::KS, UW = 32 / LPU;
   constexpr int GSH = Gr == 3 ? 1 : 0;  // GRU: plane 0 is the recurrent-only gate, which goes to dg0
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = CL ? warp_index() : tid >> 5;
   const int D = p.D, U = p.U, Q = U >> 2, CS = p.CS, T = p.T, B = p.B, N = p.N;
   const int n = blockIdx.z, b0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
@@ -490,13 +490,11 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, CL, LPU, KQ, TB, BT>::MAXTH, 1)
   const bool drop = p.test_drop && crank == 0;  // test hook: CTA 0 withholds its message of the second step
   bool poisoned = false;
   auto collect = [&](int j, int t) {  // CS > 1: the partial sums of step index j
-    if (!poisoned) {
-      if (!mbar_wait_bounded(&full[j & 1], (uint32_t)((j >> 1) & 1))) {
-        poisoned = true;
-        report_timeout(p.status, t);
-      }
-      else if (tid == 0 && j + 2 < T) mbar_arrive_expect_tx(&full[j & 1], rb);
+    if (!mbar_wait_warp(&full[j & 1], (uint32_t)((j >> 1) & 1), poisoned)) {
+      poisoned = true;
+      if (lane == 0) report_timeout(p.status, t);
     }
+    mbar_arrive_expect_tx_if(tid == 0 && j + 2 < T && !poisoned, &full[j & 1], rb);
     float x = 0.f, y = 0.f;
 #pragma unroll 2
     for (int c = 0; c < CS; ++c) {

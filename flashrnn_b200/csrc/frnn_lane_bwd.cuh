@@ -49,6 +49,11 @@ struct LaneBwdGeom {
   static constexpr int IN_E = GCM ? BT * CP : 0, IN_S = IN_E + (GCX ? BT * EP : 0), IN_B = IN_S + NSS * BT * SP;
   static constexpr int OFF_R = 2 * DB, OFF_I = OFF_R + 2 * RB, OFF_BAR = OFF_I + kLaneStages * IN_B;
   static constexpr size_t smem = OFF_BAR + 2 * 8;
+  // Waits by a vote (mbar_wait_warp), except where the registers that takes cost large batches more: 32 steps of B1024, GRU D = 96 231 -> 241 us, D = 192
+  // 273 -> 287.
+  static constexpr bool VOTE = CL && !(CELL == CELL_GRU && (KT == 6 || KT == 12));
+  // CTAs per SM the registers are cut for (0: as the compiler sees fit), where a few registers more would cost large batches a CTA
+  static constexpr int MINB = CL && NT == 1 && KT >= 12 && C::Gr == 1 && U == 64 ? 3 : 0;
   static constexpr bool valid = D % U == 0 && (!CL || U % 8 == 0) && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget;
 };
 
@@ -204,7 +209,7 @@ __device__ __forceinline__ void lane_bwd_io(const LoopParams& p, uint32_t d0, ui
 }
 
 template <int CELL, int KT, int U, int NT>
-__global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT>::TH) lane_bwd_kernel(const __grid_constant__ LoopParams p) {
+__global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT>::TH, LaneBwdGeom<CELL, KT, U, NT>::MINB) lane_bwd_kernel(const __grid_constant__ LoopParams p) {
   using G = LaneBwdGeom<CELL, KT, U, NT>;
   using C = Cell<CELL>;
   // packed arithmetic where it measured faster (LSTM D = 64, one CTA per head: B1024 N16, 11551 -> 9881 clk per step of all CTAs)
@@ -215,7 +220,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT>::TH) lane_bwd_ker
   constexpr bool CL = G::CL;
   constexpr int NS = acc_sets(MT * NT, W, G::KS, 4);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = G::VOTE ? warp_index() : tid >> 5;
   const int gid = lane >> 2, tig = lane & 3, a = gid & 1;
   const int T = p.T, N = p.N, B = p.B;
   const int n = blockIdx.z, bt0 = blockIdx.y * BT;
@@ -309,18 +314,19 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT>::TH) lane_bwd_ker
   // where this lane's partial sums arrive: source c at + c * (U/16) * NT * 512, batch tile nt at + nt * 512
   const uint32_t rsrc = recv + (uint32_t)((ul >> 4) * NT * 512 + (((ul & 15) >> 1) * 4 + tig) * 16 + a * 8);
   const bool drop = p.test_drop && crank == 0;  // test hook: CTA 0 withholds its first message
-  bool poisoned = false;  // a wait of this thread expired: it neither waits nor sends any more and the loop runs out
+  bool poisoned = false;  // a wait expired: it neither waits nor sends any more and the loop runs out
   F2 rec[NB];             // matrix part of dh of the step about to run (CS == 1: handed over in registers)
 #pragma unroll
   for (int nb = 0; nb < NB; ++nb) rec[nb] = v_pair<F2>(0.f, 0.f);
 
   auto wait_partials = [&](int j, int t) {  // sums produced in step index j
-    if (!poisoned) {
-      if (!mbar_wait_bounded(&full[j & 1], (uint32_t)((j >> 1) & 1))) {
-        poisoned = true;
-        report_timeout(p.status, t);
-      }
-      // re-arm for step index j + 2; never after an expired wait: that phase is still open, no arrival left to give
+    auto expired = [&]() { poisoned = true; report_timeout(p.status, t); };
+    // re-arm for step index j + 2, never after an expired wait: that phase is still open, no arrival left to give
+    if constexpr (G::VOTE) {
+      if (!mbar_wait_warp(&full[j & 1], (uint32_t)((j >> 1) & 1), poisoned)) expired();
+      mbar_arrive_expect_tx_if(tid == 0 && j + 2 < T && !poisoned, &full[j & 1], G::RB);
+    } else if (!poisoned) {
+      if (!mbar_wait_bounded(&full[j & 1], (uint32_t)((j >> 1) & 1))) expired();
       else if (tid == 0 && j + 2 < T) mbar_arrive_expect_tx(&full[j & 1], G::RB);
     }
   };

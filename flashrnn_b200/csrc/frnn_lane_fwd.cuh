@@ -51,6 +51,9 @@ struct LaneFwdGeom {
   // batch: clusters sLSTM D = 192 1134 -> 1100, Elman D = 128 835 -> 718, LSTM D = 128 1007 -> 925 (and 8-row tiles of a large
   // batch 8070 -> 9790, so that takes 16 rows, 8190); single CTAs GRU D = 64 743 -> 690, 8680 -> 8310, with 16 rows 9390 -> 7510; sLSTM D = 64
   // 9960 -> 9280.  Not LSTM D = 64 (813 -> 780, but 8940 -> 9290).
+  // Waits by a vote (mbar_wait_warp), except where the registers that takes cost large batches more: 48 steps of B200, sLSTM D = 192 124 -> 163 us (one CTA
+  // per SM instead of two), GRU D = 192 101 -> 115, Elman D = 192 in CTAs of 64 units 30.8 -> 33.1.
+  static constexpr bool VOTE = CL && !(KT == 12 && NT == 1 && (CELL == CELL_SLSTM || CELL == CELL_GRU || (!QUAD && U == 64)));
   static constexpr int MINB = CL ? (KT >= 12 || !QUAD ? 1 : CELL == CELL_LSTM && KT == 8 ? 2 : 0) : (KT == 4 && (CELL == CELL_GRU || CELL == CELL_SLSTM)) || NT == 2 ? 2 : 0;
 };
 
@@ -349,7 +352,7 @@ __global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT>::TH, LaneFwdGeom<
   constexpr bool SUMS_EARLY = QUAD && CL;
   constexpr uint32_t STEP_BYTES = (uint32_t)(CS * U * G::BT * 2);  // what one step's exchange delivers to a CTA
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = G::VOTE ? warp_index() : tid >> 5;
   const int gid = lane >> 2, tig = lane & 3, a = gid & 1;
   const int T = p.T, N = p.N, B = p.B;
   const int n = blockIdx.z, bt0 = blockIdx.y * G::BT;
@@ -438,7 +441,7 @@ __global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT>::TH, LaneFwdGeom<
     }
   }
   const int drop_t = (p.test_drop && crank == 0) ? 1 : -1;  // test hook: CTA 0 withholds its message of step 1
-  bool poisoned = false;  // a wait of this thread expired: it neither waits nor sends any more and the loop runs out
+  bool poisoned = false;  // a wait expired: it neither waits nor sends any more and the loop runs out
   auto expired = [&](int t) { poisoned = true; report_timeout(p.status, t); };
   const bool cache = p.cache != nullptr;
   float acc[MT][NT][4], accn[MT][NT][4];
@@ -448,9 +451,14 @@ __global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT>::TH, LaneFwdGeom<
   int stage = 0;
   for (int t = 0; t < T; ++t) {
     const int prv = (t + 1) & 1, nxt = t & 1;
-    if (CL && t > 0 && !poisoned) {
+    // re-arm for h_{t+1} never after an expired wait: that phase is still open and has no arrival left to give
+    if constexpr (G::VOTE) {
+      if (t > 0) {
+        if (!mbar_wait_warp(&full[prv], (uint32_t)(((t - 1) >> 1) & 1), poisoned)) expired(t);
+        mbar_arrive_expect_tx_if(tid == 0 && t + 2 < T && !poisoned, &full[prv], STEP_BYTES);
+      }
+    } else if (CL && t > 0 && !poisoned) {
       if (!mbar_wait_bounded(&full[prv], (uint32_t)(((t - 1) >> 1) & 1))) expired(t);
-      // re-arm for h_{t+1}; never after an expired wait: that phase is still open and has no arrival left to give
       else if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(&full[prv], STEP_BYTES);
     }
 #pragma unroll
