@@ -31,6 +31,16 @@ static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt) {
   }
   return LaneKernel{nullptr, 0, 0};
 }
+static LaneKernel lane_help_kernel(int cell, int kt) {
+  switch (cell) {
+    case CELL_LSTM: return lane_bwd_help_lstm(kt);
+    case CELL_GRU: return lane_bwd_help_gru(kt);
+    case CELL_ELMAN: return lane_bwd_help_elman(kt);
+    case CELL_ELMAN_CLIP: return lane_bwd_help_elmanc(kt);
+    case CELL_SLSTM: return lane_bwd_help_slstm(kt);
+  }
+  return LaneKernel{nullptr, 0, 0};
+}
 static BigKernel big_kernel(int cell, bool bwd, int u, int nt, bool dense) {
   switch (cell) {
     case CELL_LSTM: return bwd ? big_bwd_lstm(u, nt) : big_fwd_lstm(u, nt, dense);
@@ -72,6 +82,9 @@ constexpr size_t kStatusBytes = 256;
 static bool is_big(const frnn_problem& pr) { return pr.D > 256; }
 constexpr int kBigPlanUnits = 64;
 
+// Clusters of one CTA per SM that a B200 keeps resident, by their size (12: as if; the occupancy calculator says 8)
+constexpr int kResident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 14, 11, 8, 7, 8, 8, 7, 7};
+
 // Units per CTA and rows / 8 of one of those loops: the fewest turns of all clusters through the GPU, weighed with what a step takes.
 // `dense`: the form of Elman's 64-unit forward CTAs of which two fit an SM (frnn_big_fwd.cuh).
 struct BigTile { int u, nt; bool dense; };
@@ -86,13 +99,11 @@ constexpr int kBigWeight[4][2][5][2] = {
     {{{100, 156}, {106, 160}, {102, 175}, {100, 172}, {102, 172}}, {{100, 155}, {104, 162}, {107, 178}, {104, 170}, {106, 182}}},   // Elman
     {{{100, 146}, {123, 212}, {163, 320}, {126, 252}, {178, 300}}, {{100, 164}, {176, 405}, {286, 590}, {178, 401}, {310, 553}}}};  // sLSTM
 static BigTile big_tile(const frnn_problem& pr, bool bwd) {
-  // clusters of one CTA per SM that a B200 keeps resident, by their size (12: as if; the occupancy calculator says 8)
-  static const int resident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 14, 11, 8, 7, 8, 8, 7, 7};
   const bool elman = pr.cell == CELL_ELMAN;
   BigTile best = {64, 1, false};
   long long best_cost = -1;
   auto offer = [&](int i, int nt, bool dense, int weight, int per_sm, int shared) {  // shared: a step beside another CTA's, in percent of one alone
-    const long long tiles = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N, alone = resident[pr.D / (32 + 16 * i)];
+    const long long tiles = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N, alone = kResident[pr.D / (32 + 16 * i)];
     if (nt == 1 && (pr.B + 7) / 8 > kMaxTiles) return;
     const long long turns = (tiles + alone * per_sm - 1) / (alone * per_sm), cost = tiles <= alone ? weight * 100LL : turns * weight * shared;
     if (best_cost < 0 || cost < best_cost) { best = {32 + 16 * i, nt, dense}; best_cost = cost; }
@@ -173,6 +184,16 @@ static int lane_nt(const frnn_problem& pr, bool bwd, int bt, bool forced) {
   const bool two = bwd ? D >= 96 && (pr.cell == CELL_LSTM || D == 192 || (pr.cell == CELL_SLSTM && D == 256))
                        : D == 256 || (D <= 64 && pr.cell == CELL_GRU) || (D == 128 && pr.cell != CELL_GRU) || (D == 96 && pr.cell == CELL_SLSTM && tiles >= 180);
   return two ? 2 : 1;
+}
+
+// The reverse lane loop with warps that only multiply (8-row clusters of 32-unit CTAs).  Where every CTA has an SM to itself, always: us per 256 steps of one tile
+// without / with, beside the geometry.  With more CTAs only where it is ahead there too; us of B200 T48 and N * D = 768, without / with: LSTM D = 96 111 / 99, 192 176 / 167, 256
+// 215 / 195; sLSTM D = 96 122 / 110, 128 124 / 115, 192 183 / 171, 256 218 / 190; GRU D = 96 80 / 72 (B1024 T32 233 / 212), but 128 83 / 97, 192 118 / 157, 256 136 / 172; Elman D = 96 41 / 38,
+// but B1024 T32 124 / 130.
+static bool lane_help(const frnn_problem& pr, int cs, int u, int nt) {
+  if (cs < 2 || cs > 16 || u != 32 || nt != 1) return false;
+  const bool alone = (long long)((pr.B + 7) / 8) * pr.N <= kResident[cs];
+  return alone || pr.cell == CELL_LSTM || pr.cell == CELL_SLSTM || (pr.cell == CELL_GRU && pr.D == 96);
 }
 
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
@@ -285,7 +306,11 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
     return LoopLaunch{k.fn, k.threads, bwd ? kBigStages - 1 : kBigStages, k.smem(pr.D), pr.D / t.u, t.u, 8 * nt};
   }
   const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.batch_tile, pl.forced_tile);
-  const LaneKernel k = !pl.probe_noop_cell ? lane_kernel(cell, bwd, kt, u, nt) : bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
+  LaneKernel k = !pl.probe_noop_cell ? lane_kernel(cell, bwd, kt, u, nt) : bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
+  if (bwd && !pl.probe_noop_cell && lane_help(pr, pl.cluster_size, u, nt)) {
+    const LaneKernel h = lane_help_kernel(cell, kt);
+    if (h.fn) k = h;
+  }
   return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt};
 }
 // x: the CTAs of a cluster, y: tiles of the batch, z: heads

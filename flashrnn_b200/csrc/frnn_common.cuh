@@ -340,6 +340,10 @@ template <class V, class F> __device__ __forceinline__ V v_map(V a, V b, V c, F 
   const float2 x = v_get(a), y = v_get(b), z = v_get(c);
   return v_pair<V>(f(x.x, y.x, z.x), f(x.y, y.y, z.y));
 }
+// the value is computed in front of what follows in the program, not behind it
+__device__ __forceinline__ void v_pin(float& a) { asm volatile("" : "+f"(a)); }
+__device__ __forceinline__ void v_pin(S2& a) { asm volatile("" : "+f"(a.x), "+f"(a.y)); }
+__device__ __forceinline__ void v_pin(P2& a) { asm volatile("" : "+l"(a.v)); }
 template <class V> __device__ __forceinline__ V v_neg(V a) { return v_mul(a, v_const<V>(-1.f)); }
 template <class V> __device__ __forceinline__ V v_sub(V a, V b) { return v_fma(b, v_const<V>(-1.f), a); }
 template <class V> __device__ __forceinline__ V v_one_minus(V a) { return v_fma(a, v_const<V>(-1.f), v_const<V>(1.f)); }

@@ -7,24 +7,42 @@ namespace FRNN_NS {
 
 // ---- lane loops (head dims up to 256): head dim / 16, units per CTA, batch tile / 8
 #if FRNN_INST_BWD
-#define FRNN_GEOM LaneBwdGeom
-#define FRNN_KERNEL lane_bwd_kernel
+#define FRNN_GEOM(...) LaneBwdGeom<__VA_ARGS__, false>
+#define FRNN_KERNEL(...) lane_bwd_kernel<__VA_ARGS__, false>
 #else
-#define FRNN_GEOM LaneFwdGeom
-#define FRNN_KERNEL lane_fwd_kernel
+#define FRNN_GEOM(...) LaneFwdGeom<__VA_ARGS__>
+#define FRNN_KERNEL(...) lane_fwd_kernel<__VA_ARGS__>
 #endif
 
-template <int KT, int U, int NT, bool V = FRNN_GEOM<FRNN_INST_CELL, KT, U, NT>::valid>
+template <int KT, int U, int NT, bool V = FRNN_GEOM(FRNN_INST_CELL, KT, U, NT)::valid>
 struct LaneEntry {
   static LaneKernel get() { return LaneKernel{nullptr, 0, 0}; }
 };
 template <int KT, int U, int NT>
 struct LaneEntry<KT, U, NT, true> {
   static LaneKernel get() {
-    using G = FRNN_GEOM<FRNN_INST_CELL, KT, U, NT>;
-    return LaneKernel{reinterpret_cast<const void*>(&FRNN_KERNEL<FRNN_INST_CELL, KT, U, NT>), G::TH, G::smem};
+    using G = FRNN_GEOM(FRNN_INST_CELL, KT, U, NT);
+    return LaneKernel{reinterpret_cast<const void*>(&FRNN_KERNEL(FRNN_INST_CELL, KT, U, NT)), G::TH, G::smem};
   }
 };
+
+#if FRNN_INST_BWD
+// the reverse loops with warps that only multiply (clusters of 32-unit CTAs, 8 rows), null where there is none
+template <int KT, bool V = LaneBwdGeom<FRNN_INST_CELL, KT, 32, 1, true>::valid>
+struct HelpEntry {
+  static LaneKernel get() { return LaneKernel{nullptr, 0, 0}; }
+};
+template <int KT>
+struct HelpEntry<KT, true> {
+  static LaneKernel get() {
+    using G = LaneBwdGeom<FRNN_INST_CELL, KT, 32, 1, true>;
+    return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<FRNN_INST_CELL, KT, 32, 1, true>), G::TH, G::smem};
+  }
+};
+LaneKernel FRNN_INST_HELP(int kt) {
+  return kt == 6 ? HelpEntry<6>::get() : kt == 8 ? HelpEntry<8>::get() : kt == 12 ? HelpEntry<12>::get() : kt == 16 ? HelpEntry<16>::get() : LaneKernel{nullptr, 0, 0};
+}
+#endif
 
 LaneKernel FRNN_INST_LANE(int kt, int u, int nt) {
 #define FRNN_CASE(KT, U)                                         \

@@ -51,9 +51,9 @@ struct LaneFwdGeom {
   // batch: clusters sLSTM D = 192 1134 -> 1100, Elman D = 128 835 -> 718, LSTM D = 128 1007 -> 925 (and 8-row tiles of a large
   // batch 8070 -> 9790, so that takes 16 rows, 8190); single CTAs GRU D = 64 743 -> 690, 8680 -> 8310, with 16 rows 9390 -> 7510; sLSTM D = 64
   // 9960 -> 9280.  Not LSTM D = 64 (813 -> 780, but 8940 -> 9290).
-  // Waits by a vote (mbar_wait_warp), except where the registers that takes cost large batches more: 48 steps of B200, sLSTM D = 192 124 -> 163 us (one CTA
-  // per SM instead of two), GRU D = 192 101 -> 115, Elman D = 192 in CTAs of 64 units 30.8 -> 33.1.
-  static constexpr bool VOTE = CL && !(KT == 12 && NT == 1 && (CELL == CELL_SLSTM || CELL == CELL_GRU || (!QUAD && U == 64)));
+  // Waits by a vote (mbar_wait_warp), except where the registers that takes cost large batches more: 48 steps of B200, GRU D = 192
+  // 101 -> 115 us, Elman D = 192 in CTAs of 64 units 30.8 -> 33.1.
+  static constexpr bool VOTE = CL && !(KT == 12 && NT == 1 && (CELL == CELL_GRU || (!QUAD && U == 64)));
   static constexpr int MINB = CL ? (KT >= 12 || !QUAD ? 1 : CELL == CELL_LSTM && KT == 8 ? 2 : 0) : (KT == 4 && (CELL == CELL_GRU || CELL == CELL_SLSTM)) || NT == 2 ? 2 : 0;
 };
 

@@ -42,6 +42,22 @@ def test_head_dim_16_many_tiles(cuda_device, function):
     _check(function, N, 16, B, T, False)
 
 
+# reverse loops with warps that only multiply, and the same head dims where there are more clusters than SMs for them: six, eight and ten warps
+# beside each other, p tiles that divide among them and that do not, sums that stay in the CTA and that do not
+@pytest.mark.parametrize("function,N,D,B,alone", [("lstm", 1, 96, 9, True), ("gru", 3, 96, 1, True), ("elman", 2, 96, 8, True), ("gru", 1, 128, 10, True),
+                                                  ("slstm", 2, 128, 9, True), ("elman", 1, 128, 7, True), ("lstm", 3, 192, 9, True), ("gru", 2, 192, 3, True),
+                                                  ("slstm", 1, 192, 17, True), ("elman", 1, 192, 9, True), ("lstm", 2, 256, 1, True), ("gru", 1, 256, 15, True),
+                                                  ("slstm", 1, 256, 8, True), ("elman", 2, 256, 9, True), ("lstm", 23, 192, 3, True), ("slstm", 16, 256, 2, True),
+                                                  ("gru", 46, 96, 2, True), ("gru", 34, 128, 3, False), ("gru", 23, 192, 2, False), ("elman", 34, 128, 1, False)])
+def test_reverse_loops_with_multiplying_warps(cuda_device, function, N, D, B, alone):
+    from flashrnn_b200 import _native
+
+    few = _native.query_loop(_native.query(_native.make_problem(function, 8, 2, 1, D, False, True)), True).threads
+    threads = _native.query_loop(_native.query(_native.make_problem(function, B, 2, N, D, False, True)), True).threads
+    assert (threads == few) == alone
+    _check(function, N, D, B, 5, function == "slstm" and B == 9)
+
+
 # enough clusters that Elman's forward loop takes CTAs of which two share an SM (R in registers alone, in shared memory too), and that the
 # two loops split the head differently
 @pytest.mark.parametrize("function,N,D", [("elman", 4, 512), ("elman", 3, 704), ("elman", 2, 1024), ("lstm", 5, 320), ("slstm", 5, 384)])
