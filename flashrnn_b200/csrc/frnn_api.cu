@@ -88,16 +88,17 @@ constexpr int kResident[17] = {0, 148, 74, 45, 33, 26, 22, 17, 15, 14, 11, 8, 7,
 // Units per CTA and rows / 8 of one of those loops: the fewest turns of all clusters through the GPU, weighed with what a step takes.
 // `dense`: the form of Elman's 64-unit forward CTAs of which two fit an SM (frnn_big_fwd.cuh).
 struct BigTile { int u, nt; bool dense; };
-// A step alone, 8 / 16 rows, in hundredths of a 32-unit one of 8 rows: 32, 48 and 64 units up to head dim 576 (forward) and 512 (reverse), 48 and 64
-// above.  Measured, us per step: D = 384, 32, 48, 64 units: LSTM forward 1.06 / 1.54, 1.12 / 2.02, 1.68 / 2.53, reverse 1.00 / 1.63, 1.67 / 3.00, 2.60 / 5.58; GRU
-// forward 1.02 / 1.51, 1.12 / 1.95, 1.70 / 2.76, reverse 0.96 / 1.57, 1.54 / 2.63, 2.02 / 3.81; sLSTM forward 1.12 / 1.67, 1.38 / 2.38, 1.92 / 3.56, reverse
-// 1.05 / 1.73, 1.83 / 4.17, 2.98 / 6.09; Elman 0.80 / 1.25, 0.86 / 1.28, 0.82 / 1.28, reverse 0.96 / 1.44, 0.96 / 1.57, 1.03 / 1.76.  D = 768, 48, 64 units: LSTM
-// forward 2.15 / 3.86, 3.36 / 4.72, reverse 2.56 / 5.43, 4.59 / 8.45.
+// A step alone, 8 / 16 rows, relative to the others of its head dim: 32, 48 and 64 units up to head dim 576 (forward) and 512 (reverse), where a 32-unit one
+// of 8 rows is 100, then 48 and 64 above.  Measured, us per step: D = 384, 32, 48, 64 units: LSTM forward 0.94 / 1.41, 1.05 / 1.81, 1.41 / 2.21, reverse 0.86 / 1.49, 1.26 /
+// 2.36, 1.77 / 3.57; GRU forward 0.90 / 1.38, 1.05 / 1.72, 1.39 / 2.20, reverse 0.83 / 1.40, 1.20 / 2.10, 1.42 / 2.57; sLSTM forward 0.99 / 1.51, 1.13 / 1.98, 1.60 / 2.37,
+// reverse 0.87 / 1.54, 1.28 / 2.79, 1.88 / 4.76; Elman 0.80 / 1.25, 0.86 / 1.28, 0.82 / 1.28, reverse 0.96 / 1.44, 0.96 / 1.57, 1.03 / 1.76.  D = 768, 48, 64 units: LSTM
+// forward 1.74 / 3.17, 2.38 / 3.95, reverse 1.82 / 3.68, 2.71 / 6.19; GRU 1.79 / 3.10, 2.40 / 3.79, reverse 1.71 / 3.25, 1.94 / 3.87; sLSTM 1.81 / 3.38, 2.53 / 4.12, reverse 1.83 / 4.96,
+// 3.35 / 7.92.
 constexpr int kBigWeight[4][2][5][2] = {
-    {{{100, 146}, {110, 190}, {160, 240}, {106, 186}, {160, 232}}, {{100, 163}, {168, 302}, {256, 560}, {168, 356}, {300, 540}}},   // LSTM: forward, reverse
-    {{{100, 146}, {110, 191}, {160, 260}, {106, 190}, {161, 240}}, {{100, 162}, {158, 272}, {205, 395}, {145, 290}, {250, 390}}},   // GRU
+    {{{100, 150}, {112, 193}, {150, 235}, {87, 158}, {119, 198}}, {{100, 173}, {147, 274}, {206, 415}, {91, 184}, {136, 310}}},     // LSTM: forward, reverse
+    {{{100, 153}, {117, 191}, {154, 244}, {90, 155}, {120, 190}}, {{100, 169}, {145, 253}, {171, 310}, {86, 163}, {97, 194}}},      // GRU
     {{{100, 156}, {106, 160}, {102, 175}, {100, 172}, {102, 172}}, {{100, 155}, {104, 162}, {107, 178}, {104, 170}, {106, 182}}},   // Elman
-    {{{100, 146}, {123, 212}, {163, 320}, {126, 252}, {178, 300}}, {{100, 164}, {176, 405}, {286, 590}, {178, 401}, {310, 553}}}};  // sLSTM
+    {{{100, 153}, {114, 200}, {162, 239}, {91, 169}, {127, 206}}, {{100, 177}, {147, 321}, {216, 547}, {92, 248}, {168, 396}}}};    // sLSTM
 static BigTile big_tile(const frnn_problem& pr, bool bwd) {
   const bool elman = pr.cell == CELL_ELMAN;
   BigTile best = {64, 1, false};

@@ -1,6 +1,6 @@
 // Reverse time loop for head dims above 256: the reverse lane loop (frnn_lane_bwd.cuh) with the geometry of frnn_big_fwd.cuh.  A warp
 // owns up to four 16-row tiles of p and all K = Gr * U gate rows of its CTA; KRP of its k-pairs are in registers, the next in
-// shared memory, the rest comes from L2.  Twice as many warps multiply as run the cell (U / 8); the other half moves the data
+// tensor memory (see the forward loop), then in shared memory, the rest comes from L2.  Twice as many warps multiply as run the cell (U / 8); the other half moves the data
 // meanwhile.  The sums of a tile, or a pair of tiles, leave as soon as they are complete, so their exchange overlaps the products of the next.
 // K is padded to a multiple of 32 with zero fragments (the delta columns there are zero, or the GRU's input-only gate).
 //
@@ -35,8 +35,12 @@ struct BigBwdGeom {
   // tiles are multiplied MG at a time, one read of the deltas for both (U = 48, D = 768 LSTM step 5240 -> 4610 clk; with all of R^T in registers
   // one by one, in two accumulator sets: D = 512 2235 -> 2030); units of one k-pair of them per warp in shared memory, in the order of use
   static constexpr int MG = U == 32 ? 1 : 2;
+  static constexpr int KL = KP - KRP;  // k-pairs beyond those in registers
+  // of them, those in tensor memory, for each group of MG tiles: a lane's 16 words of a k-pair of a group lie in 16 columns of its own lane
+  static constexpr bool TM = MG == 2 && KL > 0;
+  static constexpr int TCOLS = TM ? 512 / (W / 4) / 16 * 16 : 0, TFIT = TCOLS / 16 / (MT / MG), KT = KL < TFIT ? KL : TFIT;
   static __host__ __device__ constexpr int fsm(int D) {
-    const int want = (tiles(D) + MG - 1) / MG * (KP - KRP), fit = ((int)kSmemBudget - off_r(D)) / (W * MG * 1024);
+    const int want = (tiles(D) + MG - 1) / MG * (KL - KT), fit = ((int)kSmemBudget - off_r(D)) / (W * MG * 1024);
     return want < fit ? want : (fit < 0 ? 0 : fit);
   }
   static __host__ __device__ constexpr size_t smem(int D) { return (size_t)off_r(D) + (size_t)fsm(D) * W * MG * 1024; }
@@ -186,6 +190,13 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
     mbar_arrive_expect_tx(&full[0], RB);             // partial sums of step index 0 (t = T-1)
     if (T > 1) mbar_arrive_expect_tx(&full[1], RB);  // step index 1
   }
+  constexpr bool TM = G::TM;
+  if constexpr (TM) {  // (the registers of the CTA leave no room for another on this SM, so there is nobody to wait for)
+    if (warp == 0) tmem_alloc(reinterpret_cast<uint32_t*>(smem_raw + 96), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+  }
   for (int i = tid; i < 2 * DB / 16; i += TH) sts128(dtile + i * 16, make_uint4(0u, 0u, 0u, 0u));  // (padding columns stay zero)
   __syncthreads();
   cluster_arrive();  // waited for before the first push
@@ -205,13 +216,31 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
 #pragma unroll
     for (int kp = 0; kp < KRP; ++kp)
       if (m < mtn) A[m][kp] = frag(m, kp);
-  // the other k-pairs, KL per MG tiles: the first fsm in shared memory, the rest read from L2
-  constexpr int MG = G::MG, KL = KP - KRP;
+  // the other k-pairs, KL per MG tiles: KT of them in tensor memory; of the others the first fsm in shared memory, the rest read from L2
+  constexpr int MG = G::MG, KT = G::KT, KL = G::KL - KT, KR = KRP + KT;
+  uint32_t tcol = 0;
+  if constexpr (TM) {
+    tcol = *reinterpret_cast<volatile uint32_t*>(smem_raw + 96) + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * G::TCOLS);
+#pragma unroll 1
+    for (int i = 0; i < MT / MG * KT; ++i) {
+      uint32_t r[16];
+#pragma unroll
+      for (int m = 0; m < MG; ++m) {
+        AFrag f;
+        f.lo = f.hi = make_uint4(0u, 0u, 0u, 0u);
+        if (i / KT * MG + m < mtn) f = frag(i / KT * MG + m, KRP + i % KT);
+        r[8 * m] = f.lo.x; r[8 * m + 1] = f.lo.y; r[8 * m + 2] = f.lo.z; r[8 * m + 3] = f.lo.w;
+        r[8 * m + 4] = f.hi.x; r[8 * m + 5] = f.hi.y; r[8 * m + 6] = f.hi.z; r[8 * m + 7] = f.hi.w;
+      }
+      tmem_st16(tcol + i * 16, r);
+    }
+    tmem_wait_st();
+  }
   const uint32_t rs = sm + G::off_r(D) + (uint32_t)(warp * fsm) * (MG * 1024) + lane * 16;
   for (int i = 0; i < fsm; ++i)
     for (int m = 0; m < MG; ++m)
       if (i / (KL > 0 ? KL : 1) * MG + m < mtn) {
-        const AFrag f = frag(i / (KL > 0 ? KL : 1) * MG + m, KRP + i % (KL > 0 ? KL : 1));
+        const AFrag f = frag(i / (KL > 0 ? KL : 1) * MG + m, KR + i % (KL > 0 ? KL : 1));
         sts128(rs + (i * MG + m) * 1024, f.lo);
         sts128(rs + (i * MG + m) * 1024 + 512, f.hi);
       }
@@ -247,6 +276,36 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
       };
 #pragma unroll
       for (int kp = 0; kp < KRP; ++kp) pair(kp, A[m0][kp], A[m0 + MG - 1][kp]);
+      if constexpr (TM) {
+        auto words = [&](int kp, const uint32_t* r) {
+          AFrag f[MG];
+#pragma unroll
+          for (int m = 0; m < MG; ++m) {
+            f[m].lo = make_uint4(r[8 * m], r[8 * m + 1], r[8 * m + 2], r[8 * m + 3]);
+            f[m].hi = make_uint4(r[8 * m + 4], r[8 * m + 5], r[8 * m + 6], r[8 * m + 7]);
+          }
+          pair(kp, f[0], f[MG - 1]);
+        };
+        constexpr int TP = U == 48 ? 2 : 1;  // k-pairs per load
+#pragma unroll
+        for (int i = 0; i + TP <= KT; i += TP) {
+          if constexpr (TP == 2) {
+            uint32_t r[32];
+            tmem_ld32(tcol + (m0 / MG * KT + i) * 16, r);
+            words(KRP + i, r);
+            words(KRP + i + 1, r + 16);
+          } else {
+            uint32_t r[16];
+            tmem_ld16(tcol + (m0 / MG * KT + i) * 16, r);
+            words(KRP + i, r);
+          }
+        }
+        if constexpr (KT % TP != 0) {
+          uint32_t r[16];
+          tmem_ld16(tcol + (m0 / MG * KT + KT - 1) * 16, r);
+          words(KRP + KT - 1, r);
+        }
+      }
       if constexpr (KL > 0) {
         const int first = m0 / MG * KL, stay = fsm - first < KL ? fsm - first : KL;
 #pragma unroll 1
@@ -254,15 +313,15 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
           AFrag f[MG];
 #pragma unroll
           for (int m = 0; m < MG; ++m) { f[m].lo = lds128(rs + ((first + i) * MG + m) * 1024); f[m].hi = lds128(rs + ((first + i) * MG + m) * 1024 + 512); }
-          pair(KRP + i, f[0], f[MG - 1]);
+          pair(KR + i, f[0], f[MG - 1]);
         }
 #pragma unroll 1
         for (int i = stay > 0 ? stay : 0; i < KL; ++i) {
           AFrag f[MG];
 #pragma unroll
           for (int m = 0; m < MG; ++m)
-            if (m0 + m < mtn) f[m] = frag(m0 + m, KRP + i);
-          pair(KRP + i, f[0], f[MG - 1]);
+            if (m0 + m < mtn) f[m] = frag(m0 + m, KR + i);
+          pair(KR + i, f[0], f[MG - 1]);
         }
       }
       if (!poisoned && !(drop && j == 0)) {
@@ -350,6 +409,9 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
   __syncwarp();
   cluster_arrive_relaxed();
   cluster_wait();
+  if constexpr (TM) {
+    if (warp == 0) tmem_dealloc(*reinterpret_cast<volatile uint32_t*>(smem_raw + 96), 512);
+  }
 }
 
 }  // namespace FRNN_NS

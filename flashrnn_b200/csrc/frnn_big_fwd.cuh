@@ -1,19 +1,22 @@
 // Forward time loop for head dims above 256 (multiples of 64 up to kBigMaxD), where R does not fit the registers of a cluster:
 // the lane loop of frnn_lane_fwd.cuh with
 //   * up to 16 CTAs of U = 32, 48 or 64 units per head (big_tile in frnn_api.cu): with few heads and rows as many SMs as a cluster can have, so that R -- 4.7 MB at
-//     head dim 768 -- lies in their registers (KRP k-pairs per warp) and shared memory (the rest of it) for all T steps; only what
-//     fits neither is re-read from L2 in every step (head dims 640 and 704, and 832 up, of the cells with three or four gates);
+//     head dim 768 -- lies in their registers (KRP k-pairs per warp), tensor memory (tsp pairs: a lane keeps its own words of a pair in its own lane, 16 columns,
+//     and loads them back into registers for the warp's MMAs) and shared memory (the rest of it) for all T steps; only what fits none of them is
+//     re-read from L2 in every step (head dims 960 and 1024 of the cells with three or four gates);
 //   * two warps per 8-unit group that split k; the second hands its sums to the first through shared memory (one named
 //     barrier of 64 threads), which runs the cell, and moves the data meanwhile (no IO warps: a 13th warp would cost the other
 //     12 a quarter of their registers).
-// D = 768 LSTM, 16 CTAs x 48 units: 12 x 24 MMAs per quadrant and 1700 shared-memory wavefronts (fragments of R 16 per k-pair and warp,
-// h 4) bound a step, beside the exchange.  Measured per step, 16 rows (before: 12 CTAs x 64 units that streamed 28 of 48 k-steps from L2 through
-// the exchange's barriers): D = 768 forward 7020 -> 3930, reverse 9410 -> 4620 clk; D = 512 5190 -> 1990, 6990 -> 2045; D = 384 3560 -> 1830,
-// 5400 -> 1780; D = 1024 9220 -> 8280, 12860 -> 10100; D = 640, where a head has 10 CTAs of 64 units, 5990 -> 5090, 8040 -> 8730.
+// D = 768 LSTM, 16 CTAs x 48 units: 12 x 24 MMAs per quadrant (1152 clk), 576 shared-memory wavefronts for h and the exchange of 12 KB per CTA bound a
+// step.  With the pairs that are now in tensor memory in shared memory it was 1700 wavefronts, and what did not fit came from L2.  us per 48 steps of 16 rows, that
+// form and this one, forward, reverse: LSTM D = 576 78, 113 -> 74, 86; 640 136, 216 -> 105, 129; 768 107, 127 -> 94, 100; 832 180, 234 -> 136, 148; 1024 216, 246 -> 168, 163; GRU D = 640 131,
+// 178 -> 105, 96; 1024 213, 205 -> 170, 117; sLSTM D = 640 142, 237 -> 112, 144; 768 119, 146 -> 96, 101; 1024 232, 273 -> 176, 192.  Two pairs per load with 48 units (94 us,
+// one by one 98), one with 64 (LSTM D = 640 16 rows B200 236, in pairs 266: registers).
 //
 // Replaces FLASHRNNCellFusedForward (reference flashrnn/flashrnn/fused/flashrnn_fused_forward.cu:146-659).
 #pragma once
 #include "frnn_lane_fwd.cuh"
+#include "frnn_tc.cuh"
 
 namespace FRNN_NS {
 
@@ -27,13 +30,18 @@ struct BigFwdGeom {
   static constexpr int NB = QUAD ? NT : 2 * NT;
   static constexpr int GCM = CacheGeom<C::GC>::MAIN;
   static constexpr bool GCX = CacheGeom<C::GC>::EXTRA;
-  // k-pairs of R per warp in registers: what the register file leaves beside the ~60 of everything else (U = 32: all there are).  DENSE (Elman, 64
+  // k-pairs of R per warp in registers: what the register file leaves beside the ~60 of everything else, and the words on their way from tensor memory (U = 32: all
+  // there are).  DENSE (Elman, 64
   // units): half of it, so that two CTAs fit an SM, 226 -> 128 registers (see big_tile in frnn_api.cu)
   static_assert(!DENSE || (!QUAD && U == 64), "the dense form is Elman's of 64 units");
-  static constexpr int KRP = QUAD ? (U == 32 ? 8 : U == 48 ? 6 : 2) : (U == 32 || DENSE ? 8 : U == 48 ? 12 : 16);
+  static constexpr int KRP = QUAD ? (U == 32 ? 8 : U == 48 ? 4 : NT == 2 ? 1 : 2) : (U == 32 || DENSE ? 8 : U == 48 ? 12 : 16);
+  // ... and in tensor memory, of which a warp has TCOLS columns of 32 lanes: a lane's 16 words of a k-pair lie in 16 columns of its own lane
+  static constexpr bool TM = QUAD && U > 32;
+  static constexpr int TCOLS = TM ? 512 / (W / 4) / 16 * 16 : 0, TMAX = TCOLS / 16, TPAIRS = U == 48 ? 2 : 1;  // TPAIRS: k-pairs per load
+  static __host__ __device__ constexpr int tsp(int D) { return D / 64 - KRP < 0 ? 0 : (D / 64 - KRP < TMAX ? D / 64 - KRP : TMAX); }
   // Buffers for the k-pairs that fit neither registers nor shared memory: reloaded from L2 as soon as they are used, so two pairs per warp
-  // are in flight all the time, the wait for h included (one at a time, loaded where it was used: D = 1024 LSTM step 10310 clk)
-  static constexpr int PB = QUAD && U == 64 ? 2 : 0;
+  // are in flight all the time, the wait for h included (one at a time, loaded where it was used: D = 1024 LSTM step 10310 clk).  Not with 16 rows, where their registers spill (B200 T32 D = 1024 451 -> 378 us)
+  static constexpr int PB = QUAD && U == 64 && NT == 1 ? 2 : 0;
   static constexpr int XSH = C::Gw == 3 ? 1 : 0, XPL = C::Gw + XSH;
   static constexpr int XP = io_pitch(U * 2), XS = XPL * BT * XP;
   static constexpr int SP = io_pitch(U * 4), CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2);
@@ -43,7 +51,7 @@ struct BigFwdGeom {
   static __host__ __device__ constexpr int off_r(int D) { return OFF_H + 2 * NT * opnd_bytes(D); }
   // k-pairs of R per warp in shared memory
   static __host__ __device__ constexpr int ksp(int D) {
-    const int want = D / 64 - KRP, fit = ((int)kSmemBudget - off_r(D)) / (W * MT * 1024);
+    const int want = D / 64 - KRP - tsp(D), fit = ((int)kSmemBudget - off_r(D)) / (W * MT * 1024);
     return want <= 0 ? 0 : (fit < 0 ? 0 : (want < fit ? want : fit));
   }
   static __host__ __device__ constexpr size_t smem(int D) { return (size_t)off_r(D) + (size_t)ksp(D) * W * MT * 1024; }
@@ -97,11 +105,18 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
     if (T > 1) mbar_arrive_expect_tx(&full[0], step_bytes);  // h_0, consumed at step 1
     if (T > 2) mbar_arrive_expect_tx(&full[1], step_bytes);  // h_1
   }
+  constexpr bool TM = G::TM;
+  if constexpr (TM) {  // (the registers of the CTA leave no room for another on this SM, so there is nobody to wait for)
+    if (warp == 0) tmem_alloc(reinterpret_cast<uint32_t*>(smem_raw + 64), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+  }
   if (p.clear_status && tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
     p.status[0] = 0u; p.status[1] = 0u; p.status[2] = 0u; p.status[3] = 0u;
   }
-  // ---- warp (grp, half): units [grp * UW, +UW), k-pairs [half * kph, +kph).  Its fragments: KRP pairs in registers, the next ksp
-  // in shared memory (each lane reads back what it wrote itself), the rest in global memory
+  // ---- warp (grp, half): units [grp * UW, +UW), k-pairs [half * kph, +kph).  Its fragments: KRP pairs in registers, the next tsp in tensor memory,
+  // the next ksp in shared memory (each lane reads back what it wrote itself), the rest in global memory
   const int half = warp >= G::GROUPS, grp = warp - half * G::GROUPS;
   const uint4* src = p.Rpack + big_frag<MT>(n, D / G::UW, (int)crank * G::GROUPS + grp, D / 32, half * kph) + lane;
   AFrag A[MT][KRP];
@@ -113,9 +128,25 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
         A[m][kp].lo = __ldg(src + (size_t)kp * (MT * 64) + m * 64);
         A[m][kp].hi = __ldg(src + (size_t)kp * (MT * 64) + m * 64 + 32);
       }
+  const int tsp = G::tsp(D), kst = KRP + tsp;  // kst: first pair in shared memory
+  uint32_t tcol = 0;
+  if constexpr (TM) {
+    static_assert(MT == 2, "a k-pair is 16 words per lane");
+    tcol = *reinterpret_cast<volatile uint32_t*>(smem_raw + 64) + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * G::TCOLS);
+    for (int i = 0; i < tsp; ++i) {
+      uint32_t r[16];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 v = __ldg(src + (size_t)(KRP + i) * (MT * 64) + q * 32);
+        r[4 * q] = v.x; r[4 * q + 1] = v.y; r[4 * q + 2] = v.z; r[4 * q + 3] = v.w;
+      }
+      tmem_st16(tcol + i * 16, r);
+    }
+    tmem_wait_st();
+  }
   constexpr int PB = G::PB, PBN = PB > 0 ? PB : 1;
-  const int rem = kph - KRP - ksp;  // pairs in global memory
-  const uint4* rsrc = src + (size_t)(KRP + ksp) * (MT * 64);
+  const int rem = kph - kst - ksp;  // pairs in global memory
+  const uint4* rsrc = src + (size_t)(kst + ksp) * (MT * 64);
   AFrag P[PBN][MT];
   auto fetch = [&](int s, int j) {  // pair j of those -> buffer s
 #pragma unroll
@@ -127,7 +158,7 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
       if (s < rem) fetch(s, s);
   }
   const uint32_t rs = sm + G::off_r(D) + (uint32_t)(warp * ksp) * (MT * 1024) + lane * 16;
-  for (int i = 0; i < ksp * MT * 2; ++i) sts128(rs + i * 512, __ldg(src + (size_t)KRP * (MT * 64) + i * 32));
+  for (int i = 0; i < ksp * MT * 2; ++i) sts128(rs + i * 512, __ldg(src + (size_t)kst * (MT * 64) + i * 32));
 
   grid_wait_previous();  // (R may be read before it: consecutive decoding steps overlap up to here)
   for (int idx = tid; idx < G::BT * (D / 2); idx += TH) {  // h_{-1} -> tile 1
@@ -174,7 +205,7 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
 #pragma unroll
         for (int s = 0; s < PB; ++s)
           if (j + s < rem) {
-            pair(KRP + ksp + j + s, P[s]);
+            pair(kst + ksp + j + s, P[s]);
             if (rem > PB) fetch(s, j + s + PB < rem ? j + s + PB : s);
           }
       }
@@ -188,19 +219,46 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
         for (int m = 0; m < MT; ++m) a[m] = A[m][kp];
         pair(kp, a);
       }
+    if constexpr (TM) {
+      auto words = [&](int kp, const uint32_t* r) {
+        AFrag a[MT];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          a[m].lo = make_uint4(r[8 * m], r[8 * m + 1], r[8 * m + 2], r[8 * m + 3]);
+          a[m].hi = make_uint4(r[8 * m + 4], r[8 * m + 5], r[8 * m + 6], r[8 * m + 7]);
+        }
+        pair(kp, a);
+      };
+      int i = 0;
+      if constexpr (G::TPAIRS == 2) {
+#pragma unroll 1
+        for (; i + 1 < tsp; i += 2) {
+          uint32_t r[32];
+          tmem_ld32(tcol + i * 16, r);
+          words(KRP + i, r);
+          words(KRP + i + 1, r + 16);
+        }
+      }
+#pragma unroll 1
+      for (; i < tsp; ++i) {
+        uint32_t r[16];
+        tmem_ld16(tcol + i * 16, r);
+        words(KRP + i, r);
+      }
+    }
 #pragma unroll 1
     for (int i = 0; i < ksp; ++i) {
       AFrag a[MT];
 #pragma unroll
       for (int m = 0; m < MT; ++m) { a[m].lo = lds128(rs + (i * MT + m) * 1024); a[m].hi = lds128(rs + (i * MT + m) * 1024 + 512); }
-      pair(KRP + i, a);
+      pair(kst + i, a);
     }
     if constexpr (PB > 0) {
 #pragma unroll 1
       for (int j = PB; j < rem; j += PB) buffered(j);
     } else {
 #pragma unroll 1
-      for (int kp = KRP + ksp; kp < kph; ++kp) {
+      for (int kp = kst + ksp; kp < kph; ++kp) {
         AFrag a[MT];
 #pragma unroll
         for (int m = 0; m < MT; ++m) { a[m].lo = __ldg(src + (size_t)kp * (MT * 64) + m * 64); a[m].hi = __ldg(src + (size_t)kp * (MT * 64) + m * 64 + 32); }
@@ -298,6 +356,10 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
   }
   // Every message to this CTA has been waited for; only after an expired wait can one still be in flight, and then the barrier covers it.
   if (T > 1) { __syncwarp(); cluster_arrive_relaxed(); cluster_wait(); }
+  if constexpr (TM) {
+    __syncthreads();  // (every warp has done its last load; one that reached the cluster's barrier above has, too, but T may be 1)
+    if (warp == 0) tmem_dealloc(*reinterpret_cast<volatile uint32_t*>(smem_raw + 64), 512);
+  }
 }
 
 }  // namespace FRNN_NS

@@ -60,7 +60,9 @@ def test_reverse_loops_with_multiplying_warps(cuda_device, function, N, D, B, al
 
 # enough clusters that Elman's forward loop takes CTAs of which two share an SM (R in registers alone, in shared memory too), and that the
 # two loops split the head differently
-@pytest.mark.parametrize("function,N,D", [("elman", 4, 512), ("elman", 3, 704), ("elman", 2, 1024), ("lstm", 5, 320), ("slstm", 5, 384)])
+@pytest.mark.parametrize("function,N,D", [("elman", 4, 512), ("elman", 3, 704), ("elman", 2, 1024), ("lstm", 5, 320), ("slstm", 5, 384)] +
+                         # R in tensor memory: an odd number of k-pairs, with shared memory behind it, with L2 behind that, 8 and 16 rows
+                         [("gru", 2, 576), ("lstm", 2, 832), ("gru", 1, 832), ("lstm", 1, 960), ("gru", 2, 960), ("slstm", 1, 704)])
 def test_head_dims_above_256_many_clusters(cuda_device, function, N, D):
     _check(function, N, D, 147, 3, False)
 
