@@ -12,7 +12,8 @@
 //   * warp 4, one lane: per chunk 2 MT + D/64 bulk loads into a 3- or 4-stage ring (mbarrier byte counts), then 4 MT
 //     tcgen05.mma (M128, N = D, K16) accumulating in tensor memory; tcgen05.commit frees the stage;
 //   * h_{t-1} of t = 0 is the initial state, which is not a row of `states`: the copy starts at t = -1, that row reads
-//     as zero, and the missing products delta[b,0] * h_{-1}[b] are added by the draining threads from global memory;
+//     as zero, and warp 0 writes h_{-1}[b], which it has fetched by then, into it before the chunk is multiplied (products of that row
+//     added by the draining threads, one by one: us, T64, LSTM B1024 N8 D128 492 -> 212, B512 N4 D256 369 -> 124);
 //   * warps 0-3 read their tensor-memory lanes and add the tile into the fp32 gradient workspace with atomics.
 // Every wait is bounded; on expiry the CTA records it, stops issuing and waits (bounded) for the copies in flight.
 //
@@ -32,8 +33,6 @@ constexpr int DT_THREADS = 160;                // warps 0-3 drain tensor memory;
 constexpr uint32_t DT_BLK = 64 * DT_KC * 2;    // bytes of one [64 t][64] bf16 block
 
 struct DrTmaParams {
-  const elem_t* dWx;  // [B,T,Gw,N,D]
-  const elem_t* dg0;  // [B,T,N,D] (GRU)
   const elem_t* s0;   // [S,B,1,N,D]; only s = 0 is read
   float* dR;                 // [Gr,N,D,D] fp32
   unsigned* status;
@@ -59,7 +58,9 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + (size_t)NS * stage_bytes);          // [DT_STAGES] bytes have landed
   uint64_t* empty = full + DT_STAGES;                                                  // [DT_STAGES] MMAs have read the stage
   uint64_t* done = empty + DT_STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  uint64_t* landed = done + 1;   // a chunk that starts at t = 0 has landed
+  uint64_t* filled = landed + 1;  // 32 arrivals: h_{-1} is in its first row of h
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(filled + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n = blockIdx.y;
@@ -72,10 +73,13 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
   if (c_end > total_chunks) c_end = total_chunks;
   if (c_begin >= c_end) return;  // uniform for the CTA
   const int nchunks = (int)(c_end - c_begin);
+  const int skip = (int)(c_begin % p.chunks_per_b), first = skip ? p.chunks_per_b - skip : 0;  // the first chunk of this CTA that starts at t = 0
 
   if (tid == 0) {
     for (int s = 0; s < DT_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(done, 1);
+    mbar_init(landed, 1);
+    mbar_init(filled, 32);
     fence_mbar_init();
   }
   if (warp == 4) tmem_alloc(tmem_slot, (uint32_t)p.tmem_cols);
@@ -117,9 +121,17 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
       bool ok = true;
       int s = 0, ps = 0;         // ring stage of chunk ci and of chunk ci - 1
       uint32_t par = 0, ppar = 0;  // and the parities of their barrier phases
+      int next = first;            // the next chunk that starts at t = 0
+      uint32_t npar = 0;
       for (int ci = 0; ci < nchunks; ++ci) {
         if (!mbar_wait_bounded(&full[s], par)) { ok = false; report_timeout(p.status, ci); break; }
         seen = ci + 1;
+        if (ci == next) {
+          mbar_arrive(landed);
+          if (!mbar_wait_bounded(filled, npar)) { ok = false; report_timeout(p.status, ci); break; }
+          next += p.chunks_per_b;
+          npar ^= 1u;
+        }
         const uint32_t s_lo = ((base + (uint32_t)s * stage_bytes) >> 4) | LBO, b_lo = s_lo + (uint32_t)MT * ((2 * DT_BLK) >> 4);
         for (int mt = 0; mt < MT; ++mt) {
           const uint32_t a_lo = s_lo + (uint32_t)mt * ((2 * DT_BLK) >> 4), acc = tmem + (uint32_t)(mt * DW);
@@ -145,48 +157,38 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
           mbar_wait_bounded(&full[i % NS], (uint32_t)((i / NS) & 1));
     }
   } else {
+    // ---- h_{-1}: lane i has 16-byte piece i of the row, in 64-wide block i / 8; in row 0 of a block nothing is permuted
+    if (warp == 0) {
+      const int cb = ctile * nbw + (lane >> 3) < nb ? ctile * nbw + (lane >> 3) : nb - 1;
+      const elem_t* src = p.s0 + (size_t)n * D + cb * 64 + (lane & 7) * 8;
+      int b = (int)((c_begin + first) / p.chunks_per_b);
+      uint32_t par = 0;
+      for (int ci = first; ci < nchunks; ci += p.chunks_per_b, ++b, par ^= 1u) {
+        const uint4 h = (lane >> 3) < nbw ? *reinterpret_cast<const uint4*>(src + (size_t)b * N * D) : make_uint4(0u, 0u, 0u, 0u);
+        if (!mbar_wait_bounded(landed, par)) { report_timeout(p.status, ci); break; }
+        if ((lane >> 3) < nbw) sts128(base + (uint32_t)(ci % NS) * stage_bytes + (uint32_t)(2 * MT + (lane >> 3)) * DT_BLK + (lane & 7) * 16, h);
+        fence_proxy_async_smem();  // the row is read by the tensor core
+        mbar_arrive(filled);
+      }
+      __syncwarp();
+    }
     // ---- drain: row m of tile mt = (block 2 mt + m / 64, d = 64 * dblk + m % 64)
     const bool fin = mbar_wait_bounded(done, 0);
     if (!fin) report_timeout(p.status, nchunks);
     tc_fence_after();
     const int m = warp * 32 + lane;
-    // delta[b, t = 0] of a row is needed for the batch rows whose first chunk belongs to this CTA
-    const int b_first = (int)((c_begin + p.chunks_per_b - 1) / p.chunks_per_b), b_last = (int)((c_end - 1) / p.chunks_per_b);
-    const size_t ND = (size_t)N * D;
     for (int mt = 0; mt < MT; ++mt) {
     const int rb = rbase + 2 * mt + (m >> 6);
     const bool row_ok = fin && rb < RB;
     const int rbc = row_ok ? rb : RB - 1, g = rbc / nb, d = (rbc - g * nb) * 64 + (m & 63);
     float* out = p.dR + (((size_t)g * N + n) * D + d) * D;
-    const bool from_dg0 = p.cell == CELL_GRU && g == 0;
-    const elem_t* d0src = from_dg0 ? p.dg0 + (size_t)n * D + d
-                                          : p.dWx + (size_t)((p.cell == CELL_GRU) ? g - 1 : g) * ND + (size_t)n * D + d;
-    const size_t d0stride = (from_dg0 ? (size_t)1 : (size_t)p.Gw) * ND * T;  // elements between batch rows at t = 0
     for (int cw = 0; cw < DW; cw += 32) {
       uint32_t r[32];
       tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * DW + cw), r);
       const int col0 = ctile * DW + cw;
       if (!row_ok || col0 >= D) continue;
-      float v[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-      for (int b = b_first; b <= b_last; ++b) {  // h_{-1}: the products the zero row at t = -1 left out
-        const float dv = elem_to_float(d0src[(size_t)b * d0stride]);
-        const uint4* hs = reinterpret_cast<const uint4*>(p.s0 + ((size_t)b * N + n) * D + col0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint4 w = hs[q];
-          const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 h2 = unpack_x2(ww[e]);
-            v[q * 8 + 2 * e] = fmaf(dv, h2.x, v[q * 8 + 2 * e]);
-            v[q * 8 + 2 * e + 1] = fmaf(dv, h2.y, v[q * 8 + 2 * e + 1]);
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) red_add_f32x4(out + col0 + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
+      for (int j = 0; j < 32; j += 4) red_add_f32x4(out + col0 + j, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
     }
     }
   }
@@ -222,8 +224,6 @@ cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int 
     if (!encode_tiles16(&tm_st, states, dims, str, box)) return cudaErrorNotSupported;
   }
   DrTmaParams p;
-  p.dWx = static_cast<const elem_t*>(dWx);
-  p.dg0 = static_cast<const elem_t*>(dg0);
   p.s0 = static_cast<const elem_t*>(s0);
   p.dR = dR;
   p.status = status;
@@ -237,9 +237,6 @@ cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int 
   if (mt > tiles) mt = tiles;
   while (mt > 1 && 3 * (size_t)(2 * mt + nbw) * DT_BLK > (size_t)200 * 1024) --mt;
   mt = (tiles + (tiles + mt - 1) / mt - 1) / ((tiles + mt - 1) / mt);  // same number of CTAs, evenly filled
-#ifdef FRNN_DR_ONE_TILE  // development aid: one tile per CTA
-  mt = 1;
-#endif
   p.mt = mt;
   p.ct = ct;
   p.nbw = nbw;
@@ -257,7 +254,7 @@ cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int 
   if (splits > 65535) splits = 65535;
   p.chunks_per_split = (int)((chunks + splits - 1) / splits);
   splits = (chunks + p.chunks_per_split - 1) / p.chunks_per_split;
-  const size_t smem = (size_t)p.stages * (2 * mt + nbw) * DT_BLK + 8 * (2 * DT_STAGES + 1) + 16 + 1024;
+  const size_t smem = (size_t)p.stages * (2 * mt + nbw) * DT_BLK + 8 * (2 * DT_STAGES + 3) + 16 + 1024;
   cudaError_t e = cudaFuncSetAttribute(recurrent_grad_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);  // fixed maximum, so that concurrent host threads never lower each other's setting
   if (e != cudaSuccess) return e;
   recurrent_grad_tma_kernel<<<dim3((unsigned)(mtiles * ct), (unsigned)N, (unsigned)splits), DT_THREADS, smem, stream>>>(tm_dwx, tm_dg0,

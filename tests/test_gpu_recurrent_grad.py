@@ -21,13 +21,14 @@ def test_recurrent_grad_edges(cuda_device, function, D, N, B, T, state_f32):
 
 # the tensor-map kernel (16-bit states, head dims 128, 192, 256; above, where rows are many: one to three column tiles, of which the last may be partly
 # empty): sequences shorter than, equal to
-# and just beyond the 64 steps of its copies, initial states (the h_{-1} term that is added outside the MMA), batches that do not fill a
+# and just beyond the 64 steps of its copies, initial states (the row of h_{-1} that is filled in), batches that do not fill a
 # split evenly, and the GRU, whose first gate's deltas come from a buffer of their own
 @pytest.mark.parametrize("function,B,T,N,D", [
     ("lstm", 3, 1, 2, 128), ("lstm", 5, 64, 1, 256), ("lstm", 2, 65, 2, 128), ("lstm", 9, 130, 1, 192),
     ("gru", 4, 1, 3, 128), ("gru", 7, 63, 1, 192), ("gru", 3, 129, 2, 256),
     ("slstm", 6, 66, 1, 128), ("elman", 5, 70, 2, 256), ("elman", 11, 2, 1, 128),
     ("elman", 3, 129, 2, 128), ("lstm", 10, 64, 1, 768), ("gru", 7, 129, 1, 768), ("lstm", 21, 65, 1, 512), ("slstm", 50, 70, 1, 320),
+    ("lstm", 75, 9, 2, 128), ("gru", 40, 130, 2, 128),
 ])
 def test_parameter_gradients_at_chunk_edges(cuda_device, function, B, T, N, D):
     Wx, R, b, s0 = make_inputs(function, B, T, N, D, seed=B * T + D, random_init=True)
