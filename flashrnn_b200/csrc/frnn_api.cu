@@ -41,6 +41,14 @@ static LaneKernel lane_help_kernel(int cell, int kt) {
   }
   return LaneKernel{nullptr, 0, 0};
 }
+static LaneKernel lane_dr_kernel(int cell) {
+  switch (cell) {
+    case CELL_LSTM: return lane_bwd_dr_lstm();
+    case CELL_GRU: return lane_bwd_dr_gru();
+    case CELL_SLSTM: return lane_bwd_dr_slstm();
+  }
+  return LaneKernel{nullptr, 0, 0};
+}
 static BigKernel big_kernel(int cell, bool bwd, int u, int nt, bool dense) {
   switch (cell) {
     case CELL_LSTM: return bwd ? big_bwd_lstm(u, nt) : big_fwd_lstm(u, nt, dense);
@@ -197,6 +205,17 @@ static bool lane_help(const frnn_problem& pr, int cs, int u, int nt) {
   return alone || pr.cell == CELL_LSTM || pr.cell == CELL_SLSTM || (pr.cell == CELL_GRU && pr.D == 96);
 }
 
+// Whether the reverse lane loop forms dR as well (lane_bwd_dr): head dim 64 with one CTA per head, 8 rows and 16-bit states.  Not for the shortest
+// sequences: a CTA adds its 48 or 64 KB of sums to the gradient once.  Backward pass, us, dR in its own kernel / in the loop, B1024 N16: LSTM T16 162 / 172, T20 192 /
+// 190, T24 218 / 209, T32 264 / 247, GRU T24 205 / 191, sLSTM T24 268 / 249.  The sLSTM's loop gets 23 to 27 us per 512 steps longer, which only pays once its own
+// kernel takes that: T512 B8 N2 239 / 253, B16 N12 261 / 259, B48 N16 302 / 261; LSTM 235 / 234, 255 / 239, 296 / 239; GRU 229 / 181, 243 / 182, 288 / 183.
+constexpr int kDrMinSteps = 24, kDrMinTilesSlstm = 24;
+static bool lane_dr(const frnn_plan& pl, int nt) {
+  const frnn_problem& pr = pl.prob;
+  if (pr.D != 64 || pl.cluster_size != 1 || nt != 1 || pr.cell == CELL_ELMAN || pr.dtype_state == FRNN_DTYPE_F32 || pl.forced_tile) return false;
+  return pr.T >= kDrMinSteps && (pr.cell != CELL_SLSTM || (long long)((pr.B + 7) / 8) * pr.N >= kDrMinTilesSlstm);
+}
+
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
   const int D = pr.D;
   if (bt == kWideBatchTile) return cs == 1 && wide_problem(pr);  // 128-row tensor-core loops: one CTA per head and tile
@@ -294,6 +313,7 @@ struct LoopLaunch {
   int threads, stages;
   size_t smem;
   int cs, u, rows;
+  bool dr;  // the reverse loop forms dR, too
 };
 static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
   const frnn_problem& pr = pl.prob;
@@ -308,11 +328,14 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
   }
   const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.batch_tile, pl.forced_tile);
   LaneKernel k = !pl.probe_noop_cell ? lane_kernel(cell, bwd, kt, u, nt) : bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
-  if (bwd && !pl.probe_noop_cell && lane_help(pr, pl.cluster_size, u, nt)) {
+  const bool dr = bwd && !pl.probe_noop_cell && lane_dr(pl, nt);
+  if (dr) {
+    k = lane_dr_kernel(cell);
+  } else if (bwd && !pl.probe_noop_cell && lane_help(pr, pl.cluster_size, u, nt)) {
     const LaneKernel h = lane_help_kernel(cell, kt);
     if (h.fn) k = h;
   }
-  return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt};
+  return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt, dr};
 }
 // x: the CTAs of a cluster, y: tiles of the batch, z: heads
 static int loop_tiles(const LoopLaunch& k, const frnn_problem& pr) { return (pr.B + k.rows - 1) / k.rows; }
@@ -646,6 +669,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
   lp.dg0 = reinterpret_cast<elem_t*>(ws + w.dg0);
   lp.ds0 = a->ds0;
   lp.dbias = grads + nR;
+  lp.dR = grads;
   lp.status = reinterpret_cast<unsigned*>(ws);
   lp.B = pr.B; lp.T = pr.T; lp.N = pr.N; lp.D = pr.D;
   lp.state_f32 = pr.dtype_state == FRNN_DTYPE_F32;
@@ -656,6 +680,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
     rc = launch_loop(*plan, true, lp, stream);
     if (rc) return rc;
   }
+  if (loop_of(*plan, true).dr) return FRNN_OK;  // nothing left to do for the dR part
   // dR.  Small heads: what counts is reading whole runs of neighbouring heads (frnn_dr_small.cu).  From head dim 128 up, 16-bit states: both
   // operands are [64 steps][64] tiles a tensor-map copy delivers ready for the MMA (LSTM B16 T1024 N4 D256 0.087 ms against 0.167 ms for the cp.async-fed
   // kernel; above 256, in column tiles, LSTM B16 T1024 N1 D768 0.445 -> 0.138 ms, against the warp-MMA kernel).  Above 256 the warp-MMA kernel is ahead

@@ -28,6 +28,7 @@ struct BigKernel {
   LaneKernel lane_fwd_##cell(int kt, int u, int nt);    \
   LaneKernel lane_bwd_##cell(int kt, int u, int nt);    \
   LaneKernel lane_bwd_help_##cell(int kt);              \
+  LaneKernel lane_bwd_dr_##cell();                      \
   BigKernel big_fwd_##cell(int u, int nt, bool dense);  \
   BigKernel big_bwd_##cell(int u, int nt);              \
   cudaError_t big_pack_##cell(const void* R, void* out, int N, int D, cudaStream_t stream);

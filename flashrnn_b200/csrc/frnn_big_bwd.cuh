@@ -25,6 +25,8 @@ struct BigBwdGeom {
   static constexpr int NSS = C::NNEED + C::NEXT;
   static constexpr int KRP_WANT = U == 32 ? 4 : U == 48 ? 3 : 2, KRP = KRP_WANT < KP ? KRP_WANT : KP;
   static constexpr int DCOLS = C::Gr == 3 ? 4 * U : KP * 32, DT = opnd_bytes(DCOLS), DB = NT * DT;
+  static constexpr bool DR = false;
+  static __host__ __device__ constexpr uint32_t doff(uint32_t row, uint32_t k) { return opnd_off(row, k); }
   static constexpr int CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2), SP = io_pitch(U * 4);
   static constexpr int IN_E = GCM ? BT * CP : 0, IN_S = IN_E + (GCX ? BT * EP : 0), IN_B = IN_S + NSS * BT * SP;
   // shared memory: barriers | delta tiles | input ring | 2 x partial sums received | fragments of R^T

@@ -60,6 +60,7 @@ struct LoopParams {
   elem_t* dg0;        // [B,T,N,D]   GRU only: delta of the recurrent-only gate
   void* ds0;                 // [S,B,1,N,D]
   float* dbias;              // fp32 [Gt,N,D] accumulated with atomics
+  float* dR;                 // fp32 [Gr,N,D,D], the same (reverse lane loops that form dR themselves)
   void* last;                // [S,B,1,N,D] forward: the states after the last step, or null
   unsigned* status;
   int clear_status;          // forward: CTA 0 zeroes the status block first

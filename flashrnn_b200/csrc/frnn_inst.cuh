@@ -7,8 +7,8 @@ namespace FRNN_NS {
 
 // ---- lane loops (head dims up to 256): head dim / 16, units per CTA, batch tile / 8
 #if FRNN_INST_BWD
-#define FRNN_GEOM(...) LaneBwdGeom<__VA_ARGS__, false>
-#define FRNN_KERNEL(...) lane_bwd_kernel<__VA_ARGS__, false>
+#define FRNN_GEOM(...) LaneBwdGeom<__VA_ARGS__, false, false>
+#define FRNN_KERNEL(...) lane_bwd_kernel<__VA_ARGS__, false, false>
 #else
 #define FRNN_GEOM(...) LaneFwdGeom<__VA_ARGS__>
 #define FRNN_KERNEL(...) lane_fwd_kernel<__VA_ARGS__>
@@ -28,20 +28,23 @@ struct LaneEntry<KT, U, NT, true> {
 
 #if FRNN_INST_BWD
 // the reverse loops with warps that only multiply (clusters of 32-unit CTAs, 8 rows), null where there is none
-template <int KT, bool V = LaneBwdGeom<FRNN_INST_CELL, KT, 32, 1, true>::valid>
-struct HelpEntry {
+template <int KT, int U, bool HELP, bool DR, bool V = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, DR>::valid>
+struct BwdEntry {
   static LaneKernel get() { return LaneKernel{nullptr, 0, 0}; }
 };
-template <int KT>
-struct HelpEntry<KT, true> {
+template <int KT, int U, bool HELP, bool DR>
+struct BwdEntry<KT, U, HELP, DR, true> {
   static LaneKernel get() {
-    using G = LaneBwdGeom<FRNN_INST_CELL, KT, 32, 1, true>;
-    return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<FRNN_INST_CELL, KT, 32, 1, true>), G::TH, G::smem};
+    using G = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, DR>;
+    return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<FRNN_INST_CELL, KT, U, 1, HELP, DR>), G::TH, G::smem};
   }
 };
 LaneKernel FRNN_INST_HELP(int kt) {
-  return kt == 6 ? HelpEntry<6>::get() : kt == 8 ? HelpEntry<8>::get() : kt == 12 ? HelpEntry<12>::get() : kt == 16 ? HelpEntry<16>::get() : LaneKernel{nullptr, 0, 0};
+  return kt == 6 ? BwdEntry<6, 32, true, false>::get() : kt == 8 ? BwdEntry<8, 32, true, false>::get() : kt == 12 ? BwdEntry<12, 32, true, false>::get()
+       : kt == 16 ? BwdEntry<16, 32, true, false>::get() : LaneKernel{nullptr, 0, 0};
 }
+// the reverse loop with a warp that forms dR (head dim 64, one CTA per head)
+LaneKernel FRNN_INST_DR() { return BwdEntry<4, 64, false, true>::get(); }
 #endif
 
 LaneKernel FRNN_INST_LANE(int kt, int u, int nt) {

@@ -14,8 +14,8 @@ static LaneKernel floor_fwd() {
 }
 template <int CELL, int KT, int U>
 static LaneKernel floor_bwd() {
-  using G = LaneBwdGeom<CELL | kNoopCell, KT, U, 1, true>;
-  return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<CELL | kNoopCell, KT, U, 1, true>), G::TH, G::smem};
+  using G = LaneBwdGeom<CELL | kNoopCell, KT, U, 1, true, false>;
+  return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<CELL | kNoopCell, KT, U, 1, true, false>), G::TH, G::smem};
 }
 
 // lstm head dim 256, gru head dim 128, slstm head dim 192: 32 units per CTA, 8-row batch tiles

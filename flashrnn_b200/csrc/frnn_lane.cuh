@@ -23,18 +23,24 @@ struct AFrag { uint4 lo, hi; };
 // acc[m][nt][.] (+)= sum over k of A[m][.] (rows of this lane's MT tiles) times the operand tile: KS k-steps of 16, NT tiles of 8
 // batch rows (`nt_bytes` apart).  INIT: acc holds the start value, else it starts from zero.  NS independent accumulator sets (see
 // acc_sets).  The loads run PF k-pairs ahead of the products: without it every pair waited for its own 36 clk load.
-template <int MT, int KS, int NT, int NS, bool INIT, class L>
+// BP: bytes between the tile's blocks; other than 128, the rows of a block are not permuted.
+template <int BP>
+__device__ __forceinline__ uint32_t lane_opnd(int gid, int tig) {
+  return (uint32_t)tig * BP + ((uint32_t)(BP == 128 ? gid ^ (int)opnd_swz((uint32_t)tig) : gid) << 4);
+}
+template <int MT, int KS, int NT, int NS, bool INIT, int BP = 128, class L>
 __device__ __forceinline__ void lane_mma(const AFrag (&A)[MT][(KS + 1) / 2], uint32_t tile, int nt_bytes, int gid, int tig, float (&acc)[MT][NT][4],
                                          L late) {
   constexpr int KP = KS / 2, PF = KP < 4 ? (KP < 1 ? 1 : KP) : (NT > 1 ? 3 : 4);
   static_assert(NS <= KS, "every set gets a product");
+  static_assert(BP == 128 || KS % 2 == 0, "whole k-pairs");
   float part[NS][MT][NT][4];
-  const uint32_t base = tile + (uint32_t)tig * 128u + ((uint32_t)(gid ^ (int)opnd_swz((uint32_t)tig)) << 4);
+  const uint32_t base = tile + lane_opnd<BP>(gid, tig);
   uint4 b[PF][NT];
 #pragma unroll
   for (int i = 0; i < PF && i < KP; ++i)
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) b[i][nt] = lds128(base + (uint32_t)(i * 512 + nt * nt_bytes));
+    for (int nt = 0; nt < NT; ++nt) b[i][nt] = lds128(base + (uint32_t)(i * 4 * BP + nt * nt_bytes));
   uint2 bo[NT];
   if constexpr ((KS & 1) != 0) {  // odd last k-step: four k per lane, in blocks 4 KP + (tig >> 1)
     const uint32_t blk = (uint32_t)(tig >> 1);
@@ -60,7 +66,7 @@ __device__ __forceinline__ void lane_mma(const AFrag (&A)[MT][(KS + 1) / 2], uin
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       cur[nt] = b[kp % PF][nt];
-      if (kp + PF < KP) b[kp % PF][nt] = lds128(base + (uint32_t)((kp + PF) * 512 + nt * nt_bytes));
+      if (kp + PF < KP) b[kp % PF][nt] = lds128(base + (uint32_t)((kp + PF) * 4 * BP + nt * nt_bytes));
     }
 #pragma unroll
     for (int m = 0; m < MT; ++m)

@@ -25,10 +25,11 @@
 // and gradientBiasAggregationKernel (flashrnn_fused_backward.cu:626-665).
 #pragma once
 #include "frnn_lane.cuh"
+#include "frnn_tc.cuh"
 
 namespace FRNN_NS {
 
-template <int CELL, int KT, int U, int NT, bool HELP>
+template <int CELL, int KT, int U, int NT, bool HELP, bool DR_>
 struct LaneBwdGeom {
   using C = Cell<CELL>;
   static constexpr int D = KT * 16, CS = D / U, BT = 8 * NT;
@@ -49,23 +50,32 @@ struct LaneBwdGeom {
   static constexpr bool GCX = CacheGeom<C::GC>::EXTRA;
   static constexpr int NSS = C::NNEED + C::NEXT;  // state-typed rows per batch row
   static constexpr int IOW = io_warps(BT * U * 2 * (C::Gw + C::GC + NSS)), IOT = 32 * IOW;
-  static constexpr int TH = 32 * WP + IOT;
+  static constexpr int TH = 32 * WP + IOT + (DR_ ? 32 : 0);
   static constexpr int UNITS = U, STAGES = kLaneStages, NT8 = NT;
   // columns of the delta tile: the R gates in order; the GRU's input-only gate n, which no product reads, behind them
-  static constexpr int DCOLS = C::Gr == 3 ? 4 * U : K, DT = opnd_bytes(DCOLS), DB = NT * DT;
+  static constexpr int DCOLS = C::Gr == 3 ? 4 * U : K;
+  // DR (head dim 64, one CTA per head): a warp more forms dR, see lane_bwd_dr.  The delta tiles are operands of tcgen05.mma then, whose 8 x 16 byte
+  // blocks must all have their rows in one order: the blocks lie 160 bytes apart (free of bank conflicts, too) instead of having them
+  // permuted, and a tile stays until the product of its two steps is done.
+  static constexpr bool DR = DR_;
+  static constexpr int DP = DR ? 160 : 128, DT = DCOLS / 8 * DP, DB = NT * DT, NDB = DR ? 4 : 2;
+  static __host__ __device__ constexpr uint32_t doff(uint32_t row, uint32_t k) { return DR ? (k >> 3) * DP + row * 16 + (k & 7) * 2 : opnd_off(row, k); }
+  // ... and h_{t-1} is the other operand: 8 x 16 byte blocks 144 bytes apart, the tiles of eight steps, fetched HAHEAD steps ahead
+  static constexpr int HP = 144, HT = D / 8 * HP, HSLOTS = 8, HAHEAD = 4, HBYTES = DR ? HSLOTS * HT : 0;
+  static constexpr int DRT = (K + 127) / 128, DRC = DRT * D;  // row tiles of dR, tensor-memory columns of their sums
   static constexpr int RB = CL ? CS * (U / 16) * 32 * NT * 16 : 0;  // bytes of received partial sums of one step
   // input ring: [kLaneStages] x { activations [BT] | fifth ones [BT] | states and cotangents [NSS][BT] }
-  static constexpr int CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2), SP = io_pitch(U * 4);
+  static constexpr int CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2), SP = io_pitch(U * (DR ? 2 : 4));  // (DR: 16-bit states only)
   static constexpr int IN_E = GCM ? BT * CP : 0, IN_S = IN_E + (GCX ? BT * EP : 0), IN_B = IN_S + NSS * BT * SP;
-  static constexpr int OFF_R = 2 * DB, OFF_I = OFF_R + 2 * RB, OFF_BAR = OFF_I + kLaneStages * IN_B;
+  static constexpr int OFF_R = NDB * DB, OFF_I = OFF_R + 2 * RB, OFF_H = OFF_I + kLaneStages * IN_B, OFF_BAR = OFF_H + HBYTES;
   static constexpr int SLICE = (U / 16) * 32 * NT * 16;  // bytes of partial sums from one CTA
-  static constexpr size_t smem = OFF_BAR + 3 * 8;
+  static constexpr size_t smem = OFF_BAR + 6 * 8;
   // Waits by a vote (mbar_wait_warp), except where the registers that takes cost large batches more: 32 steps of B1024, GRU D = 96 231 -> 241 us, D = 192
   // 273 -> 287.
   static constexpr bool VOTE = CL && (HELP || !(CELL == CELL_GRU && (KT == 6 || KT == 12)));
   // CTAs per SM the registers are cut for (0: as the compiler sees fit), where a few registers more would cost large batches a CTA
   static constexpr int MINB = CL && NT == 1 && KT >= 12 && C::Gr == 1 && U == 64 ? 3 : 0;
-  static constexpr bool valid = (!HELP || (CL && NT == 1 && U == 32 && KT >= 6 && BASE != CELL_ELMAN_CLIP && !(BASE == CELL_LSTM && KT == 8))) && D % U == 0 && (!CL || U % 8 == 0) && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget;
+  static constexpr bool valid = (!DR || (C::Gr >= 3 && KT == 4 && !CL && NT == 1)) && (!HELP || (CL && NT == 1 && U == 32 && KT >= 6 && BASE != CELL_ELMAN_CLIP && !(BASE == CELL_LSTM && KT == 8))) && D % U == 0 && (!CL || U % 8 == 0) && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget;
 };
 
 // Index of the first of the two 16-byte fragments (rows gid, gid + 8) of lane 0 in the packed R^T of head n, CTA c: see
@@ -169,14 +179,14 @@ __device__ __forceinline__ void bwd_io(const LoopParams& p, uint32_t d0, uint32_
 #pragma unroll
   for (int i = 0; i < TW::N; ++i) {
     const int r = TW::row(io, i), g = r / BT, bl = r - g * BT, b = bt0 + bl, c = TW::col(io, i);
-    ws[i] = d0 + (bl >> 3) * G::DT + opnd_off(bl & 7, (g + GSH) * U + c * 8);
+    ws[i] = d0 + (bl >> 3) * G::DT + G::doff(bl & 7, (g + GSH) * U + c * 8);
     wp[i] = (TW::in(io, i) && b < B) ? p.dWx + (((size_t)b * T + (T - 1)) * Gw + g) * ND + (size_t)n * D + unit0 + c * 8 : nullptr;
   }
   elem_t* gp[TE::N];
 #pragma unroll
   for (int i = 0; i < TE::N; ++i) {
     const int b = bt0 + TE::row(io, i);
-    gp[i] = (GSH && TE::in(io, i) && b < B) ? p.dg0 + ((size_t)b * T + (T - 1)) * ND + (size_t)n * D + unit0 + TE::col(io, i) * 8 : nullptr;
+    gp[i] = (GSH && !G::DR && TE::in(io, i) && b < B) ? p.dg0 + ((size_t)b * T + (T - 1)) * ND + (size_t)n * D + unit0 + TE::col(io, i) * 8 : nullptr;
   }
   auto store = [&](int x) {
 #pragma unroll
@@ -185,12 +195,12 @@ __device__ __forceinline__ void bwd_io(const LoopParams& p, uint32_t d0, uint32_
         *reinterpret_cast<uint4*>(wp[i]) = lds128(ws[i] + x * G::DB);
         wp[i] -= (size_t)Gw * ND;
       }
-    if constexpr (GSH) {
+    if constexpr (GSH && !G::DR) {
 #pragma unroll
       for (int i = 0; i < TE::N; ++i)
         if (gp[i] != nullptr) {
           const int bl = TE::row(io, i);
-          *reinterpret_cast<uint4*>(gp[i]) = lds128(d0 + x * G::DB + (bl >> 3) * G::DT + opnd_off(bl & 7, TE::col(io, i) * 8));
+          *reinterpret_cast<uint4*>(gp[i]) = lds128(d0 + x * G::DB + (bl >> 3) * G::DT + G::doff(bl & 7, TE::col(io, i) * 8));
           gp[i] -= ND;
         }
     }
@@ -213,15 +223,78 @@ __device__ __forceinline__ void lane_bwd_io(const LoopParams& p, uint32_t d0, ui
       cp_async_wait<STAGES - 2>();
       __syncthreads();
       load(T - 1 - j - STAGES, stage);
-      store(j & 1);
+      store(j & (G::NDB - 1));
       stage = stage + 1 == STAGES ? 0 : stage + 1;
     }
   });
 }
 
-template <int CELL, int KT, int U, int NT, bool HELP>
-__global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBwdGeom<CELL, KT, U, NT, HELP>::MINB) lane_bwd_kernel(const __grid_constant__ LoopParams p) {
-  using G = LaneBwdGeom<CELL, KT, U, NT, HELP>;
+// DR: the warp that forms dR beside the loop.  Its lanes fetch h_{t-1} a few steps ahead; behind the barrier of every second step its first lane has
+// the tensor core multiply the deltas of two steps, 16 rows of (b, t), as they lie in shared memory for the loop's own products, with that h.
+// The sums stay in tensor memory for the whole sequence.  So dR takes one more tile of h per step instead of a kernel that reads dWx
+// and h again; the loop's other warps do nothing for it.  Backward pass, us, with the kernel of frnn_dr_small.cu behind the loop -> so: B1024 T256 N16 LSTM
+// 1712 -> 1257, GRU 1705 -> 1132, sLSTM 2011 -> 1556; B16 T512 N12 LSTM 256 -> 239, GRU 263 -> 201; of a step, 46 clk are the tensor core's reading of shared memory.
+// Not for clusters: a CTA there needs h of the whole head, and its way into the SM lies across the exchange (LSTM B16 T1024 N4 D256 661 + 69 us -> 804: 98 for
+// fetching h, 46 for the products).
+template <class G>
+__device__ __forceinline__ void lane_bwd_dr(const LoopParams& p, uint32_t d0, uint32_t h0, int lane, uint32_t tmem, uint64_t* done, uint64_t* all_done) {
+  constexpr int D = G::D, BT = G::BT, AHEAD = G::HAHEAD;
+  using TT = IoTile<BT, D / 8, 32>;
+  const int T = p.T, n = blockIdx.z, bt0 = blockIdx.y * BT;
+  const size_t ND = (size_t)p.N * D;
+  for (uint32_t i = lane; i < G::HBYTES / 16; i += 32) sts128(h0 + i * 16, make_uint4(0u, 0u, 0u, 0u));  // (rows beyond B stay zero)
+  __syncwarp();
+  const elem_t* src = static_cast<const elem_t*>(p.states) + ((size_t)bt0 * T + T - 1) * ND + (size_t)n * D;  // the tile's first row at time T - 1
+  auto load_h = [&](int j) {  // h_{t-1} of step index j (in step order)
+    if (j < T) {
+      src = j < T - 1 ? src - ND : static_cast<const elem_t*>(p.s0) + (size_t)bt0 * ND + (size_t)n * D;
+      const size_t row = j < T - 1 ? T * ND : ND;
+#pragma unroll
+      for (int i = 0; i < TT::N; ++i) {
+        const int r = TT::row(lane, i), c = TT::col(lane, i);
+        if (bt0 + r < p.B) cp_async16_u32(h0 + (j & (G::HSLOTS - 1)) * G::HT + c * G::HP + r * 16, src + r * row + c * 8);
+      }
+    }
+    cp_async_commit();
+  };
+  // The deltas and h were written through the generic proxy, by other threads too; the barrier puts those writes before this thread's fence, and the
+  // fence puts them before the tensor core's reads.
+  auto issue = [&](int q, bool last) {  // steps 2 q and 2 q + 1
+    fence_proxy_async_smem();
+    tc_fence_after();
+    const uint32_t a0 = d0 + (2 * q & (G::NDB - 1)) * G::DB, b0 = h0 + (2 * q & (G::HSLOTS - 1)) * G::HT;
+    const uint64_t bd = smem_desc(b0, G::HT, G::HP);
+#pragma unroll
+    for (int m = 0; m < G::DRT; ++m)
+      umma_16(tmem + m * D, smem_desc(a0 + m * 16 * G::DP, G::DB, G::DP), bd, instr_desc_16(128, D, 1, 1), q > 0 ? 1u : 0u);
+    umma_commit(last ? all_done : done);
+  };
+#pragma unroll
+  for (int s = 0; s < AHEAD; ++s) load_h(s);
+  __syncthreads();  // (in front of step 0)
+  bool dead = false;
+  for (int j = 0; j < T; ++j) {
+    cp_async_wait<AHEAD - 1>();  // h of step j
+    // step j + 1 writes its deltas over those of step j - 3, and the h of step j + AHEAD lands where that of step j - 4 is
+    if (lane == 0 && (j & 1) && j >= 3 && !dead && !mbar_wait_bounded(done, (uint32_t)((j - 3) / 2 & 1))) {
+      dead = true;
+      report_timeout(p.status, T - 1 - j);
+    }
+    __syncthreads();
+    if (lane == 0 && (j & 1)) issue(j / 2, j == T - 1);
+    load_h(j + AHEAD);
+  }
+  if (T & 1) {  // the last product's second step does not exist
+    for (uint32_t i = lane; i < G::DB / 16; i += 32) sts128(d0 + (T & (G::NDB - 1)) * G::DB + i * 16, make_uint4(0u, 0u, 0u, 0u));
+    __syncwarp();
+    if (lane == 0) issue(T / 2, true);
+  }
+  cp_async_wait<0>();
+}
+
+template <int CELL, int KT, int U, int NT, bool HELP, bool DR>
+__global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP, DR>::TH, LaneBwdGeom<CELL, KT, U, NT, HELP, DR>::MINB) lane_bwd_kernel(const __grid_constant__ LoopParams p) {
+  using G = LaneBwdGeom<CELL, KT, U, NT, HELP, DR>;
   using C = Cell<CELL>;
   // packed arithmetic where it measured faster (LSTM D = 64, one CTA per head: B1024 N16, 11551 -> 9881 clk per step of all CTAs)
   using F2 = typename PairOf<CELL == CELL_LSTM && !G::CL>::type;
@@ -239,7 +312,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBw
   const int n = blockIdx.z, bt0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
   const size_t ND = (size_t)N * D;
-  const int f32 = p.state_f32;
+  const int f32 = DR ? 0 : p.state_f32;
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const uint32_t sm = smem_u32(smem_raw), recv = sm + G::OFF_R;
@@ -247,23 +320,49 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBw
   // HELP: a wait of the cell's warps expired: the others, which wait for nothing but the CTA's barrier, must stop sending too
   volatile int* gave_up = reinterpret_cast<volatile int*>(smem_raw + G::OFF_BAR + 16);
 
-  if (CL) {
+  uint64_t* dr_done = reinterpret_cast<uint64_t*>(smem_raw + G::OFF_BAR + 24);  // DR: [2] a product has been computed, all of them
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + G::OFF_BAR + 40);
+  constexpr int DRW = WP + G::IOW;  // DR: the warp that forms dR
+
+  if (DR && warp == DRW) {
+    tmem_alloc(tmem_slot, G::DRC);
+    tc_fence_before();
+  }
+  if (CL || DR) {
     if (tid == 0) {
-      *gave_up = 0;
-      mbar_init(&full[0], 1 + OWN);
-      mbar_init(&full[1], 1 + OWN);
+      if (DR) {
+        mbar_init(&dr_done[0], 1);
+        mbar_init(&dr_done[1], 1);
+      }
+      if (CL) {
+        *gave_up = 0;
+        mbar_init(&full[0], 1 + OWN);
+        mbar_init(&full[1], 1 + OWN);
+      }
       fence_mbar_init();
-      mbar_arrive_expect_tx(&full[0], STEP_BYTES);             // partial sums of step index 0 (t = T-1)
-      if (T > 1) mbar_arrive_expect_tx(&full[1], STEP_BYTES);  // step index 1
+      if (CL) {
+        mbar_arrive_expect_tx(&full[0], STEP_BYTES);             // partial sums of step index 0 (t = T-1)
+        if (T > 1) mbar_arrive_expect_tx(&full[1], STEP_BYTES);  // step index 1
+      }
     }
     __syncthreads();
-    cluster_arrive();  // waited for before the first push
+    if (CL) cluster_arrive();  // waited for before the first push
   }
 
   if (warp >= WP) {
     const int io = tid - 32 * WP;
-    if (f32) lane_bwd_io<CELL, G, 4>(p, sm, sm + G::OFF_I, io, crank);
-    else lane_bwd_io<CELL, G, 2>(p, sm, sm + G::OFF_I, io, crank);
+    if (DR && warp == DRW) {
+      tc_fence_after();
+      const uint32_t tmem = *tmem_slot;
+      if constexpr (DR) lane_bwd_dr<G>(p, sm, sm + G::OFF_H, lane, tmem, &dr_done[0], &dr_done[1]);
+      bar_sync<32 * W + 32>(3);  // dR has left tensor memory
+      tc_fence_after();
+      tmem_dealloc(tmem, G::DRC);
+    } else if (!DR && f32) {
+      lane_bwd_io<CELL, G, 4>(p, sm, sm + G::OFF_I, io, crank);
+    } else {
+      lane_bwd_io<CELL, G, 2>(p, sm, sm + G::OFF_I, io, crank);
+    }
     if (CL) {
       __syncwarp();
       cluster_wait();
@@ -304,11 +403,11 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBw
   const bool drop = p.test_drop && crank == 0;  // test hook: CTA 0 withholds its first message
   // HELP: partial dh_{t-1} of the deltas of step index j
   auto products = [&](int j, bool stop) {
-    const uint32_t tile = sm + (j & 1) * DB + (uint32_t)tig * 128u + ((uint32_t)(gid ^ (int)opnd_swz((uint32_t)tig)) << 4);
+    const uint32_t tile = sm + (j & (G::NDB - 1)) * DB + lane_opnd<G::DP>(gid, tig);
     static_assert(!HELP || G::KS % 2 == 0, "whole k-pairs");
     uint4 b[KP];
 #pragma unroll
-    for (int kp = 0; kp < KP; ++kp) b[kp] = lds128(tile + (uint32_t)(kp * 512));
+    for (int kp = 0; kp < KP; ++kp) b[kp] = lds128(tile + (uint32_t)(kp * 4 * G::DP));
     const bool send = !stop && !*gave_up && !(drop && j == 0);
     constexpr int NSP = G::KS >= 4 ? 2 : 1;  // sums of a tile in two chains: with two warps per quadrant, four
     float part[MT][2][4];
@@ -370,7 +469,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBw
     ok[nb] = b < B;
     cw[nb] = sm + G::OFF_I + r * G::CP + ul * 2 * GCM;
     sw[nb] = sm + G::OFF_I + G::IN_S + r * G::SP + ul * (f32 ? 4 : 2);
-    dloc[nb] = sm + (r >> 3) * DT + opnd_off(r & 7, ul);
+    dloc[nb] = sm + (r >> 3) * DT + G::doff(r & 7, ul);
 #pragma unroll
     for (int s = 0; s < S; ++s) car[nb][s] = v_pair<F2>(0.f, 0.f);
 #pragma unroll
@@ -382,7 +481,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBw
   }
   // gate g's word of a lane lies g * U columns on: a constant distance when U / 8 blocks leave the permutation unchanged
   auto dgate = [&](int nb, int g) -> uint32_t {
-    if constexpr (U % 32 == 0) return dloc[nb] + g * (U * 16);
+    if constexpr (DR || U % 32 == 0) return dloc[nb] + g * (U / 8 * G::DP);
     else return sm + (row_of(nb) >> 3) * DT + opnd_off(row_of(nb) & 7, g * U + ul);
   };
 
@@ -470,7 +569,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBw
   __syncthreads();  // the inputs of the first step have landed
   int stage = 0;
   for (int j = 0; j < T; ++j) {  // j-th step of the reverse loop, time index t = T-1-j
-    const int t = T - 1 - j, buf = j & 1;
+    const int t = T - 1 - j, buf = j & 1, dbuf = j & (G::NDB - 1);
     load_inputs(stage);
     form_coefs();
     if constexpr (HELP) {  // (left to itself the compiler moves part of this behind the wait: sLSTM D = 256 174 -> 197 us per 256 steps)
@@ -496,15 +595,15 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBw
       if (p.gclip > 0.f) r = v_clamp(r, p.gclip);
       cell_backward_apply<CELL>(v_add(dext0[nb], r), co[nb], car[nb], dR_, dW_, dB_);
 #pragma unroll
-      for (int g = 0; g < Gr; ++g) sts32(dgate(nb, g) + buf * DB, v_pack(dR_[g]));
-      if constexpr (Gr == 3) sts32(dgate(nb, 3) + buf * DB, v_pack(dW_[2]));
+      for (int g = 0; g < Gr; ++g) sts32(dgate(nb, g) + dbuf * DB, v_pack(dR_[g]));
+      if constexpr (Gr == 3) sts32(dgate(nb, 3) + dbuf * DB, v_pack(dW_[2]));
 #pragma unroll
       for (int g = 0; g < Gt; ++g) dbacc[g] = v_add(dbacc[g], dB_[g]);
     }
     __syncthreads();
     // ---- partial dh_{t-1}
     float acc[MT][NT][4];
-    if constexpr (!HELP) lane_mma<MT, G::KS, NT, NS, false>(A, sm + buf * DB, DT, gid, tig, acc, []() {});
+    if constexpr (!HELP) lane_mma<MT, G::KS, NT, NS, false, G::DP>(A, sm + dbuf * DB, DT, gid, tig, acc, []() {});
     if constexpr (HELP) {
       if (j == 0) cluster_wait();
       products(j, poisoned);
@@ -547,6 +646,28 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP>::TH, LaneBw
     const float2 v = v_get(dbacc[g]);
     atomicAdd(p.dbias + (size_t)g * ND + nd, v.x);
     atomicAdd(p.dbias + (size_t)g * ND + nd + 1, v.y);
+  }
+  if constexpr (DR) {  // dR: row 128 m + 32 warp + lane of the CTA's gate rows lies in this lane's columns [m D, (m + 1) D)
+    if (!mbar_wait_bounded(&dr_done[1], 0)) report_timeout(p.status, -1);
+    tc_fence_after();
+    const uint32_t tcol = *tmem_slot + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+    for (int m = 0; m < G::DRT; ++m) {
+      const int row = m * 128 + warp * 32 + lane, g = row / U;
+      float* out = p.dR + (((size_t)g * N + n) * D + (int)crank * U + (row - g * U)) * D;
+#pragma unroll 1
+      for (int c = 0; c < D; c += 32) {
+        uint32_t r[32];
+        tmem_ld32(tcol + m * D + c, r);
+        if (row < G::K) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            red_add_f32x4(out + c + i, __uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+        }
+      }
+    }
+    tc_fence_before();
+    bar_sync<32 * W + 32>(3);
   }
   // every message to this CTA has been waited for; only after an expired wait can one still be in flight, and then the barrier
   // covers it

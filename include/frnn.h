@@ -204,6 +204,7 @@ int frnn_backward(const frnn_plan* plan, const frnn_bwd_args* args, void* stream
 /* The two halves of frnn_backward, for callers that want to time or overlap them separately:
  * FRNN_PART_LOOP = zero the fp32 gradients, repack R^T, run the reverse time loop (dWx, ds0, db);
  * FRNN_PART_DR   = the dR reduction over all (b,t), which needs the loop's dWx.  frnn_backward = both, in order.
+ * Where the loop forms dR itself (the 128-row loops, most of head dim 64) the second half has nothing left to do.
  * Same reference counterpart as frnn_backward (the reference also runs these as separate launches,
  * flashrnn/flashrnn/fused/flashrnn_fused_backward.cu:947-1000 and 1049-1058). */
 enum { FRNN_PART_LOOP = 1, FRNN_PART_DR = 2 };
