@@ -20,24 +20,25 @@ static bool cell_dims(int cell, CellDims* d) {
   return false;
 }
 
-// The lane loops (head dims up to 256) and those for larger head dims of a kernel family (kernel_cell) and direction.
-static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt) {
+// The lane loops (head dims up to 256) and those for larger head dims of a kernel family (kernel_cell) and direction.  s16: the form
+// for 16-bit states, null where there is none (states16_form)
+static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt, bool s16 = false) {
   switch (cell) {
-    case CELL_LSTM: return bwd ? lane_bwd_lstm(kt, u, nt) : lane_fwd_lstm(kt, u, nt);
-    case CELL_GRU: return bwd ? lane_bwd_gru(kt, u, nt) : lane_fwd_gru(kt, u, nt);
-    case CELL_ELMAN: return bwd ? lane_bwd_elman(kt, u, nt) : lane_fwd_elman(kt, u, nt);
-    case CELL_ELMAN_CLIP: return bwd ? lane_bwd_elmanc(kt, u, nt) : lane_fwd_elmanc(kt, u, nt);
-    case CELL_SLSTM: return bwd ? lane_bwd_slstm(kt, u, nt) : lane_fwd_slstm(kt, u, nt);
+    case CELL_LSTM: return bwd ? lane_bwd_lstm(kt, u, nt, s16) : lane_fwd_lstm(kt, u, nt, s16);
+    case CELL_GRU: return bwd ? lane_bwd_gru(kt, u, nt, s16) : lane_fwd_gru(kt, u, nt, s16);
+    case CELL_ELMAN: return bwd ? lane_bwd_elman(kt, u, nt, s16) : lane_fwd_elman(kt, u, nt, s16);
+    case CELL_ELMAN_CLIP: return bwd ? lane_bwd_elmanc(kt, u, nt, s16) : lane_fwd_elmanc(kt, u, nt, s16);
+    case CELL_SLSTM: return bwd ? lane_bwd_slstm(kt, u, nt, s16) : lane_fwd_slstm(kt, u, nt, s16);
   }
   return LaneKernel{nullptr, 0, 0};
 }
-static LaneKernel lane_help_kernel(int cell, int kt) {
+static LaneKernel lane_help_kernel(int cell, int kt, bool s16) {
   switch (cell) {
-    case CELL_LSTM: return lane_bwd_help_lstm(kt);
-    case CELL_GRU: return lane_bwd_help_gru(kt);
-    case CELL_ELMAN: return lane_bwd_help_elman(kt);
-    case CELL_ELMAN_CLIP: return lane_bwd_help_elmanc(kt);
-    case CELL_SLSTM: return lane_bwd_help_slstm(kt);
+    case CELL_LSTM: return lane_bwd_help_lstm(kt, s16);
+    case CELL_GRU: return lane_bwd_help_gru(kt, s16);
+    case CELL_ELMAN: return lane_bwd_help_elman(kt, s16);
+    case CELL_ELMAN_CLIP: return lane_bwd_help_elmanc(kt, s16);
+    case CELL_SLSTM: return lane_bwd_help_slstm(kt, s16);
   }
   return LaneKernel{nullptr, 0, 0};
 }
@@ -78,6 +79,8 @@ static int kernel_cell(const frnn_problem& pr) {
 static int cache_slots_of(const frnn_problem& pr, const CellDims& cd) {
   return (pr.cell == CELL_ELMAN && !(pr.forward_clip > 0.f)) ? 0 : cd.GC;
 }
+
+static int sm_count_cached();
 
 constexpr int kMaxTiles = 65535;  // blocks in y of a launch
 
@@ -216,6 +219,15 @@ static bool lane_dr(const frnn_plan& pl, int nt) {
   return pr.T >= kDrMinSteps && (pr.cell != CELL_SLSTM || (long long)((pr.B + 7) / 8) * pr.N >= kDrMinTilesSlstm);
 }
 
+// Whether a lane loop takes its form for 16-bit states where there is one (states16_form).  Two of them need registers that cost a CTA per SM, or the
+// larger part of the gain, once CTAs queue up: LSTM, us, D = 64 forward B150 N12 T64 50 -> 44, B400 N12 T128 204 -> 208, B1024 N16 T64 285 -> 296; D = 32 reverse B16 N8 T512 159 ->
+// 140, B1024 N24 T64 239 -> 244.
+static bool lane_states16(const frnn_problem& pr, bool bwd, int u, int nt) {
+  if (pr.dtype_state == FRNN_DTYPE_F32) return false;
+  const bool few = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N * (pr.D / u) <= 2LL * sm_count_cached();
+  return few || pr.cell != CELL_LSTM || pr.D != (bwd ? 32 : 64);
+}
+
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
   const int D = pr.D;
   if (bt == kWideBatchTile) return cs == 1 && wide_problem(pr);  // 128-row tensor-core loops: one CTA per head and tile
@@ -235,8 +247,6 @@ static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) 
     if (!lane_kernel(kernel_cell(pr), false, D / 16, U, nt).fn || !lane_kernel(kernel_cell(pr), true, D / 16, U, nt).fn) return false;
   return true;
 }
-
-static int sm_count_cached();
 
 // Default tile per problem.  Small-batch problems are bound by the per-step latency of the serial chain, so
 // the head is spread over as many SMs as a portable cluster allows; large-batch problems already fill the
@@ -331,9 +341,13 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
   const bool dr = bwd && !pl.probe_noop_cell && lane_dr(pl, nt);
   if (dr) {
     k = lane_dr_kernel(cell);
-  } else if (bwd && !pl.probe_noop_cell && lane_help(pr, pl.cluster_size, u, nt)) {
-    const LaneKernel h = lane_help_kernel(cell, kt);
-    if (h.fn) k = h;
+  } else if (!pl.probe_noop_cell) {
+    const bool help = bwd && lane_help(pr, pl.cluster_size, u, nt) && lane_help_kernel(cell, kt, false).fn;
+    if (help) k = lane_help_kernel(cell, kt, false);
+    if (lane_states16(pr, bwd, u, nt)) {
+      const LaneKernel h = help ? lane_help_kernel(cell, kt, true) : lane_kernel(cell, bwd, kt, u, nt, true);
+      if (h.fn) k = h;
+    }
   }
   return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt, dr};
 }

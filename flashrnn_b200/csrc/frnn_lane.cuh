@@ -116,6 +116,34 @@ template <int GC> struct CacheGeom {
   static constexpr bool EXTRA = GC > 4;
 };
 
+// Lane loops that also exist with 16-bit states fixed at compile time (S16): the fp32 alternative of every state access costs registers and issue slots, and
+// where the compiler makes more of their absence the form is used.  It does not everywhere (GRU D = 128 forward 228 -> 246 us, LSTM D = 192 reverse of
+// 16 rows 392 -> 465), so each was measured; those listed are ahead by 1 to 23 % (us, few CTAs, T512, or GPU filled; * 16 rows).
+//   forward  LSTM D = 16 101 -> 97, * 129 -> 121, 32 168 -> 140, 64 210 -> 200, 96 85 -> 83, 128 231 -> 224, 256 * 610 -> 592; GRU 16 91 -> 89, 32 154 -> 150, * 178 -> 163, 64 * 240 -> 226, 96
+//            157 -> 155; sLSTM 32 176 -> 148, 64 251 -> 243, 96 259 -> 249, * 461 -> 406, 256 149 -> 145, * 654 -> 629; Elman 16 56 -> 52, * 35.5 -> 33.6, 32 63 -> 58, 64 79 -> 73, 128 179 -> 171, in
+//            one CTA 21.1 -> 19.1, 256 228 -> 222
+//   reverse  LSTM 16 142 -> 132, 32 159 -> 140, 96 * 410 -> 403, 128 263 -> 249 and 106 -> 82, 192 292 -> 286, 256 337 -> 330, * 703 -> 694; GRU 96 155 -> 141, 128 (with warps that only multiply) 235 -> 228,
+//            192 280 -> 264, * 257 -> 249, 256 (without) 97 -> 95; sLSTM 16 153 -> 126, 32 165 -> 162, 96 265 -> 228, 128 279 -> 265, 256 * 716 -> 695; Elman 16 66 -> 65, * 48 -> 44.5, 32 78 -> 62, 128 208 -> 201, in
+//            one CTA 29.0 -> 27.3, 192 239 -> 230, 256 in CTAs of 64 190 -> 185
+__host__ __device__ constexpr bool states16_form(int cell, bool bwd, int kt, int u, int nt, bool help) {
+  const int d = kt * 16;
+  const bool one = nt == 1, dflt = u == (d <= 64 ? d : 32);  // (CTAs the tile table makes)
+  if (cell == CELL_ELMAN && one && !help && ((d == 128 && u == 128) || (bwd && d == 256 && u == 64))) return true;
+  if (!dflt) return false;
+  if (!bwd) {
+    if (cell == CELL_LSTM) return one ? d <= 128 : d == 16 || d == 256;
+    if (cell == CELL_GRU) return one ? d == 16 || d == 32 || d == 96 : d == 32 || d == 64;
+    if (cell == CELL_SLSTM) return one ? d == 32 || d == 64 || d == 96 || d == 256 : d == 96 || d == 256;
+    if (cell == CELL_ELMAN) return one ? d <= 64 || d == 128 || d == 256 : d == 16;
+    return false;
+  }
+  if (cell == CELL_LSTM) return one ? d == 16 || d == 32 || (d == 128 && !help) || (d >= 192 && help) : d == 96 || d == 256;
+  if (cell == CELL_GRU) return one ? ((d == 96 || d == 128) && help) || d == 192 || (d == 256 && !help) : d == 192;
+  if (cell == CELL_SLSTM) return one ? d == 16 || d == 32 || ((d == 96 || d == 128) && help) : d == 256;
+  if (cell == CELL_ELMAN) return one ? d == 16 || d == 32 || ((d == 128 || d == 192) && help) : d == 16;
+  return false;
+}
+
 // ---- IO warps.  A lane's values belong to 8 batch rows per warp instruction (the MMA's accumulator layout), and the L1 charges
 // a global access per row touched: with the compute lanes loading Wx and storing states and cache themselves the LSTM D = 64 forward
 // step spent ~700 of 1380 clk on it.  So one or two extra warps move everything between global memory and padded tiles in shared

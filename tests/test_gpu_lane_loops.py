@@ -25,6 +25,13 @@ def test_head_dims_above_256_edges(cuda_device, function, N, D, B, T, state_f32)
     _check(function, N, D, B, T, state_f32)
 
 
+# the tiles the table picks, with the forms for 16-bit states where there are: few CTAs, and Elman's whole heads per CTA where CTAs fill the GPU
+@pytest.mark.parametrize("function", ["lstm", "gru", "elman", "slstm"])
+@pytest.mark.parametrize("N,D,B,T", [(2, 16, 9, 7), (1, 32, 9, 8), (3, 64, 1, 5), (2, 96, 9, 7), (1, 128, 17, 6), (1, 192, 9, 7), (32, 128, 33, 3), (19, 256, 57, 2)])
+def test_lane_loops_own_tiles(cuda_device, function, N, D, B, T):
+    _check(function, N, D, B, T, False)
+
+
 # the clusters that large batches run with 16 rows
 @pytest.mark.parametrize("function,D,cs", [("slstm", 96, 3), ("lstm", 96, 3), ("slstm", 128, 4), ("lstm", 128, 4), ("gru", 192, 6), ("gru", 256, 8)])
 def test_lane_loops_16_rows(cuda_device, function, D, cs):
