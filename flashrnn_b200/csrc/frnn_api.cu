@@ -6,6 +6,7 @@
 #include <mutex>
 
 #include "frnn_aux.cuh"
+#include "frnn_lane.cuh"
 
 namespace FRNN_NS {
 
@@ -20,25 +21,25 @@ static bool cell_dims(int cell, CellDims* d) {
   return false;
 }
 
-// The lane loops (head dims up to 256) and those for larger head dims of a kernel family (kernel_cell) and direction.  s16: the form
-// for 16-bit states, null where there is none (states16_form)
-static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt, bool s16 = false) {
+// The lane loops (head dims up to 256) and those for larger head dims of a kernel family (kernel_cell) and direction.  es: bytes of a
+// state element, 0: known at run time only; the others are null where there is none (states_form)
+static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt, int es) {
   switch (cell) {
-    case CELL_LSTM: return bwd ? lane_bwd_lstm(kt, u, nt, s16) : lane_fwd_lstm(kt, u, nt, s16);
-    case CELL_GRU: return bwd ? lane_bwd_gru(kt, u, nt, s16) : lane_fwd_gru(kt, u, nt, s16);
-    case CELL_ELMAN: return bwd ? lane_bwd_elman(kt, u, nt, s16) : lane_fwd_elman(kt, u, nt, s16);
-    case CELL_ELMAN_CLIP: return bwd ? lane_bwd_elmanc(kt, u, nt, s16) : lane_fwd_elmanc(kt, u, nt, s16);
-    case CELL_SLSTM: return bwd ? lane_bwd_slstm(kt, u, nt, s16) : lane_fwd_slstm(kt, u, nt, s16);
+    case CELL_LSTM: return bwd ? lane_bwd_lstm(kt, u, nt, es) : lane_fwd_lstm(kt, u, nt, es);
+    case CELL_GRU: return bwd ? lane_bwd_gru(kt, u, nt, es) : lane_fwd_gru(kt, u, nt, es);
+    case CELL_ELMAN: return bwd ? lane_bwd_elman(kt, u, nt, es) : lane_fwd_elman(kt, u, nt, es);
+    case CELL_ELMAN_CLIP: return bwd ? lane_bwd_elmanc(kt, u, nt, es) : lane_fwd_elmanc(kt, u, nt, es);
+    case CELL_SLSTM: return bwd ? lane_bwd_slstm(kt, u, nt, es) : lane_fwd_slstm(kt, u, nt, es);
   }
   return LaneKernel{nullptr, 0, 0};
 }
-static LaneKernel lane_help_kernel(int cell, int kt, bool s16) {
+static LaneKernel lane_help_kernel(int cell, int kt, int es) {
   switch (cell) {
-    case CELL_LSTM: return lane_bwd_help_lstm(kt, s16);
-    case CELL_GRU: return lane_bwd_help_gru(kt, s16);
-    case CELL_ELMAN: return lane_bwd_help_elman(kt, s16);
-    case CELL_ELMAN_CLIP: return lane_bwd_help_elmanc(kt, s16);
-    case CELL_SLSTM: return lane_bwd_help_slstm(kt, s16);
+    case CELL_LSTM: return lane_bwd_help_lstm(kt, es);
+    case CELL_GRU: return lane_bwd_help_gru(kt, es);
+    case CELL_ELMAN: return lane_bwd_help_elman(kt, es);
+    case CELL_ELMAN_CLIP: return lane_bwd_help_elmanc(kt, es);
+    case CELL_SLSTM: return lane_bwd_help_slstm(kt, es);
   }
   return LaneKernel{nullptr, 0, 0};
 }
@@ -219,13 +220,14 @@ static bool lane_dr(const frnn_plan& pl, int nt) {
   return pr.T >= kDrMinSteps && (pr.cell != CELL_SLSTM || (long long)((pr.B + 7) / 8) * pr.N >= kDrMinTilesSlstm);
 }
 
-// Whether a lane loop takes its form for 16-bit states where there is one (states16_form).  Two of them need registers that cost a CTA per SM, or the
-// larger part of the gain, once CTAs queue up: LSTM, us, D = 64 forward B150 N12 T64 50 -> 44, B400 N12 T128 204 -> 208, B1024 N16 T64 285 -> 296; D = 32 reverse B16 N8 T512 159 ->
-// 140, B1024 N24 T64 239 -> 244.
-static bool lane_states16(const frnn_problem& pr, bool bwd, int u, int nt) {
-  if (pr.dtype_state == FRNN_DTYPE_F32) return false;
+// The lane loop of a plan's tile: with the type of its states fixed where there is such a form and it pays, else the general one.
+static LaneKernel lane_loop(const frnn_problem& pr, bool bwd, int u, int nt, bool help) {
+  const int cell = kernel_cell(pr), kt = pr.D / 16, es = pr.dtype_state == FRNN_DTYPE_F32 ? 4 : 2;
+  auto get = [&](int s) { return help ? lane_help_kernel(cell, kt, s) : lane_kernel(cell, bwd, kt, u, nt, s); };
+  const LaneKernel form = get(es), general = get(0);
+  if (!form.fn || !general.fn) return form.fn ? form : general;
   const bool few = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N * (pr.D / u) <= 2LL * sm_count_cached();
-  return few || pr.cell != CELL_LSTM || pr.D != (bwd ? 32 : 64);
+  return few || !states_form_for_few(cell, bwd, kt, es) ? form : general;
 }
 
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
@@ -244,7 +246,7 @@ static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) 
   if (threads > (D < 192 ? 512 : D < 256 ? 384 : 256)) return false;
   if (bt == 32 && cd.Gr * U > 192) return false;
   for (int nt = 1; nt <= (bt < 16 ? 1 : 2); ++nt)
-    if (!lane_kernel(kernel_cell(pr), false, D / 16, U, nt).fn || !lane_kernel(kernel_cell(pr), true, D / 16, U, nt).fn) return false;
+    if (!lane_loop(pr, false, U, nt, false).fn || !lane_loop(pr, true, U, nt, false).fn) return false;
   return true;
 }
 
@@ -337,18 +339,12 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
     return LoopLaunch{k.fn, k.threads, bwd ? kBigStages - 1 : kBigStages, k.smem(pr.D), pr.D / t.u, t.u, 8 * nt};
   }
   const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.batch_tile, pl.forced_tile);
-  LaneKernel k = !pl.probe_noop_cell ? lane_kernel(cell, bwd, kt, u, nt) : bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
   const bool dr = bwd && !pl.probe_noop_cell && lane_dr(pl, nt);
-  if (dr) {
-    k = lane_dr_kernel(cell);
-  } else if (!pl.probe_noop_cell) {
-    const bool help = bwd && lane_help(pr, pl.cluster_size, u, nt) && lane_help_kernel(cell, kt, false).fn;
-    if (help) k = lane_help_kernel(cell, kt, false);
-    if (lane_states16(pr, bwd, u, nt)) {
-      const LaneKernel h = help ? lane_help_kernel(cell, kt, true) : lane_kernel(cell, bwd, kt, u, nt, true);
-      if (h.fn) k = h;
-    }
-  }
+  LaneKernel k = {nullptr, 0, 0};
+  if (pl.probe_noop_cell) k = bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
+  else if (dr) k = lane_dr_kernel(cell);
+  else if (bwd && lane_help(pr, pl.cluster_size, u, nt)) k = lane_loop(pr, true, u, nt, true);
+  if (!k.fn && !pl.probe_noop_cell) k = lane_loop(pr, bwd, u, nt, false);
   return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt, dr};
 }
 // x: the CTAs of a cluster, y: tiles of the batch, z: heads
@@ -553,7 +549,7 @@ int FRNN_ENTRY(frnn_query_loop)(const frnn_plan* plan, int backward, frnn_loop_s
   const LoopLaunch k = loop_of(*plan, backward != 0);
   if (!k.fn) return FRNN_ERR_PLAN;
   const dim3 g = loop_grid(k, pr);
-  *out = {is_big(pr) ? FRNN_LOOP_BIG : FRNN_LOOP_LANE, k.cs, k.u, k.rows, k.threads, k.stages, {g.x, g.y, g.z}};
+  *out = {is_big(pr) ? FRNN_LOOP_BIG : FRNN_LOOP_LANE, k.cs, k.u, k.rows, k.threads - (k.dr ? 32 : 0), k.stages, {g.x, g.y, g.z}};
   return FRNN_OK;
 }
 

@@ -25,9 +25,9 @@ struct BigKernel {
 
 // defined once per (cell, direction) in frnn_inst_*.cu
 #define FRNN_DECLARE(cell)                              \
-  LaneKernel lane_fwd_##cell(int kt, int u, int nt, bool s16); \
-  LaneKernel lane_bwd_##cell(int kt, int u, int nt, bool s16); \
-  LaneKernel lane_bwd_help_##cell(int kt, bool s16);    \
+  LaneKernel lane_fwd_##cell(int kt, int u, int nt, int es);  \
+  LaneKernel lane_bwd_##cell(int kt, int u, int nt, int es);  \
+  LaneKernel lane_bwd_help_##cell(int kt, int es);      \
   LaneKernel lane_bwd_dr_##cell();                      \
   BigKernel big_fwd_##cell(int u, int nt, bool dense);  \
   BigKernel big_bwd_##cell(int u, int nt);              \

@@ -24,7 +24,8 @@ template <int CELL, int U, int NT, bool DENSE>
 struct BigFwdGeom {
   using C = Cell<CELL>;
   static constexpr int BT = 8 * NT, NT8 = NT, UNITS = U, STAGES = kBigStages;
-  static constexpr bool QUAD = C::Gr > 1, CL = true, S16 = false;
+  static constexpr bool QUAD = C::Gr > 1, CL = true;
+  static constexpr int ES = 0;
   static constexpr int MT = QUAD ? 2 : 1, UW = QUAD ? 8 : 16;
   static constexpr int GROUPS = U / UW, W = 2 * GROUPS, IOT = 32 * GROUPS, TH = 32 * W;
   static constexpr int NB = QUAD ? NT : 2 * NT;

@@ -7,55 +7,55 @@ namespace FRNN_NS {
 
 // ---- lane loops (head dims up to 256): head dim / 16, units per CTA, batch tile / 8
 #if FRNN_INST_BWD
-#define FRNN_GEOM(KT, U, NT, S16) LaneBwdGeom<FRNN_INST_CELL, KT, U, NT, false, S16, false>
-#define FRNN_KERNEL(KT, U, NT, S16) lane_bwd_kernel<FRNN_INST_CELL, KT, U, NT, false, S16, false>
+#define FRNN_GEOM(KT, U, NT, ES) LaneBwdGeom<FRNN_INST_CELL, KT, U, NT, false, ES, false>
+#define FRNN_KERNEL(KT, U, NT, ES) lane_bwd_kernel<FRNN_INST_CELL, KT, U, NT, false, ES, false>
 #else
-#define FRNN_GEOM(KT, U, NT, S16) LaneFwdGeom<FRNN_INST_CELL, KT, U, NT, S16>
-#define FRNN_KERNEL(KT, U, NT, S16) lane_fwd_kernel<FRNN_INST_CELL, KT, U, NT, S16>
+#define FRNN_GEOM(KT, U, NT, ES) LaneFwdGeom<FRNN_INST_CELL, KT, U, NT, ES>
+#define FRNN_KERNEL(KT, U, NT, ES) lane_fwd_kernel<FRNN_INST_CELL, KT, U, NT, ES>
 #endif
 
-// s16: the form for 16-bit states, where there is one, else null
-template <int KT, int U, int NT, bool S16, bool V = FRNN_GEOM(KT, U, NT, S16)::valid && (!S16 || states16_form(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false))>
+// ES: bytes of a state element, 0: known at run time only; which exist: states_form, states_general.  Null for the others.
+template <int KT, int U, int NT, int ES, bool V = FRNN_GEOM(KT, U, NT, ES)::valid && (ES ? states_form(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false, ES) : states_general(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false))>
 struct LaneEntry {
   static LaneKernel get() { return LaneKernel{nullptr, 0, 0}; }
 };
-template <int KT, int U, int NT, bool S16>
-struct LaneEntry<KT, U, NT, S16, true> {
+template <int KT, int U, int NT, int ES>
+struct LaneEntry<KT, U, NT, ES, true> {
   static LaneKernel get() {
-    using G = FRNN_GEOM(KT, U, NT, S16);
-    return LaneKernel{reinterpret_cast<const void*>(&FRNN_KERNEL(KT, U, NT, S16)), G::TH, G::smem};
+    using G = FRNN_GEOM(KT, U, NT, ES);
+    return LaneKernel{reinterpret_cast<const void*>(&FRNN_KERNEL(KT, U, NT, ES)), G::TH, G::smem};
   }
 };
 
 #if FRNN_INST_BWD
-template <int KT, int U, bool HELP, bool S16, bool DR,
-          bool V = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, S16, DR>::valid && (!S16 || DR || states16_form(FRNN_INST_CELL, true, KT, U, 1, HELP))>
+template <int KT, int U, bool HELP, int ES, bool DR,
+          bool V = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, ES, DR>::valid && (DR || (ES ? states_form(FRNN_INST_CELL, true, KT, U, 1, HELP, ES) : states_general(FRNN_INST_CELL, true, KT, U, 1, HELP)))>
 struct BwdEntry {
   static LaneKernel get() { return LaneKernel{nullptr, 0, 0}; }
 };
-template <int KT, int U, bool HELP, bool S16, bool DR>
-struct BwdEntry<KT, U, HELP, S16, DR, true> {
+template <int KT, int U, bool HELP, int ES, bool DR>
+struct BwdEntry<KT, U, HELP, ES, DR, true> {
   static LaneKernel get() {
-    using G = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, S16, DR>;
-    return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<FRNN_INST_CELL, KT, U, 1, HELP, S16, DR>), G::TH, G::smem};
+    using G = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, ES, DR>;
+    return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<FRNN_INST_CELL, KT, U, 1, HELP, ES, DR>), G::TH, G::smem};
   }
 };
 // the reverse loops with warps that only multiply (clusters of 32-unit CTAs, 8 rows), null where there is none
-template <bool S16>
+template <int ES>
 static LaneKernel help_entry(int kt) {
-  return kt == 6 ? BwdEntry<6, 32, true, S16, false>::get() : kt == 8 ? BwdEntry<8, 32, true, S16, false>::get() : kt == 12 ? BwdEntry<12, 32, true, S16, false>::get()
-       : kt == 16 ? BwdEntry<16, 32, true, S16, false>::get() : LaneKernel{nullptr, 0, 0};
+  return kt == 6 ? BwdEntry<6, 32, true, ES, false>::get() : kt == 8 ? BwdEntry<8, 32, true, ES, false>::get() : kt == 12 ? BwdEntry<12, 32, true, ES, false>::get()
+       : kt == 16 ? BwdEntry<16, 32, true, ES, false>::get() : LaneKernel{nullptr, 0, 0};
 }
-LaneKernel FRNN_INST_HELP(int kt, bool s16) { return s16 ? help_entry<true>(kt) : help_entry<false>(kt); }
+LaneKernel FRNN_INST_HELP(int kt, int es) { return es == 2 ? help_entry<2>(kt) : es == 4 ? help_entry<4>(kt) : help_entry<0>(kt); }
 // the reverse loop with a warp that forms dR (head dim 64, one CTA per head)
-LaneKernel FRNN_INST_DR() { return BwdEntry<4, 64, false, true, true>::get(); }
+LaneKernel FRNN_INST_DR() { return BwdEntry<4, 64, false, 2, true>::get(); }
 #endif
 
-template <bool S16>
+template <int ES>
 static LaneKernel lane_entry(int kt, int u, int nt) {
 #define FRNN_CASE(KT, U)                                         \
-  if (kt == KT && u == U && nt == 1) return LaneEntry<KT, U, 1, S16>::get(); \
-  if (kt == KT && u == U && nt == 2) return LaneEntry<KT, U, 2, S16>::get();
+  if (kt == KT && u == U && nt == 1) return LaneEntry<KT, U, 1, ES>::get(); \
+  if (kt == KT && u == U && nt == 2) return LaneEntry<KT, U, 2, ES>::get();
   FRNN_FOREACH_KT_U(FRNN_CASE)
   // wide CTAs: the one- and three-gate cells only (the others would need more than 512 threads or registers than there are)
   if constexpr (Cell<FRNN_INST_CELL>::Gr < 4) { FRNN_FOREACH_KT_U_FEW_GATES(FRNN_CASE) }
@@ -63,7 +63,7 @@ static LaneKernel lane_entry(int kt, int u, int nt) {
 #undef FRNN_CASE
   return LaneKernel{nullptr, 0, 0};
 }
-LaneKernel FRNN_INST_LANE(int kt, int u, int nt, bool s16) { return s16 ? lane_entry<true>(kt, u, nt) : lane_entry<false>(kt, u, nt); }
+LaneKernel FRNN_INST_LANE(int kt, int u, int nt, int es) { return es == 2 ? lane_entry<2>(kt, u, nt) : es == 4 ? lane_entry<4>(kt, u, nt) : lane_entry<0>(kt, u, nt); }
 
 // ---- head dims above 256: units per CTA, batch tile / 8
 #if FRNN_INST_BWD

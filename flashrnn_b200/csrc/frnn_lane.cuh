@@ -116,32 +116,46 @@ template <int GC> struct CacheGeom {
   static constexpr bool EXTRA = GC > 4;
 };
 
-// Lane loops that also exist with 16-bit states fixed at compile time (S16): the fp32 alternative of every state access costs registers and issue slots, and
-// where the compiler makes more of their absence the form is used.  It does not everywhere (GRU D = 128 forward 228 -> 246 us, LSTM D = 192 reverse of
-// 16 rows 392 -> 465), so each was measured; those listed are ahead by 1 to 23 % (us, few CTAs, T512, or GPU filled; * 16 rows).
-//   forward  LSTM D = 16 101 -> 97, * 129 -> 121, 32 168 -> 140, 64 210 -> 200, 96 85 -> 83, 128 231 -> 224, 256 * 610 -> 592; GRU 16 91 -> 89, 32 154 -> 150, * 178 -> 163, 64 * 240 -> 226, 96
-//            157 -> 155; sLSTM 32 176 -> 148, 64 251 -> 243, 96 259 -> 249, * 461 -> 406, 256 149 -> 145, * 654 -> 629; Elman 16 56 -> 52, * 35.5 -> 33.6, 32 63 -> 58, 64 79 -> 73, 128 179 -> 171, in
-//            one CTA 21.1 -> 19.1, 256 228 -> 222
-//   reverse  LSTM 16 142 -> 132, 32 159 -> 140, 96 * 410 -> 403, 128 263 -> 249 and 106 -> 82, 192 292 -> 286, 256 337 -> 330, * 703 -> 694; GRU 96 155 -> 141, 128 (with warps that only multiply) 235 -> 228,
-//            192 280 -> 264, * 257 -> 249, 256 (without) 97 -> 95; sLSTM 16 153 -> 126, 32 165 -> 162, 96 265 -> 228, 128 279 -> 265, 256 * 716 -> 695; Elman 16 66 -> 65, * 48 -> 44.5, 32 78 -> 62, 128 208 -> 201, in
-//            one CTA 29.0 -> 27.3, 192 239 -> 230, 256 in CTAs of 64 190 -> 185
-__host__ __device__ constexpr bool states16_form(int cell, bool bwd, int kt, int u, int nt, bool help) {
+// Lane loops with the type of the states fixed at compile time (es = 2 or 4 bytes): the other type's side of every state access costs registers and issue
+// slots, and where the compiler makes more of its absence such a form is used.  It does not everywhere (16 bits: GRU D = 128 forward 228 -> 246 us, LSTM D = 192
+// reverse of 16 rows 392 -> 465; fp32: LSTM D = 16 forward 99 -> 134), so each was measured; those listed are ahead by 1 to 26 % (us; T512 and few CTAs, or the GPU
+// filled; * 16 rows, + with warps that only multiply).
+//   16 bits, forward  LSTM D = 16 101 -> 97, * 129 -> 121, 32 168 -> 140, 64 210 -> 200, 96 85 -> 83, 128 231 -> 224, 256 * 610 -> 592; GRU 16 91 -> 89, 32 154 -> 150, * 178 -> 163, 64 * 240 ->
+//            226, 96 157 -> 155; sLSTM 32 176 -> 148, 64 251 -> 243, 96 259 -> 249, * 461 -> 406, 256 149 -> 145, * 654 -> 629; Elman 16 56 -> 52, * 35.5 -> 33.6, 32 63 -> 58, 64 79 ->
+//            73, 128 179 -> 171, in one CTA 21.1 -> 19.1, 256 228 -> 222
+//   16 bits, reverse  LSTM 16 142 -> 132, 32 159 -> 140, 96 * 410 -> 403, 128 263 -> 249 and 106 -> 82, 192 + 292 -> 286, 256 + 337 -> 330, * 703 -> 694; GRU 96 + 155 -> 141, 128 + 235 ->
+//            228, 192 + 280 -> 264, * 257 -> 249, 256 97 -> 95; sLSTM 16 153 -> 126, 32 165 -> 162, 96 + 265 -> 228, 128 + 279 -> 265, 256 * 716 -> 695; Elman 16 66 -> 65, * 48 ->
+//            44.5, 32 78 -> 62, 128 + 208 -> 201, in one CTA 29.0 -> 27.3, 192 + 239 -> 230, 256 in CTAs of 64 190 -> 185
+//   fp32, forward     LSTM 32 217 -> 204, 64 278 -> 241, 96 255 -> 248, 128 243 -> 234, 192 263 -> 254, 256 298 -> 295, * 607 -> 589; GRU 16 91 -> 89, 64 183 -> 179, 96 156 -> 154, 192 247 -> 245,
+//            256 * 573 -> 563; sLSTM 32 230 -> 214, 96 264 -> 253, * 447 -> 435, 128 275 -> 266, 192 281 -> 278 and 327 -> 302, 256 318 -> 312, * 636 -> 630; Elman 16 56 -> 50, 32 62 -> 58, 64 87 ->
+//            81, 96 159 -> 155, 128 179 -> 168, in one CTA 21.4 -> 21.0, 192 206 -> 200, 256 234 -> 224
+//   fp32, reverse     LSTM 32 156 -> 136, 64 245 -> 208, 96 * 436 -> 408, 128 278 -> 272, 192 + 304 -> 299, * 397 -> 293; GRU 32 193 -> 158, 64 218 -> 207, 96 + 164 -> 153, 128 + 246 -> 234, 192 + 283 ->
+//            267, * 259 -> 256; sLSTM 16 144 -> 125, 32 163 -> 146, 64 251 -> 234, 96 + 276 -> 242, 128 + 288 -> 278, 256 * 723 -> 708; Elman 16 64 -> 60, * 67.4 -> 66.2, 32 74 -> 72, 64 130 -> 125, 128 +
+//            208 -> 202, in one CTA 56 -> 52
+__host__ __device__ constexpr bool states_form(int cell, bool bwd, int kt, int u, int nt, bool help, int es) {
   const int d = kt * 16;
-  const bool one = nt == 1, dflt = u == (d <= 64 ? d : 32);  // (CTAs the tile table makes)
-  if (cell == CELL_ELMAN && one && !help && ((d == 128 && u == 128) || (bwd && d == 256 && u == 64))) return true;
+  const bool one = nt == 1, dflt = u == (d <= 64 ? d : 32), h = es == 2;  // (CTAs the tile table makes)
+  if (cell == CELL_ELMAN && one && !help && ((d == 128 && u == 128) || (h && bwd && d == 256 && u == 64))) return true;
   if (!dflt) return false;
   if (!bwd) {
-    if (cell == CELL_LSTM) return one ? d <= 128 : d == 16 || d == 256;
-    if (cell == CELL_GRU) return one ? d == 16 || d == 32 || d == 96 : d == 32 || d == 64;
-    if (cell == CELL_SLSTM) return one ? d == 32 || d == 64 || d == 96 || d == 256 : d == 96 || d == 256;
-    if (cell == CELL_ELMAN) return one ? d <= 64 || d == 128 || d == 256 : d == 16;
+    if (cell == CELL_LSTM) return one ? (h ? d <= 128 : d >= 32) : (h && d == 16) || d == 256;
+    if (cell == CELL_GRU) return one ? d == 16 || (h && d == 32) || (!h && (d == 64 || d == 192)) || d == 96 : h ? d == 32 || d == 64 : d == 256;
+    if (cell == CELL_SLSTM) return one ? d == 32 || (h && d == 64) || d == 96 || (!h && (d == 128 || d == 192)) || d == 256 : d == 96 || d == 256;
+    if (cell == CELL_ELMAN) return one ? !h || d <= 64 || d == 128 || d == 256 : h && d == 16;
     return false;
   }
-  if (cell == CELL_LSTM) return one ? d == 16 || d == 32 || (d == 128 && !help) || (d >= 192 && help) : d == 96 || d == 256;
-  if (cell == CELL_GRU) return one ? ((d == 96 || d == 128) && help) || d == 192 || (d == 256 && !help) : d == 192;
-  if (cell == CELL_SLSTM) return one ? d == 16 || d == 32 || ((d == 96 || d == 128) && help) : d == 256;
-  if (cell == CELL_ELMAN) return one ? d == 16 || d == 32 || ((d == 128 || d == 192) && help) : d == 16;
+  if (cell == CELL_LSTM) return one ? (h && d == 16) || d == 32 || (!h && d == 64) || (d == 128 && !help) || (d == 192 && help) || (h && d == 256 && help) : d == 96 || d == (h ? 256 : 192);
+  if (cell == CELL_GRU) return one ? (!h && (d == 32 || d == 64)) || ((d == 96 || d == 128) && help) || (d == 192 && (h || help)) || (h && d == 256 && !help) : d == 192;
+  if (cell == CELL_SLSTM) return one ? d == 16 || d == 32 || (!h && d == 64) || ((d == 96 || d == 128) && help) : d == 256;
+  if (cell == CELL_ELMAN) return one ? d == 16 || d == 32 || (!h && d == 64) || (d == 128 && help) || (h && d == 192 && help) : d == 16;
   return false;
+}
+// Two of these forms need registers that cost a CTA per SM, or most of the gain, once CTAs queue up; the general form runs then.  LSTM, us, D = 64 forward, 16 bits: B150 N12
+// T64 50 -> 44, B400 N12 T128 204 -> 208, B1024 N16 T64 285 -> 296, fp32: B16 N12 T512 278 -> 241, B400 233 -> 241, B1024 325 -> 336; D = 32 reverse, 16 bits: B16 N8 T512 159 -> 140, B1024 N24 T64 239 -> 244.
+__host__ __device__ constexpr bool states_form_for_few(int cell, bool bwd, int kt, int es) { return cell == CELL_LSTM && (bwd ? kt == 2 && es == 2 : kt == 4); }
+// whether the form that reads the type of the states at run time is needed
+__host__ __device__ constexpr bool states_general(int cell, bool bwd, int kt, int u, int nt, bool help) {
+  return !states_form(cell, bwd, kt, u, nt, help, 2) || !states_form(cell, bwd, kt, u, nt, help, 4) || states_form_for_few(cell, bwd, kt, 2) || states_form_for_few(cell, bwd, kt, 4);
 }
 
 // ---- IO warps.  A lane's values belong to 8 batch rows per warp instruction (the MMA's accumulator layout), and the L1 charges

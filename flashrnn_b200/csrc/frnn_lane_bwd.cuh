@@ -29,7 +29,7 @@
 
 namespace FRNN_NS {
 
-template <int CELL, int KT, int U, int NT, bool HELP, bool S16, bool DR_>
+template <int CELL, int KT, int U, int NT, bool HELP, int ES, bool DR_>
 struct LaneBwdGeom {
   using C = Cell<CELL>;
   static constexpr int D = KT * 16, CS = D / U, BT = 8 * NT;
@@ -65,7 +65,7 @@ struct LaneBwdGeom {
   static constexpr int DRT = (K + 127) / 128, DRC = DRT * D;  // row tiles of dR, tensor-memory columns of their sums
   static constexpr int RB = CL ? CS * (U / 16) * 32 * NT * 16 : 0;  // bytes of received partial sums of one step
   // input ring: [kLaneStages] x { activations [BT] | fifth ones [BT] | states and cotangents [NSS][BT] }
-  static constexpr int CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2), SP = io_pitch(U * (S16 ? 2 : 4));  // S16: 16-bit states only
+  static constexpr int CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2), SP = io_pitch(U * (ES ? ES : 4));  // ES: bytes of a state element, 0: known at run time only
   static constexpr int IN_E = GCM ? BT * CP : 0, IN_S = IN_E + (GCX ? BT * EP : 0), IN_B = IN_S + NSS * BT * SP;
   static constexpr int OFF_R = NDB * DB, OFF_I = OFF_R + 2 * RB, OFF_H = OFF_I + kLaneStages * IN_B, OFF_BAR = OFF_H + HBYTES;
   static constexpr int SLICE = (U / 16) * 32 * NT * 16;  // bytes of partial sums from one CTA
@@ -75,7 +75,7 @@ struct LaneBwdGeom {
   static constexpr bool VOTE = CL && (HELP || !(CELL == CELL_GRU && (KT == 6 || KT == 12)));
   // CTAs per SM the registers are cut for (0: as the compiler sees fit), where a few registers more would cost large batches a CTA
   static constexpr int MINB = CL && NT == 1 && KT >= 12 && C::Gr == 1 && U == 64 ? 3 : 0;
-  static constexpr bool valid = (!DR || (S16 && C::Gr >= 3 && KT == 4 && !CL && NT == 1)) && (!HELP || (CL && NT == 1 && U == 32 && KT >= 6 && BASE != CELL_ELMAN_CLIP && !(BASE == CELL_LSTM && KT == 8))) && D % U == 0 && (!CL || U % 8 == 0) && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget;
+  static constexpr bool valid = (!DR || (ES == 2 && C::Gr >= 3 && KT == 4 && !CL && NT == 1)) && (!HELP || (CL && NT == 1 && U == 32 && KT >= 6 && BASE != CELL_ELMAN_CLIP && !(BASE == CELL_LSTM && KT == 8))) && D % U == 0 && (!CL || U % 8 == 0) && CS <= 16 && TH <= 512 + 64 && smem <= kSmemBudget;
 };
 
 // Index of the first of the two 16-byte fragments (rows gid, gid + 8) of lane 0 in the packed R^T of head n, CTA c: see
@@ -292,9 +292,9 @@ __device__ __forceinline__ void lane_bwd_dr(const LoopParams& p, uint32_t d0, ui
   cp_async_wait<0>();
 }
 
-template <int CELL, int KT, int U, int NT, bool HELP, bool S16, bool DR>
-__global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP, S16, DR>::TH, LaneBwdGeom<CELL, KT, U, NT, HELP, S16, DR>::MINB) lane_bwd_kernel(const __grid_constant__ LoopParams p) {
-  using G = LaneBwdGeom<CELL, KT, U, NT, HELP, S16, DR>;
+template <int CELL, int KT, int U, int NT, bool HELP, int ES, bool DR>
+__global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP, ES, DR>::TH, LaneBwdGeom<CELL, KT, U, NT, HELP, ES, DR>::MINB) lane_bwd_kernel(const __grid_constant__ LoopParams p) {
+  using G = LaneBwdGeom<CELL, KT, U, NT, HELP, ES, DR>;
   using C = Cell<CELL>;
   // packed arithmetic where it measured faster (LSTM D = 64, one CTA per head: B1024 N16, 11551 -> 9881 clk per step of all CTAs)
   using F2 = typename PairOf<CELL == CELL_LSTM && !G::CL>::type;
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP, S16, DR>::T
   const int n = blockIdx.z, bt0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
   const size_t ND = (size_t)N * D;
-  const int f32 = S16 ? 0 : p.state_f32;
+  const int f32 = ES ? ES == 4 : p.state_f32;
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const uint32_t sm = smem_u32(smem_raw), recv = sm + G::OFF_R;
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP, S16, DR>::T
       bar_sync<32 * W + 32>(3);  // dR has left tensor memory
       tc_fence_after();
       tmem_dealloc(tmem, G::DRC);
-    } else if (!S16 && f32) {
+    } else if (ES == 4 || (ES == 0 && f32)) {
       lane_bwd_io<CELL, G, 4>(p, sm, sm + G::OFF_I, io, crank);
     } else {
       lane_bwd_io<CELL, G, 2>(p, sm, sm + G::OFF_I, io, crank);

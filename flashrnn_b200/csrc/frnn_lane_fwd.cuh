@@ -24,11 +24,12 @@
 
 namespace FRNN_NS {
 
-template <int CELL, int KT, int U, int NT, bool S16_>
+template <int CELL, int KT, int U, int NT, int ES_>
 struct LaneFwdGeom {
   using C = Cell<CELL>;
   static constexpr int D = KT * 16, CS = D / U, BT = 8 * NT;
-  static constexpr bool QUAD = C::Gr > 1, CL = CS > 1, S16 = S16_;  // S16: 16-bit states only
+  static constexpr bool QUAD = C::Gr > 1, CL = CS > 1;
+  static constexpr int ES = ES_;  // bytes of a state element, 0: known at run time only
   static constexpr int MT = QUAD ? 2 : 1;
   static constexpr int UW = QUAD ? 4 * MT : 16 * MT;  // units per warp
   static constexpr int W = U / UW;                    // compute warps
@@ -42,7 +43,7 @@ struct LaneFwdGeom {
   // shared memory: 2 h tiles | Wx ring [kLaneStages][gates][BT] | results, 2 x { states [S][BT] | activations [BT] | fifth ones [BT] } | barriers
   static constexpr int XSH = C::Gw == 3 ? 1 : 0, XPL = C::Gw + XSH;  // GRU: plane 0 of the Wx tile stands for its recurrent-only gate, zero
   static constexpr int XP = io_pitch(U * 2), XS = XPL * BT * XP;
-  static constexpr int SP = io_pitch(U * (S16 ? 2 : 4)), CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2);
+  static constexpr int SP = io_pitch(U * (ES ? ES : 4)), CP = io_pitch(U * 2 * GCM), EP = io_pitch(U * 2);
   static constexpr int OUT_C = C::S * BT * SP, OUT_E = OUT_C + (GCM ? BT * CP : 0), OUT_B = OUT_E + (GCX ? BT * EP : 0);
   static constexpr int OFF_X = 2 * HB, OFF_O = OFF_X + kLaneStages * XS, OFF_BAR = OFF_O + 2 * OUT_B;
   static constexpr size_t smem = OFF_BAR + 2 * 8;
@@ -213,7 +214,7 @@ struct FwdLane {
   // ul: first unit within the CTA, unit: within the head; ht: bytes of an 8-row h tile
   __device__ __forceinline__ void init(const LoopParams& p, uint32_t x0, uint32_t o0, int ht, int lane, int ul, int unit, int n, int bt0_) {
     const size_t ND = (size_t)p.N * p.D;
-    a = (lane >> 2) & 1; tig = lane & 3; bt0 = bt0_; f32 = G::S16 ? 0 : p.state_f32;
+    a = (lane >> 2) & 1; tig = lane & 3; bt0 = bt0_; f32 = G::ES ? G::ES == 4 : p.state_f32;
     nd = (size_t)n * p.D + unit;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
@@ -336,9 +337,9 @@ struct FwdLane {
   }
 };
 
-template <int CELL, int KT, int U, int NT, bool S16>
-__global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT, S16>::TH, LaneFwdGeom<CELL, KT, U, NT, S16>::MINB) lane_fwd_kernel(const __grid_constant__ LoopParams p) {
-  using G = LaneFwdGeom<CELL, KT, U, NT, S16>;
+template <int CELL, int KT, int U, int NT, int ES>
+__global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT, ES>::TH, LaneFwdGeom<CELL, KT, U, NT, ES>::MINB) lane_fwd_kernel(const __grid_constant__ LoopParams p) {
+  using G = LaneFwdGeom<CELL, KT, U, NT, ES>;
   using C = Cell<CELL>;
   // packed arithmetic where it measured faster (LSTM D = 128 step 1023 -> 975 clk; D = 64, one CTA, 847 -> 890)
   using F2 = typename PairOf<CELL == CELL_LSTM && G::CL>::type;
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT, S16>::TH, LaneFwd
   const int T = p.T, N = p.N, B = p.B;
   const int n = blockIdx.z, bt0 = blockIdx.y * G::BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
-  const int f32 = S16 ? 0 : p.state_f32;
+  const int f32 = ES ? ES == 4 : p.state_f32;
   const size_t ND = (size_t)N * D;
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(LaneFwdGeom<CELL, KT, U, NT, S16>::TH, LaneFwd
 
   if (warp >= G::W) {
     const int io = tid - 32 * G::W;
-    if (!S16 && f32) lane_fwd_io<CELL, G, 4>(p, sm + G::OFF_X, sm + G::OFF_O, full, io, crank);
+    if (ES == 4 || (ES == 0 && f32)) lane_fwd_io<CELL, G, 4>(p, sm + G::OFF_X, sm + G::OFF_O, full, io, crank);
     else lane_fwd_io<CELL, G, 2>(p, sm + G::OFF_X, sm + G::OFF_O, full, io, crank);
     if (CL) {
       __syncwarp();

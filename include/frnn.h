@@ -184,7 +184,7 @@ typedef struct frnn_loop_shape {
   int32_t cluster_size;      /* CTAs that share one (head, batch tile)                                 */
   int32_t units_per_cta;
   int32_t batch_rows;        /* batch rows per CTA                                                     */
-  int32_t threads;           /* per CTA                                                                */
+  int32_t threads;           /* per CTA, of the loop itself: a warp that forms dR beside it comes on top */
   int32_t input_stages;      /* time steps of inputs in flight in shared memory (0: none kept there)   */
   uint32_t grid[3];          /* CTAs                                                                   */
 } frnn_loop_shape;
