@@ -275,7 +275,7 @@ wide_fwd_elman_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
     const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
     int hw = 0;  // tile that receives h_t
     for (int t = 0; t < T; ++t) {
-      if (!mbar_wait_warp(&acc_full[t & 1], (uint32_t)((t >> 1) & 1))) { report_timeout(p.status, t); break; }
+      if (!mbar_wait_bounded(&acc_full[t & 1], (uint32_t)((t >> 1) & 1))) { report_timeout(p.status, t); break; }
       tc_fence_after();
       uint32_t r0[32], r1[32];
       tmem_ld64(trow + (t & 1) * WD, r0, r1);
@@ -529,7 +529,7 @@ wide_fwd_gates_kernel(const __grid_constant__ CUtensorMap tm_wx, const __grid_co
     elem_t* c_e = p.states + (((size_t)B + (ok_e ? be : 0)) * T) * ND + (size_t)n * WD + 32 * half + (odd ? 16 : 0);
     elem_t* c_o = c_e + (size_t)T * ND;
     for (int t = 0; t < T; ++t) {
-      if (!mbar_wait_warp(&acc_full[t & 1], (uint32_t)((t >> 1) & 1))) { report_timeout(p.status, t); break; }
+      if (!mbar_wait_bounded(&acc_full[t & 1], (uint32_t)((t >> 1) & 1))) { report_timeout(p.status, t); break; }
       tc_fence_after();
       unsigned char* hdst = sm + WL_OFF_H + (uint32_t)(t & 1) * WTILE;
       const uint32_t acc = trow + (uint32_t)(t & 1) * (WL_G * WD);
@@ -920,9 +920,9 @@ wide_bwd_elman_kernel(const __grid_constant__ CUtensorMap tm_states, const __gri
     int dw = 0;  // tile that receives delta of step index j
     for (int j = 0; j < T; ++j) {
       const int tt = T - 1 - j, hr = ((T + 1) >> 1) - 1 - (tt >> 1);  // time of the step; PAIR: its h box
-      if (!mbar_wait_warp(&acc_full[j & 1], (uint32_t)((j >> 1) & 1)) ||
-          !(PAIR ? mbar_wait_warp(&h_full[hr & 1], (uint32_t)((hr >> 1) & 1))
-                  : mbar_wait_warp(&h_full[j % WB_STAGES], (uint32_t)((j / WB_STAGES) & 1)))) {
+      if (!mbar_wait_bounded(&acc_full[j & 1], (uint32_t)((j >> 1) & 1)) ||
+          !(PAIR ? mbar_wait_bounded(&h_full[hr & 1], (uint32_t)((hr >> 1) & 1))
+                  : mbar_wait_bounded(&h_full[j % WB_STAGES], (uint32_t)((j / WB_STAGES) & 1)))) {
         report_timeout(p.status, j);
         ok = false;
         break;
