@@ -771,11 +771,8 @@ __global__ void __launch_bounds__(XTHREADS) x32_dr_kernel(const XDrParams p) {
     const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
     if (m >= GD) continue;
     const int g = m / D, d = m - g * D;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int pc = p0 + tx * 4 + j;
-      if (pc < D) atomicAdd(p.dR + (((size_t)g * N + n) * D + d) * D + pc, acc[i][j]);
-    }
+    const int pc = p0 + tx * 4;  // (head dims are multiples of 4)
+    if (pc < D) red_add_f32x4(p.dR + (((size_t)g * N + n) * D + d) * D + pc, acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
   }
 }
 
@@ -1210,7 +1207,9 @@ __attribute__((visibility("hidden"))) int frnn_backward_parts_f32(const frnn_pla
     const int mt = (d.Gr * pr.D + DR_M - 1) / DR_M, pt = (pr.D + DR_P - 1) / DR_P;
     long long splits = 592 / ((long long)mt * pt * pr.N);  // about four CTAs per SM
     if (splits < 1) splits = 1;
-    if (splits > (q.K + 127) / 128) splits = (q.K + 127) / 128;
+    // at least 32 rows each: on few rows a CTA's chain of loads is what takes the time, not the sums it adds (backward pass, us, with 128, 64, 32: LSTM B4 T256 N2 D64 100.7, 95.8, 93.8, B8
+    // T128 N4 D32 49.5, 44.6, 42.5, Elman B3 T300 N2 D128 198.7, 193.9, 191.8, GRU B16 T100 N8 D20 42.4, 42.3, 43.3; with four scalar atomics for one of four words 1 to 2 us more)
+    if (splits > (q.K + 31) / 32) splits = (q.K + 31) / 32;
     if ((long long)pr.N * splits > 65535) splits = 65535 / pr.N;
     q.rows_per_split = (int)(((q.K + splits - 1) / splits + DR_K - 1) / DR_K * DR_K);
     splits = (q.K + q.rows_per_split - 1) / q.rows_per_split;
