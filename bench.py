@@ -475,7 +475,7 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
                     "more CTAs than SMs: issue slots of the cells and memory bound this workload" if min(s.grid[0] * s.grid[1] * s.grid[2] for s in loops.values()) > 148 else
                     "the serial chain of 2T dependent steps (chain_floor), not HBM or the tensor pipe, bounds this workload"},
         # loops, dR and cast; in front: fragments of R^T (16-bit), of R (head dims above 256), R^T (float32 but for the lane loop)
-        "clocks": clk.summary(), "launches_per_step": 3 if wide else 4 + (nv.LOOPS[loops["forward"].loop] != "f32_lane") if job.f32io else 6 if D > 256 else 5,
+        "clocks": clk.summary(), "launches_per_step": 3 if wide else 4 + (nv.LOOPS[loops["forward"].loop] != "f32_lane") if job.f32io else 6 if D > 256 else 5 - (dr_ms < 0.003),  # (no kernel between those events where the loop forms dR)
     }
     if keep is not None:
         keep.update(Wx=Wx, R=R, b=b, s0=s0, gcnt=gcnt)
