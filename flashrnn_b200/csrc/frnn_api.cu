@@ -21,36 +21,29 @@ static bool cell_dims(int cell, CellDims* d) {
   return false;
 }
 
-// The lane loops (head dims up to 256) and those for larger head dims of a kernel family (kernel_cell) and direction.  es: bytes of a
-// state element, 0: known at run time only; the others are null where there is none (states_form)
-static LaneKernel lane_kernel(int cell, bool bwd, int kt, int u, int nt, int es) {
-  switch (cell) {
-    case CELL_LSTM: return bwd ? lane_bwd_lstm(kt, u, nt, es) : lane_fwd_lstm(kt, u, nt, es);
-    case CELL_GRU: return bwd ? lane_bwd_gru(kt, u, nt, es) : lane_fwd_gru(kt, u, nt, es);
-    case CELL_ELMAN: return bwd ? lane_bwd_elman(kt, u, nt, es) : lane_fwd_elman(kt, u, nt, es);
-    case CELL_ELMAN_CLIP: return bwd ? lane_bwd_elmanc(kt, u, nt, es) : lane_fwd_elmanc(kt, u, nt, es);
-    case CELL_SLSTM: return bwd ? lane_bwd_slstm(kt, u, nt, es) : lane_fwd_slstm(kt, u, nt, es);
-  }
-  return LaneKernel{nullptr, 0, 0};
+// The lane loops (head dims up to 256) of a kernel family (kernel_cell), direction and tile, null: none; those with warps that only multiply, null: none
+constexpr LaneTiles kLaneTileAt;
+static const LaneForms* lane_forms(int cell, bool bwd, int kt, int u, int nt) {
+  static const LaneForms (*const tables[5][2])[2] = {{lane_fwd_lstm, lane_bwd_lstm}, {lane_fwd_gru, lane_bwd_gru}, {lane_fwd_elman, lane_bwd_elman},
+                                                     {lane_fwd_slstm, lane_bwd_slstm}, {lane_fwd_elmanc, lane_bwd_elmanc}};  // by CELL_*
+  const int at = u % 16 == 0 && u <= 128 ? kLaneTileAt.at[kt][u / 16] : -1;
+  return at < 0 ? nullptr : &tables[cell][bwd][at][nt - 1];
 }
-static LaneKernel lane_help_kernel(int cell, int kt, int es) {
-  switch (cell) {
-    case CELL_LSTM: return lane_bwd_help_lstm(kt, es);
-    case CELL_GRU: return lane_bwd_help_gru(kt, es);
-    case CELL_ELMAN: return lane_bwd_help_elman(kt, es);
-    case CELL_ELMAN_CLIP: return lane_bwd_help_elmanc(kt, es);
-    case CELL_SLSTM: return lane_bwd_help_slstm(kt, es);
-  }
-  return LaneKernel{nullptr, 0, 0};
+static const LaneForms* lane_help_forms(int cell, int kt) {
+  static const LaneForms* const tables[5] = {lane_bwd_help_lstm, lane_bwd_help_gru, lane_bwd_help_elman, lane_bwd_help_slstm, lane_bwd_help_elmanc};
+  for (int i = 0; i < 4; ++i)
+    if (kHelpKTs[i] == kt) return &tables[cell][i];
+  return nullptr;
 }
 static LaneKernel lane_dr_kernel(int cell) {
   switch (cell) {
-    case CELL_LSTM: return lane_bwd_dr_lstm();
-    case CELL_GRU: return lane_bwd_dr_gru();
-    case CELL_SLSTM: return lane_bwd_dr_slstm();
+    case CELL_LSTM: return lane_bwd_dr_lstm;
+    case CELL_GRU: return lane_bwd_dr_gru;
+    case CELL_SLSTM: return lane_bwd_dr_slstm;
   }
   return LaneKernel{nullptr, 0, 0};
 }
+// The head dims above 256
 static BigKernel big_kernel(int cell, bool bwd, int u, int nt, bool dense) {
   switch (cell) {
     case CELL_LSTM: return bwd ? big_bwd_lstm(u, nt) : big_fwd_lstm(u, nt, dense);
@@ -222,12 +215,15 @@ static bool lane_dr(const frnn_plan& pl, int nt) {
 
 // The lane loop of a plan's tile: with the type of its states fixed where there is such a form and it pays, else the general one.
 static LaneKernel lane_loop(const frnn_problem& pr, bool bwd, int u, int nt, bool help) {
-  const int cell = kernel_cell(pr), kt = pr.D / 16, es = pr.dtype_state == FRNN_DTYPE_F32 ? 4 : 2;
-  auto get = [&](int s) { return help ? lane_help_kernel(cell, kt, s) : lane_kernel(cell, bwd, kt, u, nt, s); };
-  const LaneKernel form = get(es), general = get(0);
-  if (!form.fn || !general.fn) return form.fn ? form : general;
-  const bool few = (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N * (pr.D / u) <= 2LL * sm_count_cached();
-  return few || !states_form_for_few(cell, bwd, kt, es) ? form : general;
+  const int cell = kernel_cell(pr), kt = pr.D / 16, f32 = pr.dtype_state == FRNN_DTYPE_F32;
+  const LaneForms* f = help ? lane_help_forms(cell, kt) : lane_forms(cell, bwd, kt, u, nt);
+  if (!f) return LaneKernel{nullptr, 0, 0};
+  if (f->few[f32].fn == f->many[f32].fn) return f->few[f32];
+  return (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N * (pr.D / u) <= 2LL * sm_count_cached() ? f->few[f32] : f->many[f32];
+}
+static bool lane_exists(const frnn_problem& pr, bool bwd, int u, int nt) {
+  const LaneForms* f = lane_forms(kernel_cell(pr), bwd, pr.D / 16, u, nt);
+  return f && f->few[pr.dtype_state == FRNN_DTYPE_F32].fn;
 }
 
 static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) {
@@ -246,7 +242,7 @@ static bool tile_ok(const frnn_problem& pr, const CellDims& cd, int cs, int bt) 
   if (threads > (D < 192 ? 512 : D < 256 ? 384 : 256)) return false;
   if (bt == 32 && cd.Gr * U > 192) return false;
   for (int nt = 1; nt <= (bt < 16 ? 1 : 2); ++nt)
-    if (!lane_loop(pr, false, U, nt, false).fn || !lane_loop(pr, true, U, nt, false).fn) return false;
+    if (!lane_exists(pr, false, U, nt) || !lane_exists(pr, true, U, nt)) return false;
   return true;
 }
 
@@ -345,7 +341,7 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
   else if (dr) k = lane_dr_kernel(cell);
   else if (bwd && lane_help(pr, pl.cluster_size, u, nt)) k = lane_loop(pr, true, u, nt, true);
   if (!k.fn && !pl.probe_noop_cell) k = lane_loop(pr, bwd, u, nt, false);
-  return LoopLaunch{k.fn, k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt, dr};
+  return LoopLaunch{reinterpret_cast<const void*>(k.fn), k.threads, kLaneStages, k.smem, pl.cluster_size, u, 8 * nt, dr};
 }
 // x: the CTAs of a cluster, y: tiles of the batch, z: heads
 static int loop_tiles(const LoopLaunch& k, const frnn_problem& pr) { return (pr.B + k.rows - 1) / k.rows; }

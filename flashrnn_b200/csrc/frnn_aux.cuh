@@ -13,10 +13,30 @@ constexpr int kNumKT = 7;
 constexpr int kKTs[kNumKT] = {1, 2, 4, 6, 8, 12, 16};
 
 struct LaneKernel {
-  const void* fn;  // kernel entry; null: no such instantiation
+  void (*fn)(LoopParams);  // kernel entry; null: no such instantiation
   int threads;
   size_t smem;
 };
+// The lane loop of a tile for 16-bit ([0]) and fp32 ([1]) states: where few CTAs run, and where they queue up (states_form_for_few).  Tables that the compiler
+// fills: every launch looks its loops up, the validation of its plan those of both directions.  Host time of frnn_query_loop, ns (the checks and the lookups of a launch), GRU B1 N12 D64 /
+// LSTM B16 N4 D256: 61 / 94 with one `if` per tile and form, 26 / 26 so.
+struct LaneForms { LaneKernel few[2], many[2]; };
+#define FRNN_COUNT(KT, U) +1
+constexpr int kLaneTiles = FRNN_FOREACH_KT_U(FRNN_COUNT) FRNN_FOREACH_KT_U_FEW_GATES(FRNN_COUNT) FRNN_FOREACH_KT_U_ONE_GATE(FRNN_COUNT);
+#undef FRNN_COUNT
+// place of (head dim / 16, units per CTA) in those tables, -1: none
+struct LaneTiles {
+  signed char at[17][9];
+  constexpr LaneTiles() : at() {
+    for (int k = 0; k < 17; ++k)
+      for (int u = 0; u < 9; ++u) at[k][u] = -1;
+    signed char i = 0;
+#define FRNN_PLACE(KT, U) at[KT][U / 16] = i++;
+    FRNN_FOREACH_KT_U(FRNN_PLACE) FRNN_FOREACH_KT_U_FEW_GATES(FRNN_PLACE) FRNN_FOREACH_KT_U_ONE_GATE(FRNN_PLACE)
+#undef FRNN_PLACE
+  }
+};
+constexpr int kHelpKTs[4] = {6, 8, 12, 16};  // head dims / 16 of the reverse loops with warps that only multiply
 struct BigKernel {
   const void* fn;
   int threads;
@@ -25,10 +45,10 @@ struct BigKernel {
 
 // defined once per (cell, direction) in frnn_inst_*.cu
 #define FRNN_DECLARE(cell)                              \
-  LaneKernel lane_fwd_##cell(int kt, int u, int nt, int es);  \
-  LaneKernel lane_bwd_##cell(int kt, int u, int nt, int es);  \
-  LaneKernel lane_bwd_help_##cell(int kt, int es);      \
-  LaneKernel lane_bwd_dr_##cell();                      \
+  extern const LaneForms lane_fwd_##cell[kLaneTiles][2];  /* [tile][rows / 8 - 1] */ \
+  extern const LaneForms lane_bwd_##cell[kLaneTiles][2];                             \
+  extern const LaneForms lane_bwd_help_##cell[4];                                    \
+  extern const LaneKernel lane_bwd_dr_##cell;                                        \
   BigKernel big_fwd_##cell(int u, int nt, bool dense);  \
   BigKernel big_bwd_##cell(int u, int nt);              \
   cudaError_t big_pack_##cell(const void* R, void* out, int N, int D, cudaStream_t stream);

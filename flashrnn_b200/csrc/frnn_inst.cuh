@@ -15,55 +15,51 @@ namespace FRNN_NS {
 #endif
 
 // ES: bytes of a state element, 0: known at run time only; which exist: states_form, states_general.  Null for the others.
-template <int KT, int U, int NT, int ES, bool V = FRNN_GEOM(KT, U, NT, ES)::valid && (ES ? states_form(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false, ES) : states_general(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false))>
-struct LaneEntry {
-  static LaneKernel get() { return LaneKernel{nullptr, 0, 0}; }
-};
 template <int KT, int U, int NT, int ES>
-struct LaneEntry<KT, U, NT, ES, true> {
-  static LaneKernel get() {
-    using G = FRNN_GEOM(KT, U, NT, ES);
-    return LaneKernel{reinterpret_cast<const void*>(&FRNN_KERNEL(KT, U, NT, ES)), G::TH, G::smem};
-  }
-};
-
-#if FRNN_INST_BWD
-template <int KT, int U, bool HELP, int ES, bool DR,
-          bool V = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, ES, DR>::valid && (DR || (ES ? states_form(FRNN_INST_CELL, true, KT, U, 1, HELP, ES) : states_general(FRNN_INST_CELL, true, KT, U, 1, HELP)))>
-struct BwdEntry {
-  static LaneKernel get() { return LaneKernel{nullptr, 0, 0}; }
-};
-template <int KT, int U, bool HELP, int ES, bool DR>
-struct BwdEntry<KT, U, HELP, ES, DR, true> {
-  static LaneKernel get() {
-    using G = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, ES, DR>;
-    return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<FRNN_INST_CELL, KT, U, 1, HELP, ES, DR>), G::TH, G::smem};
-  }
-};
-// the reverse loops with warps that only multiply (clusters of 32-unit CTAs, 8 rows), null where there is none
-template <int ES>
-static LaneKernel help_entry(int kt) {
-  return kt == 6 ? BwdEntry<6, 32, true, ES, false>::get() : kt == 8 ? BwdEntry<8, 32, true, ES, false>::get() : kt == 12 ? BwdEntry<12, 32, true, ES, false>::get()
-       : kt == 16 ? BwdEntry<16, 32, true, ES, false>::get() : LaneKernel{nullptr, 0, 0};
-}
-LaneKernel FRNN_INST_HELP(int kt, int es) { return es == 2 ? help_entry<2>(kt) : es == 4 ? help_entry<4>(kt) : help_entry<0>(kt); }
-// the reverse loop with a warp that forms dR (head dim 64, one CTA per head)
-LaneKernel FRNN_INST_DR() { return BwdEntry<4, 64, false, 2, true>::get(); }
-#endif
-
-template <int ES>
-static LaneKernel lane_entry(int kt, int u, int nt) {
-#define FRNN_CASE(KT, U)                                         \
-  if (kt == KT && u == U && nt == 1) return LaneEntry<KT, U, 1, ES>::get(); \
-  if (kt == KT && u == U && nt == 2) return LaneEntry<KT, U, 2, ES>::get();
-  FRNN_FOREACH_KT_U(FRNN_CASE)
-  // wide CTAs: the one- and three-gate cells only (the others would need more than 512 threads or registers than there are)
-  if constexpr (Cell<FRNN_INST_CELL>::Gr < 4) { FRNN_FOREACH_KT_U_FEW_GATES(FRNN_CASE) }
-  if constexpr (Cell<FRNN_INST_CELL>::Gr == 1) { FRNN_FOREACH_KT_U_ONE_GATE(FRNN_CASE) }
-#undef FRNN_CASE
+constexpr LaneKernel lane_entry() {
+  using G = FRNN_GEOM(KT, U, NT, ES);
+  if constexpr (G::valid && (ES ? states_form(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false, ES) : states_general(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false)))
+    return LaneKernel{&FRNN_KERNEL(KT, U, NT, ES), G::TH, G::smem};
   return LaneKernel{nullptr, 0, 0};
 }
-LaneKernel FRNN_INST_LANE(int kt, int u, int nt, int es) { return es == 2 ? lane_entry<2>(kt, u, nt) : es == 4 ? lane_entry<4>(kt, u, nt) : lane_entry<0>(kt, u, nt); }
+// the typed form where there is one, else the general one; where CTAs queue up, the general one of the forms that are for few
+constexpr LaneForms lane_forms(int cell, bool bwd, int kt, LaneKernel general, LaneKernel h, LaneKernel f) {
+  LaneForms r = {{h.fn ? h : general, f.fn ? f : general}, {}};
+  r.many[0] = general.fn && states_form_for_few(cell, bwd, kt, 2) ? general : r.few[0];
+  r.many[1] = general.fn && states_form_for_few(cell, bwd, kt, 4) ? general : r.few[1];
+  return r;
+}
+template <int KT, int U, int NT, bool ON>
+constexpr LaneForms tile_forms() {
+  if constexpr (ON) return lane_forms(FRNN_INST_CELL, FRNN_INST_BWD, KT, lane_entry<KT, U, NT, 0>(), lane_entry<KT, U, NT, 2>(), lane_entry<KT, U, NT, 4>());
+  return LaneForms{};
+}
+#define FRNN_ROW(KT, U) {tile_forms<KT, U, 1, true>(), tile_forms<KT, U, 2, true>()},
+// wide CTAs: the one- and three-gate cells only (the others would need more than 512 threads or registers than there are)
+#define FRNN_ROW_FEW(KT, U) {tile_forms<KT, U, 1, (Cell<FRNN_INST_CELL>::Gr < 4)>(), tile_forms<KT, U, 2, (Cell<FRNN_INST_CELL>::Gr < 4)>()},
+#define FRNN_ROW_ONE(KT, U) {tile_forms<KT, U, 1, (Cell<FRNN_INST_CELL>::Gr == 1)>(), tile_forms<KT, U, 2, (Cell<FRNN_INST_CELL>::Gr == 1)>()},
+constexpr LaneForms FRNN_INST_LANE[kLaneTiles][2] = {FRNN_FOREACH_KT_U(FRNN_ROW) FRNN_FOREACH_KT_U_FEW_GATES(FRNN_ROW_FEW) FRNN_FOREACH_KT_U_ONE_GATE(FRNN_ROW_ONE)};
+#undef FRNN_ROW
+#undef FRNN_ROW_FEW
+#undef FRNN_ROW_ONE
+
+#if FRNN_INST_BWD
+template <int KT, int U, bool HELP, int ES, bool DR>
+constexpr LaneKernel bwd_entry() {
+  using G = LaneBwdGeom<FRNN_INST_CELL, KT, U, 1, HELP, ES, DR>;
+  if constexpr (G::valid && (DR || (ES ? states_form(FRNN_INST_CELL, true, KT, U, 1, HELP, ES) : states_general(FRNN_INST_CELL, true, KT, U, 1, HELP))))
+    return LaneKernel{&lane_bwd_kernel<FRNN_INST_CELL, KT, U, 1, HELP, ES, DR>, G::TH, G::smem};
+  return LaneKernel{nullptr, 0, 0};
+}
+// the reverse loops with warps that only multiply (clusters of 32-unit CTAs, 8 rows)
+template <int KT>
+constexpr LaneForms help_forms() {
+  return lane_forms(FRNN_INST_CELL, true, KT, bwd_entry<KT, 32, true, 0, false>(), bwd_entry<KT, 32, true, 2, false>(), bwd_entry<KT, 32, true, 4, false>());
+}
+constexpr LaneForms FRNN_INST_HELP[4] = {help_forms<kHelpKTs[0]>(), help_forms<kHelpKTs[1]>(), help_forms<kHelpKTs[2]>(), help_forms<kHelpKTs[3]>()};
+// the reverse loop with a warp that forms dR (head dim 64, one CTA per head)
+constexpr LaneKernel FRNN_INST_DR = bwd_entry<4, 64, false, 2, true>();
+#endif
 
 // ---- head dims above 256: units per CTA, batch tile / 8
 #if FRNN_INST_BWD

@@ -10,12 +10,12 @@ namespace FRNN_NS {
 template <int CELL, int KT, int U>
 static LaneKernel floor_fwd() {
   using G = LaneFwdGeom<CELL | kNoopCell, KT, U, 1, 0>;
-  return LaneKernel{reinterpret_cast<const void*>(&lane_fwd_kernel<CELL | kNoopCell, KT, U, 1, 0>), G::TH, G::smem};
+  return LaneKernel{&lane_fwd_kernel<CELL | kNoopCell, KT, U, 1, 0>, G::TH, G::smem};
 }
 template <int CELL, int KT, int U>
 static LaneKernel floor_bwd() {
   using G = LaneBwdGeom<CELL | kNoopCell, KT, U, 1, true, 0, false>;
-  return LaneKernel{reinterpret_cast<const void*>(&lane_bwd_kernel<CELL | kNoopCell, KT, U, 1, true, 0, false>), G::TH, G::smem};
+  return LaneKernel{&lane_bwd_kernel<CELL | kNoopCell, KT, U, 1, true, 0, false>, G::TH, G::smem};
 }
 
 // lstm head dim 256, gru head dim 128, slstm head dim 192: 32 units per CTA, 8-row batch tiles

@@ -374,3 +374,48 @@ def test_plans_report_the_loops_they_run():
                  mk("gru", 1024, 8, 16, 64, False, False), mk("gru", 1024, 8, 16, 64, False, True)):
         plan = _native.query(prob)
         assert plan.wx_stages == _native.query_loop(plan, False).input_stages
+
+
+def test_looking_a_loop_up_costs_little_beside_the_checks(tmp_path):
+    """A decoding step is bound by the host, and every launch validates its plan and looks its time loop up.  Both together take 3 to 4.7 times as long as a call that the
+    first checks refuse (tables; 6.5 to 8.3 with one branch per tile and form).  Smallest of many repeats, so that other load on the machine does not count."""
+    import subprocess
+
+    (tmp_path / "lookup.c").write_text(r'''
+#include <dlfcn.h>
+#include <stdio.h>
+#include <time.h>
+#include "frnn.h"
+static double now(void) { struct timespec t; clock_gettime(CLOCK_MONOTONIC, &t); return t.tv_sec * 1e9 + t.tv_nsec; }
+int main(int argc, char** argv) {
+  void* lib = dlopen(argv[1], RTLD_NOW);
+  if (argc != 2 || !lib) return 1;
+  int (*query)(const frnn_problem*, frnn_plan*) = (int (*)(const frnn_problem*, frnn_plan*))dlsym(lib, "frnn_query");
+  int (*loop)(const frnn_plan*, int, frnn_loop_shape*) = (int (*)(const frnn_plan*, int, frnn_loop_shape*))dlsym(lib, "frnn_query_loop");
+  static const int sizes[][4] = {{FRNN_CELL_GRU, 1, 12, 64}, {FRNN_CELL_LSTM, 16, 4, 256}, {FRNN_CELL_LSTM, 16, 4, 64}, {FRNN_CELL_ELMAN, 16, 4, 64}};
+  for (int i = 0; i < 4; ++i) {
+    frnn_problem p = {sizes[i][0], sizes[i][1], 1, sizes[i][2], sizes[i][3], FRNN_DTYPE_BF16, FRNN_DTYPE_BF16, 0, 0.f, 0.f, 0};
+    frnn_plan good, bad;
+    frnn_loop_shape s;
+    if (query(&p, &good)) return 2;
+    bad = good;
+    bad.cluster_size = 17;
+    double tg = 1e12, tb = 1e12;
+    for (int r = 0; r < 200; ++r) {
+      const double t0 = now();
+      for (int k = 0; k < 2000; ++k) if (loop(&good, 0, &s)) return 3;
+      const double t1 = now();
+      for (int k = 0; k < 2000; ++k) if (!loop(&bad, 0, &s)) return 4;
+      const double t2 = now();
+      if (t1 - t0 < tg) tg = t1 - t0;
+      if (t2 - t1 < tb) tb = t2 - t1;
+    }
+    printf("%f\n", tg / tb);
+  }
+  return 0;
+}''')
+    exe = tmp_path / "lookup"
+    subprocess.run(["gcc", "-O2", "-I", str(ROOT / "include"), str(tmp_path / "lookup.c"), "-o", str(exe), "-ldl"], check=True)
+    out = subprocess.run([str(exe), str(_native.LIB_PATH)], check=True, capture_output=True, text=True).stdout
+    ratios = [float(x) for x in out.split()]
+    assert len(ratios) == 4 and max(ratios) < 5.5, ratios
