@@ -203,14 +203,18 @@ static bool lane_help(const frnn_problem& pr, int cs, int u, int nt) {
 }
 
 // Whether the reverse lane loop forms dR as well (lane_bwd_dr): head dim 64 with one CTA per head, 8 rows and 16-bit states.  Not for the shortest
-// sequences: a CTA adds its 48 or 64 KB of sums to the gradient once.  Backward pass, us, dR in its own kernel / in the loop, B1024 N16: LSTM T16 162 / 172, T20 192 /
-// 190, T24 218 / 209, T32 264 / 247, GRU T24 205 / 191, sLSTM T24 268 / 249.  The sLSTM's loop gets 23 to 27 us per 512 steps longer, which only pays once its own
-// kernel takes that: T512 B8 N2 239 / 253, B16 N12 261 / 259, B48 N16 302 / 261; LSTM 235 / 234, 255 / 239, 296 / 239; GRU 229 / 181, 243 / 182, 288 / 183.
-constexpr int kDrMinSteps = 24, kDrMinTilesSlstm = 24;
+// sequences: a CTA adds its 48 or 64 KB of sums to the gradient once.  Backward pass, us, dR in its own kernel / in the loop, B1024 N16: LSTM T16 162 / 172, T20 192 / 190, T24 229 /
+// 222, T32 281 / 262, GRU T24 212 / 179, sLSTM T24 260 / 241.  A step of the LSTM's and the sLSTM's loop takes 20 to 60 ns longer with it, which on long sequences
+// only pays once their own kernel takes that.  LSTM, tiles: T256 2 132 / 134, 8 136 / 133, 24 144 / 134, T512 2 240 / 246, 8 245 / 247, 16 251 / 253, 24 261 / 251, T2048 16 918 /
+// 943, 24 959 / 949, 32 980 / 951.  sLSTM: T64 24 58 / 51, T256 8 138 / 144, 24 150 / 146, T512 24 267 / 273, 48 284 / 275, T2048 24 986 / 1036, 48 1043 / 1043, 64 1070 /
+// 1043.  GRU, any: T512 1 232 / 193, 24 249 / 196, T2048 24 917 / 727.
+constexpr int kDrMinSteps = 24, kDrShort = 256;
 static bool lane_dr(const frnn_plan& pl, int nt) {
   const frnn_problem& pr = pl.prob;
   if (pr.D != 64 || pl.cluster_size != 1 || nt != 1 || pr.cell == CELL_ELMAN || pr.dtype_state == FRNN_DTYPE_F32 || pl.forced_tile) return false;
-  return pr.T >= kDrMinSteps && (pr.cell != CELL_SLSTM || (long long)((pr.B + 7) / 8) * pr.N >= kDrMinTilesSlstm);
+  const long long tiles = (long long)((pr.B + 7) / 8) * pr.N;
+  const int enough = pr.cell == CELL_GRU ? 0 : pr.cell == CELL_LSTM ? (pr.T <= kDrShort ? 0 : 24) : pr.T <= kDrShort ? 24 : 48;
+  return pr.T >= kDrMinSteps && tiles >= enough;
 }
 
 // The lane loop of a plan's tile: with the type of its states fixed where there is such a form and it pays, else the general one.

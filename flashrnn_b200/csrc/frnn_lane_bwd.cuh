@@ -233,7 +233,7 @@ __device__ __forceinline__ void lane_bwd_io(const LoopParams& p, uint32_t d0, ui
 // the tensor core multiply the deltas of two steps, 16 rows of (b, t), as they lie in shared memory for the loop's own products, with that h.
 // The sums stay in tensor memory for the whole sequence.  So dR takes one more tile of h per step instead of a kernel that reads dWx
 // and h again; the loop's other warps do nothing for it.  Backward pass, us, with the kernel of frnn_dr_small.cu behind the loop -> so: B1024 T256 N16 LSTM
-// 1712 -> 1257, GRU 1705 -> 1132, sLSTM 2011 -> 1556; B16 T512 N12 LSTM 256 -> 239, GRU 263 -> 201; of a step, 46 clk are the tensor core's reading of shared memory.
+// 1710 -> 1263, GRU 1626 -> 1082, sLSTM 2022 -> 1533; B48 T512 N16 302 -> 255, 292 -> 200, 310 -> 277; of a step, 46 clk are the tensor core's reading of shared memory.
 // Not for clusters: a CTA there needs h of the whole head, and its way into the SM lies across the exchange (LSTM B16 T1024 N4 D256 661 + 69 us -> 804: 98 for
 // fetching h, 46 for the products).
 template <class G>
@@ -257,10 +257,10 @@ __device__ __forceinline__ void lane_bwd_dr(const LoopParams& p, uint32_t d0, ui
     }
     cp_async_commit();
   };
-  // The deltas and h were written through the generic proxy, by other threads too; the barrier puts those writes before this thread's fence, and the
-  // fence puts them before the tensor core's reads.
+  // The deltas and h are written through the generic proxy and read by the tensor core through the async one: each thread that writes some of
+  // them fences its own writes, the cell's warps those of two steps at once, before the barrier behind which they are multiplied.  (In every step LSTM B1024
+  // T256 N16 1309 -> 1363 us, sLSTM 1572 -> 1650; behind the loop's own products, for the barrier of the next step, 1372, 1868.)
   auto issue = [&](int q, bool last) {  // steps 2 q and 2 q + 1
-    fence_proxy_async_smem();
     tc_fence_after();
     const uint32_t a0 = d0 + (2 * q & (G::NDB - 1)) * G::DB, b0 = h0 + (2 * q & (G::HSLOTS - 1)) * G::HT;
     const uint64_t bd = smem_desc(b0, G::HT, G::HP);
@@ -275,6 +275,7 @@ __device__ __forceinline__ void lane_bwd_dr(const LoopParams& p, uint32_t d0, ui
   bool dead = false;
   for (int j = 0; j < T; ++j) {
     cp_async_wait<AHEAD - 1>();  // h of step j
+    fence_proxy_async_smem();
     // step j + 1 writes its deltas over those of step j - 3, and the h of step j + AHEAD lands where that of step j - 4 is
     if (lane == 0 && (j & 1) && j >= 3 && !dead && !mbar_wait_bounded(done, (uint32_t)((j - 3) / 2 & 1))) {
       dead = true;
@@ -286,6 +287,7 @@ __device__ __forceinline__ void lane_bwd_dr(const LoopParams& p, uint32_t d0, ui
   }
   if (T & 1) {  // the last product's second step does not exist
     for (uint32_t i = lane; i < G::DB / 16; i += 32) sts128(d0 + (T & (G::NDB - 1)) * G::DB + i * 16, make_uint4(0u, 0u, 0u, 0u));
+    fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) issue(T / 2, true);
   }
@@ -599,6 +601,9 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP, ES, DR>::TH
       if constexpr (Gr == 3) sts32(dgate(nb, 3) + dbuf * DB, v_pack(dW_[2]));
 #pragma unroll
       for (int g = 0; g < Gt; ++g) dbacc[g] = v_add(dbacc[g], dB_[g]);
+    }
+    if constexpr (DR) {  // the deltas of this step and the one before, see lane_bwd_dr
+      if ((j & 1) || j == T - 1) fence_proxy_async_smem();
     }
     __syncthreads();
     // ---- partial dh_{t-1}

@@ -73,6 +73,27 @@ def test_reverse_loops_that_form_dr(cuda_device, function, N, B, T):
     _check(function, N, 64, B, T, False)
 
 
+# the same loops where every SM holds several of their CTAs: dR against the products of the very deltas and h it is formed of.  The returned dR is rounded to
+# 8 bits; its fp32 sums are chains of at most T / 2 products of 16 rows and one addition per CTA of the head, each to 2^-22 of the sum of absolute values.
+@pytest.mark.parametrize("function", ["lstm", "slstm"])
+@pytest.mark.parametrize("T", [24, 33])
+def test_loops_that_form_dr_on_a_full_gpu(cuda_device, function, T):
+    from flashrnn_b200 import flashrnn
+
+    B, N, D = 1024, 16, 64
+    g = torch.Generator(device=cuda_device).manual_seed(T)
+    randn = lambda *shape: torch.randn(*shape, generator=g, device=cuda_device, dtype=torch.bfloat16)
+    Wx, R, b = randn(B, T, 4, N, D), randn(4, N, D, D) / D ** 0.5, randn(4, N, D) / 8
+    leaves = [t.requires_grad_(True) for t in (Wx, R, b)]
+    states, _ = flashrnn(*leaves, function=function)
+    dWx, dR, _ = torch.autograd.grad(states[0], leaves, randn(B, T, N, D))
+    h = torch.cat([torch.zeros_like(states[0][:, :1]), states[0].detach()[:, :-1]], 1)
+    product = lambda x, y: torch.stack([torch.stack([x[:, :, q, n].reshape(-1, D).double().T @ y[:, :, n].reshape(-1, D).double() for n in range(N)]) for q in range(4)])
+    want, size = product(dWx, h), product(dWx.abs(), h.abs())
+    bound = 2.0 ** -8 * want.abs() + (T / 2 + 16 + B / 8) * 2.0 ** -22 * size + 2.0 ** -126
+    assert bool(((dR.double() - want).abs() <= bound).all())
+
+
 # enough clusters that Elman's forward loop takes CTAs of which two share an SM (R in registers alone, in shared memory too), and that the
 # two loops split the head differently
 @pytest.mark.parametrize("function,N,D", [("elman", 4, 512), ("elman", 3, 704), ("elman", 2, 1024), ("lstm", 5, 320), ("slstm", 5, 384)] +
