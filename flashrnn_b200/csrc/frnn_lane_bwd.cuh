@@ -382,26 +382,32 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP, ES, DR>::TH
     return j < KT ? j : j - KT;
   };
   AFrag A[MT][KP];
-#pragma unroll
-  for (int m = 0; m < MT; ++m) {
-    const int mt = tile_of(m);
-#pragma unroll
-    for (int kp = 0; kp < KP; ++kp) {
-      const uint4* src = p.Rpack + rt_frag(n, CS, (int)crank, KT, mt, KP, kp) + lane;
-      A[m][kp].lo = __ldg(src);
-      A[m][kp].hi = __ldg(src + 32);
-    }
-  }
-
   uint32_t dst[MT], dbar[MT];  // shared::cluster address of this lane's slot for tile m in the CTA that owns the tile, and of its barrier
-  if constexpr (CL) {
+  auto load_fragments = [&]() {
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
-      const int mt = tile_of(m), owner = mt * 16 / U, tl = mt - owner * (U / 16);
-      dst[m] = map_to_cta(recv + (uint32_t)((((int)crank * (U / 16) + tl) * NT * 32 + lane) * 16), (uint32_t)owner);
-      dbar[m] = map_to_cta(smem_u32(&full[0]), (uint32_t)owner);
+      const int mt = tile_of(m);
+#pragma unroll
+      for (int kp = 0; kp < KP; ++kp) {
+        const uint4* src = p.Rpack + rt_frag(n, CS, (int)crank, KT, mt, KP, kp) + lane;
+        A[m][kp].lo = __ldg(src);
+        A[m][kp].hi = __ldg(src + 32);
+      }
     }
-  }
+    if constexpr (CL) {
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const int mt = tile_of(m), owner = mt * 16 / U, tl = mt - owner * (U / 16);
+        dst[m] = map_to_cta(recv + (uint32_t)((((int)crank * (U / 16) + tl) * NT * 32 + lane) * 16), (uint32_t)owner);
+        dbar[m] = map_to_cta(smem_u32(&full[0]), (uint32_t)owner);
+      }
+    }
+  };
+  // The place decides what registers the compiler gives the loop.  Backward pass, us, in front of the rest / behind it: the general form, sLSTM D = 64 B1 T512 N1 242 / 234, LSTM D = 64 B256
+  // T512 N12 867 / 765, GRU D = 64 B8 T2048 N2 865 / 846; forms of one type of states, LSTM D = 96 B1024 T32 N8 331 / 355, GRU D = 64 fp32 B8 T512 N2 222 / 239, sLSTM D = 64
+  // with dR B1024 T32 N12 226 / 234, but LSTM D = 32 B8 T512 N2 154 / 142.
+  constexpr bool FRAGMENTS_FIRST = HELP || ES != 0;
+  if constexpr (FRAGMENTS_FIRST) load_fragments();
   const bool drop = p.test_drop && crank == 0;  // test hook: CTA 0 withholds its first message
   // HELP: partial dh_{t-1} of the deltas of step index j
   auto products = [&](int j, bool stop) {
@@ -487,6 +493,7 @@ __global__ void __launch_bounds__(LaneBwdGeom<CELL, KT, U, NT, HELP, ES, DR>::TH
     else return sm + (row_of(nb) >> 3) * DT + opnd_off(row_of(nb) & 7, g * U + ul);
   };
 
+  if constexpr (!FRAGMENTS_FIRST) load_fragments();
   // where this lane's partial sums arrive: source c at + c * (U/16) * NT * 512, batch tile nt at + nt * 512
   const uint32_t rsrc = recv + (uint32_t)((ul >> 4) * NT * 512 + (((ul & 15) >> 1) * 4 + tig) * 16 + a * 8);
   bool poisoned = false;  // a wait expired: it neither waits nor sends any more and the loop runs out
