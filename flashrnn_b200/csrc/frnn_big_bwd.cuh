@@ -45,7 +45,7 @@ struct BigBwdGeom {
     const int want = (tiles(D) + MG - 1) / MG * (KL - KT), fit = ((int)kSmemBudget - off_r(D)) / (W * MG * 1024);
     return want < fit ? want : (fit < 0 ? 0 : fit);
   }
-  static __host__ __device__ constexpr size_t smem(int D) { return (size_t)off_r(D) + (size_t)fsm(D) * W * MG * 1024; }
+  static __host__ __device__ constexpr size_t smem(int D) { return tmem_alone(TM, (size_t)off_r(D) + (size_t)fsm(D) * W * MG * 1024); }
 };
 
 // One compute lane: two adjacent units of NB batch rows.  (lane_bwd_kernel has the same in local variables.  With this struct in its place
@@ -193,7 +193,8 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
     if (T > 1) mbar_arrive_expect_tx(&full[1], RB);  // step index 1
   }
   constexpr bool TM = G::TM;
-  if constexpr (TM) {  // (the registers of the CTA leave no room for another on this SM, so there is nobody to wait for)
+  if constexpr (TM) {  // (see tmem_alone)
+    __syncwarp();
     if (warp == 0) tmem_alloc(reinterpret_cast<uint32_t*>(smem_raw + 96), 512);
     tc_fence_before();
     __syncthreads();
@@ -223,6 +224,7 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
   uint32_t tcol = 0;
   if constexpr (TM) {
     tcol = *reinterpret_cast<volatile uint32_t*>(smem_raw + 96) + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * G::TCOLS);
+    __syncwarp();  // tensor memory is accessed by whole warps
 #pragma unroll 1
     for (int i = 0; i < MT / MG * KT; ++i) {
       uint32_t r[16];
@@ -289,6 +291,7 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
           pair(kp, f[0], f[MG - 1]);
         };
         constexpr int TP = U == 48 ? 2 : 1;  // k-pairs per load
+        __syncwarp();  // (the lanes may have left the barrier, or the branch around the sends before, one by one)
 #pragma unroll
         for (int i = 0; i + TP <= KT; i += TP) {
           if constexpr (TP == 2) {
@@ -409,9 +412,12 @@ __global__ void __launch_bounds__(BigBwdGeom<CELL, U, NT>::TH, 1) big_bwd_kernel
     lx.store_grads(p, rec);
   }
   __syncwarp();
+  if constexpr (TM) tc_fence_before();
   cluster_arrive_relaxed();
   cluster_wait();
   if constexpr (TM) {
+    tc_fence_after();
+    __syncwarp();
     if (warp == 0) tmem_dealloc(*reinterpret_cast<volatile uint32_t*>(smem_raw + 96), 512);
   }
 }

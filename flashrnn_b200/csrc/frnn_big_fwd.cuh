@@ -55,7 +55,7 @@ struct BigFwdGeom {
     const int want = D / 64 - KRP - tsp(D), fit = ((int)kSmemBudget - off_r(D)) / (W * MT * 1024);
     return want <= 0 ? 0 : (fit < 0 ? 0 : (want < fit ? want : fit));
   }
-  static __host__ __device__ constexpr size_t smem(int D) { return (size_t)off_r(D) + (size_t)ksp(D) * W * MT * 1024; }
+  static __host__ __device__ constexpr size_t smem(int D) { return tmem_alone(TM, (size_t)off_r(D) + (size_t)ksp(D) * W * MT * 1024); }
 };
 
 // Index (16-byte fragments) of lane 0's first fragment of unit group `grp`, k-pair kp in the packed R of head n: [n][grp][kp][m][lo, hi][lane]
@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
     if (T > 2) mbar_arrive_expect_tx(&full[1], step_bytes);  // h_1
   }
   constexpr bool TM = G::TM;
-  if constexpr (TM) {  // (the registers of the CTA leave no room for another on this SM, so there is nobody to wait for)
+  if constexpr (TM) {  // (see tmem_alone)
+    __syncwarp();
     if (warp == 0) tmem_alloc(reinterpret_cast<uint32_t*>(smem_raw + 64), 512);
     tc_fence_before();
     __syncthreads();
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
   if constexpr (TM) {
     static_assert(MT == 2, "a k-pair is 16 words per lane");
     tcol = *reinterpret_cast<volatile uint32_t*>(smem_raw + 64) + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * G::TCOLS);
+    __syncwarp();  // tensor memory is accessed by whole warps
     for (int i = 0; i < tsp; ++i) {
       uint32_t r[16];
 #pragma unroll
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
       }
       else if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(&full[(t + 1) & 1], step_bytes);
     }
+    if constexpr (TM) __syncwarp();  // (the lanes may have left the wait one by one)
   };
   float part[NS][MT][NT][4];
   auto products = [&](uint32_t hb) {  // part += this warp's rows and k range of R times the h tile
@@ -358,7 +361,10 @@ __global__ void __launch_bounds__(BigFwdGeom<CELL, U, NT, DENSE>::TH, DENSE ? 2 
   // Every message to this CTA has been waited for; only after an expired wait can one still be in flight, and then the barrier covers it.
   if (T > 1) { __syncwarp(); cluster_arrive_relaxed(); cluster_wait(); }
   if constexpr (TM) {
+    tc_fence_before();
     __syncthreads();  // (every warp has done its last load; one that reached the cluster's barrier above has, too, but T may be 1)
+    tc_fence_after();
+    __syncwarp();
     if (warp == 0) tmem_dealloc(*reinterpret_cast<volatile uint32_t*>(smem_raw + 64), 512);
   }
 }

@@ -6,6 +6,13 @@
 namespace FRNN_NS {
 
 // ---- tensor memory
+// A CTA that takes all 512 columns waits in the allocation for whoever holds some, and a CTA of a cluster that waits keeps the rest of its cluster waiting.  Two
+// clusters on the same SMs, each holding what the other waits for, would never end.  So a kernel of clusters that takes tensor memory asks for
+// more than half of an SM's shared memory: no two of their CTAs share an SM, and what else holds some waits for nobody and ends.
+constexpr size_t kTmemAloneSmem = 116 * 1024;
+static_assert(2 * (kTmemAloneSmem + 1024) > 228 * 1024 && kTmemAloneSmem <= kSmemBudget, "more than half of 228 KB, of which a CTA's own 1 KB is part");
+__host__ __device__ constexpr size_t tmem_alone(bool tmem, size_t smem) { return tmem && smem < kTmemAloneSmem ? kTmemAloneSmem : smem; }
+
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");

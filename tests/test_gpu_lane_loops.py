@@ -120,3 +120,29 @@ def _check(function, N, D, B, T, state_f32, **tile):
     ref = run_oracle(function, Wx, R, b, s0, cot=cot, clip=opts.get("gradient_recurrent_clipval", 0.0),
                      forward_clip=opts.get("forward_clipval", 0.0))
     assert_parity(function, got, ref, tag=f"{function} N{N} D{D} {tile} B{B} T{T}", zero_init=False)
+
+
+# two clusters whose CTAs each take all of an SM's tensor memory must not share SMs: forward and reverse loops of both, on two streams at once
+def test_head_dims_above_256_on_two_streams(cuda_device):
+    from flashrnn_b200 import flashrnn
+
+    calls = []
+    for function, N, D in (("lstm", 4, 640), ("gru", 4, 768)):
+        Wx, R, b, s0 = [t.to(cuda_device, torch.bfloat16) for t in make_inputs(function, 33, 24, N, D, seed=D)]
+        calls.append((function, [Wx.requires_grad_(True), R, b, s0]))
+
+    def passes(function, args):
+        states, _ = flashrnn(*args, function=function)
+        return states.detach(), torch.autograd.grad(states[0], args[0], torch.ones_like(states[0]))[0]
+
+    alone = [passes(*c) for c in calls]
+    streams = [torch.cuda.Stream(cuda_device) for _ in calls]
+    torch.cuda.synchronize()
+    together = []
+    for _ in range(5):
+        for stream, c in zip(streams, calls):
+            with torch.cuda.stream(stream):
+                together.append(passes(*c))
+    torch.cuda.synchronize()
+    for i, got in enumerate(together):
+        assert all(torch.equal(x, y) for x, y in zip(got, alone[i % 2]))
