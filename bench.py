@@ -424,6 +424,8 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
     # ---- floor of the serial chain: the same loops with the gate arithmetic taken out (frnn_plan.probe_noop_cell)
     chain = None
     loops = {name: nv.query_loop(plan, name == "reverse") for name in ("forward", "reverse")}
+    dr_in_loop, dr_threads = nv.query_dr(plan)
+    on_top = {"forward": 0, "reverse": dr_threads}
     wide = nv.LOOPS[loops["reverse"].loop] == "wide"
     if floor and not wide:
         probe = nv.FrnnPlan.from_buffer_copy(plan)
@@ -459,7 +461,7 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
         "kernel_ms": {"forward_loop": fwd_ms, "backward_loop": bwd_ms, "recurrent_grad": dr_ms},
         "us_per_time_step": {"forward": 1e3 * fwd_ms / T, "backward": 1e3 * bwd_ms / T},
         "tile": {name: {"loop": nv.LOOPS[s.loop], "cluster_size": s.cluster_size, "units_per_cta": s.units_per_cta, "batch_rows": s.batch_rows,
-                        "threads": s.threads, "ctas": s.grid[0] * s.grid[1] * s.grid[2]} for name, s in loops.items()},  # as launched
+                        "threads": s.threads + on_top[name], "ctas": s.grid[0] * s.grid[1] * s.grid[2]} for name, s in loops.items()},  # as launched
         "roofline": {
             "bound": "hbm", "kernel": REVERSE_KERNELS[nv.LOOPS[loops["reverse"].loop]] + (" (reverse time loop, dR and db inside)" if wide else " (reverse time loop)"),
             "achieved": achieved, "peak": job.hbm_peak, "unit": "GB/s", "frac": achieved / job.hbm_peak, "peak_source": job.peak_source,
@@ -475,7 +477,7 @@ def measure(job: Job, function, B, T, N, D, f32, *, allreduce, group=True, clust
                     "more CTAs than SMs: issue slots of the cells and memory bound this workload" if min(s.grid[0] * s.grid[1] * s.grid[2] for s in loops.values()) > 148 else
                     "the serial chain of 2T dependent steps (chain_floor), not HBM or the tensor pipe, bounds this workload"},
         # loops, dR and cast; in front: fragments of R^T (16-bit), of R (head dims above 256), R^T (float32 but for the lane loop)
-        "clocks": clk.summary(), "launches_per_step": 3 if wide else 4 + (nv.LOOPS[loops["forward"].loop] != "f32_lane") if job.f32io else 6 if D > 256 else 5 - (dr_ms < 0.003),  # (no kernel between those events where the loop forms dR)
+        "clocks": clk.summary(), "launches_per_step": 3 if wide else 4 + (nv.LOOPS[loops["forward"].loop] != "f32_lane") if job.f32io else 6 if D > 256 else 5 - dr_in_loop,
     }
     if keep is not None:
         keep.update(Wx=Wx, R=R, b=b, s0=s0, gcnt=gcnt)

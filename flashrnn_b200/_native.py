@@ -24,7 +24,7 @@ DTYPE_BF16, DTYPE_F32, DTYPE_F16 = 0, 1, 2
 
 # every symbol include/frnn.h declares
 EXPORTS = (
-    "frnn_abi_version", "frnn_query", "frnn_query_tile", "frnn_query_loop", "frnn_forward", "frnn_backward", "frnn_backward_parts",
+    "frnn_abi_version", "frnn_query", "frnn_query_tile", "frnn_query_loop", "frnn_query_dr", "frnn_forward", "frnn_backward", "frnn_backward_parts",
     "frnn_forward_noalloc",
     "frnn_finalize_grads", "frnn_read_device_status", "frnn_status_string",
 )
@@ -108,6 +108,7 @@ def lib() -> ctypes.CDLL:
         L.frnn_query_tile.argtypes = [ctypes.POINTER(FrnnProblem), ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                       ctypes.POINTER(FrnnPlan)]
         L.frnn_query_loop.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.c_int, ctypes.POINTER(FrnnLoopShape)]
+        L.frnn_query_dr.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int32)]
         L.frnn_forward.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.POINTER(FrnnFwdArgs), ctypes.c_void_p]
         L.frnn_backward.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.POINTER(FrnnBwdArgs), ctypes.c_void_p]
         L.frnn_backward_parts.argtypes = [ctypes.POINTER(FrnnPlan), ctypes.POINTER(FrnnBwdArgs), ctypes.c_void_p, ctypes.c_int]
@@ -194,3 +195,10 @@ def query_loop(plan: FrnnPlan, backward: bool) -> FrnnLoopShape:
     shape = FrnnLoopShape()
     check("frnn_query_loop", lib().frnn_query_loop(ctypes.byref(plan), int(backward), ctypes.byref(shape)))
     return shape
+
+
+def query_dr(plan: FrnnPlan) -> tuple[bool, int]:
+    """Whether the plan's reverse loop forms dR itself, and the threads per CTA it is launched with for that on top of ``query_loop``'s."""
+    in_loop, threads = ctypes.c_int32(), ctypes.c_int32()
+    check("frnn_query_dr", lib().frnn_query_dr(ctypes.byref(plan), ctypes.byref(in_loop), ctypes.byref(threads)))
+    return bool(in_loop.value), threads.value

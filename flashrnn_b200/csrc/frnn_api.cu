@@ -208,7 +208,7 @@ static bool lane_help(const frnn_problem& pr, int cs, int u, int nt) {
 // only pays once their own kernel takes that.  LSTM, tiles: T256 2 132 / 134, 8 136 / 133, 24 144 / 134, T512 2 240 / 246, 8 245 / 247, 16 251 / 253, 24 261 / 251, T2048 16 918 /
 // 943, 24 959 / 949, 32 980 / 951.  sLSTM: T64 24 58 / 51, T256 8 138 / 144, 24 150 / 146, T512 24 267 / 273, 48 284 / 275, T2048 24 986 / 1036, 48 1043 / 1043, 64 1070 /
 // 1043.  GRU, any: T512 1 232 / 193, 24 249 / 196, T2048 24 917 / 727.
-constexpr int kDrMinSteps = 24, kDrShort = 256;
+constexpr int kDrMinSteps = 24, kDrShort = 256, kDrThreads = 32;
 static bool lane_dr(const frnn_plan& pl, int nt) {
   const frnn_problem& pr = pl.prob;
   if (pr.D != 64 || pl.cluster_size != 1 || nt != 1 || pr.cell == CELL_ELMAN || pr.dtype_state == FRNN_DTYPE_F32 || pl.forced_tile) return false;
@@ -489,6 +489,7 @@ extern "C" {
 int frnn_query_f16(const frnn_problem*, frnn_plan*);
 int frnn_query_tile_f16(const frnn_problem*, int, int, int, frnn_plan*);
 int frnn_query_loop_f16(const frnn_plan*, int, frnn_loop_shape*);
+int frnn_query_dr_f16(const frnn_plan*, int32_t*, int32_t*);
 int frnn_forward_f16(const frnn_plan*, const frnn_fwd_args*, void*);
 int frnn_backward_parts_f16(const frnn_plan*, const frnn_bwd_args*, void*, int);
 int frnn_finalize_grads_f16(const frnn_plan*, const void*, void*, void*, void*);
@@ -549,7 +550,19 @@ int FRNN_ENTRY(frnn_query_loop)(const frnn_plan* plan, int backward, frnn_loop_s
   const LoopLaunch k = loop_of(*plan, backward != 0);
   if (!k.fn) return FRNN_ERR_PLAN;
   const dim3 g = loop_grid(k, pr);
-  *out = {is_big(pr) ? FRNN_LOOP_BIG : FRNN_LOOP_LANE, k.cs, k.u, k.rows, k.threads - (k.dr ? 32 : 0), k.stages, {g.x, g.y, g.z}};
+  *out = {is_big(pr) ? FRNN_LOOP_BIG : FRNN_LOOP_LANE, k.cs, k.u, k.rows, k.threads - (k.dr ? kDrThreads : 0), k.stages, {g.x, g.y, g.z}};
+  return FRNN_OK;
+}
+
+int FRNN_ENTRY(frnn_query_dr)(const frnn_plan* plan, int32_t* in_loop, int32_t* threads_on_top) {
+  FRNN_FORWARD_F16(wants_f16(plan), frnn_query_dr_f16(plan, in_loop, threads_on_top));
+  frnn_loop_shape s;
+  const int rc = frnn_query_loop(plan, 1, &s);
+  if (rc) return rc;
+  if (!in_loop || !threads_on_top) return FRNN_ERR_NULL;
+  const bool lane = s.loop == FRNN_LOOP_LANE && loop_of(*plan, true).dr;
+  *in_loop = lane || s.loop == FRNN_LOOP_WIDE;
+  *threads_on_top = lane ? kDrThreads : 0;
   return FRNN_OK;
 }
 

@@ -184,7 +184,7 @@ typedef struct frnn_loop_shape {
   int32_t cluster_size;      /* CTAs that share one (head, batch tile)                                 */
   int32_t units_per_cta;
   int32_t batch_rows;        /* batch rows per CTA                                                     */
-  int32_t threads;           /* per CTA, of the loop itself: a warp that forms dR beside it comes on top */
+  int32_t threads;           /* per CTA, of the loop itself (a warp that forms dR beside it comes on top: frnn_query_dr) */
   int32_t input_stages;      /* time steps of inputs in flight in shared memory (0: none kept there)   */
   uint32_t grid[3];          /* CTAs                                                                   */
 } frnn_loop_shape;
@@ -192,6 +192,10 @@ typedef struct frnn_loop_shape {
 /* Pure host function: what the forward (backward = 0) or reverse time loop of a plan is launched with.  No counterpart in
  * the reference. */
 int frnn_query_loop(const frnn_plan* plan, int backward, frnn_loop_shape* out);
+
+/* Pure host function: whether the reverse loop of a plan forms dR itself (*in_loop = 1: FRNN_PART_DR launches nothing; 0: a kernel of its own does), and
+ * the threads per CTA it is launched with for that on top of frnn_loop_shape.threads.  FRNN_ERR_TRAINING without training.  No counterpart in the reference. */
+int frnn_query_dr(const frnn_plan* plan, int32_t* in_loop, int32_t* threads_on_top);
 
 /* Whole-sequence forward: one persistent launch (head dims above 256: plus a small weight-repack launch).
  * Replaces ForwardPass::Run (flashrnn/flashrnn/fused/flashrnn_fused_forward.cu:772-975). */

@@ -78,9 +78,10 @@ def test_reverse_loops_that_form_dr(cuda_device, function, N, B, T):
 @pytest.mark.parametrize("function", ["lstm", "slstm"])
 @pytest.mark.parametrize("T", [24, 33])
 def test_loops_that_form_dr_on_a_full_gpu(cuda_device, function, T):
-    from flashrnn_b200 import flashrnn
+    from flashrnn_b200 import _native, flashrnn
 
     B, N, D = 1024, 16, 64
+    assert _native.query_dr(_native.query(_native.make_problem(function, B, T, N, D, False, True)))[0]
     g = torch.Generator(device=cuda_device).manual_seed(T)
     randn = lambda *shape: torch.randn(*shape, generator=g, device=cuda_device, dtype=torch.bfloat16)
     Wx, R, b = randn(B, T, 4, N, D), randn(4, N, D, D) / D ** 0.5, randn(4, N, D) / 8

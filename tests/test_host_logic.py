@@ -419,3 +419,24 @@ int main(int argc, char** argv) {
     out = subprocess.run([str(exe), str(_native.LIB_PATH)], check=True, capture_output=True, text=True).stdout
     ratios = [float(x) for x in out.split()]
     assert len(ratios) == 4 and max(ratios) < 5.5, ratios
+
+
+def test_plans_report_which_kernel_forms_dr():
+    """Both sides of each line of the rule; the threads of the warp that forms dR come on top of the loop's."""
+    mk = lambda function, B, T, N, D=64, state_f32=False, training=True, **kw: _native.make_problem(function, B, T, N, D, state_f32, training, **kw)
+    dr = lambda *a, **kw: _native.query_dr(_native.query(mk(*a, **kw)))
+    own, loop, wide = (False, 0), (True, 32), (True, 0)
+    assert [dr("lstm", 8, T, 16) for T in (23, 24, 256, 257)] == [own, loop, loop, own]
+    assert [dr("lstm", 8, 257, N) for N in (23, 24)] == [own, loop]
+    assert [dr("slstm", 8, T, N) for T, N in ((23, 48), (24, 23), (24, 24), (256, 24), (257, 47), (257, 48))] == [own, own, loop, loop, own, loop]
+    assert [dr("gru", 1, T, 1) for T in (23, 24, 5000)] == [own, loop, loop]
+    for kw in ({}, {"f16": True}):
+        assert dr("lstm", 1024, 512, 16, **kw) == loop and dr("lstm", 1024, 512, 16, state_f32=True, **kw) == own
+    assert dr("elman", 1024, 512, 16) == wide and dr("elman", 8, 512, 16) == own
+    assert dr("lstm", 16, 64, 4, 256) == own and dr("lstm", 16, 64, 1, 512) == own and dr("lstm", 16, 64, 4, 64, True, f32=True) == own
+    assert _native.query_dr(_native.query(mk("lstm", 8, 64, 16), 1, 8)) == own
+    plan = _native.query(mk("lstm", 1024, 512, 16))
+    assert _native.query_loop(plan, True).threads + _native.query_dr(plan)[1] == 224
+    with pytest.raises(_native.FrnnError) as e:
+        dr("lstm", 8, 64, 16, training=False)
+    assert e.value.code == -7
