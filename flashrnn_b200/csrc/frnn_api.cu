@@ -341,7 +341,7 @@ static LoopLaunch loop_of(const frnn_plan& pl, bool bwd) {
   const int kt = pr.D / 16, u = pl.units_per_cta, nt = lane_nt(pr, bwd, pl.batch_tile, pl.forced_tile);
   const bool dr = bwd && !pl.probe_noop_cell && lane_dr(pl, nt);
   LaneKernel k = {nullptr, 0, 0};
-  if (pl.probe_noop_cell) k = bwd ? lane_bwd_floor(pr.cell, kt, u, nt) : lane_fwd_floor(pr.cell, kt, u, nt);
+  if (pl.probe_noop_cell) k = lane_floor(pr.cell, bwd, kt, u, nt, pr.dtype_state == FRNN_DTYPE_F32 ? 4 : 2);
   else if (dr) k = lane_dr_kernel(cell);
   else if (bwd && lane_help(pr, pl.cluster_size, u, nt)) k = lane_loop(pr, true, u, nt, true);
   if (!k.fn && !pl.probe_noop_cell) k = lane_loop(pr, bwd, u, nt, false);

@@ -56,8 +56,7 @@ FRNN_DECLARE(lstm) FRNN_DECLARE(gru) FRNN_DECLARE(elman) FRNN_DECLARE(elmanc) FR
 #undef FRNN_DECLARE
 
 // chain-floor variants (frnn_inst_floor.cu); fn == nullptr for any tile but the benchmark configurations
-LaneKernel lane_fwd_floor(int cell, int kt, int u, int nt);
-LaneKernel lane_bwd_floor(int cell, int kt, int u, int nt);
+LaneKernel lane_floor(int cell, bool bwd, int kt, int u, int nt, int es);
 
 // in front of a reverse loop: R^T as the fragments of its CTAs (U units each), fp32 gradients and status block zeroed
 size_t rt_pack_bytes(int Gr, int N, int D, int U);
