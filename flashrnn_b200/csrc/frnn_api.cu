@@ -199,7 +199,7 @@ static int lane_nt(const frnn_problem& pr, bool bwd, int bt, bool forced) {
 static bool lane_help(const frnn_problem& pr, int cs, int u, int nt) {
   if (cs < 2 || cs > 16 || u != 32 || nt != 1) return false;
   const bool alone = (long long)((pr.B + 7) / 8) * pr.N <= kResident[cs];
-  return alone || pr.cell == CELL_LSTM || pr.cell == CELL_SLSTM || (pr.cell == CELL_GRU && pr.D == 96);
+  return alone || help_always(kernel_cell(pr), pr.D / 16);
 }
 
 // Whether the reverse lane loop forms dR as well (lane_bwd_dr): head dim 64 with one CTA per head, 8 rows and 16-bit states.  Not for the shortest
@@ -226,6 +226,7 @@ static LaneKernel lane_loop(const frnn_problem& pr, bool bwd, int u, int nt, boo
   return (long long)((pr.B + 8 * nt - 1) / (8 * nt)) * pr.N * (pr.D / u) <= 2LL * sm_count_cached() ? f->few[f32] : f->many[f32];
 }
 static bool lane_exists(const frnn_problem& pr, bool bwd, int u, int nt) {
+  if (bwd && u == 32 && nt == 1 && help_always(kernel_cell(pr), pr.D / 16)) return true;
   const LaneForms* f = lane_forms(kernel_cell(pr), bwd, pr.D / 16, u, nt);
   return f && f->few[pr.dtype_state == FRNN_DTYPE_F32].fn;
 }

@@ -48,12 +48,12 @@ struct BigKernel {
   extern const LaneForms lane_fwd_##cell[kLaneTiles][2];  /* [tile][rows / 8 - 1] */ \
   extern const LaneForms lane_bwd_##cell[kLaneTiles][2];                             \
   extern const LaneForms lane_bwd_help_##cell[4];                                    \
-  extern const LaneKernel lane_bwd_dr_##cell;                                        \
   BigKernel big_fwd_##cell(int u, int nt, bool dense);  \
   BigKernel big_bwd_##cell(int u, int nt);              \
   cudaError_t big_pack_##cell(const void* R, void* out, int N, int D, cudaStream_t stream);
 FRNN_DECLARE(lstm) FRNN_DECLARE(gru) FRNN_DECLARE(elman) FRNN_DECLARE(elmanc) FRNN_DECLARE(slstm)
 #undef FRNN_DECLARE
+extern const LaneKernel lane_bwd_dr_lstm, lane_bwd_dr_gru, lane_bwd_dr_slstm;
 
 // chain-floor variants (frnn_inst_floor.cu); fn == nullptr for any tile but the benchmark configurations
 LaneKernel lane_floor(int cell, bool bwd, int kt, int u, int nt, int es);

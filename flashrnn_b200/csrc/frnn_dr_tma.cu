@@ -36,7 +36,7 @@ struct DrTmaParams {
   const elem_t* s0;   // [S,B,1,N,D]; only s = 0 is read
   float* dR;                 // [Gr,N,D,D] fp32
   unsigned* status;
-  int cell, B, T, N, D, Gr, Gw;
+  int cell, B, N, D, Gr;
   int chunks_per_b;          // ceil(T / 64)
   int chunks_per_split;
   int tmem_cols;             // power of two >= mt * D, >= 32
@@ -52,7 +52,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* sm = smem_raw + (base - raw);
-  const int D = p.D, N = p.N, T = p.T, nb = D >> 6;  // nb = 64-wide blocks per gate (rows) / of p (columns)
+  const int D = p.D, N = p.N, nb = D >> 6;  // nb = 64-wide blocks per gate (rows) / of p (columns)
   const int MT = p.mt, NS = p.stages, nbw = p.nbw, DW = nbw * 64, ctile = blockIdx.x % p.ct;
   const uint32_t stage_bytes = (uint32_t)(2 * MT + nbw) * DT_BLK;
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + (size_t)NS * stage_bytes);          // [DT_STAGES] bytes have landed
@@ -227,7 +227,7 @@ cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int 
   p.s0 = static_cast<const elem_t*>(s0);
   p.dR = dR;
   p.status = status;
-  p.cell = cell; p.B = B; p.T = T; p.N = N; p.D = D; p.Gr = Gr; p.Gw = Gw;
+  p.cell = cell; p.B = B; p.N = N; p.D = D; p.Gr = Gr;
   p.chunks_per_b = (T + DT_KC - 1) / DT_KC;
   // tiles of 128 rows per CTA: as many as share one fetch of h, within 512 tensor-memory columns and a ring of at least
   // three stages in shared memory

@@ -18,7 +18,8 @@ namespace FRNN_NS {
 template <int KT, int U, int NT, int ES>
 constexpr LaneKernel lane_entry() {
   using G = FRNN_GEOM(KT, U, NT, ES);
-  if constexpr (G::valid && (ES ? states_form(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false, ES) : states_general(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false)))
+  if constexpr (FRNN_INST_BWD && U == 32 && NT == 1 && help_always(FRNN_INST_CELL, KT)) return LaneKernel{nullptr, 0, 0};
+  else if constexpr (G::valid && (ES ? states_form(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false, ES) : states_general(FRNN_INST_CELL, FRNN_INST_BWD, KT, U, NT, false)))
     return LaneKernel{&FRNN_KERNEL(KT, U, NT, ES), G::TH, G::smem};
   return LaneKernel{nullptr, 0, 0};
 }
@@ -57,8 +58,9 @@ constexpr LaneForms help_forms() {
   return lane_forms(FRNN_INST_CELL, true, KT, bwd_entry<KT, 32, true, 0, false>(), bwd_entry<KT, 32, true, 2, false>(), bwd_entry<KT, 32, true, 4, false>());
 }
 constexpr LaneForms FRNN_INST_HELP[4] = {help_forms<kHelpKTs[0]>(), help_forms<kHelpKTs[1]>(), help_forms<kHelpKTs[2]>(), help_forms<kHelpKTs[3]>()};
-// the reverse loop with a warp that forms dR (head dim 64, one CTA per head)
+#ifdef FRNN_INST_DR  // the reverse loop with a warp that forms dR (head dim 64, one CTA per head)
 constexpr LaneKernel FRNN_INST_DR = bwd_entry<4, 64, false, 2, true>();
+#endif
 #endif
 
 // ---- head dims above 256: units per CTA, batch tile / 8

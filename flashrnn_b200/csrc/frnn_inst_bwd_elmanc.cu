@@ -3,6 +3,5 @@
 #define FRNN_INST_BWD 1
 #define FRNN_INST_LANE lane_bwd_elmanc
 #define FRNN_INST_HELP lane_bwd_help_elmanc
-#define FRNN_INST_DR lane_bwd_dr_elmanc
 #define FRNN_INST_BIG big_bwd_elmanc
 #include "frnn_inst.cuh"

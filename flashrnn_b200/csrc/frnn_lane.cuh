@@ -153,6 +153,10 @@ __host__ __device__ constexpr bool states_form(int cell, bool bwd, int kt, int u
 // Two of these forms need registers that cost a CTA per SM, or most of the gain, once CTAs queue up; the general form runs then.  LSTM, us, D = 64 forward, 16 bits: B150 N12
 // T64 50 -> 44, B400 N12 T128 204 -> 208, B1024 N16 T64 285 -> 296, fp32: B16 N12 T512 278 -> 241, B400 233 -> 241, B1024 325 -> 336; D = 32 reverse, 16 bits: B16 N8 T512 159 -> 140, B1024 N24 T64 239 -> 244.
 __host__ __device__ constexpr bool states_form_for_few(int cell, bool bwd, int kt, int es) { return cell == CELL_LSTM && (bwd ? kt == 2 && es == 2 : kt == 4); }
+// Whether the reverse loops of 32-unit clusters and 8 rows are always those with warps that only multiply (lane_help in frnn_api.cu): there is no other form then.
+__host__ __device__ constexpr bool help_always(int cell, int kt) {
+  return cell == CELL_LSTM ? kt == 6 || kt == 12 || kt == 16 : cell == CELL_SLSTM ? kt == 6 || kt == 8 || kt == 12 || kt == 16 : cell == CELL_GRU && kt == 6;
+}
 // whether the form that reads the type of the states at run time is needed
 __host__ __device__ constexpr bool states_general(int cell, bool bwd, int kt, int u, int nt, bool help) {
   return !states_form(cell, bwd, kt, u, nt, help, 2) || !states_form(cell, bwd, kt, u, nt, help, 4) || states_form_for_few(cell, bwd, kt, 2) || states_form_for_few(cell, bwd, kt, 4);

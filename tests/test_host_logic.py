@@ -440,3 +440,26 @@ def test_plans_report_which_kernel_forms_dr():
     with pytest.raises(_native.FrnnError) as e:
         dr("lstm", 8, 64, 16, training=False)
     assert e.value.code == -7
+
+
+def test_every_accepted_tile_has_both_loops():
+    """Tiles of 32-unit clusters with 8 rows have a reverse loop with multiplying warps, another one, or both; whatever a plan names, there is a kernel for it."""
+    asked = 0
+    for function in ("lstm", "gru", "elman", "slstm"):
+        for D in (16, 32, 64, 96, 128, 192, 256):
+            for state_f32 in (False, True):
+                for clip in (0.0, 0.5):
+                    for B, N in ((1, 1), (8, 4), (9, 60), (200, 12), (1024, 24)):
+                        for cs, bt in ((0, 0), *((cs, bt) for cs in (1, 2, 3, 4, 6, 8, 16) for bt in (8, 16, 32) if D % cs == 0)):
+                            prob = _native.make_problem(function, B, 40, N, D, state_f32, True)
+                            prob.forward_clip = clip
+                            try:
+                                plan = _native.query(prob, cs, bt)
+                            except _native.FrnnError:
+                                assert cs or bt
+                                continue
+                            for backward in (False, True):
+                                s = _native.query_loop(plan, backward)
+                                assert s.threads >= 32 and s.cluster_size * s.units_per_cta == D
+                            asked += 1
+    assert asked == 4140
