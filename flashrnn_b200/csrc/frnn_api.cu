@@ -718,7 +718,7 @@ int FRNN_ENTRY(frnn_backward_parts)(const frnn_plan* plan, const frnn_bwd_args* 
                                     sm_count_cached(), stream);
   else if ((parts & FRNN_PART_DR) && recurrent_grad_tma_supported(pr.D, lp.state_f32) && tma_pays)
     e = launch_recurrent_grad_tma(pr.cell, pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, a->dWx, ws + w.dg0, a->states, a->s0, grads,
-                                  reinterpret_cast<unsigned*>(ws), sm_count_cached(), stream);
+                                  reinterpret_cast<unsigned*>(ws), plan->test_drop_exchange, sm_count_cached(), stream);
   else if ((parts & FRNN_PART_DR) && pr.D <= 256)
     e = launch_recurrent_grad_tc(pr.cell, pr.B, pr.T, pr.N, pr.D, cd.Gr, cd.Gw, lp.state_f32, a->dWx, ws + w.dg0, a->states,
                                  a->s0, grads, reinterpret_cast<unsigned*>(ws), sm_count_cached(), stream);

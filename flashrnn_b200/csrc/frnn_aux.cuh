@@ -88,7 +88,7 @@ cudaError_t launch_wide_gates_forward(int cell, const void* Wx, long long wx_sb,
 // dR fed by tensor-map bulk copies (frnn_dr_tma.cu): 16-bit states, head dims of 128 up that are multiples of 64
 bool recurrent_grad_tma_supported(int D, int state_f32);
 cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int Gr, int Gw, const void* dWx, const void* dg0,
-                                      const void* states, const void* s0, float* dR, unsigned* status, int sm_count,
+                                      const void* states, const void* s0, float* dR, unsigned* status, int test_drop, int sm_count,
                                       cudaStream_t stream);
 // dR for head dims 16, 32, 64, 96 (frnn_dr_small.cu)
 bool recurrent_grad_small_supported(int D);

@@ -36,6 +36,7 @@ struct DrTmaParams {
   const elem_t* s0;   // [S,B,1,N,D]; only s = 0 is read
   float* dR;                 // [Gr,N,D,D] fp32
   unsigned* status;
+  int test_drop;  // test hook: of the first chunk that starts at t = 0, 1: its row of h_{-1} is never reported as filled, 2: it is never reported as landed
   int cell, B, N, D, Gr;
   int chunks_per_b;          // ceil(T / 64)
   int chunks_per_split;
@@ -127,7 +128,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
         if (!mbar_wait_bounded(&full[s], par)) { ok = false; report_timeout(p.status, ci); break; }
         seen = ci + 1;
         if (ci == next) {
-          mbar_arrive(landed);
+          if (!(p.test_drop == 2 && ci == first)) mbar_arrive(landed);
           if (!mbar_wait_bounded(filled, npar)) { ok = false; report_timeout(p.status, ci); break; }
           next += p.chunks_per_b;
           npar ^= 1u;
@@ -168,7 +169,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
         if (!mbar_wait_bounded(landed, par)) { report_timeout(p.status, ci); break; }
         if ((lane >> 3) < nbw) sts128(base + (uint32_t)(ci % NS) * stage_bytes + (uint32_t)(2 * MT + (lane >> 3)) * DT_BLK + (lane & 7) * 16, h);
         fence_proxy_async_smem();  // the row is read by the tensor core
-        mbar_arrive(filled);
+        if (!(p.test_drop == 1 && ci == first && lane == 0)) mbar_arrive(filled);
       }
       __syncwarp();
     }
@@ -205,7 +206,7 @@ recurrent_grad_tma_kernel(const __grid_constant__ CUtensorMap tm_dwx, const __gr
 bool recurrent_grad_tma_supported(int D, int state_f32) { return !state_f32 && D >= 128 && D % 64 == 0; }
 
 cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int Gr, int Gw, const void* dWx, const void* dg0,
-                                      const void* states, const void* s0, float* dR, unsigned* status, int sm_count,
+                                      const void* states, const void* s0, float* dR, unsigned* status, int test_drop, int sm_count,
                                       cudaStream_t stream) {
   const uint64_t row = (uint64_t)D * 2;
   CUtensorMap tm_dwx, tm_dg0, tm_st;
@@ -227,6 +228,7 @@ cudaError_t launch_recurrent_grad_tma(int cell, int B, int T, int N, int D, int 
   p.s0 = static_cast<const elem_t*>(s0);
   p.dR = dR;
   p.status = status;
+  p.test_drop = test_drop;
   p.cell = cell; p.B = B; p.N = N; p.D = D; p.Gr = Gr;
   p.chunks_per_b = (T + DT_KC - 1) / DT_KC;
   // tiles of 128 rows per CTA: as many as share one fetch of h, within 512 tensor-memory columns and a ring of at least

@@ -267,7 +267,7 @@ __device__ __forceinline__ void lane_bwd_dr(const LoopParams& p, uint32_t d0, ui
 #pragma unroll
     for (int m = 0; m < G::DRT; ++m)
       umma_16(tmem + m * D, smem_desc(a0 + m * 16 * G::DP, G::DB, G::DP), bd, instr_desc_16(128, D, 1, 1), q > 0 ? 1u : 0u);
-    umma_commit(last ? all_done : done);
+    if (!(p.test_drop == 1 && q == 0) && !(p.test_drop == 2 && last)) umma_commit(last ? all_done : done);  // (test hook: the first, the last product is never reported)
   };
 #pragma unroll
   for (int s = 0; s < AHEAD; ++s) load_h(s);

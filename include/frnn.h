@@ -85,7 +85,9 @@ typedef struct frnn_plan {
                                  (forward: its h of step 1; backward: its first message) so that its peers' bounded
                                  waits expire; the kernels then finish with invalid results and report it in the
                                  status block (float32 cluster loops: the message of step 1 in both loops).  With the 128-row loops (batch_tile 128, or wide_forward): one tile copy (step
-                                 index 2) is announced to its barrier and never issued.  Exercises the failure-detection path
+                                 index 2) is announced to its barrier and never issued.  Reverse loops that form dR themselves (frnn_query_dr): the
+                                 first of its products is never reported as done (2: the last one).  The dR kernel of 16-bit states from head dim 128 up: the row of
+                                 h_{-1} is never reported as filled in (2: its tile as landed).  Exercises the failure-detection path
                                  without faulting the GPU.                                                          */
   int32_t keep_packed_r;      /* 0: frnn_forward clears the status block and, where its loop needs it, repacks R into the
                                  workspace (default).

@@ -157,3 +157,45 @@ def test_wide_lstm_forward_reports_a_copy_that_never_lands(cuda_device):
     with torch.no_grad():
         states, _ = flashrnn(Wx, R, b, s0, function="lstm", config=ok)
     assert torch.isfinite(states.float()).all()
+
+
+@pytest.mark.parametrize("hook", [1, 2])
+@pytest.mark.parametrize("function,D,T,part", [("lstm", 64, 40, 1), ("gru", 64, 25, 1), ("lstm", 128, 70, 2), ("gru", 192, 9, 2)])
+def test_dr_reports_what_never_arrives(cuda_device, function, D, T, part, hook):
+    """The waits of the dR sums, in the reverse loop (head dim 64) and in the tensor-map kernel (part 2): a product that is never reported as done, a tile or
+    the row of h_{-1} in it that never arrives.  Each wait gives up and reports it, the kernel ends, and a clean run follows in the same context."""
+    B, N = 9, 2
+    Wx, R, b, s0 = [t.to(cuda_device, torch.bfloat16) for t in make_inputs(function, B, T, N, D, seed=35, random_init=True)]
+    plan = nv.query(nv.make_problem(function, B, T, N, D, False, True))
+    assert nv.query_dr(plan)[0] == (part == 1)
+    P = lambda t: ctypes.c_void_p(t.data_ptr())
+    stream = ctypes.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)
+    states = torch.zeros(s0.shape[0], B, T, N, D, device=cuda_device, dtype=torch.bfloat16)
+    cache = torch.zeros(int(plan.cache_bytes), device=cuda_device, dtype=torch.uint8)
+    ws = torch.zeros(int(plan.workspace_bytes), device=cuda_device, dtype=torch.uint8)
+    L, st = nv.lib(), nv.FrnnDevStatus()
+    fa = nv.FrnnFwdArgs(P(Wx), P(R), P(b), P(s0), P(states), P(cache), P(ws))
+    nv.check("frnn_forward", L.frnn_forward(ctypes.byref(plan), ctypes.byref(fa), stream))
+    dst, dWx, ds0 = torch.ones_like(states), torch.zeros_like(Wx), torch.zeros_like(s0)
+    ba = nv.FrnnBwdArgs(P(R), P(s0), P(states), P(cache), P(dst), P(dWx), P(ds0), P(ws))
+
+    def backward(parts):
+        nv.check("frnn_backward_parts", L.frnn_backward_parts(ctypes.byref(plan), ctypes.byref(ba), stream, parts))
+        nv.check("status", L.frnn_read_device_status(P(ws), stream, ctypes.byref(st)))
+        return st.code
+
+    def gradient():
+        return ws[int(plan.grads_offset):][: R.numel() * 4].view(torch.float32).clone()
+
+    if part == 2:
+        assert backward(1) == 0
+    t0 = time.time()
+    plan.test_drop_exchange = hook
+    assert backward(part) == 1
+    assert time.time() - t0 < 20.0  # bounded: about a second per expired wait
+    plan.test_drop_exchange = 0
+    assert backward(3) == 0
+    want = gradient()
+    assert torch.isfinite(want).all() and float(want.abs().max()) > 0
+    assert backward(3) == 0
+    assert torch.allclose(gradient(), want, rtol=1e-4, atol=1e-4 * float(want.abs().max()))  # (the order of the additions differs)
