@@ -56,9 +56,9 @@ REVERSE_KERNELS = {"lane": "lane_bwd_kernel", "big": "big_bwd_kernel", "wide": "
                    "f32_cluster": "x32c_bwd_kernel", "f32_stream": "x32_bwd_kernel"}  # by what frnn_query_loop says
 METRIC = "fwd+bwd tokens/sec (B*T/s)"
 # DRAM bytes (read + write) of ONE launch of the reverse time loop, from an ncu capture (SpeedOfLight, MemoryWorkloadAnalysis) of
-# `python bench.py --workload C2 --steps 1 --warmup 3 --min-seconds 0 --no-cpu` on a B200; reported with its provenance.
-NCU_TRAFFIC = {"C2": {"bytes": 344_170_000, "source": "ncu capture of lane_bwd_kernel<lstm,KT16,U32,NT1> on this command line with --steps 1 "
-                      "--min-seconds 0, 2026-12-02: 472.6 GB/s for 728.3 us"}}
+# `python bench.py --workload C2 --steps 1 --warmup 3 --min-seconds 0 --no-cpu --headline-only` on a B200; reported with its provenance.
+NCU_TRAFFIC = {"C2": {"bytes": 342_584_000, "source": "ncu capture of lane_bwd_kernel<lstm,KT16,U32,NT1> with multiplying warps and 16-bit states on this command "
+                      "line with --steps 1 --min-seconds 0 --headline-only, 2026-12-05: 237.1 MB read, 105.5 MB written in 643.6 us"}}
 # fwd+bwd of the reference's own CUDA backend on a B200 of this pool, measured by `bench.py --impl reference_gpu`
 # (tokens/s; None: not measured).  The live arm is the source of truth; this record lets the default line carry the ratio.
 REFERENCE_GPU_RECORD = {

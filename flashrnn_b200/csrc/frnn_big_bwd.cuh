@@ -1,6 +1,7 @@
 // Reverse time loop for head dims above 256: the reverse lane loop (frnn_lane_bwd.cuh) with the geometry of frnn_big_fwd.cuh.  A warp
 // owns up to four 16-row tiles of p and all K = Gr * U gate rows of its CTA; KRP of its k-pairs are in registers, the next in
-// tensor memory (see the forward loop), then in shared memory, the rest comes from L2.  Twice as many warps multiply as run the cell (U / 8); the other half moves the data
+// tensor memory (see the forward loop), then in shared memory, the rest comes from L2 (CTAs of 64 units: with 8 rows LSTM from head dim 960, sLSTM from 704 up,
+// with 16 rows LSTM from 576, sLSTM from 448 up).  Twice as many warps multiply as run the cell (U / 8); the other half moves the data
 // meanwhile.  The sums of a tile, or a pair of tiles, leave as soon as they are complete, so their exchange overlaps the products of the next.
 // K is padded to a multiple of 32 with zero fragments (the delta columns there are zero, or the GRU's input-only gate).
 //

@@ -3,7 +3,7 @@
 //   * up to 16 CTAs of U = 32, 48 or 64 units per head (big_tile in frnn_api.cu): with few heads and rows as many SMs as a cluster can have, so that R -- 4.7 MB at
 //     head dim 768 -- lies in their registers (KRP k-pairs per warp), tensor memory (tsp pairs: a lane keeps its own words of a pair in its own lane, 16 columns,
 //     and loads them back into registers for the warp's MMAs) and shared memory (the rest of it) for all T steps; only what fits none of them is
-//     re-read from L2 in every step (head dims 960 and 1024 of the cells with three or four gates);
+//     re-read from L2 in every step (CTAs of 64 units, three or four gates: with 8 rows head dims 960 and 1024, with 16 rows LSTM and sLSTM 768, GRU 832 and up);
 //   * two warps per 8-unit group that split k; the second hands its sums to the first through shared memory (one named
 //     barrier of 64 threads), which runs the cell, and moves the data meanwhile (no IO warps: a 13th warp would cost the other
 //     12 a quarter of their registers).
