@@ -150,9 +150,13 @@ __host__ __device__ constexpr bool states_form(int cell, bool bwd, int kt, int u
   if (cell == CELL_ELMAN) return one ? d == 16 || d == 32 || (!h && d == 64) || (d == 128 && help) || (h && d == 192 && help) : d == 16;
   return false;
 }
-// Three of these forms need registers that cost a CTA per SM, or most of the gain, once CTAs queue up; the general form runs then.  LSTM, us, D = 64 forward, 16 bits: B150 N12
+// Some of these forms need registers that cost a CTA per SM, or most of the gain, once CTAs queue up; the general form runs then.  LSTM, us, D = 64 forward, 16 bits: B150 N12
 // T64 50 -> 44, B400 N12 T128 204 -> 208, B1024 N16 T64 285 -> 296, fp32: B16 N12 T512 278 -> 241, B400 233 -> 241, B1024 325 -> 336; D = 32 reverse, 16 bits: B16 N8 T512 159 -> 140, B1024 N24 T64 239 -> 244.
-__host__ __device__ constexpr bool states_form_for_few(int cell, bool bwd, int kt, int es) { return cell == CELL_LSTM && (bwd ? kt == 2 && es == 2 : kt == 4); }
+// D = 32 forward, fp32: LSTM B64 N24 T256 130 -> 124, B1024 N24 T32 132 -> 138, sLSTM 146 -> 134, 138 -> 146 (without gradients), B200 N24 T64 87 -> 93.
+__host__ __device__ constexpr bool states_form_for_few(int cell, bool bwd, int kt, int es) {
+  if (cell == CELL_LSTM) return bwd ? kt == 2 && es == 2 : kt == 4 || (kt == 2 && es == 4);
+  return cell == CELL_SLSTM && !bwd && kt == 2 && es == 4;
+}
 // Whether the reverse loops of 32-unit clusters and 8 rows are always those with warps that only multiply (lane_help in frnn_api.cu): there is no other form then.
 __host__ __device__ constexpr bool help_always(int cell, int kt) {
   return cell == CELL_LSTM ? kt == 6 || kt == 12 || kt == 16 : cell == CELL_SLSTM ? kt == 6 || kt == 8 || kt == 12 || kt == 16 : cell == CELL_GRU && kt == 6;
