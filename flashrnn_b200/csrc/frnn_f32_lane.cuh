@@ -81,6 +81,9 @@ struct XFwdGeom {
   static constexpr int MAXQ = CL ? 8 : 16, MAXTH = 4 * LPU * MAXQ + kXIo;  // unit quads per CTA, threads, at most
   static constexpr int NR = C::Gr == 1 ? 4 : C::Gr;  // rows of R per lane: a unit's gates, Elman: four units
   static constexpr int GP = NR * KQ * BT > 128 ? 1 : NR * KQ * BT > 64 && KQ == 8 ? 2 : NR;  // of them, those multiplied in one pass over h (registers)
+  // Waits by a vote (mbar_wait_warp), except with 2 rows of three or four gates up to head dim 128: us of T256, a vote / a branch per lane, LSTM B8 N2 D = 100 173 / 167, GRU B1 N1 D = 128 164 /
+  // 160; with more rows it is the other way round, GRU B64 N4 T64 D = 128 89 / 91.
+  static constexpr bool VOTE = CL && !(C::Gr > 1 && LPU == 4 && BT == 2);
   static constexpr int NL = (C::Gw * BT * MAXQ + kXIo - 1) / kXIo, NS = ((C::S + C::GC) * BT * MAXQ + kXIo - 1) / kXIo;  // chunks per IO lane
   static __host__ __device__ constexpr int plane(int U) { return U / 4 * BT * 16; }
   static __host__ __device__ constexpr int off_x() { return 128 + 2 * HB; }
@@ -93,7 +96,7 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32
   using G = XFwdGeom<CELL, CL, LPU, KQ, BT>;
   using C = Cell<CELL>;
   constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, HB = G::HB, UW = 32 / LPU, GP = G::GP, NR = G::NR, KS = G::KS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = CL ? warp_index() : tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = G::VOTE ? warp_index() : tid >> 5;
   const int D = p.D, U = p.U, Q = U >> 2, CS = p.CS, T = p.T, B = p.B, N = p.N;
   const int n = blockIdx.z, b0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
@@ -230,7 +233,7 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32
   const uint32_t hr = ht + (uint32_t)(kk * BT) * 16u, sw = (uint32_t)(kk * BT >> 3) & (BT - 1);
   const int drop_t = (p.test_drop && crank == 0) ? 1 : -1;  // test hook: CTA 0 withholds its message of step 1
   const bool cache = GC > 0 && p.cache != nullptr;
-  bool poisoned = false;  // a wait of this warp expired: it neither waits nor sends any more and the loop runs out
+  bool poisoned = false;  // a wait expired: it neither waits nor sends any more and the loop runs out
   __syncthreads();        // Wx of steps 0 and 1 has landed
   int stage = 0;
   for (int t = 0; t < T; ++t) {
@@ -238,12 +241,20 @@ __global__ void __launch_bounds__(XFwdGeom<CELL, CL, LPU, KQ, BT>::MAXTH, 1) x32
     float wx[Gw];
 #pragma unroll
     for (int g = 0; g < Gw; ++g) wx[g] = __uint_as_float(lds32(ring + stage * xs + g * plane + word));
-    if (CL && t > 0) {
-      if (!mbar_wait_warp(&full[prv], (uint32_t)(((t - 1) >> 1) & 1), poisoned)) {
-        poisoned = true;
-        if (lane == 0) report_timeout(p.status, t);
+    if constexpr (G::VOTE) {
+      if (t > 0) {
+        if (!mbar_wait_warp(&full[prv], (uint32_t)(((t - 1) >> 1) & 1), poisoned)) {
+          poisoned = true;
+          if (lane == 0) report_timeout(p.status, t);
+        }
+        mbar_arrive_expect_tx_if(tid == 0 && t + 2 < T && !poisoned, &full[prv], step_bytes);
       }
-      mbar_arrive_expect_tx_if(tid == 0 && t + 2 < T && !poisoned, &full[prv], step_bytes);
+    } else if (CL && t > 0 && !poisoned) {
+      if (!mbar_wait_bounded(&full[prv], (uint32_t)(((t - 1) >> 1) & 1))) {
+        poisoned = true;
+        report_timeout(p.status, t);
+      }
+      else if (tid == 0 && t + 2 < T) mbar_arrive_expect_tx(&full[prv], step_bytes);
     }
     float v[NR][BT], pre[Gr], gx[Gt];
 #pragma unroll
@@ -321,6 +332,9 @@ struct XBwdGeom {
   using C = Cell<CELL>;
   static constexpr int PL = C::Gr == 3 ? 4 : C::Gr;  // planes of the delta tile: the R gates; the GRU's input-only gate behind them
   static constexpr int NIN = C::GC + C::NNEED + C::NEXT;
+  // Waits by a vote (mbar_wait_warp), except with three column tasks per warp (head dims 100 and 120) and four gates: us, a vote / a branch per lane, sLSTM D = 100 B8
+  // T256 N2 329 / 316, LSTM D = 100 B256 T32 N6 945 / 920; elsewhere 2 to 4 % the other way round, LSTM B8 T256 N2 D = 128 241 / 249.
+  static constexpr bool VOTE = CL && !(TB == 3 && C::Gr == 4);
   static constexpr int KS = CL ? 8 : 4 * LPU;
   static constexpr int MAXQ = CL ? 8 : 16, MAXTH = 4 * LPU * MAXQ + kXIo;
   static constexpr int NL = (NIN * BT * MAXQ + kXIo - 1) / kXIo, NS = ((C::Gw + (C::Gr == 3 ? 1 : 0)) * BT * MAXQ + kXIo - 1) / kXIo;
@@ -337,7 +351,7 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, CL, LPU, KQ, TB, BT>::MAXTH, 1)
   using C = Cell<CELL>;
   constexpr int Gr = C::Gr, Gw = C::Gw, Gt = C::Gt, S = C::S, GC = C::GC, GCA = GC > 0 ? GC : 1, NNEED = C::NNEED, NEXT = C::NEXT, NIN = G::NIN, KS = G::KS, UW = 32 / LPU;
   constexpr int GSH = Gr == 3 ? 1 : 0;  // GRU: plane 0 is the recurrent-only gate, which goes to dg0
-  const int tid = threadIdx.x, lane = tid & 31, warp = CL ? warp_index() : tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = G::VOTE ? warp_index() : tid >> 5;
   const int D = p.D, U = p.U, Q = U >> 2, CS = p.CS, T = p.T, B = p.B, N = p.N;
   const int n = blockIdx.z, b0 = blockIdx.y * BT;
   const uint32_t crank = CL ? cluster_ctarank() : 0u;
@@ -490,11 +504,19 @@ __global__ void __launch_bounds__(XBwdGeom<CELL, CL, LPU, KQ, TB, BT>::MAXTH, 1)
   const bool drop = p.test_drop && crank == 0;  // test hook: CTA 0 withholds its message of the second step
   bool poisoned = false;
   auto collect = [&](int j, int t) {  // CS > 1: the partial sums of step index j
-    if (!mbar_wait_warp(&full[j & 1], (uint32_t)((j >> 1) & 1), poisoned)) {
-      poisoned = true;
-      if (lane == 0) report_timeout(p.status, t);
+    if constexpr (G::VOTE) {
+      if (!mbar_wait_warp(&full[j & 1], (uint32_t)((j >> 1) & 1), poisoned)) {
+        poisoned = true;
+        if (lane == 0) report_timeout(p.status, t);
+      }
+      mbar_arrive_expect_tx_if(tid == 0 && j + 2 < T && !poisoned, &full[j & 1], rb);
+    } else if (!poisoned) {
+      if (!mbar_wait_bounded(&full[j & 1], (uint32_t)((j >> 1) & 1))) {
+        poisoned = true;
+        report_timeout(p.status, t);
+      }
+      else if (tid == 0 && j + 2 < T) mbar_arrive_expect_tx(&full[j & 1], rb);
     }
-    mbar_arrive_expect_tx_if(tid == 0 && j + 2 < T && !poisoned, &full[j & 1], rb);
     float x = 0.f, y = 0.f;
 #pragma unroll 2
     for (int c = 0; c < CS; ++c) {
